@@ -5,8 +5,8 @@
 //
 // Two kernels:
 //
-//  k_residual -- every coded TB of every picture, fully parallel (one warp
-//     per TB).  TBs whose prediction is already in the plane (inter TBs,
+//  k_residual -- every coded TB of every picture, fully parallel (a lane, eight
+//     lanes or a warp per TB by its size).  TBs whose prediction is already in the plane (inter TBs,
 //     prediction-in-plane pictures) are added and clipped into the plane
 //     right away; intra TBs leave an int16 residual in a residual plane.
 //     (int16 is exact: for 8-bit the reference itself truncates to i16,
@@ -45,33 +45,17 @@ __constant__ int16_t c_inv_angle[15] = {-4096, -1638, -910, -630, -482, -390, -3
 __constant__ int32_t c_dequant_scale[6] = {40, 45, 51, 57, 64, 72};
 // transform.rs:30 DST4
 __constant__ int8_t c_dst4[4][4] = {{29, 55, 74, 84}, {74, 74, 0, -74}, {84, -29, -74, 55}, {55, -84, 74, -29}};
-// H.265 DCT basis magnitudes by angle j (units of pi/64); see dct_entry().
-__constant__ int8_t c_dct_mag[33] = {64, 90, 90, 90, 89, 88, 87, 85, 83, 82, 80, 78, 75, 73, 70, 67, 64,
-                                     61, 57, 54, 50, 46, 43, 38, 36, 31, 25, 22, 18, 13, 9,  4,  0};
-
 constexpr int kScr = 33;  // padded row stride of the transform scratch
 // Inverse-transform variants of k_residual (schedule knob; pixels identical).
 constexpr int kIdctMatrix = 0;     // matrix product, all-zero rows / columns skipped
 constexpr int kIdctButterfly = 1;  // even-odd butterflies for 16x16 and 32x32 TBs
 constexpr int kIdctTensor = 2;     // integer tensor-core products (int8 halves) for 16x16 and 32x32 TBs
 
-__device__ __forceinline__ int dct_entry(int n, int k, int m) {
-    if (k == 0) return 64;
-    const int k32 = k * (32 / n);
-    int j = (k32 * (2 * m + 1)) & 127;
-    int sign = 1;
-    if (j > 64) j = 128 - j;
-    if (j > 32) {
-        j = 64 - j;
-        sign = -1;
-    }
-    return sign * c_dct_mag[j];
-}
-
 __device__ __forceinline__ int sat16(int v) { return v < -32768 ? -32768 : (v > 32767 ? 32767 : v); }
 
-// The same basis entry as a compile-time constant, for fully unrolled
-// butterflies (the multiplier becomes an immediate operand).
+// Entry (k, m) of the n-point H.265 DCT basis as a compile-time constant (the
+// multipliers of the unrolled butterflies, the tables below); mag: the basis
+// magnitudes by angle j, in units of pi/64.
 __host__ __device__ constexpr int dct_c(int n, int k, int m) {
     constexpr int8_t mag[33] = {64, 90, 90, 90, 89, 88, 87, 85, 83, 82, 80, 78, 75, 73, 70, 67, 64,
                                 61, 57, 54, 50, 46, 43, 38, 36, 31, 25, 22, 18, 13, 9,  4,  0};
@@ -190,88 +174,133 @@ __device__ __forceinline__ void mma16(int (&d)[4], uint32_t a0, uint32_t a1, uin
                      : "r"(a0), "r"(a1), "r"(b0));
 }
 
-// Basis fragments, per lane, in shared memory (index [entry][lane]):
+// Basis fragments, per lane (index [entry][lane]):
 //   s1a32: T^T as the A operand of stage 1, 32x32: 2 row tiles x 4 registers
 //   s2b32: T as the B operand of stage 2, 32x32: 4 column tiles x 2 registers
 //   s1a16: T^T, 16x16: 2 registers;  s2b16: T, 16x16: 2 column tiles x 1 register
+// Stage 2 takes stage 1's accumulators as its A operand without moving them
+// between lanes: byte i of lane t's register holds column 8 * (i / 2) + 2t +
+// (i & 1) of its half instead of column 4t + i, and the rows of the stage-2
+// basis are permuted the same way (a sum over K in another order).
 constexpr int kFragS1A32 = 0, kFragS2B32 = 8, kFragS1A16 = 16, kFragS2B16 = 18, kFragEntries = 20;
 
-__device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
-    return (uint32_t)(a & 0xff) | ((uint32_t)(b & 0xff) << 8) | ((uint32_t)(c & 0xff) << 16) | ((uint32_t)(d & 0xff) << 24);
-}
-
-__device__ void build_basis_frags(uint32_t* frags, int tid, int nthreads) {
-    for (int e = tid; e < kFragEntries * 32; e += nthreads) {
+// The basis as the kernels stage it into shared memory, computed at compile
+// time (building it in every CTA cost a launch several microseconds of
+// serialised constant reads).
+struct BasisTables {
+    uint32_t frags[kFragEntries * 32];
+    int16_t dct[32 * 32];
+};
+constexpr BasisTables make_basis() {
+    BasisTables B{};
+    for (int i = 0; i < 32 * 32; ++i) B.dct[i] = (int16_t)dct_c(32, i / 32, i % 32);
+    for (int e = 0; e < kFragEntries * 32; ++e) {
         const int entry = e >> 5, lane = e & 31, g = lane >> 2, t = lane & 3;
-        int v[4];
-        if (entry < kFragS2B32) {  // A of stage 1, n = 32: A[m][k] = T[k][m]
-            const int mt = entry >> 2, reg = entry & 3;
-            const int m = mt * 16 + g + (reg & 1) * 8, k0 = (reg >> 1) * 16 + 4 * t;
-            for (int i = 0; i < 4; ++i) v[i] = dct_entry(32, k0 + i, m);
-        } else if (entry < kFragS1A16) {  // B of stage 2, n = 32: B[k][m] = T[k][m]
-            const int nt = (entry - kFragS2B32) >> 1, reg = (entry - kFragS2B32) & 1;
-            const int m = nt * 8 + g, k0 = reg * 16 + 4 * t;
-            for (int i = 0; i < 4; ++i) v[i] = dct_entry(32, k0 + i, m);
-        } else if (entry < kFragS2B16) {  // A of stage 1, n = 16
-            const int reg = entry - kFragS1A16;
-            const int m = g + reg * 8, k0 = 4 * t;
-            for (int i = 0; i < 4; ++i) v[i] = dct_entry(16, k0 + i, m);
-        } else {  // B of stage 2, n = 16
-            const int nt = entry - kFragS2B16;
-            const int m = nt * 8 + g, k0 = 4 * t;
-            for (int i = 0; i < 4; ++i) v[i] = dct_entry(16, k0 + i, m);
+        uint32_t w = 0;
+        for (int i = 0; i < 4; ++i) {
+            int n = 0, k = 0, m = 0;
+            if (entry < kFragS2B32) {  // A of stage 1, n = 32: A[m][k] = T[k][m]
+                const int mt = entry >> 2, reg = entry & 3;
+                n = 32, m = mt * 16 + g + (reg & 1) * 8, k = (reg >> 1) * 16 + 4 * t + i;
+            } else if (entry < kFragS1A16) {  // B of stage 2, n = 32 (permuted rows)
+                const int nt = (entry - kFragS2B32) >> 1, reg = (entry - kFragS2B32) & 1;
+                n = 32, m = nt * 8 + g, k = reg * 16 + (i >> 1) * 8 + 2 * t + (i & 1);
+            } else if (entry < kFragS2B16) {  // A of stage 1, n = 16
+                n = 16, m = g + (entry - kFragS1A16) * 8, k = 4 * t + i;
+            } else {  // B of stage 2, n = 16 (permuted rows)
+                n = 16, m = (entry - kFragS2B16) * 8 + g, k = (i >> 1) * 8 + 2 * t + (i & 1);
+            }
+            w |= (uint32_t)(dct_c(n, k, m) & 0xff) << (8 * i);
         }
-        frags[e] = pack4(v[0], v[1], v[2], v[3]);
+        B.frags[e] = w;
     }
+    return B;
+}
+__device__ const __align__(16) BasisTables g_basis = make_basis();
+
+// Copies `bytes` (a multiple of 16) of a table into shared memory.
+__device__ __forceinline__ void stage_table(void* dst, const void* src, int bytes) {
+    for (int i = threadIdx.x; i < bytes / 16; i += blockDim.x) ((uint4*)dst)[i] = ((const uint4*)src)[i];
 }
 
-// Four int16 values split into their high bytes (s8) and low bytes (u8).
+// Four int16 values (each in the low half of its word) split into their high
+// bytes (s8) and low bytes (u8).
 __device__ __forceinline__ void split4(int a, int b, int c, int d, uint32_t& hi, uint32_t& lo) {
-    hi = pack4(a >> 8, b >> 8, c >> 8, d >> 8);
-    lo = pack4(a, b, c, d);
+    const uint32_t ab = __byte_perm((uint32_t)a, (uint32_t)b, 0x5410), cd = __byte_perm((uint32_t)c, (uint32_t)d, 0x5410);
+    lo = __byte_perm(ab, cd, 0x6420);
+    hi = __byte_perm(ab, cd, 0x7531);
 }
+
+// Four 8x8 matrices of 16-bit entries from shared memory, transposed: lane l
+// passes the address of row l % 8 of matrix l / 8 and receives entries
+// (2t, g) and (2t + 1, g) of each.
+__device__ __forceinline__ void ldmatrix_x4_trans(const int16_t* row, uint32_t (&r)[4]) {
+    const unsigned a = (unsigned)__cvta_generic_to_shared(row);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+
+// Row stride of the dequantised block in shared memory: rows stay 16-byte
+// aligned and eight consecutive rows of a column block fall into different
+// banks.
+__host__ __device__ constexpr int tensor_stride(int n) { return n == 32 ? 40 : 24; }
 
 // Both stages of an n x n (16 or 32) inverse DCT by one warp: buf holds the
-// dequantised coefficients (row k, column c, stride kScr), tmp receives
-// stage 1; emit(r, m, v) gets every output with the reference's storage.
+// dequantised coefficients (row k, column c, stride tensor_stride(n));
+// emit(mt, out) gets, per 16-row tile, out[nt][e] = row mt * 16 + g + 8 *
+// (e / 2), column nt * 8 + 2t + (e & 1), before the storage wrap.  Stage 1's
+// operand fragments are four rows of one column: two transposed 8x8 loads
+// whose row addresses interleave rows 4t, 4t + 1 and 4t + 2, 4t + 3.
 template <int N, typename Emit>
-__device__ __forceinline__ void idct_tensor(const int16_t* buf, int16_t* tmp, const uint32_t* frags, int bd, bool i16s,
-                                            int lane, Emit emit) {
+__device__ __forceinline__ void idct_tensor(const int16_t* buf, const uint32_t* frags, int bd, int lane, Emit emit) {
     constexpr int MT = N / 16, NT = N / 8;  // row tiles, column tiles
-    const int g = lane >> 2, t = lane & 3;
+    constexpr int STR = tensor_stride(N);
     // ---- stage 1: tmp[m][c] = clip((sum_k T[k][m] D[k][c] + 64) >> 7) ----
+    uint32_t tmp[MT][NT][2];  // two int16 per word: columns 2t, 2t + 1 of rows g and g + 8
+    const int mat = lane >> 3, li = lane & 7;
+    const int row = 4 * (li >> 1) + (li & 1) + 2 * (mat & 1);
+    uint32_t bh[NT][N / 16], bl[NT][N / 16];
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        const int c = nt * 8 + g;
-        uint32_t bh[2], bl[2];
+    for (int q = 0; q < NT * (N / 16) / 2; ++q) {
+        // N = 16: one load covers both column tiles; N = 32: one column tile,
+        // both 16-row halves
+        uint32_t r[4];
+        if constexpr (N == 16)
+            ldmatrix_x4_trans(buf + row * STR + 8 * (mat >> 1), r);
+        else
+            ldmatrix_x4_trans(buf + (row + 16 * (mat >> 1)) * STR + 8 * q, r);
 #pragma unroll
-        for (int reg = 0; reg < (N == 32 ? 2 : 1); ++reg) {
-            const int k0 = reg * 16 + 4 * t;
-            split4(buf[k0 * kScr + c], buf[(k0 + 1) * kScr + c], buf[(k0 + 2) * kScr + c], buf[(k0 + 3) * kScr + c],
-                   bh[reg], bl[reg]);
-        }
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-            int dh[4] = {0, 0, 0, 0}, dl[4] = {0, 0, 0, 0};
-            if constexpr (N == 32) {
-                const uint32_t a[4] = {frags[(kFragS1A32 + mt * 4 + 0) * 32 + lane], frags[(kFragS1A32 + mt * 4 + 1) * 32 + lane],
-                                       frags[(kFragS1A32 + mt * 4 + 2) * 32 + lane], frags[(kFragS1A32 + mt * 4 + 3) * 32 + lane]};
-                mma32(dh, a, bh[0], bh[1], false, false);
-                mma32(dl, a, bl[0], bl[1], false, true);
-            } else {
-                const uint32_t a0 = frags[(kFragS1A16 + 0) * 32 + lane], a1 = frags[(kFragS1A16 + 1) * 32 + lane];
-                mma16(dh, a0, a1, bh[0], false, false);
-                mma16(dl, a0, a1, bl[0], false, true);
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int m = mt * 16 + g + (e >> 1) * 8, cc = nt * 8 + 2 * t + (e & 1);
-                const int acc = dh[e] * 256 + dl[e];
-                tmp[m * kScr + cc] = (int16_t)clamp3i((acc + 64) >> 7, -32768, 32767);
-            }
+        for (int h = 0; h < 2; ++h) {
+            const int nt = N == 16 ? h : q, reg = N == 16 ? 0 : h;
+            bl[nt][reg] = __byte_perm(r[2 * h], r[2 * h + 1], 0x6420);
+            bh[nt][reg] = __byte_perm(r[2 * h], r[2 * h + 1], 0x7531);
         }
     }
-    __syncwarp();
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+        uint32_t a[4];
+#pragma unroll
+        for (int i = 0; i < (N == 32 ? 4 : 2); ++i)
+            a[i] = frags[((N == 32 ? kFragS1A32 + mt * 4 : kFragS1A16) + i) * 32 + lane];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            int dh[4] = {0, 0, 0, 0}, dl[4] = {0, 0, 0, 0};
+            if constexpr (N == 32) {
+                mma32(dh, a, bh[nt][0], bh[nt][1], false, false);
+                mma32(dl, a, bl[nt][0], bl[nt][1], false, true);
+            } else {
+                mma16(dh, a[0], a[1], bh[nt][0], false, false);
+                mma16(dl, a[0], a[1], bl[nt][0], false, true);
+            }
+            int v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = clamp3i((dh[e] * 256 + dl[e] + 64) >> 7, -32768, 32767);
+            tmp[mt][nt][0] = __byte_perm((uint32_t)v[0], (uint32_t)v[1], 0x5410);
+            tmp[mt][nt][1] = __byte_perm((uint32_t)v[2], (uint32_t)v[3], 0x5410);
+        }
+    }
     // ---- stage 2: out[r][m] = (sum_k tmp[r][k] T[k][m] + add2) >> shift2 ----
     const int shift2 = 20 - bd;
     const int add2 = 1 << (shift2 - 1);
@@ -279,11 +308,14 @@ __device__ __forceinline__ void idct_tensor(const int16_t* buf, int16_t* tmp, co
     for (int mt = 0; mt < MT; ++mt) {
         uint32_t ah[4], al[4];
 #pragma unroll
-        for (int reg = 0; reg < (N == 32 ? 4 : 2); ++reg) {
-            const int r = mt * 16 + g + (reg & 1) * 8, k0 = (reg >> 1) * 16 + 4 * t;
-            const int16_t* row = tmp + r * kScr + k0;
-            split4(row[0], row[1], row[2], row[3], ah[reg], al[reg]);
-        }
+        for (int half = 0; half < N / 16; ++half)
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+                const uint32_t p = tmp[mt][2 * half][rr], q = tmp[mt][2 * half + 1][rr];
+                al[2 * half + rr] = __byte_perm(p, q, 0x6420);
+                ah[2 * half + rr] = __byte_perm(p, q, 0x7531);
+            }
+        int out[NT][4];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             int dh[4] = {0, 0, 0, 0}, dl[4] = {0, 0, 0, 0};
@@ -297,14 +329,10 @@ __device__ __forceinline__ void idct_tensor(const int16_t* buf, int16_t* tmp, co
                 mma16(dl, al[0], al[1], b0, true, false);
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int r = mt * 16 + g + (e >> 1) * 8, m = nt * 8 + 2 * t + (e & 1);
-                const int v = (dh[e] * 256 + dl[e] + add2) >> shift2;
-                emit(r, m, i16s ? (int)(int16_t)v : v);
-            }
+            for (int e = 0; e < 4; ++e) out[nt][e] = (dh[e] * 256 + dl[e] + add2) >> shift2;
         }
+        emit(mt, out);
     }
-    __syncwarp();
 }
 
 // ===========================================================================
@@ -319,8 +347,7 @@ constexpr int kResWarps = 8;
 // path for chroma TBs with cross-component prediction, decode.rs:5313-5316).
 template <int kIdct, typename Emit>
 __device__ void tb_residual_warp(const DevPic& P, const hpvcd_tu& t, const int16_t* dct, int16_t* buf,
-                                 int16_t* tmp, int lane, Emit emit, bool allow16 = true,
-                                 const uint32_t* frags = nullptr) {
+                                 int16_t* tmp, int lane, Emit emit, bool allow16 = true) {
     const int n = 1 << t.log2n;
     const bool luma = t.comp == 0;
     const int bd = luma ? P.bd : P.bd_c;
@@ -475,13 +502,6 @@ __device__ void tb_residual_warp(const DevPic& P, const hpvcd_tu& t, const int16
     for (int o = 16; o; o >>= 1) rows = max(rows, __shfl_xor_sync(0xffffffffu, rows, o));
     __syncwarp();
     const bool dst = luma && n == 4 && (t.flags & HPVCD_TU_INTRA);
-    if (kIdct == kIdctTensor && n >= 16) {
-        if (n == 16)
-            idct_tensor<16>(buf, tmp, frags, bd, i16s, lane, emit);
-        else
-            idct_tensor<32>(buf, tmp, frags, bd, i16s, lane, emit);
-        return;
-    }
     if (kIdct == kIdctButterfly && n >= 16) {
         // stage 1, lane = column: rows >= `rows` are zero
         auto st1 = [](int acc) { return clamp3i((acc + 64) >> 7, -32768, 32767); };
@@ -545,16 +565,49 @@ __device__ void tb_residual_warp(const DevPic& P, const hpvcd_tu& t, const int16
     __syncwarp();
 }
 
-// Records per warp step of k_residual: a warp loads 32 consecutive records
-// at once (one per lane, coalesced), finds their pictures in parallel and
-// prefetches their coefficients into L2, then transforms them one by one.
-constexpr int kResChunk = 32;
-
 // Dequantisation scale m_levelScale[qs % 6] (transform.rs:701-725) without a
 // table: lanes of one warp index it differently, which a constant-bank read
 // would serialise.
 __device__ __forceinline__ int level_scale(int r) {
     return r == 0 ? 40 : (r == 1 ? 45 : (r == 2 ? 51 : (r == 3 ? 57 : (r == 4 ? 64 : 72))));
+}
+
+// Dequantisation of one TB in 32-bit arithmetic (transform.rs:764-858):
+// clip((l * (s << q) * m + 2^(b - 1)) >> b) to int16 with s = levelScale, q =
+// qP / 6, m the scaling factor (16 when flat) and b = bd + log2n - 5.  The
+// common factor 2^min(q, b) cancels exactly: with b > q the result is (l s m
+// + 2^(b - q - 1)) >> (b - q), else (l s m) << (q - b).  |l s m| <= 32768 *
+// 72 * 255 < 2^30; before a left shift the product is clamped to +-32768,
+// which the final clip cannot tell from the full value.
+struct Dequant {
+    int s, lim, left, right, rnd;
+    __device__ __forceinline__ Dequant(const DevPic& P, const hpvcd_tu& t, int log2n) {
+        const int c = t.comp, bd = c ? P.bd_c : P.bd;
+        int qpp;
+        if (c == 0) {
+            qpp = qp_prime(t.qp_y, bd);
+        } else {
+            const int pps_off = c == 1 ? P.pps_cb_qp_offset : P.pps_cr_qp_offset;
+            qpp = qp_prime(qpc_map(t.qp_y + pps_off + t.cqp_off, P.idc, bd), bd);
+        }
+        const int qs = clamp3i(qpp, 0, 51 + 6 * (bd - 8));
+        const int q = qs / 6, b = bd + log2n - 5;
+        s = level_scale(qs - 6 * q);
+        left = max(q - b, 0);
+        right = max(b - q, 0);
+        rnd = right ? 1 << (right - 1) : 0;
+        lim = left ? 32768 : 0x7fffffff;
+    }
+    __device__ __forceinline__ int operator()(int l, int m) const {
+        const int x = min(max(l * (s * m), -lim), lim);
+        return clamp3i(((x << left) + rnd) >> right, -32768, 32767);
+    }
+};
+
+// Scaling list of a TB (transform.rs:668-683), NULL when flat.
+__device__ __forceinline__ const uint8_t* scaling_of(const DevPic& P, const hpvcd_tu& t, int log2n) {
+    if (!P.scaling) return nullptr;
+    return P.scaling->m[log2n - 2][min((int)t.comp, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
 }
 
 // One 4-point inverse transform, DST-VII (kDst) or DCT, with the basis as
@@ -605,43 +658,67 @@ __device__ __forceinline__ void idct4_thread(int (&d)[16], int shift2) {
     }
 }
 
-// A record k_residual's per-lane paths take: a coded, valid TB of size
-// 2^log2n with a transform (no transform skip, bypass, I_PCM or RExt residual
-// tool) whose residual is not k_ccp's.
-__device__ __forceinline__ bool tb_lanes_ok(const DevPic& P, const hpvcd_tu& t, int log2n) {
+// Four horizontally adjacent samples of a plane at an address aligned to
+// four samples.
+__device__ __forceinline__ void ld_row4(const void* plane, int bps, size_t idx, int (&v)[4]) {
+    if (bps == 1) {
+        const uint32_t w = *(const uint32_t*)((const uint8_t*)plane + idx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = (w >> (8 * i)) & 0xff;
+    } else {
+        const uint2 w = *(const uint2*)((const uint16_t*)plane + idx);
+        v[0] = w.x & 0xffff; v[1] = w.x >> 16; v[2] = w.y & 0xffff; v[3] = w.y >> 16;
+    }
+}
+__device__ __forceinline__ void st_row4(void* plane, int bps, size_t idx, const int (&v)[4]) {
+    if (bps == 1)
+        *(uint32_t*)((uint8_t*)plane + idx) =
+            (uint32_t)v[0] | ((uint32_t)v[1] << 8) | ((uint32_t)v[2] << 16) | ((uint32_t)v[3] << 24);
+    else
+        *(uint2*)((uint16_t*)plane + idx) =
+            make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
+}
+
+// A plain coded TB of size 2^log2n: valid, with a transform (no transform
+// skip, bypass, I_PCM or RExt residual tool) and a residual that is not
+// k_ccp's.
+__device__ __forceinline__ bool tb_plain(const DevPic& P, const hpvcd_tu& t) {
     constexpr uint32_t kOther = HPVCD_TU_TSKIP | HPVCD_TU_TQB | HPVCD_TU_ROTATE | HPVCD_TU_RDPCM_H |
                                 HPVCD_TU_RDPCM_V | HPVCD_TU_PCM;
-    if (!(t.flags & HPVCD_TU_CBF) || (t.flags & kOther) || t.log2n != log2n) return false;
+    if (!(t.flags & HPVCD_TU_CBF) || (t.flags & kOther) || t.log2n < 2 || t.log2n > 5) return false;
     if ((P.flags & HPVCD_PIC_CROSS_COMPONENT) && t.comp && t.res_scale) return false;
     const int ncomp = P.idc ? 3 : 1;
     if (t.comp >= ncomp) return false;
     const int pw = t.comp ? P.cw : P.w, ph = t.comp ? P.ch : P.h;
-    return (int)t.x < pw && (int)t.y < ph && (uint64_t)t.coeff_off + (1u << (2 * log2n)) <= P.n_coeffs;
+    return (int)t.x < pw && (int)t.y < ph && (uint64_t)t.coeff_off + (1u << (2 * t.log2n)) <= P.n_coeffs;
 }
 
-// Residual of one such 4x4 TB by one thread (the 4x4 case of
-// tb_residual_warp: dequantisation transform.rs:764-858 with the same
-// per-coefficient factor, then idct4_thread), stored where the warp path
-// stores it: added to the plane and clipped for TBs predicted in the
-// plane, else into the int16 residual plane.
+// TBs whose prediction is already in the plane (inter TBs and
+// prediction-in-plane pictures); the others leave their residual in the int16
+// residual plane.
+__device__ __forceinline__ bool tb_in_plane(const DevPic& P, const hpvcd_tu& t) {
+    return (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
+}
+
+// Residual of one plain 4x4 TB by one thread (the 4x4 case of
+// tb_residual_warp), stored where the warp path stores it: added to the plane
+// and clipped for TBs predicted in the plane, else into the int16 residual
+// plane.
 __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
     const int c = t.comp;
-    const bool luma = c == 0;
-    const int bd = luma ? P.bd : P.bd_c;
-    int qpp;
-    if (luma) {
-        qpp = qp_prime(t.qp_y, bd);
-    } else {
-        const int pps_off = c == 1 ? P.pps_cb_qp_offset : P.pps_cr_qp_offset;
-        qpp = qp_prime(qpc_map(t.qp_y + pps_off + t.cqp_off, P.idc, bd), bd);
+    const int bd = c ? P.bd_c : P.bd;
+    const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
+    const int x0 = t.x, y0 = t.y;
+    const bool in_plane = tb_in_plane(P, t);
+    // the plane's rows are read up front, beside the levels
+    int pv[4][4];
+    void* pl = P.rec[c];
+    const size_t p0 = (size_t)y0 * pw + x0;
+    const bool pvec = in_plane && x0 + 4 <= pw && y0 + 4 <= ph && (p0 & 3) == 0 && (pw & 3) == 0;
+    if (pvec) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r) ld_row4(pl, P.bps, p0 + (size_t)r * pw, pv[r]);
     }
-    const int bd_shift = bd + 2 + 10 - 15;
-    const int qs = clamp3i(qpp, 0, 51 + 6 * (bd - 8));
-    const long long base = (long long)level_scale(qs % 6) * (1ll << (qs / 6));
-    const long long add = 1ll << (bd_shift - 1);
-    const uint8_t* sm = nullptr;
-    if (P.scaling) sm = P.scaling->m[0][min(c, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
-    const int nx = (t.nx == 0 || t.nx > 4) ? 4 : t.nx;
     int d[16];
     const bool c8 = (P.flags & HPVCD_PIC_COEFF8) != 0;
     if (c8) {
@@ -667,31 +744,37 @@ __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
             for (int i = 0; i < 16; ++i) d[i] = lv[i];
         }
     }
+    const Dequant dq(P, t, 2);
+    const uint8_t* sm = scaling_of(P, t, 2);
+    const int nx = (t.nx == 0 || t.nx > 4) ? 4 : t.nx;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const long long f = sm ? base * sm[i] : base * 16;
-        const long long v = ((long long)d[i] * f + add) >> bd_shift;
-        d[i] = (i & 3) < nx ? (int)(v < -32768 ? -32768 : (v > 32767 ? 32767 : v)) : 0;
-    }
+    for (int i = 0; i < 16; ++i) d[i] = (i & 3) < nx ? dq(d[i], sm ? sm[i] : 16) : 0;
     const int shift2 = 20 - bd;
-    if (luma && (t.flags & HPVCD_TU_INTRA))
+    if (c == 0 && (t.flags & HPVCD_TU_INTRA))
         idct4_thread<true>(d, shift2);
     else
         idct4_thread<false>(d, shift2);
-    const bool i16s = bd <= 8;
-    const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
-    const int x0 = t.x, y0 = t.y;
-    const bool in_plane = (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
-    if (in_plane) {  // reconstruct.rs:214-251: add and clip into the plane
-        void* pl = P.rec[c];
-        const int mx = (1 << bd) - 1;
+    if (bd <= 8) {  // the reference's int16 storage
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int x = x0 + (i & 3), y = y0 + (i >> 2);
-            if (x < pw && y < ph) {
-                const int v = i16s ? (int)(int16_t)d[i] : d[i];
-                const size_t idx = (size_t)y * pw + x;
-                store_sample(pl, P.bps, idx, clamp3i(load_sample(pl, P.bps, idx) + v, 0, mx));
+        for (int i = 0; i < 16; ++i) d[i] = (int)(int16_t)d[i];
+    }
+    if (in_plane) {  // reconstruct.rs:214-251: add and clip into the plane
+        const int mx = (1 << bd) - 1;
+        if (pvec) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) pv[r][m] = clamp3i(pv[r][m] + d[4 * r + m], 0, mx);
+                st_row4(pl, P.bps, p0 + (size_t)r * pw, pv[r]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int x = x0 + (i & 3), y = y0 + (i >> 2);
+                if (x < pw && y < ph) {
+                    const size_t idx = (size_t)y * pw + x;
+                    store_sample(pl, P.bps, idx, clamp3i(load_sample(pl, P.bps, idx) + d[i], 0, mx));
+                }
             }
         }
     } else {  // the int16 residual plane k_recon adds to its prediction
@@ -704,7 +787,7 @@ __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
             int16_t* row = rp + (size_t)y * rs + x0;
             int16_t v4[4];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) v4[m] = (int16_t)sat16(i16s ? (int)(int16_t)d[4 * r + m] : d[4 * r + m]);
+            for (int m = 0; m < 4; ++m) v4[m] = (int16_t)sat16(d[4 * r + m]);
             if (x0 + 4 <= pw && ((uintptr_t)row & 7) == 0) {
                 *(uint2*)row = make_uint2((uint32_t)(uint16_t)v4[0] | ((uint32_t)(uint16_t)v4[1] << 16),
                                           (uint32_t)(uint16_t)v4[2] | ((uint32_t)(uint16_t)v4[3] << 16));
@@ -715,10 +798,6 @@ __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
             }
         }
     }
-}
-
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
 // 8-point inverse DCT with the basis as immediates, even-odd form:
@@ -737,37 +816,27 @@ __device__ __forceinline__ void inv8(const int (&in)[8], int (&o)[8]) {
     o[3] = e3 + o3; o[4] = e3 - o3;
 }
 
-// Stage 1 of a plain coded 8x8 TB by lane q (0..7) of its group of eight:
-// column q dequantised (the 8x8 case of tb_residual_warp: factor
-// base * m[r][q] or base * 16, columns >= nx zero) and inverse transformed,
-// (sum + 64) >> 7 clipped to int16 into the group's scratch S[m * 9 + q].
-__device__ void tb8_cols(const DevPic& P, const hpvcd_tu& t, int q, int16_t* S) {
-    const int c = t.comp;
-    const int bd = c ? P.bd_c : P.bd;
-    int qpp;
-    if (c == 0) {
-        qpp = qp_prime(t.qp_y, bd);
-    } else {
-        const int pps_off = c == 1 ? P.pps_cb_qp_offset : P.pps_cr_qp_offset;
-        qpp = qp_prime(qpc_map(t.qp_y + pps_off + t.cqp_off, P.idc, bd), bd);
-    }
-    const int bd_shift = bd + 3 + 10 - 15;
-    const int qs = clamp3i(qpp, 0, 51 + 6 * (bd - 8));
-    const long long base = (long long)level_scale(qs % 6) * (1ll << (qs / 6));
-    const long long add = 1ll << (bd_shift - 1);
-    const uint8_t* sm = nullptr;
-    if (P.scaling) sm = P.scaling->m[1][min(c, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
-    const int nx = (t.nx == 0 || t.nx > 8) ? 8 : t.nx;
+// Stage 1 of a plain 8x8 TB by lane q (0..7) of its group of eight: column q
+// dequantised (the 8x8 case of tb_residual_warp, columns >= nx zero) and
+// inverse transformed, (sum + 64) >> 7 clipped to int16 into the group's
+// scratch S[m * 9 + q].
+__device__ __forceinline__ void tb8_cols(const DevPic& P, const hpvcd_tu& t, int q, int16_t* S) {
     const bool c8 = (P.flags & HPVCD_PIC_COEFF8) != 0;
     int in[8];
+    if (c8) {
+        const int8_t* lv = (const int8_t*)P.coeffs + t.coeff_off + q;
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int i = r * 8 + q;
-        const int l = c8 ? (int)((const int8_t*)P.coeffs + t.coeff_off)[i] : (int)(P.coeffs + t.coeff_off)[i];
-        const long long f = sm ? base * sm[i] : base * 16;
-        const long long v = ((long long)l * f + add) >> bd_shift;
-        in[r] = q < nx ? (int)(v < -32768 ? -32768 : (v > 32767 ? 32767 : v)) : 0;
+        for (int r = 0; r < 8; ++r) in[r] = lv[r * 8];
+    } else {
+        const int16_t* lv = P.coeffs + t.coeff_off + q;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) in[r] = lv[r * 8];
     }
+    const Dequant dq(P, t, 3);
+    const uint8_t* sm = scaling_of(P, t, 3);
+    const int nx = (t.nx == 0 || t.nx > 8) ? 8 : t.nx;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) in[r] = q < nx ? dq(in[r], sm ? sm[r * 8 + q] : 16) : 0;
     int o[8];
     inv8(in, o);
 #pragma unroll
@@ -777,9 +846,21 @@ __device__ void tb8_cols(const DevPic& P, const hpvcd_tu& t, int q, int16_t* S) 
 // Stage 2 of the same TB by lane q: row q of the stage-1 result, inverse
 // transformed, + 2^(shift2 - 1) >> shift2, stored as tb4_thread stores
 // (added to the plane, or into the int16 residual plane).
-__device__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int q, const int16_t* S) {
+__device__ __forceinline__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int q, const int16_t* S) {
     const int c = t.comp;
     const int bd = c ? P.bd_c : P.bd;
+    const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
+    const int x0 = t.x, y = t.y + q;
+    if (y >= ph) return;
+    const bool in_plane = tb_in_plane(P, t);
+    void* pl = P.rec[c];
+    const size_t p0 = (size_t)y * pw + x0;
+    const bool pvec = in_plane && x0 + 8 <= pw && (p0 & 3) == 0;
+    int pv[2][4];
+    if (pvec) {
+        ld_row4(pl, P.bps, p0, pv[0]);
+        ld_row4(pl, P.bps, p0 + 4, pv[1]);
+    }
     const int shift2 = 20 - bd, add2 = 1 << (shift2 - 1);
     const bool i16s = bd <= 8;
     int in[8], o[8];
@@ -791,18 +872,20 @@ __device__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int q, const int16_
         const int v = (o[m] + add2) >> shift2;
         o[m] = i16s ? (int)(int16_t)v : v;
     }
-    const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
-    const int x0 = t.x, y = t.y + q;
-    if (y >= ph) return;
-    const bool in_plane = (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
     if (in_plane) {  // reconstruct.rs:214-251: add and clip into the plane
-        void* pl = P.rec[c];
         const int mx = (1 << bd) - 1;
+        if (pvec) {
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            if (x0 + m >= pw) break;
-            const size_t idx = (size_t)y * pw + x0 + m;
-            store_sample(pl, P.bps, idx, clamp3i(load_sample(pl, P.bps, idx) + o[m], 0, mx));
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int m = 0; m < 4; ++m) pv[h][m] = clamp3i(pv[h][m] + o[4 * h + m], 0, mx);
+                st_row4(pl, P.bps, p0 + 4 * h, pv[h]);
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                if (x0 + m < pw)
+                    store_sample(pl, P.bps, p0 + m, clamp3i(load_sample(pl, P.bps, p0 + m) + o[m], 0, mx));
         }
     } else {
         int16_t* row = P.res[c] + (size_t)y * P.res_stride[c] + x0;
@@ -820,137 +903,276 @@ __device__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int q, const int16_
     }
 }
 
-template <int kIdct>
-__global__ void __launch_bounds__(kResWarps * 32)
-k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, uint32_t n_pics,
-           uint32_t* dev_err) {
-    __shared__ int16_t dct[32 * 32];
-    __shared__ __align__(16) int16_t scr[kResWarps][2][32 * kScr];  // per warp: buf, tmp (contiguous)
-    __shared__ uint32_t frags[kIdct == kIdctTensor ? kFragEntries * 32 : 1];
-    for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) dct[i] = (int16_t)dct_entry(32, i / 32, i % 32);
-    if (kIdct == kIdctTensor) build_basis_frags(frags, threadIdx.x, blockDim.x);
-    __syncthreads();
-    constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t first = rec_prefix[0], total = rec_prefix[n_pics];
-    const uint32_t n_chunks = (total - first + kResChunk - 1) / kResChunk;
-    for (uint32_t ch = blockIdx.x * kResWarps + warp; ch < n_chunks; ch += gridDim.x * kResWarps) {
-        const uint32_t g0 = first + ch * kResChunk;
-        // ---- this lane's record: its picture (binary search in the prefix),
-        // the record, and an L2 prefetch of its coefficients ----
-        const uint32_t gl = g0 + lane;
-        uint32_t pic = 0;
-        uint4 r4 = make_uint4(0u, 0u, 0u, 0u);
-        bool mine4 = false;  // a plain coded 4x4 TB: this lane transforms it on its own
-        bool mine8 = false;  // a plain coded 8x8 TB: a group of eight lanes transforms it
-        if (gl < total) {
-            uint32_t lo = 0, hi = n_pics;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (rec_prefix[mid] <= gl) lo = mid; else hi = mid;
+// Residual of one plain 16x16 or 32x32 TB by one warp on the integer tensor
+// pipe: eight levels per lane and load (all loads in flight together),
+// dequantised into shared memory, both stages in registers (idct_tensor),
+// two adjacent samples per store.  x0 is even (the caller's class test).
+template <int N>
+__device__ __forceinline__ void tb_tensor(const DevPic& P, const hpvcd_tu& t, int16_t* buf, const uint32_t* frags,
+                                          int lane) {
+    constexpr int LOG2N = N == 32 ? 5 : 4, STR = tensor_stride(N), PASS = N * N / 256;
+    const int c = t.comp;
+    const int bd = c ? P.bd_c : P.bd;
+    const bool c8 = (P.flags & HPVCD_PIC_COEFF8) != 0;
+    uint4 raw[PASS];  // eight levels: four words of two int16, or two words of four int8
+    if (c8) {
+        const int8_t* lv = (const int8_t*)P.coeffs + t.coeff_off;
+        const bool al = ((uintptr_t)lv & 7) == 0;
+#pragma unroll
+        for (int p = 0; p < PASS; ++p) {
+            const int8_t* q = lv + (p * 32 + lane) * 8;
+            uint2 w;
+            if (al) {
+                w = *(const uint2*)q;
+            } else {
+                memcpy(&w, q, 8);  // byte loads
             }
-            pic = lo;
-            const DevPic& P = pics[lo];
-            r4 = *(const uint4*)(P.tus + (gl - rec_prefix[lo]));  // records are 16-byte aligned
-            hpvcd_tu t;
-            memcpy(&t, &r4, sizeof(t));
-            if (tb_lanes_ok(P, t, 2)) {
-                mine4 = true;
-            } else if (tb_lanes_ok(P, t, 3)) {
-                mine8 = true;
-            } else if ((t.flags & HPVCD_TU_CBF) && t.log2n >= 2 && t.log2n <= 5) {
-                const uint32_t esz = (P.flags & HPVCD_PIC_COEFF8) ? 1u : 2u;
-                const uint64_t n2 = 1ull << (2 * t.log2n);
-                if ((uint64_t)t.coeff_off + n2 <= P.n_coeffs) {
-                    const char* b = (const char*)P.coeffs + (uint64_t)t.coeff_off * esz;
-                    const char* e = b + n2 * esz;
-                    for (const char* q = (const char*)((uintptr_t)b & ~(uintptr_t)127); q < e; q += 128) prefetch_l2(q);
+            raw[p] = make_uint4(w.x, w.y, 0u, 0u);
+        }
+    } else {
+        const int16_t* lv = P.coeffs + t.coeff_off;
+        const bool al = ((uintptr_t)lv & 15) == 0;
+#pragma unroll
+        for (int p = 0; p < PASS; ++p) {
+            const int16_t* q = lv + (p * 32 + lane) * 8;
+            if (al) {
+                raw[p] = *(const uint4*)q;
+            } else {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    w[i] = (uint32_t)(uint16_t)q[2 * i] | ((uint32_t)(uint16_t)q[2 * i + 1] << 16);
+                raw[p] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+    }
+    const Dequant dq(P, t, LOG2N);
+    const uint8_t* sm = scaling_of(P, t, LOG2N);
+    const int nx = (t.nx == 0 || t.nx > N) ? N : t.nx;
+#pragma unroll
+    for (int p = 0; p < PASS; ++p) {
+        const int i0 = (p * 32 + lane) * 8, r = i0 >> LOG2N, col = i0 & (N - 1);
+        const uint32_t w[4] = {raw[p].x, raw[p].y, raw[p].z, raw[p].w};
+        uint32_t o[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            int d[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int j = 2 * h + u;
+                const int l = c8 ? (int)(int8_t)(w[j >> 2] >> (8 * (j & 3))) : (int)(int16_t)(w[j >> 1] >> (16 * (j & 1)));
+                int m = 16;
+                if (sm) {  // the 8x8 list upsampled, with its DC entry
+                    m = sm[(r >> (LOG2N - 3)) * 8 + ((col + j) >> (LOG2N - 3))];
+                    if (i0 + j == 0)
+                        m = P.scaling->dc[LOG2N - 2][min(c, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
+                }
+                d[u] = col + j < nx ? dq(l, m) : 0;
+            }
+            o[h] = __byte_perm((uint32_t)d[0], (uint32_t)d[1], 0x5410);
+        }
+        *(uint4*)(buf + r * STR + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    __syncwarp();
+    const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
+    const int x0 = t.x, y0 = t.y;
+    const int g = lane >> 2, tq = lane & 3;
+    const bool in_plane = tb_in_plane(P, t);
+    const bool i16s = bd <= 8;
+    const int mx = (1 << bd) - 1, bps = P.bps;
+    void* pl = P.rec[c];
+    int16_t* rp = P.res[c];
+    const int rs = P.res_stride[c];
+    // plane widths are even, so a pair starting at an even column is inside
+    // or outside as a whole
+    idct_tensor<N>(buf, frags, bd, lane, [&](int mt, int (&out)[N / 8][4]) {
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+            const int y = y0 + mt * 16 + g + 8 * rr;
+            if (y >= ph) continue;
+            if (in_plane) {  // reconstruct.rs:214-251: add and clip into the plane
+                uint32_t pv[N / 8];
+                const size_t row = (size_t)y * pw;
+#pragma unroll
+                for (int nt = 0; nt < N / 8; ++nt) {
+                    const int x = x0 + nt * 8 + 2 * tq;
+                    pv[nt] = 0u;
+                    if (x < pw)
+                        pv[nt] = bps == 1 ? (uint32_t) * (const uint16_t*)((const uint8_t*)pl + row + x)
+                                          : *(const uint32_t*)((const uint16_t*)pl + row + x);
+                }
+#pragma unroll
+                for (int nt = 0; nt < N / 8; ++nt) {
+                    const int x = x0 + nt * 8 + 2 * tq;
+                    int v0 = out[nt][2 * rr], v1 = out[nt][2 * rr + 1];
+                    if (i16s) v0 = (int)(int16_t)v0, v1 = (int)(int16_t)v1;
+                    if (x >= pw) continue;
+                    if (bps == 1) {
+                        const uint32_t a = (uint32_t)clamp3i((int)(pv[nt] & 0xff) + v0, 0, mx);
+                        const uint32_t b = (uint32_t)clamp3i((int)(pv[nt] >> 8) + v1, 0, mx);
+                        *(uint16_t*)((uint8_t*)pl + row + x) = (uint16_t)(a | (b << 8));
+                    } else {
+                        const uint32_t a = (uint32_t)clamp3i((int)(pv[nt] & 0xffff) + v0, 0, mx);
+                        const uint32_t b = (uint32_t)clamp3i((int)(pv[nt] >> 16) + v1, 0, mx);
+                        *(uint32_t*)((uint16_t*)pl + row + x) = a | (b << 16);
+                    }
+                }
+            } else {
+                int16_t* row = rp + (size_t)y * rs + x0;
+#pragma unroll
+                for (int nt = 0; nt < N / 8; ++nt) {
+                    const int x = nt * 8 + 2 * tq;
+                    int v0 = out[nt][2 * rr], v1 = out[nt][2 * rr + 1];
+                    if (i16s) v0 = (int)(int16_t)v0, v1 = (int)(int16_t)v1;
+                    if (x0 + x < pw)
+                        *(uint32_t*)(row + x) = (uint32_t)(uint16_t)sat16(v0) | ((uint32_t)(uint16_t)sat16(v1) << 16);
                 }
             }
         }
-        // ---- the plain coded 4x4 TBs (most coded TBs): one per lane, in
-        // registers ----
-        if (mine4) {
+    });
+    __syncwarp();
+}
+
+// Residual of any other coded TB (transform skip, bypass, I_PCM, RExt tools;
+// every 16x16 / 32x32 TB of the matrix and butterfly schedules) by one warp.
+template <int kIdct>
+__device__ __noinline__ void tb_general(const DevPic& P, const hpvcd_tu& t, const int16_t* dct, int16_t* scr,
+                                        uint32_t* dev_err, int lane) {
+    if ((P.flags & HPVCD_PIC_CROSS_COMPONENT) && t.comp && t.res_scale) return;  // k_ccp's
+    const int c = t.comp;
+    const int ncomp = P.idc ? 3 : 1;
+    const int n = 1 << t.log2n;
+    const int pw = c < 3 && c ? P.cw : P.w, ph = c < 3 && c ? P.ch : P.h;
+    if (c >= ncomp || t.log2n < 2 || t.log2n > 5 || (int)t.x >= pw || (int)t.y >= ph ||
+        (uint64_t)t.coeff_off + (uint64_t)n * n > P.n_coeffs) {
+        if (lane == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
+        return;
+    }
+    const int x0 = t.x, y0 = t.y;
+    if (tb_in_plane(P, t)) {  // prediction already in the plane: add + clip (reconstruct.rs:214-251)
+        void* pl = P.rec[c];
+        const int mx = (1 << (c ? P.bd_c : P.bd)) - 1;
+        const int keep = (t.flags & HPVCD_TU_PCM) ? 0 : 1;  // I_PCM samples replace the plane's
+        tb_residual_warp<kIdct>(P, t, dct, scr, scr + 32 * kScr, lane, [&](int r, int m, int v) {
+            const int x = x0 + m, y = y0 + r;
+            if (x < pw && y < ph) {
+                const size_t idx = (size_t)y * pw + x;
+                store_sample(pl, P.bps, idx, clamp3i(keep * load_sample(pl, P.bps, idx) + v, 0, mx));
+            }
+        });
+    } else {
+        int16_t* rp = P.res[c];
+        const int rs = P.res_stride[c];
+        tb_residual_warp<kIdct>(P, t, dct, scr, scr + 32 * kScr, lane, [&](int r, int m, int v) {
+            const int x = x0 + m, y = y0 + r;
+            if (x < pw && y < ph) rp[(size_t)y * rs + x] = (int16_t)sat16(v);
+        });
+    }
+    __syncwarp();
+}
+
+// Classes of coded records, in the order their warp tasks are taken: the
+// longest first, so that the last tasks of a CTA are short.
+constexpr int kCls32 = 0, kCls16 = 1, kClsGeneral = 2, kCls8 = 3, kCls4 = 4, kClasses = 5;
+constexpr uint32_t kResMaxChunk = 256;  // records of a CTA step (one per thread)
+
+// One CTA takes `chunk` consecutive records at a time: every thread loads one,
+// finds its picture (one search per CTA, then a short walk) and files it
+// under its class; the warps then take tasks off the class lists: one 32x32,
+// 16x16 or general TB, four 8x8 (eight lanes each) or thirty-two 4x4 (one
+// lane each).  What bounds a launch is the latency of its longest chain of
+// tasks, so the chunk is chosen by the record count (hpvcd_launch_residual)
+// to spread small pictures over all SMs.  One warp taking 32 consecutive
+// records one after another, one sample per lane and step, took 150 us on
+// any picture of 512x512 and up; the whole call on a residual-only 512x512
+// picture went from 191 to 38.5 us, the 4032x3024 grid from 1522 to 1373 us.
+template <int kIdct>
+__global__ void __launch_bounds__(kResWarps * 32, 4)
+k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, uint32_t n_pics,
+           uint32_t* dev_err, uint32_t chunk) {
+    __shared__ __align__(16) BasisTables basis;
+    __shared__ __align__(16) int16_t scr[kResWarps][2 * 32 * kScr];  // per warp
+    __shared__ __align__(16) uint4 s_rec[kResMaxChunk];
+    __shared__ uint32_t s_pic[kResMaxChunk];
+    __shared__ uint8_t s_list[kClasses][kResMaxChunk];
+    __shared__ uint32_t s_cnt[kClasses], s_next;
+    static_assert(kResMaxChunk <= kResWarps * 32, "one record per thread");
+    static_assert(tensor_stride(32) * 32 <= 2 * 32 * kScr, "the tensor path's block fits the scratch");
+    stage_table(&basis, &g_basis, (int)sizeof(basis));
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t first = rec_prefix[0], total = rec_prefix[n_pics];
+    for (uint32_t g0 = first + blockIdx.x * chunk; g0 < total; g0 += gridDim.x * chunk) {
+        __syncthreads();  // the previous step's lists are done with (and, first, the tables staged)
+        if (threadIdx.x < kClasses) s_cnt[threadIdx.x] = 0u;
+        if (threadIdx.x == kClasses) s_next = 0u;
+        __syncthreads();
+        const uint32_t gl = g0 + threadIdx.x;
+        if (threadIdx.x < chunk && gl < total) {
+            uint32_t pic = 0, hi = n_pics;
+            while (hi - pic > 1) {  // the picture of the step's first record (uniform)
+                const uint32_t mid = (pic + hi) >> 1;
+                if (rec_prefix[mid] <= g0) pic = mid; else hi = mid;
+            }
+            while (rec_prefix[pic + 1] <= gl) ++pic;
+            const DevPic& P = pics[pic];
+            const uint4 r4 = *(const uint4*)(P.tus + (gl - rec_prefix[pic]));  // records are 16-byte aligned
             hpvcd_tu t;
             memcpy(&t, &r4, sizeof(t));
-            tb4_thread(pics[pic], t);
-        }
-        const uint32_t done4 = __ballot_sync(kAll, mine4);
-        // ---- the plain coded 8x8 TBs: four per pass, eight lanes each
-        // (lane q of a group takes column q, then row q; the transpose goes
-        // through the warp's scratch) ----
-        const uint32_t done8 = __ballot_sync(kAll, mine8);
-        for (uint32_t mask8 = done8; mask8;) {
-            const int grp = lane >> 3, q = lane & 7;
-            uint32_t m = mask8;
-            for (int i = 0; i < grp; ++i) m &= m - 1u;
-            const int src = m ? __ffs(m) - 1 : 0;
-            const uint32_t pj = __shfl_sync(kAll, pic, src);
-            uint4 w4;
-            w4.x = __shfl_sync(kAll, r4.x, src);
-            w4.y = __shfl_sync(kAll, r4.y, src);
-            w4.z = __shfl_sync(kAll, r4.z, src);
-            w4.w = __shfl_sync(kAll, r4.w, src);
-            hpvcd_tu t;
-            memcpy(&t, &w4, sizeof(t));
-            int16_t* S = scr[warp][0] + grp * 72;
-            if (m) tb8_cols(pics[pj], t, q, S);
-            __syncwarp();
-            if (m) tb8_rows(pics[pj], t, q, S);
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) mask8 &= mask8 - 1u;
-        }
-        // ---- the chunk's other records one by one ----
-        const uint32_t nrec = min((uint32_t)kResChunk, total - g0);
-        for (uint32_t j = 0; j < nrec; ++j) {
-            if (((done4 | done8) >> j) & 1u) continue;
-            const uint32_t pj = __shfl_sync(kAll, pic, j);
-            uint4 w4;
-            w4.x = __shfl_sync(kAll, r4.x, j);
-            w4.y = __shfl_sync(kAll, r4.y, j);
-            w4.z = __shfl_sync(kAll, r4.z, j);
-            w4.w = __shfl_sync(kAll, r4.w, j);
-            hpvcd_tu t;
-            memcpy(&t, &w4, sizeof(t));
-            const DevPic& P = pics[pj];
-            if (!(t.flags & HPVCD_TU_CBF)) continue;
-            if ((P.flags & HPVCD_PIC_CROSS_COMPONENT) && t.comp && t.res_scale) continue;  // k_ccp's
-            const int c = t.comp;
-            const int ncomp = P.idc ? 3 : 1;
-            const int n = 1 << t.log2n;
-            const int pw = c < 3 && c ? P.cw : P.w, ph = c < 3 && c ? P.ch : P.h;
-            if (c >= ncomp || t.log2n < 2 || t.log2n > 5 || (int)t.x >= pw || (int)t.y >= ph ||
-                (uint64_t)t.coeff_off + (uint64_t)n * n > P.n_coeffs) {
-                if (lane == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
-                continue;
+            if (t.flags & HPVCD_TU_CBF) {
+                int cls = kClsGeneral;
+                if (tb_plain(P, t)) {
+                    if (t.log2n <= 3)
+                        cls = t.log2n == 2 ? kCls4 : kCls8;
+                    else if (kIdct == kIdctTensor && (t.x & 1) == 0)
+                        cls = t.log2n == 4 ? kCls16 : kCls32;
+                }
+                s_rec[threadIdx.x] = r4;
+                s_pic[threadIdx.x] = pic;
+                s_list[cls][atomicAdd(&s_cnt[cls], 1u)] = (uint8_t)threadIdx.x;
             }
-            const int x0 = t.x, y0 = t.y;
-            const bool in_plane = (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
-            if (in_plane) {  // prediction already in the plane: add + clip (reconstruct.rs:214-251)
-                void* pl = P.rec[c];
-                const int mx = (1 << (c ? P.bd_c : P.bd)) - 1;
-                const int keep = (t.flags & HPVCD_TU_PCM) ? 0 : 1;  // I_PCM samples replace the plane's
-                tb_residual_warp<kIdct>(
-                    P, t, dct, scr[warp][0], scr[warp][1], lane,
-                    [&](int r, int m, int v) {
-                        const int x = x0 + m, y = y0 + r;
-                        if (x < pw && y < ph) {
-                            const size_t idx = (size_t)y * pw + x;
-                            store_sample(pl, P.bps, idx, clamp3i(keep * load_sample(pl, P.bps, idx) + v, 0, mx));
-                        }
-                    },
-                    true, frags);
+        }
+        __syncthreads();
+        const uint32_t e32 = s_cnt[kCls32], e16 = e32 + s_cnt[kCls16], eg = e16 + s_cnt[kClsGeneral];
+        const uint32_t n8 = s_cnt[kCls8], n4 = s_cnt[kCls4];
+        const uint32_t e8 = eg + (n8 + 3) / 4, e4 = e8 + (n4 + 31) / 32;
+        for (;;) {
+            uint32_t task = 0;
+            if (lane == 0) task = atomicAdd(&s_next, 1u);
+            task = __shfl_sync(kAll, task, 0);
+            if (task >= e4) break;
+            hpvcd_tu t;
+            if (task < eg) {
+                const int cls = task < e32 ? kCls32 : (task < e16 ? kCls16 : kClsGeneral);
+                const uint32_t j = s_list[cls][task - (cls == kCls32 ? 0u : (cls == kCls16 ? e32 : e16))];
+                memcpy(&t, &s_rec[j], sizeof(t));
+                const DevPic& P = pics[s_pic[j]];
+                if (kIdct == kIdctTensor && cls == kCls32)
+                    tb_tensor<32>(P, t, scr[warp], basis.frags, lane);
+                else if (kIdct == kIdctTensor && cls == kCls16)
+                    tb_tensor<16>(P, t, scr[warp], basis.frags, lane);
+                else
+                    tb_general<kIdct == kIdctButterfly ? kIdctButterfly : kIdctMatrix>(P, t, basis.dct, scr[warp],
+                                                                                       dev_err, lane);
+            } else if (task < e8) {
+                const uint32_t k = (task - eg) * 4 + (lane >> 3);
+                const int q = lane & 7;
+                const uint32_t j = k < n8 ? s_list[kCls8][k] : s_list[kCls8][0];
+                memcpy(&t, &s_rec[j], sizeof(t));
+                const DevPic& P = pics[s_pic[j]];
+                int16_t* S = scr[warp] + (lane >> 3) * 72;
+                if (k < n8) tb8_cols(P, t, q, S);
+                __syncwarp();
+                if (k < n8) tb8_rows(P, t, q, S);
+                __syncwarp();
             } else {
-                int16_t* rp = P.res[c];
-                const int rs = P.res_stride[c];
-                tb_residual_warp<kIdct>(
-                    P, t, dct, scr[warp][0], scr[warp][1], lane,
-                    [&](int r, int m, int v) {
-                        const int x = x0 + m, y = y0 + r;
-                        if (x < pw && y < ph) rp[(size_t)y * rs + x] = (int16_t)sat16(v);
-                    },
-                    true, frags);
+                const uint32_t k = (task - e8) * 32 + lane;
+                if (k < n4) {
+                    const uint32_t j = s_list[kCls4][k];
+                    memcpy(&t, &s_rec[j], sizeof(t));
+                    tb4_thread(pics[s_pic[j]], t);
+                }
+                __syncwarp();
             }
         }
     }
@@ -970,10 +1192,10 @@ constexpr int kCcpWarps = 4;
 __global__ void __launch_bounds__(kCcpWarps * 32)
 k_ccp(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, uint32_t n_pics,
       uint32_t* dev_err) {
-    __shared__ int16_t dct[32 * 32];
+    __shared__ __align__(16) int16_t dct[32 * 32];
     __shared__ __align__(16) int16_t scr[kCcpWarps][2][32 * kScr];
     __shared__ int32_t ry_all[kCcpWarps][32 * 32];
-    for (int i = threadIdx.x; i < 32 * 32; i += blockDim.x) dct[i] = (int16_t)dct_entry(32, i / 32, i % 32);
+    stage_table(dct, g_basis.dct, (int)sizeof(dct));
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t* ry = ry_all[warp];
@@ -2179,20 +2401,24 @@ extern "C" cudaError_t hpvcd_launch_residual(const hpvcd::DevPic* pics, const ui
                                              uint32_t n_pics, uint32_t total_records, uint32_t* dev_err,
                                              int sms, int idct, cudaStream_t stream) {
     if (total_records == 0) return cudaSuccess;
-    const uint32_t chunks = (total_records + hpvcd::kResChunk - 1) / hpvcd::kResChunk;
-    const uint32_t blocks_needed = (chunks + hpvcd::kResWarps - 1) / hpvcd::kResWarps;
-    const uint32_t cap = (uint32_t)sms * 8u;
-    const int grid = (int)(blocks_needed < cap ? blocks_needed : cap);
+    // Records of a CTA step: at least kResMinChunk (a warp's worth), doubled
+    // while twice as many still give every SM two CTAs, so that a small
+    // picture spreads over the whole chip and a large one fills the lanes of
+    // its 4x4 tasks.
+    constexpr uint32_t kResMinChunk = 32;
+    uint32_t chunk = kResMinChunk;
+    while (chunk < hpvcd::kResMaxChunk && total_records / (2 * chunk) >= 2u * (uint32_t)sms) chunk *= 2;
+    const uint32_t steps = (total_records + chunk - 1) / chunk;
+    const uint32_t cap = (uint32_t)sms * 4u;  // resident CTAs
+    const int grid = (int)(steps < cap ? steps : cap), threads = hpvcd::kResWarps * 32;
     // schedule value: 0 integer tensor cores (the default), 1 butterflies, 2 matrix product
     if (idct == 0)
-        hpvcd::k_residual<hpvcd::kIdctTensor><<<grid, hpvcd::kResWarps * 32, 0, stream>>>(pics, rec_prefix, n_pics,
-                                                                                        dev_err);
+        hpvcd::k_residual<hpvcd::kIdctTensor><<<grid, threads, 0, stream>>>(pics, rec_prefix, n_pics, dev_err, chunk);
     else if (idct == 1)
-        hpvcd::k_residual<hpvcd::kIdctButterfly><<<grid, hpvcd::kResWarps * 32, 0, stream>>>(pics, rec_prefix,
-                                                                                          n_pics, dev_err);
+        hpvcd::k_residual<hpvcd::kIdctButterfly><<<grid, threads, 0, stream>>>(pics, rec_prefix, n_pics, dev_err,
+                                                                             chunk);
     else
-        hpvcd::k_residual<hpvcd::kIdctMatrix><<<grid, hpvcd::kResWarps * 32, 0, stream>>>(pics, rec_prefix, n_pics,
-                                                                                       dev_err);
+        hpvcd::k_residual<hpvcd::kIdctMatrix><<<grid, threads, 0, stream>>>(pics, rec_prefix, n_pics, dev_err, chunk);
     hpvcd_note_launches(1);
     return cudaGetLastError();
 }
