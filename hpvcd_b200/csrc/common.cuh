@@ -39,7 +39,7 @@ struct DevPic {
     void* fin[3];
     int16_t* res[3];        // int16 residual planes of intra TBs (k_residual -> k_recon)
     int32_t res_stride[3];  // row stride of res[c] in samples (multiple of 16)
-    uint32_t* ready;  // wavefront progress: 4 words per CTU, one level (0..4) per component
+    unsigned long long* edges;  // wavefront: edge words of every CTU (edge_words_per_ctu), zero at launch
     // output placement on its RGB canvas
     int32_t dst_x, dst_y, crop_w, crop_h;
     uint64_t canvas_off;  // byte offset of the picture's canvas in the output
@@ -48,6 +48,16 @@ struct DevPic {
     int32_t needs_wavefront;
     int32_t write_fin;  // the tile filter kernel writes the final planes (else only the canvas)
 };
+
+// Edge words of one CTU: its right column and bottom row per component, four
+// samples per 64-bit word (16 bits each, the top bit of the word set once it
+// is written), which neighbouring CTUs poll and read.
+__host__ __device__ inline int edge_words_of(int ctb, int sub_w, int sub_h, int c) {
+    return c ? ctb / sub_w / 4 + ctb / sub_h / 4 : ctb / 2;
+}
+__host__ __device__ inline int edge_words_per_ctu(int ctb, int idc, int sub_w, int sub_h) {
+    return edge_words_of(ctb, sub_w, sub_h, 0) + (idc ? 2 * edge_words_of(ctb, sub_w, sub_h, 1) : 0);
+}
 
 // Work item of the reconstruction kernel: one CTU of one picture.
 struct CtuItem {
@@ -72,19 +82,16 @@ __device__ __forceinline__ void store_sample(void* plane, int bps, size_t idx, i
     else
         ((uint16_t*)plane)[idx] = (uint16_t)v;
 }
-// L2-only load (bypasses L1): used for samples another CTA published.
-__device__ __forceinline__ int load_sample_cg(const void* plane, int bps, size_t idx) {
-    return bps == 1 ? (int)__ldcg((const unsigned char*)plane + idx)
-                    : (int)__ldcg((const unsigned short*)plane + idx);
-}
-
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// Edge words: single-copy atomic 64-bit accesses at device scope.  A word
+// carries its samples and their validity together, so neither side needs a
+// fence or a second access.
+__device__ __forceinline__ unsigned long long ld_edge(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_edge(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // qp helpers: decode.rs:5753-5771, :5868-5871, :7599-7613

@@ -1297,8 +1297,6 @@ constexpr int kRecCap420 = 256 + 64 + 2 * 64;
 constexpr int kRecCap422 = 256 + 64 + 2 * 128;
 constexpr int kRecCap444 = 256 + 64 + 2 * 256;
 constexpr int kListCap = 256;  // intra TBs of luma in one CTU (all 4x4)
-// list entry: record index (< 1024) | kListEvent for a wavefront event
-constexpr uint32_t kListRec = 0x3ffu, kListEvent = 0x8000u;
 constexpr uint32_t kNoStamp = 0xffffffffu;
 
 struct ReconLayout {
@@ -1321,7 +1319,7 @@ struct ReconLayout {
         off_stamp = o; o += 256 * sizeof(uint32_t);
         off_lists = o; o += (size_t)(kListCap + 2 * list_c) * sizeof(uint16_t);
         o = (o + 15) & ~(size_t)15;
-        off_misc = o;  o += 128;  // claimed item, list counts, edge masks, neighbour levels
+        off_misc = o;  o += 128;  // claimed item, list counts, have bits, covered words, done flags
         total = o;
     }
     __host__ __device__ int list_off(int c) const { return c == 0 ? 0 : kListCap + (c - 1) * list_c; }
@@ -1462,57 +1460,189 @@ __device__ __forceinline__ void stage_residual(const Comp& k, int log2n, int x0,
         for (int q = 0; q < chunks; ++q) cp_async16(dst + r * cr + 8 * q, src + (size_t)r * k.rs + 8 * q);
 }
 
-// ---- wavefront progress between neighbouring CTUs ----
-// Every CTU publishes, per component, a level: how many of its quadrants
-// (z-order: top-left, top-right, bottom-left, bottom-right) are
-// reconstructed with their edge samples in the plane.  Other CTUs only read
-// a CTU's right column and bottom row, so the levels that matter are 2 (top
-// half of the right column), 3 (left half of the bottom row) and 4 (all).
-// A CTU reads seven edge segments of its neighbours, each needing one level
-// of one neighbour (0 left, 1 above-left, 2 above, 3 above-right):
-//   bit 0 above-left corner        above-left  >= 4
-//   bit 1 above row, left half      above       >= 3
-//   bit 2 above row, right half     above       >= 4
-//   bit 3 above-right, left half    above-right >= 3
-//   bit 4 above-right, right half   above-right >= 4
-//   bit 5 left column, top half     left        >= 2
-//   bit 6 left column, bottom half  left        >= 4
-constexpr int kSegs = 7;
-constexpr uint32_t kSegMask = (1u << kSegs) - 1u;
+// ---- edges between neighbouring CTUs ----
+// Other CTUs only read a CTU's right column and bottom row.  A CTU publishes
+// them as 64-bit edge words of four samples (common.cuh), each word as soon
+// as the TB that covers it is reconstructed: plain stores, nothing to wait
+// for.  The CTA's edge warp polls the words of the left, above-left, above
+// and above-right CTUs, unpacks them into the canvases and sets a bit per
+// word in shared memory, where the walking warps look before a TB on the
+// CTU's top or left edge.  So a CTU's lag behind its neighbours is a few TBs
+// and a walking warp never waits for a round trip to L2.
+//
+// Have bits of a component: word 0, bit i: row above, samples 4i .. 4i + 3
+// (i < 2S / 4); word 1, bit i < 16: left column, rows 4i .. 4i + 3, bit 16:
+// the corner.  Words outside the picture count as present.
+constexpr uint32_t kHaveCorner = 1u << 16;
 
-__device__ __forceinline__ int seg_nb(int s) { return s == 0 ? 1 : (s <= 2 ? 2 : (s <= 4 ? 3 : 0)); }
-__device__ __forceinline__ uint32_t seg_level(int s) { return s == 5 ? 2u : ((s == 1 || s == 3) ? 3u : 4u); }
-__device__ __forceinline__ int seg_len(int s, int S, int Sh) { return s == 0 ? 1 : (s <= 4 ? S >> 1 : Sh >> 1); }
-
-// Segments of neighbour nb readable once it has reached level v.
-__device__ __forceinline__ uint32_t segs_at(int nb, uint32_t v) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int s = 0; s < kSegs; ++s)
-        if (seg_nb(s) == nb && seg_level(s) <= v) m |= 1u << s;
-    return m;
+// The right-column and bottom-row words of component c of CTU (cx, cy).
+__device__ __forceinline__ unsigned long long* edge_words(const DevPic& P, int cx, int cy, int c) {
+    const int ctb = 1 << P.log2_ctb;
+    const int per = edge_words_per_ctu(ctb, P.idc, P.sub_w, P.sub_h);
+    unsigned long long* w = P.edges + ((size_t)cy * P.ctb_cols + cx) * per;
+    return c ? w + edge_words_of(ctb, P.sub_w, P.sub_h, 0) + (c - 1) * edge_words_of(ctb, P.sub_w, P.sub_h, 1) : w;
+}
+__device__ __forceinline__ unsigned long long edge_pack(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    return (unsigned long long)(a | (b << 16)) | ((unsigned long long)(c | (d << 16) | 0x80000000u) << 32);
 }
 
-// Edge segments an n x n TB at (x, y) of a component CTU S x Sh reads from
-// its neighbours: the row above spans x - 1 .. x + 2n - 1 (intra.rs:84-148),
-// the left column y - 1 .. y + 2n - 1, below-left never past the CTU.
-__device__ __forceinline__ uint32_t segs_needed(int x, int y, int n, int S, int Sh) {
-    uint32_t m = 0;
-    const int hs = S >> 1, hh = Sh >> 1;
-    if (y == 0) {
-        if (x == 0) m |= 1u;
-        const int lo = max(x - 1, 0), hi = min(x + 2 * n, S);
-        if (lo < hs) m |= 2u;
-        if (hi > hs) m |= 4u;
-        if (x + 2 * n > S) m |= 8u;
-        if (x + 2 * n > S + hs) m |= 16u;
+// Publishes the edge words a finished n x n TB at (x0, y0) covers: lanes
+// 0..15 the right column, lanes 16..31 the bottom row.
+__device__ __forceinline__ void publish_tb(const uint16_t* can, int row, int S, int Sh, int x0, int y0, int n,
+                                           unsigned long long* words, int lane) {
+    const bool bottom = lane >= 16;
+    const int i = lane & 15;
+    if (i < (n >> 2) && (bottom ? y0 + n == Sh : x0 + n == S)) {
+        const int x = bottom ? x0 + 4 * i : S - 1, y = bottom ? Sh - 1 : y0 + 4 * i, st = bottom ? 1 : row;
+        const uint16_t* q = can + can_in(S, x, y);
+        st_edge(words + (bottom ? (Sh >> 2) + (x >> 2) : y >> 2), edge_pack(q[0], q[st], q[2 * st], q[3 * st]));
     }
-    if (x == 0) {
-        const int lo = max(y - 1, 0), hi = min(y + 2 * n, Sh);
-        if (lo < hh) m |= 32u;
-        if (hi > hh) m |= 64u;
+}
+
+// One component's place in the CTU, for the edge warp.
+struct EdgeGeo {
+    int ox, oy, S, Sh, pw, ph;
+};
+__device__ __forceinline__ EdgeGeo edge_geo(const DevPic& P, int c, int cx, int cy) {
+    const int ctb = 1 << P.log2_ctb;
+    EdgeGeo e;
+    e.S = c ? ctb / P.sub_w : ctb;
+    e.Sh = c ? ctb / P.sub_h : ctb;
+    e.ox = cx * e.S;
+    e.oy = cy * e.Sh;
+    e.pw = c ? P.cw : P.w;
+    e.ph = c ? P.ch : P.h;
+    return e;
+}
+// Whether this lane's word of the row above / of the left column (lane 16:
+// the corner) lies inside the picture.
+__device__ __forceinline__ bool edge_top_in(const EdgeGeo& e, int lane) {
+    return e.oy > 0 && 4 * lane < 2 * e.S && e.ox + 4 * lane < e.pw;
+}
+__device__ __forceinline__ bool edge_left_in(const EdgeGeo& e, int lane) {
+    if (lane == 16) return e.ox > 0 && e.oy > 0;
+    return e.ox > 0 && 4 * lane < e.Sh && e.oy + 4 * lane < e.ph;
+}
+
+// The edge warp of a CTU: first publishes the edge words no intra TB covers
+// (inter samples, final in the canvas), then receives the neighbours' words
+// until every one has arrived or the walking warps are done.  A wait here
+// cannot outlast them: theirs are bounded.
+template <class CanOf>
+__device__ void edge_service(const DevPic& P, int cx, int cy, int ncomp, CanOf can_of, const uint32_t* cov,
+                             volatile uint32_t* s_have, volatile uint32_t* s_done, int walkers, int lane) {
+    const unsigned long long* tp[3];
+    const unsigned long long* lp[3];
+    uint32_t pend = 0;  // bit 2c: this lane's word above, 2c + 1: left / corner
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        tp[c] = lp[c] = nullptr;
+        if (c >= ncomp) continue;
+        const EdgeGeo e = edge_geo(P, c, cx, cy);
+        const uint32_t full = ((1u << (e.Sh >> 2)) - 1u) | (((1u << (e.S >> 2)) - 1u) << 16);
+        const uint32_t miss = full & ~cov[c];
+        if (miss >> lane & 1u) {
+            const uint16_t* can = can_of(c);
+            const bool bottom = lane >= 16;
+            const int i = lane & 15, st = bottom ? 1 : can_row(e.S);
+            const uint16_t* q = can + (bottom ? can_in(e.S, 4 * i, e.Sh - 1) : can_in(e.S, e.S - 1, 4 * i));
+            st_edge(edge_words(P, cx, cy, c) + (bottom ? (e.Sh >> 2) + i : i),
+                    edge_pack(q[0] & 0x7fffu, q[st] & 0x7fffu, q[2 * st] & 0x7fffu, q[3 * st] & 0x7fffu));
+        }
+        if (edge_top_in(e, lane)) {
+            const int w = e.S >> 2;
+            tp[c] = (lane < w ? edge_words(P, cx, cy - 1, c) + lane : edge_words(P, cx + 1, cy - 1, c) + lane - w) + (e.Sh >> 2);
+            pend |= 1u << (2 * c);
+        }
+        if (edge_left_in(e, lane)) {
+            lp[c] = lane == 16 ? edge_words(P, cx - 1, cy - 1, c) + (e.Sh >> 2) + (e.S >> 2) - 1
+                               : edge_words(P, cx - 1, cy, c) + lane;
+            pend |= 2u << (2 * c);
+        }
     }
-    return m;
+    uint32_t nap = 32;
+    for (;;) {
+        unsigned long long t[3], l[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            t[c] = l[c] = 0ull;
+            if (pend >> (2 * c) & 1u) t[c] = ld_edge(tp[c]);
+            if (pend >> (2 * c) & 2u) l[c] = ld_edge(lp[c]);
+        }
+        bool news = false;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (c >= ncomp) continue;
+            const int S = c ? (1 << P.log2_ctb) / P.sub_w : 1 << P.log2_ctb;
+            uint16_t* can = can_of(c);
+            const bool gt = (long long)t[c] < 0, gl = (long long)l[c] < 0;
+            if (gt) {  // can_at(S, 4 * lane, -1): 8-byte aligned
+                t[c] &= ~(1ull << 63);
+                *(uint2*)(can + 8 + 4 * lane) = make_uint2((uint32_t)t[c], (uint32_t)(t[c] >> 32));
+            }
+            if (gl) {
+                l[c] &= ~(1ull << 63);
+                if (lane == 16) {
+                    can[7] = (uint16_t)(l[c] >> 48);  // can_at(S, -1, -1)
+                } else {
+                    uint16_t* q = can + can_in(S, -1, 4 * lane);
+                    const int row = can_row(S);
+                    q[0] = (uint16_t)l[c];
+                    q[row] = (uint16_t)(l[c] >> 16);
+                    q[2 * row] = (uint16_t)(l[c] >> 32);
+                    q[3 * row] = (uint16_t)(l[c] >> 48);
+                }
+            }
+            const uint32_t bt = __ballot_sync(kFull, gt), bl = __ballot_sync(kFull, gl);
+            if (gt) pend &= ~(1u << (2 * c));
+            if (gl) pend &= ~(2u << (2 * c));
+            if (bt | bl) {
+                news = true;
+                __threadfence_block();  // the samples before their bits
+                __syncwarp();
+                if (lane == 0) {
+                    s_have[2 * c] = s_have[2 * c] | bt;
+                    s_have[2 * c + 1] = s_have[2 * c + 1] | bl;
+                }
+            }
+        }
+        if (!__any_sync(kFull, pend != 0u)) break;
+        int done = 0;
+        for (int w = 0; w < walkers; ++w) done += s_done[w] != 0u;
+        if (done == walkers) break;
+        if (news) {
+            nap = 32;
+        } else {
+            __nanosleep(nap);
+            nap = min(2 * nap, 256u);
+        }
+    }
+}
+
+// Waits (bounded, in shared memory) until the words a TB needs are in the
+// canvas; after a wait that ran out every word counts as present.
+struct Have {
+    uint32_t top, left;
+};
+__device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need_left, const volatile uint32_t* s_have,
+                                        uint32_t spin_limit, uint32_t* dev_err, int lane) {
+    uint32_t spins = 0;
+    for (;;) {
+        h.top = s_have[0];
+        h.left = s_have[1];
+        if (!((need_top & ~h.top) | (need_left & ~h.left))) break;
+        if (++spins > spin_limit) {
+            if (lane == 0) atomicOr(dev_err, DEV_ERR_TIMEOUT);
+            h.top = h.left = 0xffffffffu;
+            break;
+        }
+        if (spins > 16) __nanosleep(spins > 1024 ? 64 : 16);
+    }
+    // one lane may have seen a later state than another
+    h.top = __reduce_and_sync(kFull, h.top);
+    h.left = __reduce_and_sync(kFull, h.left);
+    __threadfence_block();
+    return h;
 }
 
 // ---- walk entries: everything about an intra TB that does not depend on
@@ -1530,30 +1660,32 @@ __device__ __forceinline__ uint32_t segs_needed(int x, int y, int n, int S, int 
 // prediction), or that has none, is flagged kTbGather and its line is gathered
 // sample by sample first.
 //   x: canvas offset of the TB | of line position 0 << 16
-//   y: canvas offset of the corner | lo << 16 | hi << 24
-//   z: x | y << 8 (in the CTU) | log2n << 16 | mode << 20 | kTb* flags
-//   w: edge segments read | quadrant << 8 | record index << 16
-// Measured (4032x3024 grid, 70 luma TBs a CTU): the walk's chain went from
-// ~87k to ~46k cycles a CTU (4x4 700 -> 500, 16x16 5100 -> 1650, 32x32 10700 ->
-// 3300 cycles); 512x512 tile 1004 -> 649 us, 3840x2160 picture 6465 -> 4705 us.
-constexpr uint32_t kTbCoded = 1u << 26, kTbFilt = 1u << 27, kTbGather = 1u << 28, kTbPcm = 1u << 29;
+//   y: canvas offset of the corner | row of the angular table << 16
+//   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbCoded | kTbFilt
+//   w: x | y << 8 (in the CTU) | record index << 16
+// Measured when the entries came in (4032x3024 grid, 70 luma TBs a CTU): the
+// walk's chain went from ~87k to ~46k cycles a CTU (4x4 700 -> 500, 16x16 5100
+// -> 1650, 32x32 10700 -> 3300 cycles); 512x512 tile 1004 -> 649 us.
+constexpr uint32_t kTbCoded = 1u << 30, kTbFilt = 1u << 31;
 
 struct TbEntry {
     uint4 w;
     __device__ __forceinline__ int org() const { return (int)(w.x & 0xffffu); }
     __device__ __forceinline__ int line0() const { return (int)(w.x >> 16); }
     __device__ __forceinline__ int corner() const { return (int)(w.y & 0xffffu); }
-    __device__ __forceinline__ int lo() const { return (int)((w.y >> 16) & 0xffu); }
-    __device__ __forceinline__ int hi() const { return (int)(w.y >> 24); }
-    __device__ __forceinline__ int x() const { return (int)(w.z & 0xffu); }
-    __device__ __forceinline__ int y() const { return (int)((w.z >> 8) & 0xffu); }
-    __device__ __forceinline__ int log2n() const { return (int)((w.z >> 16) & 0xfu); }
-    __device__ __forceinline__ int mode() const { return (int)((w.z >> 20) & 0x3fu); }
+    __device__ __forceinline__ uint32_t lut() const { return w.y >> 16; }
+    __device__ __forceinline__ int lo() const { return (int)(w.z & 0xffu); }
+    __device__ __forceinline__ int hi() const { return (int)((w.z >> 8) & 0xffu); }
+    __device__ __forceinline__ int n2() const { return (int)((w.z >> 16) & 0xffu); }
+    __device__ __forceinline__ int mode() const { return (int)((w.z >> 24) & 0x3fu); }
+    __device__ __forceinline__ int x() const { return (int)(w.w & 0xffu); }
+    __device__ __forceinline__ int y() const { return (int)((w.w >> 8) & 0xffu); }
 };
 
-// The walk entry of intra record j (t, at (x0, y0) of the CTU).
+// The walk entry of intra record j (t, at (x0, y0) of the CTU); *gather: its
+// line is not one run of available samples.
 __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, int x0, int y0, uint32_t jrec,
-                                            const uint32_t* stamp, bool coded, bool pcm) {
+                                            const uint32_t* stamp, bool coded, bool* gather) {
     const int n = 1 << t.log2n, n2 = 2 * n;
     // cells one sample apart in this component's units
     const int uw = 4 / k.sw, uh = 4 / k.sh;
@@ -1605,17 +1737,17 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
             lo = n2 + 1;
     }
     if (lo > hi) one_run = false;  // nothing available
-    uint32_t z = (uint32_t)x0 | ((uint32_t)y0 << 8) | ((uint32_t)t.log2n << 16) | ((uint32_t)t.mode << 20);
-    if (coded) z |= kTbCoded;
-    if (n > 4 && ref_filtered(k, n, t.mode)) z |= kTbFilt;
-    if (!one_run) z |= kTbGather, lo = 0, hi = 4 * n;
-    if (pcm) z |= kTbPcm;
-    const uint32_t q = (x0 >= (k.S >> 1) ? 1u : 0u) + (y0 >= (k.Sh >> 1) ? 2u : 0u);
+    if (!one_run) lo = 0, hi = 4 * n;
+    *gather = !one_run;
+    const uint32_t am = t.mode >= 2 ? t.mode - 2u : 0u;
+    const uint32_t lut = n == 4 ? am * 16u : (n == 8 ? 33u * 16u + am * 32u : 0u);
     uint4 w;
     w.x = (uint32_t)cin(k, x0, y0) | ((uint32_t)cin(k, x0 - 1, y0 + n2 - 1) << 16);
-    w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | ((uint32_t)lo << 16) | ((uint32_t)hi << 24);
-    w.z = z;
-    w.w = segs_needed(x0, y0, n, k.S, k.Sh) | (q << 8) | (jrec << 16);
+    w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (lut << 16);
+    w.z = (uint32_t)lo | ((uint32_t)hi << 8) | ((uint32_t)n2 << 16) | ((uint32_t)t.mode << 24);
+    if (coded) w.z |= kTbCoded;
+    if (n > 4 && ref_filtered(k, n, t.mode)) w.z |= kTbFilt;
+    w.w = (uint32_t)x0 | ((uint32_t)y0 << 8) | (jrec << 16);
     return w;
 }
 
@@ -1623,8 +1755,8 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
 // the two line positions it interpolates (intra.rs:305-318, the projection
 // of negative angles included) and their weights: p0 | p1 << 8 | weight of
 // p1 << 16 | weight of p0 << 24.
-struct AngularTables {
-    uint32_t t4[33][16], t8[33][64];
+struct AngularTables {  // rows of uint2: 33 x 16 lanes (4x4, .x only), then 33 x 32 lanes (8x8)
+    uint32_t t4[33][16][2], t8[33][32][2];
 };
 constexpr uint32_t angular_entry(int mode, int n, int x, int y) {
     constexpr int ang[33] = {32,  26,  21,  17,  13,  9,  5,  2,  0,  -2, -5, -9, -13, -17, -21, -26, -32,
@@ -1652,9 +1784,9 @@ constexpr uint32_t angular_entry(int mode, int n, int x, int y) {
 constexpr AngularTables make_angular() {
     AngularTables T{};
     for (int m = 0; m < 33; ++m) {
-        for (int i = 0; i < 16; ++i) T.t4[m][i] = angular_entry(m + 2, 4, i & 3, i >> 2);
+        for (int i = 0; i < 16; ++i) T.t4[m][i][0] = angular_entry(m + 2, 4, i & 3, i >> 2);
         // lane l of an 8x8 TB predicts samples (2 (l & 3) + h, l >> 2)
-        for (int i = 0; i < 64; ++i) T.t8[m][i] = angular_entry(m + 2, 8, 2 * ((i >> 1) & 3) + (i & 1), i >> 3);
+        for (int i = 0; i < 64; ++i) T.t8[m][i >> 1][i & 1] = angular_entry(m + 2, 8, 2 * ((i >> 1) & 3) + (i & 1), i >> 3);
     }
     return T;
 }
@@ -1665,10 +1797,10 @@ __device__ const __align__(16) AngularTables g_angular = make_angular();
 // [lo, hi] that substitutes unavailable samples.
 struct Line {
     int l0, ls, c0, lo, hi, n2;
-    __device__ __forceinline__ Line(const TbEntry& E, int row) {
-        n2 = 2 << E.log2n();
+    __device__ __forceinline__ Line(const TbEntry& E, int stride) {
+        n2 = E.n2();
         l0 = E.line0();
-        ls = (E.w.z & kTbGather) ? -1 : row;  // a gathered line lies upwards in the warp's scratch
+        ls = stride;
         c0 = E.corner() - n2;
         lo = E.lo();
         hi = E.hi();
@@ -1719,13 +1851,16 @@ __device__ __forceinline__ void walk_tb4(uint16_t* can, int row, int org, int mo
     __syncwarp();
 }
 
-// 8x8 intra TB: v is line position `lane`, v_hi position 32 (the same in
-// every lane); [1 2 1] filtering (intra.rs:151-219; no strong filter below
+// 8x8 intra TB: v is line position `lane`, v_hi position 32 where it is
+// available (the same in every lane; else position 31 stands in for it);
+// [1 2 1] filtering (intra.rs:151-219; no strong filter below
 // 32x32) and prediction (intra.rs:257-372) by shuffles, two horizontally
 // adjacent samples per lane.
 __device__ __forceinline__ void walk_tb8(uint16_t* can, int row, int org, int mode, bool coded, bool filt, bool luma,
-                                         int max_v, int v, int v_hi, uint2 lut, int lane) {
+                                         int max_v, int v, int v_hi, bool hi_ok, uint2 lut, int lane) {
     constexpr int n = 8, n2 = 16;
+    const int v31 = __shfl_sync(kFull, v, 31);
+    v_hi = hi_ok ? v_hi : v31;
     const int yy = lane >> 2, xx = 2 * (lane & 3);
     uint32_t* px = (uint32_t*)(can + org + yy * row + xx);  // canvas rows and TB columns are even
     const uint32_t rv = coded ? *px : 0u;
@@ -1935,171 +2070,36 @@ __device__ __noinline__ void gather_line(const Comp& k, int log2n, int x0, int y
     __syncwarp();
 }
 
-// One component's neighbour edges as the canvas holds them: row 0 is the
-// row above (x = -1 at index 7, x at 8 + x), column 7 the left column.
-struct EdgeGeo {
-    void* plane;
-    uint16_t* can;
-    int ox, oy, S, Sh, pw, ph;
-};
+// Warps of a k_recon CTA: warp 0 walks luma, chroma is walked by warp 1 (Cb,
+// then Cr: kCW = 1) or by warps 1 and 2 (one component each: kCW = 2), and the
+// last warp moves edge words.  At 4:2:0 a CTU's two chroma walks together are
+// shorter than its luma walk, so one warp for both loses nothing; at 4:2:2 and
+// 4:4:4 they would be the longer chain.
+__host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 
-// Loads the segments m of one component into its canvas, thread t of nt
-// taking samples t, t + nt, ... (a rolled loop: this runs inside the walk,
-// whose code competes for the instruction cache).  Samples outside the
-// picture read as 0 (they are never available).
-__device__ __forceinline__ void fetch_edges(const EdgeGeo& e, uint32_t m, int bps, int t, int nt) {
-    int total = 0;
-#pragma unroll 1
-    for (int s = 0; s < kSegs; ++s)
-        if (m >> s & 1u) total += seg_len(s, e.S, e.Sh);
-#pragma unroll 1
-    for (int i = t; i < total; i += nt) {
-        int j = i, s = 0;
-#pragma unroll 1
-        for (; s < kSegs; ++s) {
-            if (!(m >> s & 1u)) continue;
-            const int L = seg_len(s, e.S, e.Sh);
-            if (j < L) break;
-            j -= L;
-        }
-        if (s >= kSegs) break;  // unreachable: i < total
-        int dx, dy;
-        if (s == 0) {
-            dx = -1, dy = -1;
-        } else if (s <= 4) {
-            dx = (s - 1) * (e.S >> 1) + j, dy = -1;
-        } else {
-            dx = -1, dy = (s - 5) * (e.Sh >> 1) + j;
-        }
-        const int ax = e.ox + dx, ay = e.oy + dy;
-        int v = 0;
-        if (ax >= 0 && ay >= 0 && ax < e.pw && ay < e.ph) v = load_sample_cg(e.plane, bps, (size_t)ay * e.pw + ax);
-        e.can[can_at(e.S, dx, dy)] = (uint16_t)v;
-    }
-}
-
-// Writes the edge samples of quadrants [from, to) of one component to the
-// plane (lanes of one warp) and releases level `to`: the warp barrier orders
-// every lane's stores before lane 0's release store, which is cumulative.
-__device__ __forceinline__ void publish_level(const EdgeGeo& e, int bps, int from, int to, uint32_t* level,
-                                              int lane) {
-    const int rows = min(e.Sh, e.ph - e.oy), cols = min(e.S, e.pw - e.ox);
-    const int hs = e.S >> 1, hh = e.Sh >> 1;
-    const bool right = cols == e.S, bottom = rows == e.Sh;  // a neighbour exists on that side
-    // right column rows [r0, r1), bottom row cols [b0, b1)
-    const int r0 = from < 2 ? 0 : hh, r1 = to >= 4 ? e.Sh : (to >= 2 ? hh : 0);
-    const int b0 = from < 3 ? 0 : hs, b1 = to >= 4 ? e.S : (to >= 3 ? hs : 0);
-    const int nr = right ? max(0, min(r1, rows) - r0) : 0;
-    const int nb = bottom ? max(0, min(b1, cols) - b0) : 0;
-    __syncwarp();
-    for (int i = lane; i < nr + nb; i += 32) {
-        int x, y;
-        if (i < nr)
-            x = e.S - 1, y = r0 + i;
-        else
-            x = b0 + i - nr, y = e.Sh - 1;
-        store_sample(e.plane, bps, (size_t)(e.oy + y) * e.pw + e.ox + x, e.can[can_in(e.S, x, y)]);
-    }
-    __syncwarp();
-    if (lane == 0) st_release(level, (uint32_t)to);
-}
-
-// Edge geometry of component c of CTU (cx, cy) of picture P.
-__device__ __forceinline__ EdgeGeo edge_geo(const DevPic& P, uint16_t* can, int c, int cx, int cy) {
-    const int ctb = 1 << P.log2_ctb;
-    EdgeGeo e;
-    e.plane = P.rec[c];
-    e.can = can;
-    e.S = c ? ctb / P.sub_w : ctb;
-    e.Sh = c ? ctb / P.sub_h : ctb;
-    e.ox = cx * e.S;
-    e.oy = cy * e.Sh;
-    e.pw = c ? P.cw : P.w;
-    e.ph = c ? P.ch : P.h;
-    return e;
-}
-
-// The walk's rare step, taken only by TBs flagged when the lists were built
-// (a per-TB test in the loop itself costs the walk about 10 %): release the
-// quadrants before this TB's quadrant q (edge samples of quadrants from `prog`
-// on go to the plane), then make sure the canvas holds the neighbour segments
-// `miss` that the TB reads: lanes 0..3 wait (bounded) for one neighbour each
-// and the warp loads every segment the levels seen release.  Returns segments
-// held | (quadrants done << 8).
-__device__ __forceinline__ uint32_t walk_event(const DevPic& P, uint16_t* can, int c, int cx, int cy, int q,
-                                            uint32_t miss, int prog, uint32_t have, uint32_t spin_limit,
-                                            uint32_t* dev_err, int lane) {
-    const EdgeGeo e = edge_geo(P, can, c, cx, cy);
-    if (q > prog) {
-        if (q >= 2) publish_level(e, P.bps, prog, q, P.ready + ((size_t)cy * P.ctb_cols + cx) * 4 + c, lane);
-        prog = q;
-    }
-    if (miss) {
-        uint32_t lv = 0u;  // level seen (0: not polled)
-        if (lane < 4) {
-            uint32_t need = 0;
-            for (int s = 0; s < kSegs; ++s)
-                if ((miss >> s & 1u) && seg_nb(s) == lane) need = max(need, seg_level(s));
-            const int nx = cx + (lane == 3 ? 1 : (lane == 2 ? 0 : -1));
-            const int ny = cy - (lane == 0 ? 0 : 1);
-            if (nx < 0 || ny < 0 || nx >= P.ctb_cols) {
-                lv = 4u;  // outside the picture: nothing to wait for
-            } else if (need) {
-                const uint32_t* f = P.ready + ((size_t)ny * P.ctb_cols + nx) * 4 + c;
-                uint32_t spins = 0;
-                while ((lv = ld_acquire(f)) < need) {
-                    if (++spins > spin_limit) {
-                        atomicOr(dev_err, DEV_ERR_TIMEOUT);
-                        lv = need;
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-        }
-        __syncwarp();  // orders the acquires before every lane's loads
-        uint32_t got = 0;
-#pragma unroll
-        for (int nb = 0; nb < 4; ++nb) got |= segs_at(nb, __shfl_sync(kFull, lv, nb));
-        got = (got | miss) & ~have;
-        fetch_edges(e, got, P.bps, lane, 32);
-        have |= got;
-        __syncwarp();
-    }
-    return have | ((uint32_t)prog << 8);
-}
-
-// Warps of a k_recon CTA: warp 0 walks luma, chroma is walked by warp 1
-// (Cb, then Cr: kCW = 1) or by warps 1 and 2 (one component each: kCW = 2).
-// Two warps keep eight CTU walks resident per SM at 4:2:0 (shared memory
-// and registers both allow it); the third warp shortens a CTU whose chroma
-// walk is as long as its luma walk (4:4:4).
-// Register-capped build (kDense, three warps only): at most 80 registers
-// per thread so that eight CTAs of three warps fit an SM instead of five.
-// Each walk is a few percent slower, which costs a single picture whose
-// wavefront holds few CTUs at a time; a batch with thousands of CTUs ready
-// at once is bound by the walks resident per SM instead (a fused batch of
-// 256 mixed-size images: reconstruction 73 -> 61 ms).
-__host__ __device__ constexpr int recon_warps(int kCW) { return 1 + kCW; }
+// List entry flags beside the record index (< 1024): the TB reads neighbour
+// CTUs, its line must be gathered, it is an I_PCM block, it covers edge words.
+constexpr uint32_t kListRec = 0x3ffu;
+constexpr uint32_t kListEdge = 0x8000u, kListGather = 0x4000u, kListPcm = 0x2000u, kListPub = 0x1000u;
 
 // kFeat: some picture of the launch has slices / tiles, constrained intra
 // prediction, cross-component prediction or I_PCM blocks; without them the
-// availability, coded and PCM tests compile to the plain form.  fine: the
-// quadrant-level wavefront; otherwise a CTU waits for its neighbours' last
-// level before its walk and releases only its last level.
-template <int kCW, bool kFeat, bool kDense = false>
-__global__ void __launch_bounds__(32 * recon_warps(kCW), kDense ? 8 : (kCW == 1 ? 8 : 5))
+// availability, coded and PCM tests compile to the plain form.  fine: a TB
+// waits for the edge words it reads; otherwise a CTU waits for all of its
+// neighbours' words before its walk.
+template <int kCW, bool kFeat>
+__global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 7 : 5)
 k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint32_t n_items,
         uint32_t* work_counter, uint32_t* dev_err, int cfmt, uint32_t spin_limit, int fine) {
     static_assert(kCW == 1 || kCW == 2, "one or two chroma warps");
-    static_assert(!kDense || kCW == 2, "the register-capped build has three warps");
-    constexpr int kWarps = recon_warps(kCW), kThreads = 32 * kWarps;
+    constexpr int kWarps = recon_warps(kCW), kThreads = 32 * kWarps, kWalkers = kWarps - 1;
     extern __shared__ __align__(16) unsigned char smem[];
     const ReconLayout lay(cfmt, kWarps);
     uint32_t* s_item = (uint32_t*)(smem + lay.off_misc);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // components walked (and listed) by this warp: [c_lo, c_hi]
-    const int c_lo = warp == 0 ? 0 : (kCW == 1 ? 1 : warp), c_hi = warp == 0 ? 0 : (kCW == 1 ? 2 : warp);
+    // components walked (and listed) by this warp: [c_lo, c_hi], none for the edge warp
+    const int c_lo = warp == kWalkers ? 3 : (warp == 0 ? 0 : (kCW == 1 ? 1 : warp));
+    const int c_hi = warp == 0 ? 0 : (kCW == 1 ? 2 : warp);
     for (;;) {
         __syncthreads();
         if (tid == 0) *s_item = atomicAdd(work_counter, 1u);
@@ -2128,7 +2128,10 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         uint4* recs = (uint4*)(smem + lay.off_recs);
         uint32_t* stamp = (uint32_t*)(smem + lay.off_stamp);
         uint16_t* lists = (uint16_t*)(smem + lay.off_lists);
-        uint32_t* counts = (uint32_t*)(smem + lay.off_misc) + 1;
+        uint32_t* counts = (uint32_t*)(smem + lay.off_misc) + 1;  // TBs listed per component
+        uint32_t* s_have = counts + 3;                            // have bits, two words per component
+        uint32_t* s_cov = s_have + 6;                             // edge words covered by intra TBs
+        uint32_t* s_done = s_cov + 3;                             // walking warps that are done
         auto can_of = [&](int c) -> uint16_t* {
             return c == 0 ? (uint16_t*)(smem + lay.off_can_y)
                           : (uint16_t*)(smem + lay.off_can_c) + (size_t)(c - 1) * can_size(lay.cs_w, lay.cs_h);
@@ -2137,6 +2140,14 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         for (uint32_t i = tid; i < nrec; i += kThreads) cp_async16(recs + i, P.tus + r0 + i);
         asm volatile("cp.async.commit_group;" ::: "memory");
         for (int i = tid; i < 256; i += kThreads) stamp[i] = kNoStamp;
+        if (tid < 3) counts[tid] = s_cov[tid] = s_done[tid] = 0u;
+        if (warp == kWalkers)  // words outside the picture count as present
+            for (int c = 0; c < ncomp; ++c) {
+                const EdgeGeo e = edge_geo(P, c, it.cx, it.cy);
+                const uint32_t t = __ballot_sync(kFull, edge_top_in(e, lane));
+                const uint32_t l = __ballot_sync(kFull, edge_left_in(e, lane));
+                if (lane == 0) s_have[2 * c] = ~t, s_have[2 * c + 1] = ~l;
+            }
         // the CTU's own records have arrived: the decode-order build below
         // runs before the neighbour wait, off the critical path
         cp_async_wait_all();
@@ -2171,46 +2182,26 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 for (int cx = x >> 2; cx < (x1 + 3) >> 2; ++cx) atomicMin(&stamp[cy * 16 + cx], i);
         }
         for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
-            const int hs = (c ? Scw : ctb) >> 1, hh = (c ? Sch : ctb) >> 1;
             const uint32_t cap = (uint32_t)lay.list_cap(c);
             uint16_t* list = lists + lay.list_off(c);
             uint32_t cnt = 0;
-            int qmax = 0;  // quadrant of the entries listed so far (z-order: never decreases)
             for (uint32_t base = 0; base < nrec; base += 32) {
                 const uint32_t i = base + lane;
                 bool mine = false;
-                int q = -1;
-                bool edge = false;
                 if (i < nrec) {
                     hpvcd_tu t;
                     memcpy(&t, &recs[i], sizeof(t));
                     int x, y;
                     if (t.comp == c && (t.flags & HPVCD_TU_INTRA) && intra_pred_ok && rec_check(t, x, y) == 1) {
-                        if (t.mode > 34 || t.log2n > 5) {
+                        if (t.mode > 34 || t.log2n > 5)
                             atomicOr(dev_err, DEV_ERR_BITSTREAM);
-                        } else {
+                        else
                             mine = true;
-                            q = (x >= hs ? 1 : 0) + (y >= hh ? 2 : 0);
-                            edge = x == 0 || y == 0;
-                        }
                     }
                 }
-                // running maximum of q over the list order: an entry that opens
-                // a later quadrant, or sits on the CTU's top / left edge, is an
-                // event of the quadrant-level wavefront
-                int run = q;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int o = __shfl_up_sync(kFull, run, d);
-                    if (lane >= d) run = max(run, o);
-                }
-                int before = __shfl_up_sync(kFull, run, 1);
-                before = max(lane ? before : -1, qmax);
-                qmax = max(qmax, __shfl_sync(kFull, run, 31));
-                const bool event = fine && (q > before || edge);
                 const uint32_t m = __ballot_sync(kFull, mine);
                 const uint32_t pos = cnt + __popc(m & ((1u << lane) - 1u));
-                if (mine && pos < cap) list[pos] = (uint16_t)(i | (event ? kListEvent : 0u));
+                if (mine && pos < cap) list[pos] = (uint16_t)i;
                 cnt += __popc(m);
             }
             if (cnt > cap) {
@@ -2222,12 +2213,23 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         __syncthreads();
         // A CTU without intra TBs (inter pictures) has its final samples in the
         // plane already: it neither waits for its neighbours nor rewrites
-        // anything, it only releases every component for the CTUs that
-        // predict from it.
-        const bool any_intra = counts[0] + (ncomp > 1 ? counts[1] + counts[2] : 0u) > 0u;
-        uint32_t* level = P.ready + (size_t)ci * 4;  // per-component progress of this CTU
-        if (!any_intra) {
-            if (tid < ncomp) st_release(level + tid, 4u);
+        // anything, it only publishes its edge words.
+        if (!(counts[0] | counts[1] | counts[2])) {
+            for (int c = 0; c < ncomp; ++c) {
+                const EdgeGeo e = edge_geo(P, c, it.cx, it.cy);
+                const int nr = e.Sh >> 2, nw = nr + (e.S >> 2);
+                unsigned long long* words = edge_words(P, it.cx, it.cy, c);
+                for (int i = tid; i < nw; i += kThreads) {
+                    uint32_t v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int ax = e.ox + (i < nr ? e.S - 1 : 4 * (i - nr) + u);
+                        const int ay = e.oy + (i < nr ? 4 * i + u : e.Sh - 1);
+                        v[u] = ax < e.pw && ay < e.ph ? (uint32_t)load_sample(P.rec[c], P.bps, (size_t)ay * e.pw + ax) : 0u;
+                    }
+                    st_edge(words + i, edge_pack(v[0], v[1], v[2], v[3]));
+                }
+            }
             continue;
         }
         // Inter pictures: the plane holds motion-compensated + residual
@@ -2258,37 +2260,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             nb_ok = (same(cx - 1, cy) ? 1u : 0u) | (same(cx - 1, cy - 1) ? 2u : 0u) | (same(cx, cy - 1) ? 4u : 0u) |
                     (same(cx + 1, cy - 1) ? 8u : 0u);
         }
-        // ---- neighbour edges available now: one level read per neighbour
-        // and component, then every segment already released is loaded ----
-        auto geo = [&](int c) { return edge_geo(P, can_of(c), c, it.cx, it.cy); };
-        uint32_t* s_have = (uint32_t*)(smem + lay.off_misc) + 4;
-        uint32_t* s_lvl = (uint32_t*)(smem + lay.off_misc) + 8;
-        // neighbour nb of this CTU: its level words, or null outside the picture
-        auto nb_level = [&](int nb) -> const uint32_t* {
-            const int nx = it.cx + (nb == 3 ? 1 : (nb == 2 ? 0 : -1));
-            const int ny = it.cy - (nb == 0 ? 0 : 1);
-            if (nx < 0 || ny < 0 || nx >= P.ctb_cols) return nullptr;
-            return P.ready + ((size_t)ny * P.ctb_cols + nx) * 4;
-        };
-        if (tid < 4 * ncomp) {
-            const uint32_t* f = nb_level(tid & 3);
-            uint32_t v = 4u;
-            if (f) {
-                v = ld_acquire(f + (tid >> 2));
-                uint32_t spins = 0;
-                while (!fine && v < 4u) {  // whole-CTU wavefront: wait (bounded) for the last level
-                    if (++spins > spin_limit) {
-                        atomicOr(dev_err, DEV_ERR_TIMEOUT);
-                        v = 4u;
-                        break;
-                    }
-                    __nanosleep(64);
-                    v = ld_acquire(f + (tid >> 2));
-                }
-            }
-            s_lvl[tid] = v;
-        }
-        __syncthreads();
+        if (P.flags & HPVCD_PIC_INTER) __syncthreads();  // the interior before the residuals staged over it
         // Everything one walking warp needs about component c of this CTU.
         auto comp_of = [&](int c) -> Comp {
             Comp k;
@@ -2316,8 +2288,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             k.res = P.res[c] + (size_t)k.oy * k.rs + k.ox;
             return k;
         };
-        // ---- residuals into the canvas, before the walk: the copies overlap
-        // the neighbour edge loads below.  In an intra picture every sample
+        // ---- residuals into the canvas, before the walk.  In an intra picture every sample
         // of the CTU comes from the walk, so the whole visible residual block
         // of each component is copied by all threads (the areas of uncoded
         // TBs are never read); in an inter picture the canvas holds inter
@@ -2352,103 +2323,113 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 const bool coded = (t.flags & HPVCD_TU_CBF) != 0 || (k.ccp && t.res_scale);
                 const bool pcm = kFeat && (t.flags & HPVCD_TU_PCM);
                 if ((P.flags & HPVCD_PIC_INTER) && coded && !pcm) stage_residual(k, t.log2n, x, y);
-                const uint4 w = make_entry(k, t, x, y, j, stamp, coded, pcm);
-                recs[j] = w;
-                if (w.z & kTbGather) list[e] |= (uint16_t)kListEvent;
+                bool gather;
+                recs[j] = make_entry(k, t, x, y, j, stamp, coded, &gather);
+                uint32_t f = pcm ? kListPcm : 0u;
+                if (x == 0 || y == 0) f |= kListEdge;
+                if (gather) f |= kListGather;
+                const int n = 1 << t.log2n;
+                const uint32_t run = (1u << (n >> 2)) - 1u;
+                uint32_t cov = 0;
+                if (x + n == k.S) cov |= run << (y >> 2);
+                if (y + n == k.Sh) cov |= run << (16 + (x >> 2));
+                if (cov) {
+                    f |= kListPub;
+                    atomicOr(&s_cov[c], cov);
+                }
+                list[e] = (uint16_t)(j | f);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (tid < ncomp) {
-            uint32_t h = 0;
-            for (int nb = 0; nb < 4; ++nb) h |= segs_at(nb, s_lvl[tid * 4 + nb]);
-            s_have[tid] = h;
-        }
-        __syncthreads();
-        for (int c = 0; c < ncomp; ++c) fetch_edges(geo(c), s_have[c], P.bps, tid, kThreads);
         cp_async_wait_all();  // this thread's residual copies; the barrier publishes them
         __syncthreads();
+        if (warp == kWalkers) {
+            edge_service(P, it.cx, it.cy, ncomp, can_of, s_cov, s_have, s_done, kWalkers, lane);
+        }
         // ---- decode-order walk: each warp reconstructs its components ----
         WalkScratch& ws = *(WalkScratch*)(smem + lay.off_ws + (size_t)warp * kWsBytes);
         for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
             const Comp k = comp_of(c);
             const uint32_t cnt = counts[c];
             const uint16_t* list = lists + lay.list_off(c);
-            // edge segments in the canvas, quadrants released
-            uint32_t have = s_have[c];
-            int prog = 0;
             // Software pipeline: while a TB is reconstructed, the next one's
             // line address and table entry are worked out and the entry after
             // it is loaded.
             uint16_t* const can = k.can;
             const int row = can_row(k.S);
             const bool luma = c == 0;
-            auto line_at = [&](const TbEntry& E, int i) { return Line(E, row).at(i); };
-            auto first_pos = [&](const TbEntry& E) { return line_at(E, min(lane, 4 << E.log2n())); };
+            unsigned long long* const words = edge_words(P, it.cx, it.cy, c);
             auto lut_of = [&](const TbEntry& E) -> uint2 {
-                const int m = max(E.mode() - 2, 0);
-                const uint32_t* t4 = &g_angular.t4[m][lane & 14];
-                const uint32_t* t8 = &g_angular.t8[m][2 * lane];
-                uint2 u = __ldg((const uint2*)(E.log2n() == 2 ? t4 : t8));
-                if (E.log2n() == 2 && (lane & 1)) u.x = u.y;
-                return u;
+                return __ldg((const uint2*)&g_angular + E.lut() + (E.n2() == 16 ? lane : lane & 15));
             };
+            Have have{0u, 0u};
+            if (!fine && cnt) have = wait_edges(have, 0xffffffffu, 0xffffffffu, s_have + 2 * c, spin_limit, dev_err, lane);
             const uint32_t last = cnt ? cnt - 1 : 0u;
             TbEntry E{}, En{};
             uint32_t j0 = 0, j1 = 0, j2 = 0;
-            int adr = 0, adr_hi = 0;
+            int adr = 0;
             uint2 lut = make_uint2(0u, 0u);
             if (cnt) {
                 j0 = list[0], j1 = list[min(1u, last)], j2 = list[min(2u, last)];
                 E.w = recs[j0 & kListRec];
                 En.w = recs[j1 & kListRec];
-                adr = first_pos(E);
-                adr_hi = line_at(E, 32);
+                adr = Line(E, row).at(lane);  // positions past the line clamp to its last one
                 lut = lut_of(E);
             }
             for (uint32_t e = 0; e < cnt; ++e) {
-                if (j0 & kListEvent) {
-                    const int q = (int)((E.w.w >> 8) & 3u);
-                    const uint32_t miss = E.w.w & kSegMask & ~have;
-                    if (fine && (miss || q > prog)) {
-                        const uint32_t r =
-                            walk_event(P, can, c, it.cx, it.cy, q, miss, prog, have, spin_limit, dev_err, lane);
-                        have = r & kSegMask;
-                        prog = (int)(r >> 8);
+                const int n2 = E.n2(), mode = E.mode();
+                int stride = row;
+                if (j0 & (kListEdge | kListGather)) {
+                    // the words it reads: with x = 0 the left column from row
+                    // y - 1 on, with y = 0 the row above from sample x - 1 on
+                    const int x = E.x(), y = E.y();
+                    uint32_t need_top = 0u, need_left = 0u;
+                    if (y == 0) {
+                        const int lo = max(x - 1, 0) >> 2, hi = (x + n2) >> 2;
+                        need_top = (0xffffffffu >> (32 - (hi - lo))) << lo;
                     }
-                    if (E.w.z & kTbGather) {
-                        gather_line(k, E.log2n(), E.x(), E.y(), stamp, E.w.w >> 16, ws, lane);
-                        const uint32_t at = (uint32_t)(ws.s - can);
+                    if (x == 0) {
+                        const int lo = max(y - 1, 0) >> 2, hi = min(y + n2, k.Sh) >> 2;
+                        need_left = ((1u << (hi - lo)) - 1u) << lo;
+                        if (y == 0) need_left |= kHaveCorner;
+                    }
+                    if ((need_top & ~have.top) | (need_left & ~have.left))
+                        have = wait_edges(have, need_top, need_left, s_have + 2 * c, spin_limit, dev_err, lane);
+                    if (j0 & kListGather) {
+                        gather_line(k, 31 - __clz(n2) - 1, x, y, stamp, E.w.w >> 16, ws, lane);
+                        const uint32_t at = (uint32_t)(ws.s - can);  // position i at canvas offset at + i
                         E.w.x = (E.w.x & 0xffffu) | (at << 16);
-                        E.w.y = (E.w.y & 0xffff0000u) | (at + (2u << E.log2n()));
-                        adr = first_pos(E);
-                        adr_hi = line_at(E, 32);
+                        E.w.y = (E.w.y & 0xffff0000u) | (at + (uint32_t)n2);
+                        stride = -1;
+                        adr = Line(E, stride).at(lane);
                     }
                 }
-                const int v = can[adr], v_hi = can[adr_hi];
+                const int v = can[adr];
                 TbEntry Enn;
                 Enn.w = recs[j2 & kListRec];
                 const uint32_t j3 = list[min(e + 3, last)];
-                const int adr_n = first_pos(En), adr_hi_n = line_at(En, 32);
+                const int adr_n = Line(En, row).at(lane);
                 const uint2 lut_n = lut_of(En);
-                const int log2n = E.log2n(), mode = E.mode();
                 const bool coded = (E.w.z & kTbCoded) != 0u, filt = (E.w.z & kTbFilt) != 0u;
-                if (kFeat && (E.w.z & kTbPcm)) {
-                    pcm_tb(k, log2n, E.x(), E.y(), lane);
-                } else if (log2n == 2) {
+                if (kFeat && (j0 & kListPcm)) {
+                    pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
+                } else if (n2 == 8) {
                     walk_tb4(can, row, E.org(), mode, coded, luma, k.max_v, v, lut.x, lane);
-                } else if (log2n == 3) {
-                    walk_tb8(can, row, E.org(), mode, coded, filt, luma, k.max_v, v, v_hi, lut, lane);
+                } else if (n2 == 16) {
+                    const bool hi_ok = E.hi() == 32;
+                    const int v_hi = can[hi_ok ? E.corner() + 16 : 0];
+                    walk_tb8(can, row, E.org(), mode, coded, filt, luma, k.max_v, v, v_hi, hi_ok, lut, lane);
                 } else {
-                    walk_tb_big(can, row, Line(E, row), E.org(), log2n, mode, coded, filt, luma, k.strong, k.bd, ws.f,
-                                lane);
+                    walk_tb_big(can, row, Line(E, stride), E.org(), 31 - __clz(n2) - 1, mode, coded, filt, luma, k.strong,
+                                k.bd, ws.f, lane);
                 }
+                if (j0 & kListPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
                 E = En;
                 En = Enn;
                 j0 = j1, j1 = j2, j2 = j3;
-                adr = adr_n, adr_hi = adr_hi_n, lut = lut_n;
+                adr = adr_n, lut = lut_n;
             }
-            publish_level(geo(c), P.bps, prog, 4, level + c, lane);
         }
+        if (warp < kWalkers && lane == 0) *(volatile uint32_t*)&s_done[warp] = 1u;
         __syncthreads();
         // ---- write the CTU out for the filters (8 samples per store when
         // rows allow); the kernel boundary orders it before them ----
@@ -2534,21 +2515,14 @@ extern "C" cudaError_t hpvcd_launch_recon(const hpvcd::DevPic* pics, const hpvcd
     // the dynamic shared-memory limit was raised by hpvcd_recon_occupancy()
     // when the plan was built (no non-stream API call here, so launches can
     // be captured into CUDA graphs)
-    // build: 1 one chroma warp (Cb, then Cr), 2 one warp per chroma
-    // component, 3 the same in the register-capped build
+    // build: 1 one chroma warp (Cb, then Cr), 2 (and 3) one warp per chroma
+    // component
     const int cw = chroma_warps == 1 ? 1 : 2;
     const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw)).total;
     const int threads = 32 * hpvcd::recon_warps(cw);
-    // default: 2^22 polls of >= 64 ns each bound one neighbour wait to a few
-    // hundred ms
+    // default: 2^22 polls of up to 64 ns each bound one wait to a few hundred ms
     if (spin == 0) spin = 1u << 22;
-    if (chroma_warps == 3 && feat)
-        hpvcd::k_recon<2, true, true><<<grid, threads, smem, stream>>>(pics, items, n_items, work_counter, dev_err,
-                                                                       cfmt, spin, fine);
-    else if (chroma_warps == 3)
-        hpvcd::k_recon<2, false, true><<<grid, threads, smem, stream>>>(pics, items, n_items, work_counter, dev_err,
-                                                                        cfmt, spin, fine);
-    else if (cw == 2 && feat)
+    if (cw == 2 && feat)
         hpvcd::k_recon<2, true><<<grid, threads, smem, stream>>>(pics, items, n_items, work_counter, dev_err, cfmt,
                                                                  spin, fine);
     else if (cw == 2)
@@ -2572,10 +2546,10 @@ namespace {
 // other on the SMs: an SM changes its L1 / shared split only when it holds
 // no CTA, so a wave that wanted a larger split than the one running could
 // start only once the other groups' waves had drained every SM.
-template <int kCW, bool kFeat, bool kDense>
+template <int kCW, bool kFeat>
 void recon_attrs(int lim) {
-    cudaFuncSetAttribute(hpvcd::k_recon<kCW, kFeat, kDense>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(hpvcd::k_recon<kCW, kFeat, kDense>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cudaFuncSetAttribute(hpvcd::k_recon<kCW, kFeat>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(hpvcd::k_recon<kCW, kFeat>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);
 }
 
@@ -2584,10 +2558,7 @@ int recon_occupancy_of(int cfmt, int chroma_warps) {
     int blocks = 0;
     const int cw = chroma_warps == 1 ? 1 : 2;
     const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw)).total;
-    if (chroma_warps == 3)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, hpvcd::k_recon<2, false, true>,
-                                                      32 * hpvcd::recon_warps(2), smem);
-    else if (cw == 2)
+    if (cw == 2)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, hpvcd::k_recon<2, false>, 32 * hpvcd::recon_warps(2),
                                                       smem);
     else
@@ -2623,12 +2594,10 @@ extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
     std::lock_guard<std::mutex> lock(g_attr_mu);
     if (dev >= 0 && g_attr_done[dev]) return g_attr_occ[dev][cf][build - 1];
     const int lim = (int)hpvcd::ReconLayout(hpvcd::kFmt444, hpvcd::recon_warps(2)).total;
-    recon_attrs<1, false, false>(lim);
-    recon_attrs<2, false, false>(lim);
-    recon_attrs<1, true, false>(lim);
-    recon_attrs<2, true, false>(lim);
-    recon_attrs<2, false, true>(lim);
-    recon_attrs<2, true, true>(lim);
+    recon_attrs<1, false>(lim);
+    recon_attrs<2, false>(lim);
+    recon_attrs<1, true>(lim);
+    recon_attrs<2, true>(lim);
     // the residual pre-pass of one group runs beside another group's waves
     cudaFuncSetAttribute(hpvcd::k_residual<hpvcd::kIdctMatrix>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);

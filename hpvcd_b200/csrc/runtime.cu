@@ -193,7 +193,7 @@ struct hpvcd_plan {
     std::vector<uint32_t> rec_prefix;  // TB records of pictures [0, i)
     uint32_t* d_prefix = nullptr;
     unsigned char* d_res = nullptr;    // int16 residual planes
-    uint32_t* d_scratch = nullptr;  // [seg counters][err][progress words...]
+    uint32_t* d_scratch = nullptr;  // [wave counters][err][edge words...]
     size_t scratch_words = 0;
     unsigned char* d_planes = nullptr;
     size_t plane_bytes = 0;
@@ -226,14 +226,11 @@ struct hpvcd_plan {
     // 3 three warps register-capped; index build - 1)
     int occ[3][3] = {{1, 1, 1}, {1, 1, 1}, {1, 1, 1}};
     // Build of a wave's wavefront kernel (hpvcd_sched.chroma_warps): 0 picks
-    // three warps, register-capped when the wave has more CTUs ready at once
-    // than the plain build's CTAs can hold (its share of them when segments
-    // run concurrently).
-    int build_of(const Wave& wv, int n_seg) const {
+    // one warp for both chroma components at 4:2:0 and 4:0:0, where their
+    // walks together are shorter than the luma walk, else one warp each.
+    int build_of(const Wave& wv) const {
         const uint32_t cw = sched.chroma_warps;
-        if (cw >= 1 && cw <= 3) return (int)cw;
-        const int slots = concurrent ? sms * occ[wv.cfmt][1] / std::max(1, n_seg) : sms * occ[wv.cfmt][1];
-        return wv.ready > (uint32_t)slots ? 3 : 2;
+        return cw >= 1 && cw <= 3 ? (int)cw : (wv.cfmt == 0 ? 1 : 2);
     }
     int occ_of(int cfmt, int build) const { return occ[cfmt][build - 1]; }
     int sms = 148;
@@ -339,6 +336,11 @@ hpvcd_status cuda_status(cudaError_t e) {
 extern "C" hpvcd_status hpvcd_internal_status(cudaError_t e) { return cuda_status(e); }
 
 namespace {
+
+// 64-bit wavefront edge words of a picture.
+size_t edge_words_of_picture(const hpvcd_picture& p, const Geo& g) {
+    return (size_t)hpvcd::edge_words_per_ctu(1 << p.log2_ctb, p.chroma_idc, g.sub_w, g.sub_h) * g.ctb_cols * g.ctb_rows;
+}
 
 // int16 residual planes of a picture, rows padded to 16 samples.
 inline int res_stride_of(int w) { return (w + 15) & ~15; }
@@ -529,8 +531,8 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
     // ---- planes + scratch layout ----
     size_t plane_bytes = 0;
     std::vector<size_t> rec_off(n), fin_off(n);
-    size_t ready_words = 0;
-    std::vector<size_t> ready_off(n);
+    size_t edge_words = 0;
+    std::vector<size_t> edge_off(n);
     for (uint32_t i = 0; i < n; ++i) {
         const Geo g = geo_of(pics[i]);
         const size_t one = align_up(g.luma_bytes, 256) + 2 * align_up(g.chroma_bytes, 256);
@@ -545,8 +547,9 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
         } else {
             fin_off[i] = rec_off[i];
         }
-        ready_off[i] = ready_words;
-        ready_words += (size_t)4 * g.ctb_cols * g.ctb_rows;  // one progress word per component
+        edge_off[i] = edge_words;
+        if (!(pics[i].flags & HPVCD_PIC_PRED_IN_PLANE))  // pictures with a wavefront
+            edge_words += (size_t)edge_words_of_picture(pics[i], g);
     }
     // segments: all pictures at once, or one per picture when any picture
     // predicts from another (its references must be final first).
@@ -611,7 +614,8 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
         s.n_waves = (uint32_t)P->waves.size() - s.wave_first;
     }
     const size_t n_waves = P->waves.size();
-    P->scratch_words = n_waves + 1 + ready_words;
+    const size_t edge_base = align_up(n_waves + 1, 64);  // 64-bit words, 256-byte aligned
+    P->scratch_words = edge_base + 2 * edge_words;
     size_t res_bytes = 0;
     std::vector<size_t> res_off(n);
     for (uint32_t i = 0; i < n; ++i) {
@@ -675,7 +679,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
         d.fin[1] = fb + align_up(g.luma_bytes, 256);
         d.fin[2] = fb + align_up(g.luma_bytes, 256) + align_up(g.chroma_bytes, 256);
         if (!p.chroma_idc) d.rec[1] = d.rec[2] = d.fin[1] = d.fin[2] = nullptr;
-        d.ready = P->d_scratch + n_waves + 1 + ready_off[i];
+        d.edges = (unsigned long long*)(P->d_scratch + edge_base) + edge_off[i];
         {
             unsigned char* rb = P->d_res + res_off[i];
             d.res_stride[0] = res_stride_of(g.w);
@@ -819,7 +823,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
 
 hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
-    // Work counters, the device error word and the wavefront progress words are
+    // Work counters, the device error word and the wavefront edge words are
     // reset by every launch that reconstructs.
     if (stages & HPVCD_STAGE_RECON) {
         e = cudaMemsetAsync(P->d_scratch, 0, P->scratch_words * sizeof(uint32_t), st);
@@ -870,7 +874,7 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
             // its own layout and work counter
             for (uint32_t w = s.wave_first; w < s.wave_first + s.n_waves; ++w) {
                 const hpvcd_plan::Wave& wv = P->waves[w];
-                const int build = P->build_of(wv, (int)n_seg);
+                const int build = P->build_of(wv);
                 int occ = P->occ_of(wv.cfmt, build);
                 if (P->sched.recon_ctas_per_sm > 0) occ = std::min<int>(occ, (int)P->sched.recon_ctas_per_sm);
                 // concurrent segments share the SMs: each gets its share of the CTAs
@@ -1904,9 +1908,9 @@ HPVCD_API hpvcd_status hpvcd_gpu_read(hpvcd_gpu* g, hpvcd_ticket t, void* dst, u
 // a frame loop with a latency budget where cudaMalloc/cudaFree would
 // synchronise the device and stall unrelated streams.  For them the scratch of
 // one picture's decode lives in one fixed array of module global memory,
-// reserved when the module loads: work counter, device error word, wavefront
-// wavefront progress words, the device picture record, the CTU work list, the int16
-// residual planes and, when SAO runs, the pre-SAO planes.  The caller owns the
+// reserved when the module loads: work counter, device error word, the device
+// picture record, the CTU work list, the int16 residual planes and, when SAO
+// runs, the pre-SAO planes (the wavefront's edge words have a second one).  The caller owns the
 // inputs (device buffers) and the output planes.
 //
 // The array is reset per call by the first kernel the call enqueues, so calls
@@ -1921,12 +1925,22 @@ static constexpr size_t kNoAllocScratchBytes = HPVCD_NOALLOC_SCRATCH_BYTES;
 static_assert(kNoAllocScratchBytes % 256 == 0, "scratch size");
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
+// Wavefront edge words of the same picture, in an array of their own so that
+// the pictures that fit the scratch stay the same.  A picture that fits has
+// at least 2.09 (4:0:0), 3.09 (4:2:0), 4.09 (4:2:2) or 6.09 (4:4:4) bytes of
+// scratch and, with 16x16 CTBs, 0.25 / 0.5 / 0.625 / 0.75 bytes of edge words
+// per luma sample of its CTBs: at most 2.1 MB of them, 3 % more where the
+// last CTB row is cropped.
+static constexpr size_t kNoAllocEdgeBytes = 2560 * 1024;
+static __device__ __align__(256) unsigned char g_noalloc_edges[kNoAllocEdgeBytes];
+
 namespace {
 
 constexpr int kNoAllocMaxDevices = 64;
 
 struct NoAllocDevice {
     unsigned char* base = nullptr;  // address of g_noalloc_scratch on this device
+    unsigned char* edges = nullptr;  // and of g_noalloc_edges
     int sms = 0;
     int occ[3] = {0, 0, 0};         // k_recon CTAs per SM (4:2:0, 4:4:4, 4:2:2 layouts)
     bool ready = false;
@@ -1935,16 +1949,16 @@ std::mutex g_noalloc_mu;
 NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
 
 // Byte offsets inside the scratch array.  Word 0 is the work counter, word 1
-// the device error word; the progress words follow at byte 256.
+// the device error word; 16 bytes per CTU after byte 256 are kept free (they
+// count in which pictures fit).
 struct NoAllocLayout {
-    uint64_t ready, pic, prefix, items, res, snap, need;
+    uint64_t pic, prefix, items, res, snap, need;
 };
 
 NoAllocLayout noalloc_layout(const hpvcd_picture& p, const Geo& g) {
     NoAllocLayout L;
     const uint64_t n_ctu = (uint64_t)g.ctb_cols * g.ctb_rows;
-    L.ready = 256;
-    L.pic = align_up(L.ready + n_ctu * 16, 256);  // four progress words per CTU
+    L.pic = align_up(256 + n_ctu * 16, 256);
     L.prefix = align_up(L.pic + sizeof(DevPic), 256);
     L.items = L.prefix + 256;
     L.res = align_up(L.items + n_ctu * sizeof(CtuItem), 256);
@@ -1963,6 +1977,10 @@ hpvcd_status noalloc_setup(int dev, NoAllocDevice** out) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_status(e);
+        void* q = nullptr;
+        e = cudaGetSymbolAddress(&q, g_noalloc_edges);
+        if (e != cudaSuccess) return cuda_status(e);
+        d.edges = (unsigned char*)q;
         e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return cuda_status(e);
         for (int f = 0; f < 3; ++f) d.occ[f] = std::max(1, hpvcd_recon_occupancy(f, 1));
@@ -1975,15 +1993,15 @@ hpvcd_status noalloc_setup(int dev, NoAllocDevice** out) {
     return HPVCD_OK;
 }
 
-// Zero the counter, error word and progress words; store the picture record and
+// Zero the counter, error word and edge words; store the picture record and
 // the TB-record prefix; write the CTU work list in wavefront order (sorted by
 // t = x + 2y, then y), the order in which every CTU's left, above-left, above
 // and above-right neighbours come earlier.
-__global__ void k_noalloc_setup(DevPic pic, uint32_t n_tus, unsigned char* base, NoAllocLayout L, int list) {
+__global__ void k_noalloc_setup(DevPic pic, uint32_t n_tus, unsigned char* base, NoAllocLayout L, int list,
+                                uint32_t edge_words) {
     const int cols = pic.ctb_cols, rows = pic.ctb_rows;
     const int n_ctu = cols * rows;
     uint32_t* words = (uint32_t*)base;
-    uint32_t* ready = (uint32_t*)(base + L.ready);
     CtuItem* items = (CtuItem*)(base + L.items);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid < 2) words[tid] = 0u;
@@ -1993,9 +2011,8 @@ __global__ void k_noalloc_setup(DevPic pic, uint32_t n_tus, unsigned char* base,
         prefix[0] = 0u;
         prefix[1] = n_tus;
     }
-    for (int i = tid; i < n_ctu; i += gridDim.x * blockDim.x) {
-        for (int c = 0; c < 4; ++c) ready[(size_t)i * 4 + c] = 0u;
-        if (!list) continue;
+    for (uint32_t i = tid; i < edge_words; i += gridDim.x * blockDim.x) pic.edges[i] = 0ull;
+    for (int i = tid; i < n_ctu && list; i += gridDim.x * blockDim.x) {
         const int x = i % cols, y = i / cols, t = x + 2 * y;
         uint32_t rank = 0;
         for (int yy = 0; yy < rows && 2 * yy <= t; ++yy) {
@@ -2091,16 +2108,20 @@ HPVCD_API hpvcd_status hpvcd_decode_noalloc(const hpvcd_picture* dev_pic, void* 
         d.res[1] = p.chroma_idc ? (int16_t*)(rb + ly) : nullptr;
         d.res[2] = p.chroma_idc ? (int16_t*)(rb + ly + lc) : nullptr;
     }
-    d.ready = (uint32_t*)(base + L.ready);
+    d.edges = (unsigned long long*)nd->edges;
     d.needs_wavefront = (p.flags & HPVCD_PIC_PRED_IN_PLANE) ? 0 : 1;
+    const size_t edge_words = d.needs_wavefront ? edge_words_of_picture(p, g) : 0;
+    if (edge_words * 8 > kNoAllocEdgeBytes) return HPVCD_ERR_LIMIT;  // no picture that fits the scratch has more
 
     cudaStream_t st = (cudaStream_t)stream;
     const uint32_t n_ctu = (uint32_t)g.ctb_cols * g.ctb_rows;
     const DevPic* dp = (const DevPic*)(base + L.pic);
     uint32_t* work_counter = (uint32_t*)base;
     uint32_t* d_err = work_counter + 1;
-    const int setup_blocks = (int)std::min<uint32_t>((n_ctu + 255) / 256, (uint32_t)nd->sms);
-    k_noalloc_setup<<<std::max(1, setup_blocks), 256, 0, st>>>(d, p.n_tus, base, L, d.needs_wavefront);
+    const uint32_t setup_items = std::max<uint32_t>(n_ctu, (uint32_t)edge_words);
+    const int setup_blocks = (int)std::min<uint32_t>((setup_items + 255) / 256, (uint32_t)nd->sms);
+    k_noalloc_setup<<<std::max(1, setup_blocks), 256, 0, st>>>(d, p.n_tus, base, L, d.needs_wavefront,
+                                                              (uint32_t)edge_words);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_status(e);
     hpvcd_note_launches(1);
