@@ -50,8 +50,8 @@ struct DevPic {
 };
 
 // Edge words of one CTU: its right column and bottom row per component, four
-// samples per 64-bit word (16 bits each, the top bit of the word set once it
-// is written), which neighbouring CTUs poll and read.
+// samples per 64-bit word (16 bits each, the top bit of each set once it is
+// written), which neighbouring CTUs poll and read.
 __host__ __device__ inline int edge_words_of(int ctb, int sub_w, int sub_h, int c) {
     return c ? ctb / sub_w / 4 + ctb / sub_h / 4 : ctb / 2;
 }
@@ -82,9 +82,9 @@ __device__ __forceinline__ void store_sample(void* plane, int bps, size_t idx, i
     else
         ((uint16_t*)plane)[idx] = (uint16_t)v;
 }
-// Edge words: single-copy atomic 64-bit accesses at device scope.  A word
-// carries its samples and their validity together, so neither side needs a
-// fence or a second access.
+// Edge words: relaxed accesses at device scope.  Every sample carries its own
+// validity, so neither side needs a fence or a second access, and a word read
+// while only some of its samples are written is simply not complete yet.
 __device__ __forceinline__ unsigned long long ld_edge(const unsigned long long* p) {
     unsigned long long v;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -92,6 +92,10 @@ __device__ __forceinline__ unsigned long long ld_edge(const unsigned long long* 
 }
 __device__ __forceinline__ void st_edge(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// One sample of a word (its own 16 bits).
+__device__ __forceinline__ void st_edge16(uint16_t* p, uint16_t v) {
+    asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"(v) : "memory");
 }
 
 // qp helpers: decode.rs:5753-5771, :5868-5871, :7599-7613

@@ -9,9 +9,9 @@
 //     lanes or a warp per TB by its size).  TBs whose prediction is already in the plane (inter TBs,
 //     prediction-in-plane pictures) are added and clipped into the plane
 //     right away; intra TBs leave an int16 residual in a residual plane.
-//     (int16 is exact: for 8-bit the reference itself truncates to i16,
-//     transform.rs:55-63; above 8 bits a residual outside +-32767 saturates
-//     the clip to [0, 2^bd - 1] exactly as the unsaturated one does.)
+//     (for 8-bit the reference itself truncates to i16, transform.rs:55-63;
+//     then every residual is clamped to +-(2^bd - 1), which the clip of the
+//     sum to [0, 2^bd - 1] cannot tell from the full value.)
 //
 //  k_recon -- the intra wavefront.  One CTA reconstructs one CTU at a time;
 //     CTUs are claimed from a global queue sorted by wavefront index
@@ -52,6 +52,11 @@ constexpr int kIdctButterfly = 1;  // even-odd butterflies for 16x16 and 32x32 T
 constexpr int kIdctTensor = 2;     // integer tensor-core products (int8 halves) for 16x16 and 32x32 TBs
 
 __device__ __forceinline__ int sat16(int v) { return v < -32768 ? -32768 : (v > 32767 ? 32767 : v); }
+
+// A residual as the residual planes hold it, mx the largest sample: clip(pred
+// + r, 0, mx) is the same for r clamped to [-mx, mx], and the sum of a sample
+// and a clamped residual fits 16 bits.
+__device__ __forceinline__ int16_t res_store(int v, int mx) { return (int16_t)clamp3i(v, -mx, mx); }
 
 // Entry (k, m) of the n-point H.265 DCT basis as a compile-time constant (the
 // multipliers of the unrolled butterflies, the tables below); mag: the basis
@@ -787,7 +792,7 @@ __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
             int16_t* row = rp + (size_t)y * rs + x0;
             int16_t v4[4];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) v4[m] = (int16_t)sat16(d[4 * r + m]);
+            for (int m = 0; m < 4; ++m) v4[m] = res_store(d[4 * r + m], (1 << bd) - 1);
             if (x0 + 4 <= pw && ((uintptr_t)row & 7) == 0) {
                 *(uint2*)row = make_uint2((uint32_t)(uint16_t)v4[0] | ((uint32_t)(uint16_t)v4[1] << 16),
                                           (uint32_t)(uint16_t)v4[2] | ((uint32_t)(uint16_t)v4[3] << 16));
@@ -893,12 +898,13 @@ __device__ __forceinline__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int
             uint32_t w[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h)
-                w[h] = (uint32_t)(uint16_t)sat16(o[2 * h]) | ((uint32_t)(uint16_t)sat16(o[2 * h + 1]) << 16);
+                w[h] = (uint32_t)(uint16_t)res_store(o[2 * h], (1 << bd) - 1) |
+                       ((uint32_t)(uint16_t)res_store(o[2 * h + 1], (1 << bd) - 1) << 16);
             *(uint4*)row = make_uint4(w[0], w[1], w[2], w[3]);
         } else {
 #pragma unroll
             for (int m = 0; m < 8; ++m)
-                if (x0 + m < pw) row[m] = (int16_t)sat16(o[m]);
+                if (x0 + m < pw) row[m] = res_store(o[m], (1 << bd) - 1);
         }
     }
 }
@@ -1025,7 +1031,8 @@ __device__ __forceinline__ void tb_tensor(const DevPic& P, const hpvcd_tu& t, in
                     int v0 = out[nt][2 * rr], v1 = out[nt][2 * rr + 1];
                     if (i16s) v0 = (int)(int16_t)v0, v1 = (int)(int16_t)v1;
                     if (x0 + x < pw)
-                        *(uint32_t*)(row + x) = (uint32_t)(uint16_t)sat16(v0) | ((uint32_t)(uint16_t)sat16(v1) << 16);
+                        *(uint32_t*)(row + x) =
+                            (uint32_t)(uint16_t)res_store(v0, mx) | ((uint32_t)(uint16_t)res_store(v1, mx) << 16);
                 }
             }
         }
@@ -1062,10 +1069,10 @@ __device__ __noinline__ void tb_general(const DevPic& P, const hpvcd_tu& t, cons
         });
     } else {
         int16_t* rp = P.res[c];
-        const int rs = P.res_stride[c];
+        const int rs = P.res_stride[c], mx = (1 << (c ? P.bd_c : P.bd)) - 1;
         tb_residual_warp<kIdct>(P, t, dct, scr, scr + 32 * kScr, lane, [&](int r, int m, int v) {
             const int x = x0 + m, y = y0 + r;
-            if (x < pw && y < ph) rp[(size_t)y * rs + x] = (int16_t)sat16(v);
+            if (x < pw && y < ph) rp[(size_t)y * rs + x] = res_store(v, mx);
         });
     }
     __syncwarp();
@@ -1246,7 +1253,7 @@ k_ccp(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, 
                 const long long s = (long long)load_sample(P.rec[c], P.bps, idx) + vv;
                 store_sample(P.rec[c], P.bps, idx, (int)(s < 0 ? 0 : (s > mx ? mx : s)));
             } else {
-                P.res[c][(size_t)y * P.res_stride[c] + x] = (int16_t)sat16(vv);
+                P.res[c][(size_t)y * P.res_stride[c] + x] = res_store(vv, mx);
             }
         };
         if (t.flags & HPVCD_TU_CBF)
@@ -1266,7 +1273,12 @@ constexpr unsigned kFull = 0xffffffffu;
 // Per-warp scratch of the decode-order walk.
 struct WalkScratch {
     uint16_t s[132];  // the substituted line of a gathered TB, position i at s[i]
-    uint16_t f[132];  // its available samples before substitution; the references of a 16x16 / 32x32 TB
+    // its available samples before substitution; the references of a 16x16 /
+    // 32x32 TB, each with the next one (angular) or on its own (planar)
+    union {
+        uint16_t f[132];
+        uint32_t pairs[66];
+    };
 };
 constexpr size_t kWsBytes = (sizeof(WalkScratch) + 15) & ~(size_t)15;
 
@@ -1275,9 +1287,9 @@ constexpr size_t kWsBytes = (sizeof(WalkScratch) + 15) & ~(size_t)15;
 // entries (index 7 = the column left of the CTU, x at x + 8).  Both row
 // lengths are multiples of 8 entries, so every interior row starts 16-byte
 // aligned.
-__host__ __device__ __forceinline__ int can_top(int S) { return 2 * S + 8; }
-__host__ __device__ __forceinline__ int can_row(int S) { return S + 8; }
-__host__ __device__ __forceinline__ int can_size(int S, int Sh) { return can_top(S) + Sh * can_row(S); }
+__host__ __device__ constexpr int can_top(int S) { return 2 * S + 8; }
+__host__ __device__ constexpr int can_row(int S) { return S + 8; }
+__host__ __device__ constexpr int can_size(int S, int Sh) { return can_top(S) + Sh * can_row(S); }
 __device__ __forceinline__ int can_at(int S, int x, int y) {
     return y < 0 ? x + 8 : can_top(S) + y * can_row(S) + x + 8;
 }
@@ -1285,8 +1297,8 @@ __device__ __forceinline__ int can_at(int S, int x, int y) {
 // test for the row above.
 __device__ __forceinline__ int can_in(int S, int x, int y) { return can_top(S) + y * can_row(S) + x + 8; }
 
-// Shared-memory layout of one CTA: the canvases, one walk scratch per warp,
-// the CTU's staged records, the 16x16 stamp map, the three TB lists.
+// Shared-memory layout of one CTA: the canvases, one walk scratch per
+// walking warp, the walk entries, the 16x16 stamp map.
 // Records of one CTU staged at once: up to 256 luma TBs, one "mark decoded"
 // record per inter CU (64 at most) and the chroma TBs (64 per component at
 // 4:2:0, 128 at 4:2:2, 256 at 4:4:4).  A CTU with more records is malformed.
@@ -1302,9 +1314,9 @@ constexpr uint32_t kNoStamp = 0xffffffffu;
 struct ReconLayout {
     int cs_w, cs_h;  // chroma canvas width and height (CTU interior)
     int rec_cap;     // staged records
-    int list_c;      // list entries per chroma component
-    size_t off_can_y, off_can_c, off_ws, off_recs, off_stamp, off_lists, off_misc, total;
-    __host__ __device__ ReconLayout(int cfmt, int warps) {
+    int list_c;      // intra TBs per chroma component
+    size_t off_can_y, off_can_c, off_ws, off_ents, off_stamp, off_misc, total;
+    __host__ __device__ ReconLayout(int cfmt, int walkers) {
         cs_w = cfmt == kFmt444 ? 64 : 32;
         cs_h = cfmt == kFmt420 ? 32 : 64;
         rec_cap = cfmt == kFmt444 ? kRecCap444 : (cfmt == kFmt422 ? kRecCap422 : kRecCap420);
@@ -1314,17 +1326,21 @@ struct ReconLayout {
         o = (o + 15) & ~(size_t)15;
         off_can_c = o; o += 2 * (size_t)can_size(cs_w, cs_h) * sizeof(uint16_t);
         o = (o + 15) & ~(size_t)15;
-        off_ws = o;    o += (size_t)warps * kWsBytes;
-        off_recs = o;  o += (size_t)rec_cap * sizeof(hpvcd_tu);
+        off_ws = o;    o += (size_t)walkers * kWsBytes;
+        off_ents = o;  o += (size_t)(kListCap + 2 * list_c) * sizeof(uint4);
         off_stamp = o; o += 256 * sizeof(uint32_t);
-        off_lists = o; o += (size_t)(kListCap + 2 * list_c) * sizeof(uint16_t);
-        o = (o + 15) & ~(size_t)15;
-        off_misc = o;  o += 128;  // claimed item, list counts, have bits, covered words, done flags
+        off_misc = o;  o += 128;  // claimed item, TB counts, have bits, covered words, done flags
         total = o;
     }
-    __host__ __device__ int list_off(int c) const { return c == 0 ? 0 : kListCap + (c - 1) * list_c; }
-    __host__ __device__ int list_cap(int c) const { return c == 0 ? kListCap : list_c; }
+    __host__ __device__ int ent_off(int c) const { return c == 0 ? 0 : kListCap + (c - 1) * list_c; }
+    __host__ __device__ int ent_cap(int c) const { return c == 0 ? kListCap : list_c; }
 };
+// The CTU's records are staged in the canvases: they are done with (turned
+// into walk entries) before any sample or residual is put there.
+static_assert(kRecCap420 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(32, 32)) * sizeof(uint16_t) &&
+                  kRecCap422 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(32, 64)) * sizeof(uint16_t) &&
+                  kRecCap444 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(64, 64)) * sizeof(uint16_t),
+              "records fit the canvases");
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1482,12 +1498,13 @@ __device__ __forceinline__ unsigned long long* edge_words(const DevPic& P, int c
     unsigned long long* w = P.edges + ((size_t)cy * P.ctb_cols + cx) * per;
     return c ? w + edge_words_of(ctb, P.sub_w, P.sub_h, 0) + (c - 1) * edge_words_of(ctb, P.sub_w, P.sub_h, 1) : w;
 }
+constexpr unsigned long long kEdgeTags = 0x8000800080008000ull;
 __device__ __forceinline__ unsigned long long edge_pack(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    return (unsigned long long)(a | (b << 16)) | ((unsigned long long)(c | (d << 16) | 0x80000000u) << 32);
+    return (unsigned long long)(a | (b << 16)) | ((unsigned long long)(c | (d << 16)) << 32) | kEdgeTags;
 }
 
-// Publishes the edge words a finished n x n TB at (x0, y0) covers: lanes
-// 0..15 the right column, lanes 16..31 the bottom row.
+// Publishes the edge words a finished n x n TB at (x0, y0) covers, from the
+// canvas: lanes 0..15 the right column, lanes 16..31 the bottom row.
 __device__ __forceinline__ void publish_tb(const uint16_t* can, int row, int S, int Sh, int x0, int y0, int n,
                                            unsigned long long* words, int lane) {
     const bool bottom = lane >= 16;
@@ -1575,13 +1592,13 @@ __device__ void edge_service(const DevPic& P, int cx, int cy, int ncomp, CanOf c
             if (c >= ncomp) continue;
             const int S = c ? (1 << P.log2_ctb) / P.sub_w : 1 << P.log2_ctb;
             uint16_t* can = can_of(c);
-            const bool gt = (long long)t[c] < 0, gl = (long long)l[c] < 0;
+            const bool gt = (t[c] & kEdgeTags) == kEdgeTags, gl = (l[c] & kEdgeTags) == kEdgeTags;
             if (gt) {  // can_at(S, 4 * lane, -1): 8-byte aligned
-                t[c] &= ~(1ull << 63);
+                t[c] &= ~kEdgeTags;
                 *(uint2*)(can + 8 + 4 * lane) = make_uint2((uint32_t)t[c], (uint32_t)(t[c] >> 32));
             }
             if (gl) {
-                l[c] &= ~(1ull << 63);
+                l[c] &= ~kEdgeTags;
                 if (lane == 16) {
                     can[7] = (uint16_t)(l[c] >> 48);  // can_at(S, -1, -1)
                 } else {
@@ -1662,11 +1679,16 @@ __device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need
 //   x: canvas offset of the TB | of line position 0 << 16
 //   y: canvas offset of the corner | row of the angular table << 16
 //   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbCoded | kTbFilt
-//   w: x | y << 8 (in the CTU) | record index << 16
+//   w: x | y << 8 (in the CTU) | record index (< 1024) << 16 | kTb* flags << 26
 // Measured when the entries came in (4032x3024 grid, 70 luma TBs a CTU): the
 // walk's chain went from ~87k to ~46k cycles a CTU (4x4 700 -> 500, 16x16 5100
 // -> 1650, 32x32 10700 -> 3300 cycles); 512x512 tile 1004 -> 649 us.
 constexpr uint32_t kTbCoded = 1u << 30, kTbFilt = 1u << 31;
+// the TB reads neighbour CTUs, its line must be gathered, it is an I_PCM
+// block, it covers edge words, line position 32 is available, it is a 4x4 or
+// 8x8 TB of an angular mode without line or edge filter and with one run of
+// available samples (each sample is a blend of two line samples)
+constexpr uint32_t kTbEdge = 1u, kTbGather = 2u, kTbPcm = 4u, kTbPub = 8u, kTbHi32 = 16u, kTbPlain = 32u;
 
 struct TbEntry {
     uint4 w;
@@ -1680,12 +1702,14 @@ struct TbEntry {
     __device__ __forceinline__ int mode() const { return (int)((w.z >> 24) & 0x3fu); }
     __device__ __forceinline__ int x() const { return (int)(w.w & 0xffu); }
     __device__ __forceinline__ int y() const { return (int)((w.w >> 8) & 0xffu); }
+    __device__ __forceinline__ uint32_t jrec() const { return (w.w >> 16) & 0x3ffu; }
+    __device__ __forceinline__ uint32_t flags() const { return w.w >> 26; }
 };
 
-// The walk entry of intra record j (t, at (x0, y0) of the CTU); *gather: its
-// line is not one run of available samples.
+// The walk entry of intra record j (t, at (x0, y0) of the CTU); `flags` gives
+// kTbPcm and kTbPub, the others are added here.
 __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, int x0, int y0, uint32_t jrec,
-                                            const uint32_t* stamp, bool coded, bool* gather) {
+                                            const uint32_t* stamp, bool coded, uint32_t flags) {
     const int n = 1 << t.log2n, n2 = 2 * n;
     // cells one sample apart in this component's units
     const int uw = 4 / k.sw, uh = 4 / k.sh;
@@ -1737,8 +1761,12 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
             lo = n2 + 1;
     }
     if (lo > hi) one_run = false;  // nothing available
-    if (!one_run) lo = 0, hi = 4 * n;
-    *gather = !one_run;
+    if (!one_run) lo = 0, hi = 4 * n, flags |= kTbGather;
+    if (x0 == 0 || y0 == 0) flags |= kTbEdge;
+    if (hi == 32) flags |= kTbHi32;
+    const bool filt = n > 4 && ref_filtered(k, n, t.mode);
+    if (n <= 8 && t.mode >= 2 && one_run && !filt && !(flags & kTbPcm) && !(k.luma && (t.mode == 10 || t.mode == 26)))
+        flags |= kTbPlain;
     const uint32_t am = t.mode >= 2 ? t.mode - 2u : 0u;
     const uint32_t lut = n == 4 ? am * 16u : (n == 8 ? 33u * 16u + am * 32u : 0u);
     uint4 w;
@@ -1746,8 +1774,8 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
     w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (lut << 16);
     w.z = (uint32_t)lo | ((uint32_t)hi << 8) | ((uint32_t)n2 << 16) | ((uint32_t)t.mode << 24);
     if (coded) w.z |= kTbCoded;
-    if (n > 4 && ref_filtered(k, n, t.mode)) w.z |= kTbFilt;
-    w.w = (uint32_t)x0 | ((uint32_t)y0 << 8) | (jrec << 16);
+    if (filt) w.z |= kTbFilt;
+    w.w = (uint32_t)x0 | ((uint32_t)y0 << 8) | (jrec << 16) | (flags << 26);
     return w;
 }
 
@@ -1811,14 +1839,18 @@ struct Line {
     }
 };
 
+// Residual add + clip (reconstruct.rs:214-251) of two samples in 16-bit halves.
+__device__ __forceinline__ uint32_t add_clip2(uint32_t pred, uint32_t res, int max_v) {
+    return __viaddmin_s16x2_relu(pred, res, (uint32_t)max_v * 0x10001u);
+}
+
 // 4x4 intra TB: v is line position `lane` (lanes 0..16), lut the lane's entry
 // of the angular table (prediction intra.rs:257-372, no filtering of 4x4
-// lines, intra.rs:174), lanes 0..15 one sample each.
-__device__ __forceinline__ void walk_tb4(uint16_t* can, int row, int org, int mode, bool coded, bool luma, int max_v,
-                                         int v, uint32_t lut, int lane) {
+// lines, intra.rs:174), lanes 0..15 one sample each, at px.
+__device__ __forceinline__ void walk_tb4(uint16_t* px, int mode, bool coded, bool luma, int max_v, int v, uint32_t lut,
+                                         int lane) {
     constexpr int n = 4, n2 = 8;
     const int yy = (lane >> 2) & 3, xx = lane & 3;
-    uint16_t* px = can + org + yy * row + xx;
     const int rv = coded ? (int)(int16_t)*px : 0;
     int pred;
     if (mode >= 2) {
@@ -1847,7 +1879,7 @@ __device__ __forceinline__ void walk_tb4(uint16_t* can, int row, int org, int mo
         const int tr = __shfl_sync(kFull, v, n2 + n + 1), bl = __shfl_sync(kFull, v, n2 - n - 1);
         pred = ((n - 1 - xx) * lft + (xx + 1) * tr + (n - 1 - yy) * abv + (yy + 1) * bl + n) >> 3;
     }
-    if (lane < 16) *px = (uint16_t)clamp3i(pred + rv, 0, max_v);
+    if (lane < 16) *px = (uint16_t)__viaddmin_s32_relu(pred, rv, max_v);
     __syncwarp();
 }
 
@@ -1855,14 +1887,13 @@ __device__ __forceinline__ void walk_tb4(uint16_t* can, int row, int org, int mo
 // available (the same in every lane; else position 31 stands in for it);
 // [1 2 1] filtering (intra.rs:151-219; no strong filter below
 // 32x32) and prediction (intra.rs:257-372) by shuffles, two horizontally
-// adjacent samples per lane.
-__device__ __forceinline__ void walk_tb8(uint16_t* can, int row, int org, int mode, bool coded, bool filt, bool luma,
-                                         int max_v, int v, int v_hi, bool hi_ok, uint2 lut, int lane) {
+// adjacent samples per lane, at px (canvas rows and TB columns are even).
+__device__ __forceinline__ void walk_tb8(uint32_t* px, int mode, bool coded, bool filt, bool luma, int max_v, int v,
+                                         int v_hi, bool hi_ok, uint2 lut, int lane) {
     constexpr int n = 8, n2 = 16;
     const int v31 = __shfl_sync(kFull, v, 31);
     v_hi = hi_ok ? v_hi : v31;
     const int yy = lane >> 2, xx = 2 * (lane & 3);
-    uint32_t* px = (uint32_t*)(can + org + yy * row + xx);  // canvas rows and TB columns are even
     const uint32_t rv = coded ? *px : 0u;
     if (filt) {
         const int up = __shfl_up_sync(kFull, v, 1);
@@ -1911,18 +1942,28 @@ __device__ __forceinline__ void walk_tb8(uint16_t* can, int row, int org, int mo
             out[h] = ((n - 1 - xx - h) * lft + (xx + h + 1) * tr + (n - 1 - yy) * abv + (yy + 1) * bl + n) >> 4;
         }
     }
-    const int s0 = clamp3i(out[0] + (int)(int16_t)rv, 0, max_v);
-    const int s1 = clamp3i(out[1] + ((int)rv >> 16), 0, max_v);
-    *px = (uint32_t)s0 | ((uint32_t)s1 << 16);
+    *px = add_clip2((uint32_t)out[0] | ((uint32_t)out[1] << 16), rv, max_v);
+    __syncwarp();
+}
+
+// Two horizontally adjacent samples of a plain 8x8 TB per lane (kTbPlain):
+// every lane reads its four line samples in place, no line, no shuffles.
+__device__ __forceinline__ void walk_plain8(uint16_t* can, const Line& L, uint32_t* px, bool coded, int max_v, uint2 lut) {
+    const int a0 = can[L.at((int)(lut.x & 0xffu))], a1 = can[L.at((int)((lut.x >> 8) & 0xffu))];
+    const int b0 = can[L.at((int)(lut.y & 0xffu))], b1 = can[L.at((int)((lut.y >> 8) & 0xffu))];
+    const uint32_t rv = coded ? *px : 0u;
+    const uint32_t p0 = ((lut.x >> 24) * a0 + ((lut.x >> 16) & 0xffu) * a1 + 16u) >> 5;
+    const uint32_t p1 = ((lut.y >> 24) * b0 + ((lut.y >> 16) & 0xffu) * b1 + 16u) >> 5;
+    *px = add_clip2(p0 | (p1 << 16), rv, max_v);
     __syncwarp();
 }
 
 // 16x16 or 32x32 intra TB by one warp, two horizontally adjacent samples per
 // lane and row step.  The reference samples a sample may read (the angular
-// projection, or the left column) are filtered on the way into `refs`; the
+// projection, or the left column) are filtered on the way into the scratch; the
 // row loops then read them at addresses that do not depend on loaded values.
 __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& L, int org, int log2n, int mode,
-                                            bool coded, bool filt, bool luma, bool strong_on, int bd, uint16_t* refs,
+                                            bool coded, bool filt, bool luma, bool strong_on, int bd, WalkScratch& ws,
                                             int lane) {
     const int n = 1 << log2n, n2 = 2 * n;
     const int max_v = (1 << bd) - 1;
@@ -1949,45 +1990,52 @@ __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& 
     const bool edge = luma && n < 32;
     uint32_t* px = (uint32_t*)(can + org + (lane >> hl) * row + x);  // canvas rows and TB columns are even
     const int step = (ys * row) >> 1;
-    auto put = [&](int p0, int p1) {  // residual add + clip (reconstruct.rs:214-251)
-        const uint32_t rv = coded ? *px : 0u;
-        const int s0 = clamp3i(p0 + (int)(int16_t)rv, 0, max_v), s1 = clamp3i(p1 + ((int)rv >> 16), 0, max_v);
-        *px = (uint32_t)s0 | ((uint32_t)s1 << 16);
+    auto put = [&](int p0, int p1) {
+        *px = add_clip2((uint32_t)p0 | ((uint32_t)p1 << 16), coded ? *px : 0u, max_v);
         px += step;
     };
     if (mode >= 2) {
         const int angle = c_intra_angle[mode - 2];
         const bool vertical = mode >= 18;
         const int inv = angle < 0 ? c_inv_angle[mode - 11] : 0;
-        // refs[k - k0] = projected reference k; k0 .. k0 + 2n - 1 is all a TB
-        // reads with a weight
+        // pairs[k - k0] = projected references k and k + 1; k0 .. k0 + 2n - 1
+        // is all a TB reads with a weight
         const int k0 = angle < 0 ? 1 - n : 1;
-        for (int q = lane; q < n2; q += 32) refs[q] = (uint16_t)R(ref_pos(k0 + q, vertical, n2, inv));
+        {
+            const int ra = R(ref_pos(k0 + lane, vertical, n2, inv));
+            int na = __shfl_down_sync(kFull, ra, 1);
+            if (n == 32) {
+                const int rb = R(ref_pos(k0 + 32 + lane, vertical, n2, inv));
+                const int b0 = __shfl_sync(kFull, rb, 0);
+                if (lane == 31) na = b0;
+                ws.pairs[lane + 32] = (uint32_t)rb | ((uint32_t)__shfl_down_sync(kFull, rb, 1) << 16);
+            }
+            ws.pairs[lane] = (uint32_t)ra | ((uint32_t)na << 16);
+        }
         __syncwarp();
+        // ((32 - f) r[k] + f r[k + 1] + 16) >> 5
+        auto blend = [](uint32_t pair, int f) { return __dp2a_lo((int)pair, 32 - f + (f << 8), 16) >> 5; };
         if (vertical) {
             const bool e26 = edge && mode == 26;
             const int a0 = e26 ? raw(n2 + 1) : 0, c0 = e26 ? raw(n2) : 0;
-            const uint16_t* base = refs + x + 1 - k0;
+            const uint32_t* base = ws.pairs + x + 1 - k0;
             int pos = ((lane >> hl) + 1) * angle;
 #pragma unroll 4
             for (int y = lane >> hl; y < n; y += ys, pos += ys * angle) {
-                const uint16_t* r = base + (pos >> 5);
-                const int f = pos & 31, r0 = r[0], r1 = r[1], r2 = r[2];
-                int p0 = (32 * r0 + f * (r1 - r0) + 16) >> 5;
-                const int p1 = (32 * r1 + f * (r2 - r1) + 16) >> 5;
+                const uint32_t* r = base + (pos >> 5);
+                int p0 = blend(r[0], pos & 31);
+                const int p1 = blend(r[1], pos & 31);
                 if (e26 && x == 0) p0 = clamp3i(a0 + ((raw(n2 - (y + 1)) - c0) >> 1), 0, max_v);
                 put(p0, p1);
             }
         } else {
             const bool e10 = edge && mode == 10;
             const int pa = (x + 1) * angle, pb = pa + angle;
-            const int fa = pa & 31, fb = pb & 31;
-            const uint16_t* ra = refs + (pa >> 5) + 1 - k0;
-            const uint16_t* rb = refs + (pb >> 5) + 1 - k0;
+            const uint32_t* ra = ws.pairs + (pa >> 5) + 1 - k0;
+            const uint32_t* rb = ws.pairs + (pb >> 5) + 1 - k0;
 #pragma unroll 4
             for (int y = lane >> hl; y < n; y += ys) {
-                const int a = ra[y], a1 = ra[y + 1], b = rb[y], b1 = rb[y + 1];
-                int p0 = (32 * a + fa * (a1 - a) + 16) >> 5, p1 = (32 * b + fb * (b1 - b) + 16) >> 5;
+                int p0 = blend(ra[y], pa & 31), p1 = blend(rb[y], pb & 31);
                 if (e10 && y == 0) {
                     const int a0 = raw(n2 - 1), c0 = raw(n2);
                     p0 = clamp3i(a0 + ((raw(n2 + x + 1) - c0) >> 1), 0, max_v);
@@ -2017,12 +2065,12 @@ __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& 
             put(p0, p1);
         }
     } else {  // planar
-        if (lane < n) refs[lane] = (uint16_t)R(n2 - 1 - lane);
+        if (lane < n) ws.f[lane] = (uint16_t)R(n2 - 1 - lane);
         const int ab0 = R(n2 + x + 1), ab1 = R(n2 + x + 2), rt = R(n2 + n + 1), lb = R(n2 - n - 1);
         __syncwarp();
 #pragma unroll 4
         for (int y = lane >> hl; y < n; y += ys) {
-            const int lf = refs[y], vb = (y + 1) * lb + n, up = n - 1 - y;
+            const int lf = ws.f[y], vb = (y + 1) * lb + n, up = n - 1 - y;
             const int p0 = ((n - 1 - x) * lf + (x + 1) * rt + up * ab0 + vb) >> (log2n + 1);
             const int p1 = ((n - 2 - x) * lf + (x + 2) * rt + up * ab1 + vb) >> (log2n + 1);
             put(p0, p1);
@@ -2077,24 +2125,19 @@ __device__ __noinline__ void gather_line(const Comp& k, int log2n, int x0, int y
 // 4:4:4 they would be the longer chain.
 __host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 
-// List entry flags beside the record index (< 1024): the TB reads neighbour
-// CTUs, its line must be gathered, it is an I_PCM block, it covers edge words.
-constexpr uint32_t kListRec = 0x3ffu;
-constexpr uint32_t kListEdge = 0x8000u, kListGather = 0x4000u, kListPcm = 0x2000u, kListPub = 0x1000u;
-
 // kFeat: some picture of the launch has slices / tiles, constrained intra
 // prediction, cross-component prediction or I_PCM blocks; without them the
 // availability, coded and PCM tests compile to the plain form.  fine: a TB
 // waits for the edge words it reads; otherwise a CTU waits for all of its
 // neighbours' words before its walk.
 template <int kCW, bool kFeat>
-__global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 7 : 5)
+__global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 5 : 4)
 k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint32_t n_items,
         uint32_t* work_counter, uint32_t* dev_err, int cfmt, uint32_t spin_limit, int fine) {
     static_assert(kCW == 1 || kCW == 2, "one or two chroma warps");
     constexpr int kWarps = recon_warps(kCW), kThreads = 32 * kWarps, kWalkers = kWarps - 1;
     extern __shared__ __align__(16) unsigned char smem[];
-    const ReconLayout lay(cfmt, kWarps);
+    const ReconLayout lay(cfmt, kWalkers);
     uint32_t* s_item = (uint32_t*)(smem + lay.off_misc);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // components walked (and listed) by this warp: [c_lo, c_hi], none for the edge warp
@@ -2125,9 +2168,9 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             if (tid == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
             nrec = (uint32_t)lay.rec_cap;
         }
-        uint4* recs = (uint4*)(smem + lay.off_recs);
+        uint4* recs = (uint4*)(smem + lay.off_can_y);  // until the walk entries are built
+        uint4* ents = (uint4*)(smem + lay.off_ents);
         uint32_t* stamp = (uint32_t*)(smem + lay.off_stamp);
-        uint16_t* lists = (uint16_t*)(smem + lay.off_lists);
         uint32_t* counts = (uint32_t*)(smem + lay.off_misc) + 1;  // TBs listed per component
         uint32_t* s_have = counts + 3;                            // have bits, two words per component
         uint32_t* s_cov = s_have + 6;                             // edge words covered by intra TBs
@@ -2154,8 +2197,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         __syncthreads();
         // ---- decode order, in parallel: every luma record stamps the 4x4
         // cells it marks decoded (decode.rs:3170-3189; cells outside the
-        // picture stay unmarked), and each warp lists the intra TBs of its
-        // components in decode order ----
+        // picture stay unmarked) ----
         const int vis_w = min(64, P.w - oxl), vis_h = min(64, P.h - oyl);
         const bool intra_pred_ok = !(P.flags & HPVCD_PIC_PRED_IN_PLANE);
         // validity of record i for component tc: -1 skip silently, 0 invalid
@@ -2181,17 +2223,60 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             for (int cy = y >> 2; cy < (y1 + 3) >> 2; ++cy)
                 for (int cx = x >> 2; cx < (x1 + 3) >> 2; ++cx) atomicMin(&stamp[cy * 16 + cx], i);
         }
+        // neighbour CTUs that intra prediction may read: same slice and tile
+        // (decode.rs:4651-4690)
+        uint32_t nb_ok = 0xfu;
+        if (kFeat && P.ctb_region) {
+            const uint16_t me = P.ctb_region[ci];
+            const int cx = it.cx, cy = it.cy;
+            auto same = [&](int nx, int ny) {
+                return nx >= 0 && ny >= 0 && nx < P.ctb_cols && P.ctb_region[(size_t)ny * P.ctb_cols + nx] == me;
+            };
+            nb_ok = (same(cx - 1, cy) ? 1u : 0u) | (same(cx - 1, cy - 1) ? 2u : 0u) | (same(cx, cy - 1) ? 4u : 0u) |
+                    (same(cx + 1, cy - 1) ? 8u : 0u);
+        }
+        // Everything one walking warp needs about component c of this CTU.
+        auto comp_of = [&](int c) -> Comp {
+            Comp k;
+            k.S = c ? Scw : ctb;
+            k.Sh = c ? Sch : ctb;
+            k.ox = c ? ocx : oxl;
+            k.oy = c ? ocy : oyl;
+            k.pw = c ? P.cw : P.w;
+            k.ph = c ? P.ch : P.h;
+            k.sw = c ? P.sub_w : 1;
+            k.sh = c ? P.sub_h : 1;
+            k.nb_ok = nb_ok;
+            k.ci_cells = kFeat && (P.flags & HPVCD_PIC_CONSTRAINED_INTRA) ? P.cells : nullptr;
+            k.gw = P.gw;
+            k.restricted = kFeat && (nb_ok != 0xfu || k.ci_cells != nullptr);
+            k.ccp = kFeat && c && (P.flags & HPVCD_PIC_CROSS_COMPONENT);
+            k.bd = c ? P.bd_c : P.bd;
+            k.max_v = (1 << k.bd) - 1;
+            k.luma = c == 0;
+            k.filt = c == 0 || P.idc == 3;
+            k.smoothing = !(P.flags & HPVCD_PIC_SMOOTHING_DISABLED);
+            k.strong = (P.flags & HPVCD_PIC_STRONG_SMOOTHING) != 0;
+            k.can = can_of(c);
+            k.rs = P.res_stride[c];
+            k.res = P.res[c] + (size_t)k.oy * k.rs + k.ox;
+            return k;
+        };
+        __syncthreads();
+        // ---- each walking warp turns the intra TBs of its components into
+        // walk entries, in decode order ----
         for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
-            const uint32_t cap = (uint32_t)lay.list_cap(c);
-            uint16_t* list = lists + lay.list_off(c);
+            const Comp k = comp_of(c);
+            const uint32_t cap = (uint32_t)lay.ent_cap(c);
+            uint4* list = ents + lay.ent_off(c);
             uint32_t cnt = 0;
             for (uint32_t base = 0; base < nrec; base += 32) {
                 const uint32_t i = base + lane;
                 bool mine = false;
+                hpvcd_tu t;
+                int x = 0, y = 0;
                 if (i < nrec) {
-                    hpvcd_tu t;
                     memcpy(&t, &recs[i], sizeof(t));
-                    int x, y;
                     if (t.comp == c && (t.flags & HPVCD_TU_INTRA) && intra_pred_ok && rec_check(t, x, y) == 1) {
                         if (t.mode > 34 || t.log2n > 5)
                             atomicOr(dev_err, DEV_ERR_BITSTREAM);
@@ -2201,8 +2286,23 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 }
                 const uint32_t m = __ballot_sync(kFull, mine);
                 const uint32_t pos = cnt + __popc(m & ((1u << lane) - 1u));
-                if (mine && pos < cap) list[pos] = (uint16_t)i;
                 cnt += __popc(m);
+                if (mine && pos < cap) {
+                    // a chroma TB with cross-component prediction has a
+                    // residual (written by k_ccp) even without coded coefficients
+                    const bool coded = (t.flags & HPVCD_TU_CBF) != 0 || (k.ccp && t.res_scale);
+                    uint32_t f = kFeat && (t.flags & HPVCD_TU_PCM) ? kTbPcm : 0u;
+                    const int n = 1 << t.log2n;
+                    const uint32_t run = (1u << (n >> 2)) - 1u;
+                    uint32_t cov = 0;
+                    if (x + n == k.S) cov |= run << (y >> 2);
+                    if (y + n == k.Sh) cov |= run << (16 + (x >> 2));
+                    if (cov) {
+                        f |= kTbPub;
+                        atomicOr(&s_cov[c], cov);
+                    }
+                    list[pos] = make_entry(k, t, x, y, i, stamp, coded, f);
+                }
             }
             if (cnt > cap) {
                 if (lane == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
@@ -2248,52 +2348,13 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 }
             }
         }
-        // neighbour CTUs that intra prediction may read: same slice and tile
-        // (decode.rs:4651-4690)
-        uint32_t nb_ok = 0xfu;
-        if (kFeat && P.ctb_region) {
-            const uint16_t me = P.ctb_region[ci];
-            const int cx = it.cx, cy = it.cy;
-            auto same = [&](int nx, int ny) {
-                return nx >= 0 && ny >= 0 && nx < P.ctb_cols && P.ctb_region[(size_t)ny * P.ctb_cols + nx] == me;
-            };
-            nb_ok = (same(cx - 1, cy) ? 1u : 0u) | (same(cx - 1, cy - 1) ? 2u : 0u) | (same(cx, cy - 1) ? 4u : 0u) |
-                    (same(cx + 1, cy - 1) ? 8u : 0u);
-        }
         if (P.flags & HPVCD_PIC_INTER) __syncthreads();  // the interior before the residuals staged over it
-        // Everything one walking warp needs about component c of this CTU.
-        auto comp_of = [&](int c) -> Comp {
-            Comp k;
-            k.S = c ? Scw : ctb;
-            k.Sh = c ? Sch : ctb;
-            k.ox = c ? ocx : oxl;
-            k.oy = c ? ocy : oyl;
-            k.pw = c ? P.cw : P.w;
-            k.ph = c ? P.ch : P.h;
-            k.sw = c ? P.sub_w : 1;
-            k.sh = c ? P.sub_h : 1;
-            k.nb_ok = nb_ok;
-            k.ci_cells = kFeat && (P.flags & HPVCD_PIC_CONSTRAINED_INTRA) ? P.cells : nullptr;
-            k.gw = P.gw;
-            k.restricted = kFeat && (nb_ok != 0xfu || k.ci_cells != nullptr);
-            k.ccp = kFeat && c && (P.flags & HPVCD_PIC_CROSS_COMPONENT);
-            k.bd = c ? P.bd_c : P.bd;
-            k.max_v = (1 << k.bd) - 1;
-            k.luma = c == 0;
-            k.filt = c == 0 || P.idc == 3;
-            k.smoothing = !(P.flags & HPVCD_PIC_SMOOTHING_DISABLED);
-            k.strong = (P.flags & HPVCD_PIC_STRONG_SMOOTHING) != 0;
-            k.can = can_of(c);
-            k.rs = P.res_stride[c];
-            k.res = P.res[c] + (size_t)k.oy * k.rs + k.ox;
-            return k;
-        };
-        // ---- residuals into the canvas, before the walk.  In an intra picture every sample
-        // of the CTU comes from the walk, so the whole visible residual block
-        // of each component is copied by all threads (the areas of uncoded
-        // TBs are never read); in an inter picture the canvas holds inter
-        // samples, so only the areas of coded intra TBs are staged (with their
-        // walk entries, one lane of the walking warp each) ----
+        // ---- residuals into the canvas, before the walk.  In an intra picture
+        // every sample of the CTU comes from the walk, so the whole visible
+        // residual block of each component is copied by all threads (the areas
+        // of uncoded TBs are never read); in an inter picture the canvas holds
+        // inter samples, so only the areas of coded intra TBs are staged (one
+        // lane of the walking warp each) ----
         if (!(P.flags & HPVCD_PIC_INTER)) {
             for (int c = 0; c < ncomp; ++c) {
                 const int S = c ? Scw : ctb, Sh = c ? Sch : ctb, ox = c ? ocx : oxl, oy = c ? ocy : oyl;
@@ -2307,126 +2368,146 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                     cp_async16(can + can_in(S, 8 * q, r), res + (size_t)r * rs + 8 * q);
                 }
             }
-        }
-        // ---- walk entries of this warp's components, over their records ----
-        for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
-            const Comp k = comp_of(c);
-            const uint32_t cnt = counts[c];
-            uint16_t* list = lists + lay.list_off(c);
-            for (uint32_t e = lane; e < cnt; e += 32) {
-                hpvcd_tu t;
-                const uint32_t j = list[e] & kListRec;
-                memcpy(&t, &recs[j], sizeof(t));
-                const int x = (int)t.x - k.ox, y = (int)t.y - k.oy;
-                // a chroma TB with cross-component prediction has a residual
-                // (written by k_ccp) even without coded coefficients
-                const bool coded = (t.flags & HPVCD_TU_CBF) != 0 || (k.ccp && t.res_scale);
-                const bool pcm = kFeat && (t.flags & HPVCD_TU_PCM);
-                if ((P.flags & HPVCD_PIC_INTER) && coded && !pcm) stage_residual(k, t.log2n, x, y);
-                bool gather;
-                recs[j] = make_entry(k, t, x, y, j, stamp, coded, &gather);
-                uint32_t f = pcm ? kListPcm : 0u;
-                if (x == 0 || y == 0) f |= kListEdge;
-                if (gather) f |= kListGather;
-                const int n = 1 << t.log2n;
-                const uint32_t run = (1u << (n >> 2)) - 1u;
-                uint32_t cov = 0;
-                if (x + n == k.S) cov |= run << (y >> 2);
-                if (y + n == k.Sh) cov |= run << (16 + (x >> 2));
-                if (cov) {
-                    f |= kListPub;
-                    atomicOr(&s_cov[c], cov);
+        } else {
+            for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
+                const Comp k = comp_of(c);
+                const uint4* list = ents + lay.ent_off(c);
+                for (uint32_t e = lane; e < counts[c]; e += 32) {
+                    TbEntry E;
+                    E.w = list[e];
+                    if ((E.w.z & kTbCoded) && !(E.flags() & kTbPcm))
+                        stage_residual(k, 31 - __clz(E.n2()) - 1, E.x(), E.y());
                 }
-                list[e] = (uint16_t)(j | f);
             }
         }
         cp_async_wait_all();  // this thread's residual copies; the barrier publishes them
         __syncthreads();
-        if (warp == kWalkers) {
+        if (warp == kWalkers)
             edge_service(P, it.cx, it.cy, ncomp, can_of, s_cov, s_have, s_done, kWalkers, lane);
-        }
         // ---- decode-order walk: each warp reconstructs its components ----
-        WalkScratch& ws = *(WalkScratch*)(smem + lay.off_ws + (size_t)warp * kWsBytes);
+        WalkScratch& ws = *(WalkScratch*)(smem + lay.off_ws + (size_t)min(warp, kWalkers - 1) * kWsBytes);
+        const int half = lane >> 4, l15 = lane & 15;
         for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
             const Comp k = comp_of(c);
-            const uint32_t cnt = counts[c];
-            const uint16_t* list = lists + lay.list_off(c);
-            // Software pipeline: while a TB is reconstructed, the next one's
-            // line address and table entry are worked out and the entry after
-            // it is loaded.
+            const uint32_t cnt = counts[c], last = cnt ? cnt - 1 : 0u;
+            const uint4* list = ents + lay.ent_off(c);
             uint16_t* const can = k.can;
-            const int row = can_row(k.S);
+            const int row = can_row(k.S), max_v = k.max_v;
             const bool luma = c == 0;
             unsigned long long* const words = edge_words(P, it.cx, it.cy, c);
-            auto lut_of = [&](const TbEntry& E) -> uint2 {
-                return __ldg((const uint2*)&g_angular + E.lut() + (E.n2() == 16 ? lane : lane & 15));
-            };
+            const int px4 = ((lane >> 2) & 3) * row + (lane & 3), px8 = (lane >> 2) * row + 2 * (lane & 3);
             Have have{0u, 0u};
             if (!fine && cnt) have = wait_edges(have, 0xffffffffu, 0xffffffffu, s_have + 2 * c, spin_limit, dev_err, lane);
-            const uint32_t last = cnt ? cnt - 1 : 0u;
-            TbEntry E{}, En{};
-            uint32_t j0 = 0, j1 = 0, j2 = 0;
-            int adr = 0;
+            // The edge words a TB reads: with x = 0 the left column from row
+            // y - 1 on, with y = 0 the row above from sample x - 1 on.
+            auto await = [&](const TbEntry& E, bool active) {
+                const int x = E.x(), y = E.y(), n2 = E.n2();
+                uint32_t need_top = 0u, need_left = 0u;
+                if (active && y == 0) {
+                    const int lo = max(x - 1, 0) >> 2, hi = (x + n2) >> 2;
+                    need_top = (0xffffffffu >> (32 - (hi - lo))) << lo;
+                }
+                if (active && x == 0) {
+                    const int lo = max(y - 1, 0) >> 2, hi = min(y + n2, k.Sh) >> 2;
+                    need_left = ((1u << (hi - lo)) - 1u) << lo;
+                    if (y == 0) need_left |= kHaveCorner;
+                }
+                need_top = __reduce_or_sync(kFull, need_top & ~have.top);
+                need_left = __reduce_or_sync(kFull, need_left & ~have.left);
+                if (need_top | need_left)
+                    have = wait_edges(have, need_top, need_left, s_have + 2 * c, spin_limit, dev_err, lane);
+            };
+            // Lanes 0..15 hold TB e, lanes 16..31 TB e + 1.  Two plain 4x4 TBs
+            // share the arithmetic of their addresses and weights (half of a
+            // 4x4 TB's instructions), each half-warp then predicts its own
+            // TB, the second after the first is stored.
+            TbEntry H;
             uint2 lut = make_uint2(0u, 0u);
+            auto lut_at = [&](uint32_t row_of, int l) { return __ldg((const uint2*)&g_angular + row_of + l); };
             if (cnt) {
-                j0 = list[0], j1 = list[min(1u, last)], j2 = list[min(2u, last)];
-                E.w = recs[j0 & kListRec];
-                En.w = recs[j1 & kListRec];
-                adr = Line(E, row).at(lane);  // positions past the line clamp to its last one
-                lut = lut_of(E);
+                H.w = list[min((uint32_t)half, last)];
+                lut = lut_at(H.lut(), l15);
             }
-            for (uint32_t e = 0; e < cnt; ++e) {
-                const int n2 = E.n2(), mode = E.mode();
-                int stride = row;
-                if (j0 & (kListEdge | kListGather)) {
-                    // the words it reads: with x = 0 the left column from row
-                    // y - 1 on, with y = 0 the row above from sample x - 1 on
-                    const int x = E.x(), y = E.y();
-                    uint32_t need_top = 0u, need_left = 0u;
-                    if (y == 0) {
-                        const int lo = max(x - 1, 0) >> 2, hi = (x + n2) >> 2;
-                        need_top = (0xffffffffu >> (32 - (hi - lo))) << lo;
+            for (uint32_t e = 0; e < cnt;) {
+                const bool plain4 = (H.flags() & kTbPlain) && H.n2() == 8;
+                const uint32_t b4 = __ballot_sync(kFull, plain4);
+                uint32_t next;
+                if (b4 & 1u) {
+                    const bool two = (b4 >> 16) && e < last;
+                    const bool active = two || half == 0;
+                    next = e + (two ? 2u : 1u);
+                    if (__any_sync(kFull, active && (H.flags() & kTbEdge))) await(H, active);
+                    const int lo = H.lo(), hi = H.hi(), l0 = H.line0(), c0 = H.corner() - 8;
+                    const int q0 = min(max((int)(lut.x & 0xffu), lo), hi), q1 = min(max((int)((lut.x >> 8) & 0xffu), lo), hi);
+                    const uint16_t* r0 = can + (q0 < 8 ? l0 - q0 * row : c0 + q0);
+                    const uint16_t* r1 = can + (q1 < 8 ? l0 - q1 * row : c0 + q1);
+                    uint16_t* const px = can + H.org() + px4;
+                    const int w0 = (int)(lut.x >> 24), w1 = (int)((lut.x >> 16) & 0xffu);
+                    int rv = 0, s = 0;
+                    if (plain4) {  // (the other half's TB may be of another kind: its addresses mean nothing here)
+                        if (H.w.z & kTbCoded) rv = (int)(int16_t)*px;
+                        s = __viaddmin_s32_relu((w0 * *r0 + w1 * *r1 + 16) >> 5, rv, max_v);
+                        if (half == 0) *px = (uint16_t)s;
                     }
-                    if (x == 0) {
-                        const int lo = max(y - 1, 0) >> 2, hi = min(y + n2, k.Sh) >> 2;
-                        need_left = ((1u << (hi - lo)) - 1u) << lo;
-                        if (y == 0) need_left |= kHaveCorner;
+                    TbEntry N;
+                    N.w = list[min(next + half, last)];
+                    __syncwarp();
+                    if (two) {
+                        s = __viaddmin_s32_relu((w0 * *r0 + w1 * *r1 + 16) >> 5, rv, max_v);
+                        if (half) *px = (uint16_t)s;
                     }
-                    if ((need_top & ~have.top) | (need_left & ~have.left))
-                        have = wait_edges(have, need_top, need_left, s_have + 2 * c, spin_limit, dev_err, lane);
-                    if (j0 & kListGather) {
-                        gather_line(k, 31 - __clz(n2) - 1, x, y, stamp, E.w.w >> 16, ws, lane);
+                    lut = lut_at(N.lut(), l15);
+                    if (__any_sync(kFull, active && (H.flags() & kTbPub)) && active) {  // samples on the right column / bottom row
+                        uint16_t* const w16 = (uint16_t*)words;
+                        const int x = H.x() + (lane & 3), y = H.y() + (l15 >> 2);
+                        const uint16_t t = (uint16_t)(s | 0x8000);
+                        if (x == k.S - 1) st_edge16(w16 + y, t);
+                        if (y == k.Sh - 1) st_edge16(w16 + k.Sh + x, t);
+                    }
+                    __syncwarp();
+                    H = N;
+                } else {
+                    TbEntry E;
+                    E.w = list[e];
+                    next = e + 1;
+                    const uint32_t f = E.flags();
+                    const int n2 = E.n2(), mode = E.mode();
+                    int stride = row;
+                    if (f & kTbEdge) await(E, true);
+                    if (f & kTbGather) {
+                        gather_line(k, 31 - __clz(n2) - 1, E.x(), E.y(), stamp, E.jrec(), ws, lane);
                         const uint32_t at = (uint32_t)(ws.s - can);  // position i at canvas offset at + i
                         E.w.x = (E.w.x & 0xffffu) | (at << 16);
                         E.w.y = (E.w.y & 0xffff0000u) | (at + (uint32_t)n2);
                         stride = -1;
-                        adr = Line(E, stride).at(lane);
                     }
+                    const Line L(E, stride);
+                    const bool coded = (E.w.z & kTbCoded) != 0u, filt = (E.w.z & kTbFilt) != 0u;
+                    if (kFeat && (f & kTbPcm)) {
+                        pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
+                    } else if (n2 == 8) {
+                        // positions past the line clamp to its last one
+                        const uint2 lu = lut_at(E.lut(), l15);
+                        walk_tb4(can + E.org() + px4, mode, coded, luma, max_v, can[L.at(lane)], lu.x, lane);
+                    } else if (n2 == 16) {
+                        const uint2 lu = lut_at(E.lut(), lane);
+                        uint32_t* const px = (uint32_t*)(can + E.org() + px8);
+                        if (f & kTbPlain) {
+                            walk_plain8(can, L, px, coded, max_v, lu);
+                        } else {
+                            const bool hi_ok = (f & kTbHi32) != 0u;
+                            walk_tb8(px, mode, coded, filt, luma, max_v, can[L.at(lane)], hi_ok ? can[E.corner() + 16] : 0,
+                                     hi_ok, lu, lane);
+                        }
+                    } else {
+                        walk_tb_big(can, row, L, E.org(), 31 - __clz(n2) - 1, mode, coded, filt, luma, k.strong, k.bd, ws,
+                                    lane);
+                    }
+                    H.w = list[min(next + half, last)];
+                    lut = lut_at(H.lut(), l15);
+                    if (f & kTbPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
                 }
-                const int v = can[adr];
-                TbEntry Enn;
-                Enn.w = recs[j2 & kListRec];
-                const uint32_t j3 = list[min(e + 3, last)];
-                const int adr_n = Line(En, row).at(lane);
-                const uint2 lut_n = lut_of(En);
-                const bool coded = (E.w.z & kTbCoded) != 0u, filt = (E.w.z & kTbFilt) != 0u;
-                if (kFeat && (j0 & kListPcm)) {
-                    pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
-                } else if (n2 == 8) {
-                    walk_tb4(can, row, E.org(), mode, coded, luma, k.max_v, v, lut.x, lane);
-                } else if (n2 == 16) {
-                    const bool hi_ok = E.hi() == 32;
-                    const int v_hi = can[hi_ok ? E.corner() + 16 : 0];
-                    walk_tb8(can, row, E.org(), mode, coded, filt, luma, k.max_v, v, v_hi, hi_ok, lut, lane);
-                } else {
-                    walk_tb_big(can, row, Line(E, stride), E.org(), 31 - __clz(n2) - 1, mode, coded, filt, luma, k.strong,
-                                k.bd, ws.f, lane);
-                }
-                if (j0 & kListPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
-                E = En;
-                En = Enn;
-                j0 = j1, j1 = j2, j2 = j3;
-                adr = adr_n, lut = lut_n;
+                e = next;
             }
         }
         if (warp < kWalkers && lane == 0) *(volatile uint32_t*)&s_done[warp] = 1u;
@@ -2467,7 +2548,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
 }  // namespace hpvcd
 
 extern "C" size_t hpvcd_recon_smem_bytes(int cfmt, int chroma_warps) {
-    return hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(chroma_warps == 1 ? 1 : 2)).total;
+    return hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(chroma_warps == 1 ? 1 : 2) - 1).total;
 }
 
 extern "C" cudaError_t hpvcd_launch_residual(const hpvcd::DevPic* pics, const uint32_t* rec_prefix,
@@ -2518,7 +2599,7 @@ extern "C" cudaError_t hpvcd_launch_recon(const hpvcd::DevPic* pics, const hpvcd
     // build: 1 one chroma warp (Cb, then Cr), 2 (and 3) one warp per chroma
     // component
     const int cw = chroma_warps == 1 ? 1 : 2;
-    const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw)).total;
+    const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw) - 1).total;
     const int threads = 32 * hpvcd::recon_warps(cw);
     // default: 2^22 polls of up to 64 ns each bound one wait to a few hundred ms
     if (spin == 0) spin = 1u << 22;
@@ -2557,7 +2638,7 @@ void recon_attrs(int lim) {
 int recon_occupancy_of(int cfmt, int chroma_warps) {
     int blocks = 0;
     const int cw = chroma_warps == 1 ? 1 : 2;
-    const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw)).total;
+    const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw) - 1).total;
     if (cw == 2)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, hpvcd::k_recon<2, false>, 32 * hpvcd::recon_warps(2),
                                                       smem);
@@ -2593,7 +2674,7 @@ extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
     }
     std::lock_guard<std::mutex> lock(g_attr_mu);
     if (dev >= 0 && g_attr_done[dev]) return g_attr_occ[dev][cf][build - 1];
-    const int lim = (int)hpvcd::ReconLayout(hpvcd::kFmt444, hpvcd::recon_warps(2)).total;
+    const int lim = (int)hpvcd::ReconLayout(hpvcd::kFmt444, hpvcd::recon_warps(2) - 1).total;
     recon_attrs<1, false>(lim);
     recon_attrs<2, false>(lim);
     recon_attrs<1, true>(lim);
