@@ -1298,7 +1298,7 @@ __device__ __forceinline__ int can_at(int S, int x, int y) {
 __device__ __forceinline__ int can_in(int S, int x, int y) { return can_top(S) + y * can_row(S) + x + 8; }
 
 // Shared-memory layout of one CTA: the canvases, one walk scratch per
-// walking warp, the walk entries, the 16x16 stamp map.
+// walking warp, the walk entries, the blend table, the 16x16 stamp map.
 // Records of one CTU staged at once: up to 256 luma TBs, one "mark decoded"
 // record per inter CU (64 at most) and the chroma TBs (64 per component at
 // 4:2:0, 128 at 4:2:2, 256 at 4:4:4).  A CTU with more records is malformed.
@@ -1315,7 +1315,7 @@ struct ReconLayout {
     int cs_w, cs_h;  // chroma canvas width and height (CTU interior)
     int rec_cap;     // staged records
     int list_c;      // intra TBs per chroma component
-    size_t off_can_y, off_can_c, off_ws, off_ents, off_stamp, off_misc, total;
+    size_t off_can_y, off_can_c, off_ws, off_ents, off_tab, off_stamp, off_wf, off_misc, total;
     __host__ __device__ ReconLayout(int cfmt, int walkers) {
         cs_w = cfmt == kFmt444 ? 64 : 32;
         cs_h = cfmt == kFmt420 ? 32 : 64;
@@ -1328,12 +1328,16 @@ struct ReconLayout {
         o = (o + 15) & ~(size_t)15;
         off_ws = o;    o += (size_t)walkers * kWsBytes;
         off_ents = o;  o += (size_t)(kListCap + 2 * list_c) * sizeof(uint4);
+        off_tab = o;   o += (size_t)(64 * 64 + 2 * cs_w * cs_h) * sizeof(uint32_t);
         off_stamp = o; o += 256 * sizeof(uint32_t);
-        off_misc = o;  o += 128;  // claimed item, TB counts, have bits, covered words, done flags
+        off_wf = o;    o += (size_t)(kListCap + 2 * list_c);
+        o = (o + 15) & ~(size_t)15;
+        off_misc = o;  o += 128;  // claimed item, have bits, covered words, done flags, TB counts
         total = o;
     }
     __host__ __device__ int ent_off(int c) const { return c == 0 ? 0 : kListCap + (c - 1) * list_c; }
     __host__ __device__ int ent_cap(int c) const { return c == 0 ? kListCap : list_c; }
+    __host__ __device__ int tab_off(int c) const { return c == 0 ? 0 : 64 * 64 + (c - 1) * cs_w * cs_h; }
 };
 // The CTU's records are staged in the canvases: they are done with (turned
 // into walk entries) before any sample or residual is put there.
@@ -1677,7 +1681,7 @@ __device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need
 // prediction), or that has none, is flagged kTbGather and its line is gathered
 // sample by sample first.
 //   x: canvas offset of the TB | of line position 0 << 16
-//   y: canvas offset of the corner | row of the angular table << 16
+//   y: canvas offset of the corner | blend table offset of a plain TB << 16
 //   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbCoded | kTbFilt
 //   w: x | y << 8 (in the CTU) | record index (< 1024) << 16 | kTb* flags << 26
 // Measured when the entries came in (4032x3024 grid, 70 luma TBs a CTU): the
@@ -1695,7 +1699,7 @@ struct TbEntry {
     __device__ __forceinline__ int org() const { return (int)(w.x & 0xffffu); }
     __device__ __forceinline__ int line0() const { return (int)(w.x >> 16); }
     __device__ __forceinline__ int corner() const { return (int)(w.y & 0xffffu); }
-    __device__ __forceinline__ uint32_t lut() const { return w.y >> 16; }
+    __device__ __forceinline__ uint32_t tab() const { return w.y >> 16; }
     __device__ __forceinline__ int lo() const { return (int)(w.z & 0xffu); }
     __device__ __forceinline__ int hi() const { return (int)((w.z >> 8) & 0xffu); }
     __device__ __forceinline__ int n2() const { return (int)((w.z >> 16) & 0xffu); }
@@ -1711,46 +1715,60 @@ struct TbEntry {
 __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, int x0, int y0, uint32_t jrec,
                                             const uint32_t* stamp, bool coded, uint32_t flags) {
     const int n = 1 << t.log2n, n2 = 2 * n;
-    // cells one sample apart in this component's units
-    const int uw = 4 / k.sw, uh = 4 / k.sh;
     auto decoded = [&](int x, int y) { return stamp[((y * k.sh) >> 2) * 16 + ((x * k.sw) >> 2)] < jrec; };
     auto allowed = [&](int x, int y) { return !k.restricted || restricted_ok(k, x, y, k.ox + x, k.oy + y); };
-    bool one_run = true;
-    // left column, downwards: samples available from the top
-    int al = 0;
-    const int yend = min(min(y0 + n2, k.Sh), k.ph - k.oy);
-    if (k.ox + x0 > 0) {
-        if (x0 == 0 && !k.restricted) {
-            al = max(yend - y0, 0);
+    // Availability is per cell, but an n x n block aligned to its size is one
+    // run of the decode order, so the first and last cell of each side's n
+    // samples (the row above, above-right, left, below-left) speak for it.
+    // Where they differ, and where slices, tiles or constrained intra
+    // prediction decide per cell, every cell is looked at.
+    const int yend = min(min(y0 + n2, k.Sh), k.ph - k.oy), xend = min(y0 == 0 ? x0 + n2 : min(x0 + n2, k.S), k.pw - k.ox);
+    const bool any_l = k.ox + x0 > 0, any_a = k.oy + y0 > 0;
+    bool one_run = true, cells = k.restricted;
+    int al = 0, ar = 0;  // samples available downwards from the top left, rightwards from the left above
+    if (any_l && !cells) {
+        if (x0 == 0) {
+            al = n2;
         } else {
-            bool open = true;
-            for (int y = y0; y < yend; y += uh) {
-                const bool a = (x0 == 0 || decoded(x0 - 1, y)) && allowed(x0 - 1, y);
-                if (a && open) al = y + uh - y0;
-                if (a && !open) one_run = false;
-                open = open && a;
-            }
-            al = min(al, max(yend - y0, 0));
+            const bool a = decoded(x0 - 1, y0), b = decoded(x0 - 1, min(y0 + n, yend) - 1);
+            const bool low = y0 + n < yend;
+            const bool d = low && decoded(x0 - 1, y0 + n), e = low && decoded(x0 - 1, yend - 1);
+            cells = a != b || d != e || (d && !a);
+            al = a ? (d ? n2 : n) : 0;
         }
     }
-    // row above, rightwards (the above-right CTU is a neighbour too)
-    int ar = 0;
-    const int xend = min(y0 == 0 ? x0 + n2 : min(x0 + n2, k.S), k.pw - k.ox);
-    if (k.oy + y0 > 0) {
-        if (y0 == 0 && !k.restricted) {
-            ar = max(xend - x0, 0);
+    if (any_a && !cells) {
+        if (y0 == 0) {
+            ar = n2;
         } else {
-            bool open = true;
-            for (int x = x0; x < xend; x += uw) {
-                const bool a = (y0 == 0 || decoded(x, y0 - 1)) && allowed(x, y0 - 1);
-                if (a && open) ar = x + uw - x0;
-                if (a && !open) one_run = false;
-                open = open && a;
-            }
-            ar = min(ar, max(xend - x0, 0));
+            const bool a = decoded(x0, y0 - 1), b = decoded(min(x0 + n, xend) - 1, y0 - 1);
+            const bool right = x0 + n < xend;
+            const bool d = right && decoded(x0 + n, y0 - 1), e = right && decoded(xend - 1, y0 - 1);
+            cells = a != b || d != e || (d && !a);
+            ar = a ? (d ? n2 : n) : 0;
         }
     }
-    bool corner = k.ox + x0 > 0 && k.oy + y0 > 0 && allowed(x0 - 1, y0 - 1);
+    if (cells) {
+        const int uw = 4 / k.sw, uh = 4 / k.sh;  // a cell in this component's samples
+        al = ar = 0;
+        bool open = true;
+        for (int y = y0; any_l && y < yend; y += uh) {
+            const bool a = (x0 == 0 || decoded(x0 - 1, y)) && allowed(x0 - 1, y);
+            if (a && open) al = y + uh - y0;
+            if (a && !open) one_run = false;
+            open = open && a;
+        }
+        open = true;
+        for (int x = x0; any_a && x < xend; x += uw) {
+            const bool a = (y0 == 0 || decoded(x, y0 - 1)) && allowed(x, y0 - 1);
+            if (a && open) ar = x + uw - x0;
+            if (a && !open) one_run = false;
+            open = open && a;
+        }
+    }
+    al = min(al, max(yend - y0, 0));
+    ar = min(ar, max(xend - x0, 0));
+    bool corner = any_l && any_a && allowed(x0 - 1, y0 - 1);
     if (corner && x0 > 0 && y0 > 0) corner = decoded(x0 - 1, y0 - 1);
     int lo = n2 - al, hi = n2 + ar;
     if (!corner) {
@@ -1767,11 +1785,10 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
     const bool filt = n > 4 && ref_filtered(k, n, t.mode);
     if (n <= 8 && t.mode >= 2 && one_run && !filt && !(flags & kTbPcm) && !(k.luma && (t.mode == 10 || t.mode == 26)))
         flags |= kTbPlain;
-    const uint32_t am = t.mode >= 2 ? t.mode - 2u : 0u;
-    const uint32_t lut = n == 4 ? am * 16u : (n == 8 ? 33u * 16u + am * 32u : 0u);
+    const uint32_t tab = flags & kTbPlain ? (uint32_t)((y0 >> 2) * (k.S >> 2) + (x0 >> 2)) * 16u : 0u;
     uint4 w;
     w.x = (uint32_t)cin(k, x0, y0) | ((uint32_t)cin(k, x0 - 1, y0 + n2 - 1) << 16);
-    w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (lut << 16);
+    w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (tab << 16);
     w.z = (uint32_t)lo | ((uint32_t)hi << 8) | ((uint32_t)n2 << 16) | ((uint32_t)t.mode << 24);
     if (coded) w.z |= kTbCoded;
     if (filt) w.z |= kTbFilt;
@@ -1783,8 +1800,8 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
 // the two line positions it interpolates (intra.rs:305-318, the projection
 // of negative angles included) and their weights: p0 | p1 << 8 | weight of
 // p1 << 16 | weight of p0 << 24.
-struct AngularTables {  // rows of uint2: 33 x 16 lanes (4x4, .x only), then 33 x 32 lanes (8x8)
-    uint32_t t4[33][16][2], t8[33][32][2];
+struct AngularTables {
+    uint32_t t4[33][16], t8[33][64];
 };
 constexpr uint32_t angular_entry(int mode, int n, int x, int y) {
     constexpr int ang[33] = {32,  26,  21,  17,  13,  9,  5,  2,  0,  -2, -5, -9, -13, -17, -21, -26, -32,
@@ -1812,9 +1829,8 @@ constexpr uint32_t angular_entry(int mode, int n, int x, int y) {
 constexpr AngularTables make_angular() {
     AngularTables T{};
     for (int m = 0; m < 33; ++m) {
-        for (int i = 0; i < 16; ++i) T.t4[m][i][0] = angular_entry(m + 2, 4, i & 3, i >> 2);
-        // lane l of an 8x8 TB predicts samples (2 (l & 3) + h, l >> 2)
-        for (int i = 0; i < 64; ++i) T.t8[m][i >> 1][i & 1] = angular_entry(m + 2, 8, 2 * ((i >> 1) & 3) + (i & 1), i >> 3);
+        for (int i = 0; i < 16; ++i) T.t4[m][i] = angular_entry(m + 2, 4, i & 3, i >> 2);
+        for (int i = 0; i < 64; ++i) T.t8[m][i] = angular_entry(m + 2, 8, i & 7, i >> 3);
     }
     return T;
 }
@@ -1838,6 +1854,23 @@ struct Line {
         return i < n2 ? l0 - i * ls : c0 + i;
     }
 };
+
+// Blend table of a CTU component: one word per sample of its plain TBs, by
+// 4x4 blocks in raster order: coded | canvas byte offsets of the two line
+// samples (even, < 2^14) << 0 and << 13 | weight of the second (of 32) << 27.
+// With it the walk neither looks anything up nor clamps: it was 270 cycles a
+// 4x4 TB and 850 an 8x8 one with the table of modes and the line in the loop.
+constexpr uint32_t kBlendAdr = 0x3ffeu;
+static_assert(2 * can_size(64, 64) < 0x4000, "canvas byte offsets fit the blend words");
+__device__ __forceinline__ uint32_t blend_word(const Line& L, uint32_t ang, bool coded) {
+    return (coded ? 1u : 0u) | (uint32_t)(2 * L.at((int)(ang & 0xffu))) | ((uint32_t)(2 * L.at((int)((ang >> 8) & 0xffu))) << 13) |
+           ((ang & 0x1f0000u) << 11);
+}
+__device__ __forceinline__ int blend_of(const uint16_t* can, uint32_t w) {
+    const int a = *(const uint16_t*)((const char*)can + (w & kBlendAdr));
+    const int b = *(const uint16_t*)((const char*)can + ((w >> 13) & kBlendAdr));
+    return (32 * a + (int)(w >> 27) * (b - a) + 16) >> 5;
+}
 
 // Residual add + clip (reconstruct.rs:214-251) of two samples in 16-bit halves.
 __device__ __forceinline__ uint32_t add_clip2(uint32_t pred, uint32_t res, int max_v) {
@@ -1883,7 +1916,7 @@ __device__ __forceinline__ void walk_tb4(uint16_t* px, int mode, bool coded, boo
     __syncwarp();
 }
 
-// 8x8 intra TB: v is line position `lane`, v_hi position 32 where it is
+// 8x8 intra TB that is not plain: v is line position `lane`, v_hi position 32 where it is
 // available (the same in every lane; else position 31 stands in for it);
 // [1 2 1] filtering (intra.rs:151-219; no strong filter below
 // 32x32) and prediction (intra.rs:257-372) by shuffles, two horizontally
@@ -1946,28 +1979,30 @@ __device__ __forceinline__ void walk_tb8(uint32_t* px, int mode, bool coded, boo
     __syncwarp();
 }
 
-// Two horizontally adjacent samples of a plain 8x8 TB per lane (kTbPlain):
-// every lane reads its four line samples in place, no line, no shuffles.
-__device__ __forceinline__ void walk_plain8(uint16_t* can, const Line& L, uint32_t* px, bool coded, int max_v, uint2 lut) {
-    const int a0 = can[L.at((int)(lut.x & 0xffu))], a1 = can[L.at((int)((lut.x >> 8) & 0xffu))];
-    const int b0 = can[L.at((int)(lut.y & 0xffu))], b1 = can[L.at((int)((lut.y >> 8) & 0xffu))];
-    const uint32_t rv = coded ? *px : 0u;
-    const uint32_t p0 = ((lut.x >> 24) * a0 + ((lut.x >> 16) & 0xffu) * a1 + 16u) >> 5;
-    const uint32_t p1 = ((lut.y >> 24) * b0 + ((lut.y >> 16) & 0xffu) * b1 + 16u) >> 5;
+// Two horizontally adjacent samples of a plain 8x8 TB per lane.
+__device__ __forceinline__ void walk_plain8(const uint16_t* can, uint32_t* px, uint2 w, int max_v) {
+    const uint32_t rv = (w.x & 1u) ? *px : 0u;
+    const uint32_t p0 = (uint32_t)blend_of(can, w.x), p1 = (uint32_t)blend_of(can, w.y);
     *px = add_clip2(p0 | (p1 << 16), rv, max_v);
     __syncwarp();
 }
 
 // 16x16 or 32x32 intra TB by one warp, two horizontally adjacent samples per
-// lane and row step.  The reference samples a sample may read (the angular
-// projection, or the left column) are filtered on the way into the scratch; the
-// row loops then read them at addresses that do not depend on loaded values.
-__device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& L, int org, int log2n, int mode,
-                                            bool coded, bool filt, bool luma, bool strong_on, int bd, WalkScratch& ws,
-                                            int lane) {
-    const int n = 1 << log2n, n2 = 2 * n;
+// lane and row step.  First the line samples the prediction reads, filtered
+// (intra.rs:151-219), go to the scratch: the projected references, each with
+// the next one, or for planar and DC the line from the sample below the left
+// column to the one right of the row above.  Then one rolled row loop per kind
+// of prediction: the loops are kept small because on a loaded SM the walks
+// wait for instructions first (unrolled by four the same batch took 8 % more).
+__device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& L, int org, int mode, bool coded,
+                                            bool filt, bool luma, bool strong_on, int bd, WalkScratch& ws, int lane) {
+    const int n2 = L.n2, n = n2 >> 1, hl = 30 - __clz(n);  // hl: log2 of the pairs per row
     const int max_v = (1 << bd) - 1;
     auto raw = [&](int i) { return (int)can[L.at(i)]; };
+    const bool angular = mode >= 2, vertical = mode >= 18;
+    const int angle = angular ? (int)c_intra_angle[mode - 2] : 0;
+    const int inv = angle < 0 ? (int)c_inv_angle[mode - 11] : 0;
+    const int k0 = angle < 0 ? 1 - n : 1;  // references k0 .. k0 + 2n - 1 are all a TB reads with a weight
     bool strong = false;
     int tl = 0, tr = 0, bl = 0;
     if (filt && luma && strong_on && n == 32) {  // intra.rs:176-196
@@ -1975,17 +2010,28 @@ __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& 
         const int thr = 1 << (bd - 5);
         strong = abs(bl + tl - 2 * raw(n2 - n)) < thr && abs(tr + tl - 2 * raw(n2 + n)) < thr;
     }
-    auto R = [&](int i) -> int {  // filtered line sample (intra.rs:151-219)
-        const int s = raw(i);
-        if (!filt || i == 0 || i == 2 * n2) return s;
-        if (strong) {
-            const int q = abs(i - n2);
-            return i == n2 ? s : ((n2 - q) * tl + q * (i > n2 ? tr : bl) + n) >> 6;
+    uint16_t* const halves = (uint16_t*)ws.pairs;
+    const int count = angular ? n2 : n2 + 3;
+#pragma unroll 1
+    for (int q = lane; q < count; q += 32) {
+        const int i = angular ? ref_pos(k0 + q, vertical, n2, inv) : n2 - n - 1 + q;
+        int v = raw(i);
+        if (filt && i != 0 && i != 2 * n2) {
+            if (!strong) {
+                v = (raw(i - 1) + 2 * v + raw(i + 1) + 2) >> 2;
+            } else if (i != n2) {
+                const int d = abs(i - n2);
+                v = ((n2 - d) * tl + d * (i > n2 ? tr : bl) + n) >> 6;
+            }
         }
-        return (raw(i - 1) + 2 * s + raw(i + 1) + 2) >> 2;
-    };
+        if (angular) {  // reference q in its own pair and the one before
+            halves[2 * q] = (uint16_t)v;
+            if (q) halves[2 * q - 1] = (uint16_t)v;
+        } else {
+            ws.f[q] = (uint16_t)v;
+        }
+    }
     // this lane's column pair, first row and rows per step
-    const int hl = log2n - 1;
     const int x = 2 * (lane & ((1 << hl) - 1)), ys = 32 >> hl;
     const bool edge = luma && n < 32;
     uint32_t* px = (uint32_t*)(can + org + (lane >> hl) * row + x);  // canvas rows and TB columns are even
@@ -1994,85 +2040,50 @@ __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& 
         *px = add_clip2((uint32_t)p0 | ((uint32_t)p1 << 16), coded ? *px : 0u, max_v);
         px += step;
     };
-    if (mode >= 2) {
-        const int angle = c_intra_angle[mode - 2];
-        const bool vertical = mode >= 18;
-        const int inv = angle < 0 ? c_inv_angle[mode - 11] : 0;
-        // pairs[k - k0] = projected references k and k + 1; k0 .. k0 + 2n - 1
-        // is all a TB reads with a weight
-        const int k0 = angle < 0 ? 1 - n : 1;
-        {
-            const int ra = R(ref_pos(k0 + lane, vertical, n2, inv));
-            int na = __shfl_down_sync(kFull, ra, 1);
-            if (n == 32) {
-                const int rb = R(ref_pos(k0 + 32 + lane, vertical, n2, inv));
-                const int b0 = __shfl_sync(kFull, rb, 0);
-                if (lane == 31) na = b0;
-                ws.pairs[lane + 32] = (uint32_t)rb | ((uint32_t)__shfl_down_sync(kFull, rb, 1) << 16);
-            }
-            ws.pairs[lane] = (uint32_t)ra | ((uint32_t)na << 16);
-        }
-        __syncwarp();
-        // ((32 - f) r[k] + f r[k + 1] + 16) >> 5
-        auto blend = [](uint32_t pair, int f) { return __dp2a_lo((int)pair, 32 - f + (f << 8), 16) >> 5; };
-        if (vertical) {
-            const bool e26 = edge && mode == 26;
-            const int a0 = e26 ? raw(n2 + 1) : 0, c0 = e26 ? raw(n2) : 0;
-            const uint32_t* base = ws.pairs + x + 1 - k0;
-            int pos = ((lane >> hl) + 1) * angle;
-#pragma unroll 4
-            for (int y = lane >> hl; y < n; y += ys, pos += ys * angle) {
-                const uint32_t* r = base + (pos >> 5);
-                int p0 = blend(r[0], pos & 31);
-                const int p1 = blend(r[1], pos & 31);
-                if (e26 && x == 0) p0 = clamp3i(a0 + ((raw(n2 - (y + 1)) - c0) >> 1), 0, max_v);
-                put(p0, p1);
-            }
-        } else {
-            const bool e10 = edge && mode == 10;
-            const int pa = (x + 1) * angle, pb = pa + angle;
-            const uint32_t* ra = ws.pairs + (pa >> 5) + 1 - k0;
-            const uint32_t* rb = ws.pairs + (pb >> 5) + 1 - k0;
-#pragma unroll 4
-            for (int y = lane >> hl; y < n; y += ys) {
-                int p0 = blend(ra[y], pa & 31), p1 = blend(rb[y], pb & 31);
-                if (e10 && y == 0) {
-                    const int a0 = raw(n2 - 1), c0 = raw(n2);
-                    p0 = clamp3i(a0 + ((raw(n2 + x + 1) - c0) >> 1), 0, max_v);
-                    p1 = clamp3i(a0 + ((raw(n2 + x + 2) - c0) >> 1), 0, max_v);
-                }
-                put(p0, p1);
-            }
-        }
-    } else if (mode == 1) {  // DC
-        const int part = lane < n ? raw(n2 + 1 + lane) + raw(n2 - 1 - lane) : 0;
-        const int dc = ((int)__reduce_add_sync(kFull, (unsigned)part) + n) >> (log2n + 1);
-        // the edge samples are read before the row they are on is written
-        int e0 = 0, e1 = 0;
-        const int l1 = raw(n2 - 1), a1 = raw(n2 + 1);
-        if (edge) e0 = raw(n2 + x + 1), e1 = raw(n2 + x + 2);
-#pragma unroll 4
-        for (int y = lane >> hl; y < n; y += ys) {
-            int p0 = dc, p1 = dc;
-            if (edge) {
-                if (y == 0) {
-                    p0 = x == 0 ? (l1 + 2 * dc + a1 + 2) >> 2 : (e0 + 3 * dc + 2) >> 2;
-                    p1 = (e1 + 3 * dc + 2) >> 2;
-                } else if (x == 0) {
-                    p0 = (raw(n2 - y - 1) + 3 * dc + 2) >> 2;
-                }
+    __syncwarp();
+    if (angular) {
+        // Sample (x, y) blends references idx and idx + 1 by frac, idx * 32 +
+        // frac = 32 b + (a + 1) angle, b along the edge and a away from it.
+        int pos = vertical ? 32 * x + ((lane >> hl) + 1) * angle : 32 * (lane >> hl) + (x + 1) * angle;
+        const int dx = vertical ? 32 : angle, dy = vertical ? ys * angle : ys * 32;
+        pos += 32 * (1 - k0);
+        const bool filter0 = edge && angle == 0;  // modes 10 and 26: their first row / column
+        auto blend = [&](int at) {  // ((32 - f) r[k] + f r[k + 1] + 16) >> 5
+            return __dp2a_lo((int)ws.pairs[at >> 5], 32 + (at & 31) * 255, 16) >> 5;
+        };
+#pragma unroll 1
+        for (int y = lane >> hl; y < n; y += ys, pos += dy) {
+            int p0 = blend(pos), p1 = blend(pos + dx);
+            if (filter0 && (vertical ? x == 0 : y == 0)) {
+                const int c0 = raw(n2), a0 = raw(vertical ? n2 + 1 : n2 - 1);
+                p0 = clamp3i(a0 + ((raw(vertical ? n2 - (y + 1) : n2 + x + 1) - c0) >> 1), 0, max_v);
+                if (!vertical) p1 = clamp3i(a0 + ((raw(n2 + x + 2) - c0) >> 1), 0, max_v);
             }
             put(p0, p1);
         }
-    } else {  // planar
-        if (lane < n) ws.f[lane] = (uint16_t)R(n2 - 1 - lane);
-        const int ab0 = R(n2 + x + 1), ab1 = R(n2 + x + 2), rt = R(n2 + n + 1), lb = R(n2 - n - 1);
-        __syncwarp();
-#pragma unroll 4
+    } else {
+        // ws.f: below-left, left column upwards, corner, row above, above-right
+        const uint16_t* const left = ws.f + n;       // left[-y]
+        const uint16_t* const above = ws.f + n + 2;  // above[x]
+        const int dc = mode == 1 ? (int)(__reduce_add_sync(kFull, lane < n ? (unsigned)above[lane] + left[-lane] : 0u) + n) >> (hl + 2)
+                                 : 0;
+        const int ab0 = above[x], ab1 = above[x + 1], rt = above[n], lb = left[-n];
+#pragma unroll 1
         for (int y = lane >> hl; y < n; y += ys) {
-            const int lf = ws.f[y], vb = (y + 1) * lb + n, up = n - 1 - y;
-            const int p0 = ((n - 1 - x) * lf + (x + 1) * rt + up * ab0 + vb) >> (log2n + 1);
-            const int p1 = ((n - 2 - x) * lf + (x + 2) * rt + up * ab1 + vb) >> (log2n + 1);
+            const int lf = left[-y];
+            int p0 = dc, p1 = dc;
+            if (mode == 0) {  // planar
+                const int vb = (y + 1) * lb + n, up = n - 1 - y;
+                p0 = ((n - 1 - x) * lf + (x + 1) * rt + up * ab0 + vb) >> (hl + 2);
+                p1 = ((n - 2 - x) * lf + (x + 2) * rt + up * ab1 + vb) >> (hl + 2);
+            } else if (edge) {
+                if (y == 0) {
+                    p0 = x == 0 ? (lf + 2 * dc + ab0 + 2) >> 2 : (ab0 + 3 * dc + 2) >> 2;
+                    p1 = (ab1 + 3 * dc + 2) >> 2;
+                } else if (x == 0) {
+                    p0 = (lf + 3 * dc + 2) >> 2;
+                }
+            }
             put(p0, p1);
         }
     }
@@ -2130,6 +2141,11 @@ __host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 // availability, coded and PCM tests compile to the plain form.  fine: a TB
 // waits for the edge words it reads; otherwise a CTU waits for all of its
 // neighbours' words before its walk.
+// How the walk takes the TB at an entry: it and the next one are plain 4x4
+// TBs, it is a plain 8x8 TB, it (or the pair) reads neighbour CTUs / covers
+// edge words.
+constexpr uint32_t kWalkPair = 1u, kWalkPlain8 = 2u, kWalkEdge = 4u, kWalkPub = 8u;
+
 template <int kCW, bool kFeat>
 __global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 5 : 4)
 k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint32_t n_items,
@@ -2171,10 +2187,10 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         uint4* recs = (uint4*)(smem + lay.off_can_y);  // until the walk entries are built
         uint4* ents = (uint4*)(smem + lay.off_ents);
         uint32_t* stamp = (uint32_t*)(smem + lay.off_stamp);
-        uint32_t* counts = (uint32_t*)(smem + lay.off_misc) + 1;  // TBs listed per component
-        uint32_t* s_have = counts + 3;                            // have bits, two words per component
+        uint32_t* s_have = (uint32_t*)(smem + lay.off_misc) + 1;  // have bits, two words per component
         uint32_t* s_cov = s_have + 6;                             // edge words covered by intra TBs
         uint32_t* s_done = s_cov + 3;                             // walking warps that are done
+        uint32_t* s_wcnt = s_done + 3;                            // TBs found per warp and component
         auto can_of = [&](int c) -> uint16_t* {
             return c == 0 ? (uint16_t*)(smem + lay.off_can_y)
                           : (uint16_t*)(smem + lay.off_can_c) + (size_t)(c - 1) * can_size(lay.cs_w, lay.cs_h);
@@ -2183,7 +2199,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         for (uint32_t i = tid; i < nrec; i += kThreads) cp_async16(recs + i, P.tus + r0 + i);
         asm volatile("cp.async.commit_group;" ::: "memory");
         for (int i = tid; i < 256; i += kThreads) stamp[i] = kNoStamp;
-        if (tid < 3) counts[tid] = s_cov[tid] = s_done[tid] = 0u;
+        if (tid < 3) s_cov[tid] = s_done[tid] = 0u;
         if (warp == kWalkers)  // words outside the picture count as present
             for (int c = 0; c < ncomp; ++c) {
                 const EdgeGeo e = edge_geo(P, c, it.cx, it.cy);
@@ -2211,17 +2227,40 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             const int Sw = tc ? Scw : ctb, Sh = tc ? Sch : ctb;
             return (x < 0 || y < 0 || x + n > Sw || y + n > Sh) ? 0 : 1;
         };
-        for (uint32_t i = tid; i < nrec; i += kThreads) {
-            hpvcd_tu t;
-            memcpy(&t, &recs[i], sizeof(t));
-            int x, y;
-            const int ok = rec_check(t, x, y);
-            if (ok == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
-            if (ok != 1 || t.comp != 0) continue;
-            const int n = 1 << t.log2n;
-            const int x1 = min(x + n, vis_w), y1 = min(y + n, vis_h);
-            for (int cy = y >> 2; cy < (y1 + 3) >> 2; ++cy)
-                for (int cx = x >> 2; cx < (x1 + 3) >> 2; ++cx) atomicMin(&stamp[cy * 16 + cx], i);
+        for (uint32_t base = 32 * warp; base < nrec; base += kThreads) {
+            const uint32_t i = base + lane;
+            // cell rectangle of a luma record: x | y << 8 | width << 16 | height << 24
+            uint32_t rect = 0u;
+            if (i < nrec) {
+                hpvcd_tu t;
+                memcpy(&t, &recs[i], sizeof(t));
+                int x, y;
+                const int ok = rec_check(t, x, y);
+                if (ok == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
+                if (ok == 1 && t.comp == 0) {
+                    const int n = 1 << t.log2n;
+                    const int cx = x >> 2, cy = y >> 2;
+                    const int w = ((min(x + n, vis_w) + 3) >> 2) - cx, h = ((min(y + n, vis_h) + 3) >> 2) - cy;
+                    if (w > 0 && h > 0) {
+                        if (w * h <= 4) {
+                            for (int u = 0; u < w * h; ++u) {
+                                const int yy = u >= w ? (u - w >= w ? (u - 2 * w >= w ? 3 : 2) : 1) : 0;
+                                atomicMin(&stamp[(cy + yy) * 16 + cx + u - yy * w], i);
+                            }
+                        } else {
+                            rect = (uint32_t)cx | ((uint32_t)cy << 8) | ((uint32_t)w << 16) | ((uint32_t)h << 24);
+                        }
+                    }
+                }
+            }
+            // larger blocks by the whole warp
+            for (uint32_t m = __ballot_sync(kFull, rect != 0u); m; m &= m - 1u) {
+                const int src = __ffs(m) - 1;
+                const uint32_t r = __shfl_sync(kFull, rect, src);
+                const int cx = (int)(r & 0xffu), cy = (int)((r >> 8) & 0xffu), w = (int)((r >> 16) & 0xffu), h = (int)(r >> 24);
+                for (int u = lane; u < 16 * h; u += 32)
+                    if ((u & 15) < w) atomicMin(&stamp[(cy + (u >> 4)) * 16 + cx + (u & 15)], base + src);
+            }
         }
         // neighbour CTUs that intra prediction may read: same slice and tile
         // (decode.rs:4651-4690)
@@ -2263,58 +2302,69 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             return k;
         };
         __syncthreads();
-        // ---- each walking warp turns the intra TBs of its components into
-        // walk entries, in decode order ----
-        for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
-            const Comp k = comp_of(c);
-            const uint32_t cap = (uint32_t)lay.ent_cap(c);
-            uint4* list = ents + lay.ent_off(c);
-            uint32_t cnt = 0;
-            for (uint32_t base = 0; base < nrec; base += 32) {
-                const uint32_t i = base + lane;
-                bool mine = false;
+        // ---- the intra TBs become walk entries, listed per component in decode
+        // order: one record per thread, its place from ballots within the
+        // warp and the other warps' counts ----
+        uint32_t listed[3] = {0u, 0u, 0u};
+        for (uint32_t base = 0; base < nrec; base += kThreads) {
+            const uint32_t i = base + tid;
+            int tc = -1;
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (i < nrec) {
                 hpvcd_tu t;
-                int x = 0, y = 0;
-                if (i < nrec) {
-                    memcpy(&t, &recs[i], sizeof(t));
-                    if (t.comp == c && (t.flags & HPVCD_TU_INTRA) && intra_pred_ok && rec_check(t, x, y) == 1) {
-                        if (t.mode > 34 || t.log2n > 5)
-                            atomicOr(dev_err, DEV_ERR_BITSTREAM);
-                        else
-                            mine = true;
+                memcpy(&t, &recs[i], sizeof(t));
+                int x, y;
+                if ((t.flags & HPVCD_TU_INTRA) && intra_pred_ok && rec_check(t, x, y) == 1) {
+                    if (t.mode > 34 || t.log2n > 5) {
+                        atomicOr(dev_err, DEV_ERR_BITSTREAM);
+                    } else {
+                        tc = t.comp;
+                        const Comp k = comp_of(tc);
+                        // a chroma TB with cross-component prediction has a
+                        // residual (written by k_ccp) even without coded coefficients
+                        const bool coded = (t.flags & HPVCD_TU_CBF) != 0 || (k.ccp && t.res_scale);
+                        uint32_t f = kFeat && (t.flags & HPVCD_TU_PCM) ? kTbPcm : 0u;
+                        const int n = 1 << t.log2n;
+                        const uint32_t run = (1u << (n >> 2)) - 1u;
+                        uint32_t cov = 0;
+                        if (x + n == k.S) cov |= run << (y >> 2);
+                        if (y + n == k.Sh) cov |= run << (16 + (x >> 2));
+                        if (cov) {
+                            f |= kTbPub;
+                            atomicOr(&s_cov[tc], cov);
+                        }
+                        w = make_entry(k, t, x, y, i, stamp, coded, f);
                     }
                 }
-                const uint32_t m = __ballot_sync(kFull, mine);
-                const uint32_t pos = cnt + __popc(m & ((1u << lane) - 1u));
-                cnt += __popc(m);
-                if (mine && pos < cap) {
-                    // a chroma TB with cross-component prediction has a
-                    // residual (written by k_ccp) even without coded coefficients
-                    const bool coded = (t.flags & HPVCD_TU_CBF) != 0 || (k.ccp && t.res_scale);
-                    uint32_t f = kFeat && (t.flags & HPVCD_TU_PCM) ? kTbPcm : 0u;
-                    const int n = 1 << t.log2n;
-                    const uint32_t run = (1u << (n >> 2)) - 1u;
-                    uint32_t cov = 0;
-                    if (x + n == k.S) cov |= run << (y >> 2);
-                    if (y + n == k.Sh) cov |= run << (16 + (x >> 2));
-                    if (cov) {
-                        f |= kTbPub;
-                        atomicOr(&s_cov[c], cov);
-                    }
-                    list[pos] = make_entry(k, t, x, y, i, stamp, coded, f);
+            }
+            uint32_t pos = 0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const uint32_t m = __ballot_sync(kFull, tc == c);
+                if (tc == c) pos = listed[c] + __popc(m & ((1u << lane) - 1u));
+                if (lane == 0) s_wcnt[3 * warp + c] = (uint32_t)__popc(m);
+            }
+            __syncthreads();
+            for (int v = 0; v < kWarps; ++v)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const uint32_t nv = s_wcnt[3 * v + c];
+                    if (tc == c && v < warp) pos += nv;
+                    listed[c] += nv;
                 }
-            }
-            if (cnt > cap) {
-                if (lane == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
-                cnt = cap;
-            }
-            if (lane == 0) counts[c] = cnt;
+            if (tc >= 0 && pos < (uint32_t)lay.ent_cap(tc)) ents[lay.ent_off(tc) + pos] = w;
+            __syncthreads();  // the counts are read, the entries written
         }
-        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            if (listed[c] > (uint32_t)lay.ent_cap(c)) {
+                if (tid == 0) atomicOr(dev_err, DEV_ERR_BITSTREAM);
+                listed[c] = (uint32_t)lay.ent_cap(c);
+            }
         // A CTU without intra TBs (inter pictures) has its final samples in the
         // plane already: it neither waits for its neighbours nor rewrites
         // anything, it only publishes its edge words.
-        if (!(counts[0] | counts[1] | counts[2])) {
+        if (!(listed[0] | listed[1] | listed[2])) {
             for (int c = 0; c < ncomp; ++c) {
                 const EdgeGeo e = edge_geo(P, c, it.cx, it.cy);
                 const int nr = e.Sh >> 2, nw = nr + (e.S >> 2);
@@ -2339,8 +2389,9 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 const int S = c ? Scw : ctb, Sh = c ? Sch : ctb, ox = c ? ocx : oxl, oy = c ? ocy : oyl;
                 const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
                 uint16_t* can = can_of(c);
+                const int ls = 31 - __clz(S);
                 for (int i = tid; i < S * Sh; i += kThreads) {
-                    const int y = i / S, x = i % S;
+                    const int y = i >> ls, x = i & (S - 1);
                     const int ax = ox + x, ay = oy + y;
                     int v = 0;
                     if (ax < pw && ay < ph) v = load_sample(P.rec[c], P.bps, (size_t)ay * pw + ax);
@@ -2359,25 +2410,87 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             for (int c = 0; c < ncomp; ++c) {
                 const int S = c ? Scw : ctb, Sh = c ? Sch : ctb, ox = c ? ocx : oxl, oy = c ? ocy : oyl;
                 const int rows = min(Sh, (c ? P.ch : P.h) - oy), cols = min(S, (c ? P.cw : P.w) - ox);
-                const int chunks = (cols + 7) >> 3;
+                const int lq = 28 - __clz(S);  // 8-sample chunks of a whole CTU row
                 const int rs = P.res_stride[c];
                 const int16_t* res = P.res[c] + (size_t)oy * rs + ox;
                 uint16_t* can = can_of(c);
-                for (int i = tid; i < rows * chunks; i += kThreads) {
-                    const int r = i / chunks, q = i - r * chunks;
-                    cp_async16(can + can_in(S, 8 * q, r), res + (size_t)r * rs + 8 * q);
+                for (int i = tid; i < rows << lq; i += kThreads) {
+                    const int r = i >> lq, q = i & ((1 << lq) - 1);
+                    if (8 * q < cols) cp_async16(can + can_in(S, 8 * q, r), res + (size_t)r * rs + 8 * q);
                 }
             }
         } else {
             for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
                 const Comp k = comp_of(c);
                 const uint4* list = ents + lay.ent_off(c);
-                for (uint32_t e = lane; e < counts[c]; e += 32) {
+                const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
+                for (uint32_t e = lane; e < cnt; e += 32) {
                     TbEntry E;
                     E.w = list[e];
                     if ((E.w.z & kTbCoded) && !(E.flags() & kTbPcm))
                         stage_residual(k, 31 - __clz(E.n2()) - 1, E.x(), E.y());
                 }
+            }
+        }
+        // ---- how the walk takes each entry, and the blend table: by all warps,
+        // two TBs at a time ----
+        const int half = lane >> 4, l15 = lane & 15;
+        for (int c = 0; c < ncomp; ++c) {
+            const int S = c ? Scw : ctb, row = can_row(S);
+            uint32_t* tab = (uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
+            const uint4* list = ents + lay.ent_off(c);
+            uint8_t* wf = smem + lay.off_wf + lay.ent_off(c);
+            const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
+            // the angular words of the next TB are on their way while one is done
+            auto angles = [&](const TbEntry& E, uint32_t (&ang)[4]) {
+                if (!(E.flags() & kTbPlain)) return;
+                const bool four = E.n2() == 8;
+                const uint32_t* a = (four ? g_angular.t4[E.mode() - 2] : g_angular.t8[E.mode() - 2]) + l15;
+                ang[0] = a[0];
+                if (!four) ang[1] = a[16], ang[2] = a[32], ang[3] = a[48];
+            };
+            uint32_t e = 2 * warp + half;
+            TbEntry E{};
+            uint32_t ang[4] = {0u, 0u, 0u, 0u};
+            if (e < cnt) {
+                E.w = list[e];
+                angles(E, ang);
+            }
+            while (e < cnt) {
+                const TbEntry F{list[min(e + 1, cnt - 1)]};
+                const uint32_t en = e + 2 * kWarps;
+                TbEntry N{};
+                uint32_t ang_n[4] = {0u, 0u, 0u, 0u};
+                if (en < cnt) {
+                    N.w = list[en];
+                    angles(N, ang_n);
+                }
+                const uint32_t f = E.flags();
+                const bool plain = (f & kTbPlain) != 0u, four = E.n2() == 8;
+                if (l15 == 0) {
+                    const bool pair = e + 1 < cnt && plain && four && (F.flags() & kTbPlain) && F.n2() == 8;
+                    const uint32_t g = pair ? f | F.flags() : f;
+                    wf[e] = (uint8_t)((pair ? kWalkPair : (plain && !four ? kWalkPlain8 : 0u)) |
+                                      (g & kTbEdge ? kWalkEdge : 0u) | (g & kTbPub ? kWalkPub : 0u));
+                }
+                if (plain) {
+                    const Line L(E, row);
+                    const bool coded = (E.w.z & kTbCoded) != 0u;
+                    uint32_t* t = tab + E.tab();
+                    if (four) {
+                        t[l15] = blend_word(L, ang[0], coded);
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const int x = l15 & 7, y = 2 * u + (l15 >> 3);
+                            t[((y >> 2) * (S >> 2) + (x >> 2)) * 16 + (y & 3) * 4 + (x & 3)] = blend_word(L, ang[u], coded);
+                        }
+                    }
+                }
+                E = N;
+                e = en;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) ang[u] = ang_n[u];
             }
         }
         cp_async_wait_all();  // this thread's residual copies; the barrier publishes them
@@ -2386,28 +2499,31 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             edge_service(P, it.cx, it.cy, ncomp, can_of, s_cov, s_have, s_done, kWalkers, lane);
         // ---- decode-order walk: each warp reconstructs its components ----
         WalkScratch& ws = *(WalkScratch*)(smem + lay.off_ws + (size_t)min(warp, kWalkers - 1) * kWsBytes);
-        const int half = lane >> 4, l15 = lane & 15;
         for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
             const Comp k = comp_of(c);
-            const uint32_t cnt = counts[c], last = cnt ? cnt - 1 : 0u;
+            const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]), last = cnt ? cnt - 1 : 0u;
             const uint4* list = ents + lay.ent_off(c);
+            const uint8_t* wf = smem + lay.off_wf + lay.ent_off(c);
+            const uint32_t* tab = (const uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
             uint16_t* const can = k.can;
             const int row = can_row(k.S), max_v = k.max_v;
             const bool luma = c == 0;
             unsigned long long* const words = edge_words(P, it.cx, it.cy, c);
             const int px4 = ((lane >> 2) & 3) * row + (lane & 3), px8 = (lane >> 2) * row + 2 * (lane & 3);
+            // this lane's pair of samples in the blend table of an 8x8 TB
+            const int tab8 = ((lane >> 4) * (k.S >> 2) + ((lane >> 1) & 1)) * 16 + ((lane >> 2) & 3) * 4 + 2 * (lane & 1);
             Have have{0u, 0u};
             if (!fine && cnt) have = wait_edges(have, 0xffffffffu, 0xffffffffu, s_have + 2 * c, spin_limit, dev_err, lane);
             // The edge words a TB reads: with x = 0 the left column from row
             // y - 1 on, with y = 0 the row above from sample x - 1 on.
-            auto await = [&](const TbEntry& E, bool active) {
+            auto await = [&](const TbEntry& E) {
                 const int x = E.x(), y = E.y(), n2 = E.n2();
                 uint32_t need_top = 0u, need_left = 0u;
-                if (active && y == 0) {
+                if (y == 0) {
                     const int lo = max(x - 1, 0) >> 2, hi = (x + n2) >> 2;
                     need_top = (0xffffffffu >> (32 - (hi - lo))) << lo;
                 }
-                if (active && x == 0) {
+                if (x == 0) {
                     const int lo = max(y - 1, 0) >> 2, hi = min(y + n2, k.Sh) >> 2;
                     need_left = ((1u << (hi - lo)) - 1u) << lo;
                     if (y == 0) need_left |= kHaveCorner;
@@ -2417,63 +2533,54 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 if (need_top | need_left)
                     have = wait_edges(have, need_top, need_left, s_have + 2 * c, spin_limit, dev_err, lane);
             };
-            // Lanes 0..15 hold TB e, lanes 16..31 TB e + 1.  Two plain 4x4 TBs
-            // share the arithmetic of their addresses and weights (half of a
-            // 4x4 TB's instructions), each half-warp then predicts its own
-            // TB, the second after the first is stored.
-            TbEntry H;
-            uint2 lut = make_uint2(0u, 0u);
-            auto lut_at = [&](uint32_t row_of, int l) { return __ldg((const uint2*)&g_angular + row_of + l); };
+            // Plain 4x4 TBs are taken in pairs: lanes 0..15 hold TB e, lanes
+            // 16..31 TB e + 1, predicted after TB e is stored.  The pair's
+            // blend words and place are loaded an iteration ahead.
+            uint32_t how = 0, bw = 0;
+            int org = 0;
+            auto fetch = [&](uint32_t e) { return *(const uint2*)&list[min(e + half, last)]; };
             if (cnt) {
-                H.w = list[min((uint32_t)half, last)];
-                lut = lut_at(H.lut(), l15);
+                const uint2 h = fetch(0);
+                org = (int)(h.x & 0xffffu);
+                bw = tab[(h.y >> 16) + l15];
+                how = wf[0];
             }
             for (uint32_t e = 0; e < cnt;) {
-                const bool plain4 = (H.flags() & kTbPlain) && H.n2() == 8;
-                const uint32_t b4 = __ballot_sync(kFull, plain4);
-                uint32_t next;
-                if (b4 & 1u) {
-                    const bool two = (b4 >> 16) && e < last;
-                    const bool active = two || half == 0;
-                    next = e + (two ? 2u : 1u);
-                    if (__any_sync(kFull, active && (H.flags() & kTbEdge))) await(H, active);
-                    const int lo = H.lo(), hi = H.hi(), l0 = H.line0(), c0 = H.corner() - 8;
-                    const int q0 = min(max((int)(lut.x & 0xffu), lo), hi), q1 = min(max((int)((lut.x >> 8) & 0xffu), lo), hi);
-                    const uint16_t* r0 = can + (q0 < 8 ? l0 - q0 * row : c0 + q0);
-                    const uint16_t* r1 = can + (q1 < 8 ? l0 - q1 * row : c0 + q1);
-                    uint16_t* const px = can + H.org() + px4;
-                    const int w0 = (int)(lut.x >> 24), w1 = (int)((lut.x >> 16) & 0xffu);
-                    int rv = 0, s = 0;
-                    if (plain4) {  // (the other half's TB may be of another kind: its addresses mean nothing here)
-                        if (H.w.z & kTbCoded) rv = (int)(int16_t)*px;
-                        s = __viaddmin_s32_relu((w0 * *r0 + w1 * *r1 + 16) >> 5, rv, max_v);
-                        if (half == 0) *px = (uint16_t)s;
-                    }
-                    TbEntry N;
-                    N.w = list[min(next + half, last)];
+                if (how & kWalkPair) {
+                    if (how & kWalkEdge) await(TbEntry{list[e + half]});
+                    uint16_t* const px = can + org + px4;
+                    const int rv = (bw & 1u) ? (int)(int16_t)*px : 0;
+                    int s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);
+                    if (half == 0) *px = (uint16_t)s;
+                    const uint2 h = fetch(e + 2);
+                    const uint32_t hn = wf[min(e + 2, last)];
                     __syncwarp();
-                    if (two) {
-                        s = __viaddmin_s32_relu((w0 * *r0 + w1 * *r1 + 16) >> 5, rv, max_v);
-                        if (half) *px = (uint16_t)s;
-                    }
-                    lut = lut_at(N.lut(), l15);
-                    if (__any_sync(kFull, active && (H.flags() & kTbPub)) && active) {  // samples on the right column / bottom row
+                    s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
+                    if (half) *px = (uint16_t)s;
+                    org = (int)(h.x & 0xffffu);
+                    bw = tab[(h.y >> 16) + l15];
+                    if (how & kWalkPub) {  // samples on the CTU's right column / bottom row
+                        const TbEntry E{list[e + half]};
                         uint16_t* const w16 = (uint16_t*)words;
-                        const int x = H.x() + (lane & 3), y = H.y() + (l15 >> 2);
+                        const int x = E.x() + (lane & 3), y = E.y() + (l15 >> 2);
                         const uint16_t t = (uint16_t)(s | 0x8000);
                         if (x == k.S - 1) st_edge16(w16 + y, t);
                         if (y == k.Sh - 1) st_edge16(w16 + k.Sh + x, t);
                     }
+                    how = hn;
+                    e += 2;
                     __syncwarp();
-                    H = N;
+                    continue;
+                }
+                TbEntry E{list[e]};
+                if (how & kWalkEdge) await(E);
+                const int n2 = E.n2();
+                if (how & kWalkPlain8) {
+                    walk_plain8(can, (uint32_t*)(can + E.org() + px8), *(const uint2*)(tab + E.tab() + tab8), max_v);
                 } else {
-                    TbEntry E;
-                    E.w = list[e];
-                    next = e + 1;
                     const uint32_t f = E.flags();
-                    const int n2 = E.n2(), mode = E.mode();
+                    const int mode = E.mode();
                     int stride = row;
-                    if (f & kTbEdge) await(E, true);
                     if (f & kTbGather) {
                         gather_line(k, 31 - __clz(n2) - 1, E.x(), E.y(), stamp, E.jrec(), ws, lane);
                         const uint32_t at = (uint32_t)(ws.s - can);  // position i at canvas offset at + i
@@ -2487,27 +2594,24 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                         pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
                     } else if (n2 == 8) {
                         // positions past the line clamp to its last one
-                        const uint2 lu = lut_at(E.lut(), l15);
-                        walk_tb4(can + E.org() + px4, mode, coded, luma, max_v, can[L.at(lane)], lu.x, lane);
+                        walk_tb4(can + E.org() + px4, mode, coded, luma, max_v, can[L.at(lane)],
+                                 g_angular.t4[max(mode - 2, 0)][l15], lane);
                     } else if (n2 == 16) {
-                        const uint2 lu = lut_at(E.lut(), lane);
-                        uint32_t* const px = (uint32_t*)(can + E.org() + px8);
-                        if (f & kTbPlain) {
-                            walk_plain8(can, L, px, coded, max_v, lu);
-                        } else {
-                            const bool hi_ok = (f & kTbHi32) != 0u;
-                            walk_tb8(px, mode, coded, filt, luma, max_v, can[L.at(lane)], hi_ok ? can[E.corner() + 16] : 0,
-                                     hi_ok, lu, lane);
-                        }
+                        const bool hi_ok = (f & kTbHi32) != 0u;
+                        walk_tb8((uint32_t*)(can + E.org() + px8), mode, coded, filt, luma, max_v, can[L.at(lane)],
+                                 hi_ok ? can[E.corner() + 16] : 0, hi_ok,
+                                 *(const uint2*)&g_angular.t8[max(mode - 2, 0)][2 * lane], lane);
                     } else {
-                        walk_tb_big(can, row, L, E.org(), 31 - __clz(n2) - 1, mode, coded, filt, luma, k.strong, k.bd, ws,
-                                    lane);
+                        walk_tb_big(can, row, L, E.org(), mode, coded, filt, luma, k.strong, k.bd, ws, lane);
                     }
-                    H.w = list[min(next + half, last)];
-                    lut = lut_at(H.lut(), l15);
-                    if (f & kTbPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
                 }
-                e = next;
+                const uint32_t was = how;
+                ++e;
+                const uint2 h = fetch(e);
+                how = wf[min(e, last)];
+                org = (int)(h.x & 0xffffu);
+                bw = tab[(h.y >> 16) + l15];
+                if (was & kWalkPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
             }
         }
         if (warp < kWalkers && lane == 0) *(volatile uint32_t*)&s_done[warp] = 1u;
@@ -2520,9 +2624,10 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             const uint16_t* can = can_of(c);
             const int rows = min(Sh, ph - oy), cols = min(S, pw - ox);
             if ((pw & 7) == 0 && (cols & 7) == 0) {
-                const int chunks = cols >> 3;
-                for (int i = tid; i < rows * chunks; i += kThreads) {
-                    const int y = i / chunks, q = i % chunks;
+                const int lq = 28 - __clz(S);
+                for (int i = tid; i < rows << lq; i += kThreads) {
+                    const int y = i >> lq, q = i & ((1 << lq) - 1);
+                    if (8 * q >= cols) continue;
                     const uint4 v = *(const uint4*)(can + can_in(S, 8 * q, y));
                     const size_t off = (size_t)(oy + y) * pw + ox + 8 * q;
                     if (P.bps == 2) {
