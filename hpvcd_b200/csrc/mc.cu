@@ -40,11 +40,23 @@ __device__ __forceinline__ int dot2hi(uint32_t a, uint32_t b, int c) {
     return d;
 }
 
+// The same words column by column, the picture's first and last column
+// repeated (rare, and kept out of the unrolled rows: the kernel's code already
+// fills the instruction cache).
+template <int TAPS, int BPS>
+__device__ __noinline__ uint4 fetch_clamped(const void* plane, int pw, int x, int y) {
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    const size_t row = (size_t)y * pw;
+#pragma unroll
+    for (int i = 0; i < TAPS; ++i)
+        w[i * BPS / 4] |= (uint32_t)load_sample(plane, BPS, row + clamp3i(x + i, 0, pw - 1)) << (8 * BPS * (i & (4 / BPS - 1)));
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // TAPS samples of a row starting at column x, packed in words (four 8-bit or
 // two 16-bit samples each).  Inside the picture by aligned 32-bit loads (rows
 // and planes are multiples of four samples from an aligned start, so a word
-// holding a sample of the plane lies inside it), else column by column with
-// the picture's first and last column repeated.
+// holding a sample of the plane lies inside it).
 template <int TAPS, int BPS>
 __device__ __forceinline__ void fetch_row(const void* plane, int pw, int x, int y, bool inside,
                                           uint32_t (&w)[TAPS * BPS / 4]) {
@@ -60,14 +72,10 @@ __device__ __forceinline__ void fetch_row(const void* plane, int pw, int x, int 
 #pragma unroll
         for (int i = 0; i < W; ++i) w[i] = __funnelshift_r(r[i], r[i + 1], sh);
     } else {
-        const size_t row = (size_t)y * pw;
+        const uint4 v = fetch_clamped<TAPS, BPS>(plane, pw, x, y);
+        const uint32_t t[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int i = 0; i < W; ++i) {
-            w[i] = 0u;
-#pragma unroll
-            for (int u = 0; u < 4 / BPS; ++u)
-                w[i] |= (uint32_t)load_sample(plane, BPS, row + clamp3i(x + i * (4 / BPS) + u, 0, pw - 1)) << (8 * BPS * u);
-        }
+        for (int i = 0; i < W; ++i) w[i] = t[i];
     }
 }
 
@@ -118,9 +126,9 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
     const int pw = luma ? P.w : P.cw, ph = luma ? P.h : P.ch;
     const int bd = luma ? P.bd : P.bd_c;
     const int mx = (1 << bd) - 1;
-    int a[ROWS], b[ROWS];
+    int a[ROWS], b[ROWS];  // the lists found, in turn
     int have = 0;
-#pragma unroll
+#pragma unroll 1
     for (int l = 0; l < 2; ++l) {  // reference views per list (decode.rs:7040-7120 ref_frame_for_lists)
         if (!(u.flags & (l ? HPVCD_PU_L1 : HPVCD_PU_L0))) continue;
         const int ri = u.ref_idx[l];
@@ -139,7 +147,13 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
             ix = mvcx >> 3, iy = mvcy >> 3;
             fx = mvcx & 7, fy = mvcy & 7;
         }
-        interp_column<TAPS, ROWS, BPS>(pics[rp].fin[c], pw, ph, x + ix, y + iy, fx, fy, bd, l ? b : a);
+        int t[ROWS];
+        interp_column<TAPS, ROWS, BPS>(pics[rp].fin[c], pw, ph, x + ix, y + iy, fx, fy, bd, t);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            b[r] = t[r];
+            if (l == 0) a[r] = t[r];
+        }
     }
     const int denom = P.has_wp ? (luma ? P.wp.luma_log2_denom : P.wp.chroma_log2_denom) : 0;
     auto wpair = [&](int l, int& wgt, int& off) {
@@ -198,7 +212,7 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
 // (kMcSplit CTAs interleave, so that a run of large PUs does not end up on one
 // SM).  A warp takes four tiles of luma, or of both chroma components, at a
 // time.
-constexpr int kMcPus = 16, kMcSplit = 4, kMcWarps = 8;
+constexpr int kMcPus = 32, kMcSplit = 8, kMcWarps = 8;
 
 template <int BPS>
 __device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, const hpvcd_pu* s_pu, const uint32_t* s_pre) {
@@ -239,7 +253,7 @@ __device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, cons
     }
 }
 
-__global__ void __launch_bounds__(32 * kMcWarps) k_mc(const DevPic* __restrict__ pics, int pic_index) {
+__global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restrict__ pics, int pic_index) {
     __shared__ hpvcd_pu s_pu[kMcPus];
     __shared__ uint32_t s_pre[kMcPus + 1];  // tiles of the PUs before
     const DevPic& P = pics[pic_index];

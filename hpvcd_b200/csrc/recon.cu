@@ -1877,23 +1877,25 @@ __device__ __forceinline__ uint32_t add_clip2(uint32_t pred, uint32_t res, int m
     return __viaddmin_s16x2_relu(pred, res, (uint32_t)max_v * 0x10001u);
 }
 
-// 4x4 intra TB: v is line position `lane` (lanes 0..16), lut the lane's entry
-// of the angular table (prediction intra.rs:257-372, no filtering of 4x4
+// 4x4 intra TB that is not plain: v is line position `lane` (lanes 0..16;
+// prediction intra.rs:257-372, no filtering of 4x4
 // lines, intra.rs:174), lanes 0..15 one sample each, at px.
-__device__ __forceinline__ void walk_tb4(uint16_t* px, int mode, bool coded, bool luma, int max_v, int v, uint32_t lut,
-                                         int lane) {
+__device__ __forceinline__ void walk_tb4(uint16_t* px, int mode, bool coded, bool luma, int max_v, int v, int lane) {
     constexpr int n = 4, n2 = 8;
     const int yy = (lane >> 2) & 3, xx = lane & 3;
     const int rv = coded ? (int)(int16_t)*px : 0;
     int pred;
     if (mode >= 2) {
-        const int r0 = __shfl_sync(kFull, v, (int)lut), r1 = __shfl_sync(kFull, v, (int)(lut >> 8));
-        pred = (int)((lut >> 24) * (uint32_t)r0 + ((lut >> 16) & 0xffu) * (uint32_t)r1 + 16u) >> 5;
-        if (luma && (mode == 26 || mode == 10)) {  // vertical / horizontal edge filter (n < 32)
+        if (luma && (mode == 26 || mode == 10)) {  // straight, with the vertical / horizontal edge filter (n < 32)
+            pred = __shfl_sync(kFull, v, mode == 26 ? n2 + xx + 1 : n2 - yy - 1);
             const int c0 = __shfl_sync(kFull, v, n2);
             const int a0 = __shfl_sync(kFull, v, mode == 26 ? n2 + 1 : n2 - 1);
             const int e = __shfl_sync(kFull, v, mode == 26 ? n2 - (yy + 1) : n2 + xx + 1);
             if (mode == 26 ? xx == 0 : yy == 0) pred = clamp3i(a0 + ((e - c0) >> 1), 0, max_v);
+        } else {  // a gathered line
+            const uint32_t lut = g_angular.t4[mode - 2][lane & 15];
+            const int r0 = __shfl_sync(kFull, v, (int)lut), r1 = __shfl_sync(kFull, v, (int)(lut >> 8));
+            pred = (int)((lut >> 24) * (uint32_t)r0 + ((lut >> 16) & 0xffu) * (uint32_t)r1 + 16u) >> 5;
         }
     } else if (mode == 1) {  // DC
         const int part = ((lane >= n2 - n && lane < n2) || (lane > n2 && lane <= n2 + n)) ? v : 0;
@@ -1987,7 +1989,7 @@ __device__ __forceinline__ void walk_plain8(const uint16_t* can, uint32_t* px, u
     __syncwarp();
 }
 
-// 16x16 or 32x32 intra TB by one warp, two horizontally adjacent samples per
+// 16x16 or 32x32 intra TB by one warp, four horizontally adjacent samples per
 // lane and row step.  First the line samples the prediction reads, filtered
 // (intra.rs:151-219), go to the scratch: the projected references, each with
 // the next one, or for planar and DC the line from the sample below the left
@@ -1996,7 +1998,7 @@ __device__ __forceinline__ void walk_plain8(const uint16_t* can, uint32_t* px, u
 // wait for instructions first (unrolled by four the same batch took 8 % more).
 __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& L, int org, int mode, bool coded,
                                             bool filt, bool luma, bool strong_on, int bd, WalkScratch& ws, int lane) {
-    const int n2 = L.n2, n = n2 >> 1, hl = 30 - __clz(n);  // hl: log2 of the pairs per row
+    const int n2 = L.n2, n = n2 >> 1, hl = 29 - __clz(n);  // hl: log2 of the lanes per row
     const int max_v = (1 << bd) - 1;
     auto raw = [&](int i) { return (int)can[L.at(i)]; };
     const bool angular = mode >= 2, vertical = mode >= 18;
@@ -2031,60 +2033,81 @@ __device__ __forceinline__ void walk_tb_big(uint16_t* can, int row, const Line& 
             ws.f[q] = (uint16_t)v;
         }
     }
-    // this lane's column pair, first row and rows per step
-    const int x = 2 * (lane & ((1 << hl) - 1)), ys = 32 >> hl;
+    // this lane's columns, first row and rows per step
+    const int x = 4 * (lane & ((1 << hl) - 1)), y0 = lane >> hl, ys = 32 >> hl;
     const bool edge = luma && n < 32;
-    uint32_t* px = (uint32_t*)(can + org + (lane >> hl) * row + x);  // canvas rows and TB columns are even
-    const int step = (ys * row) >> 1;
-    auto put = [&](int p0, int p1) {
-        *px = add_clip2((uint32_t)p0 | ((uint32_t)p1 << 16), coded ? *px : 0u, max_v);
+    uint2* px = (uint2*)(can + org + y0 * row + x);  // canvas rows and TB columns are multiples of four
+    const int step = (ys * row) >> 2;
+    auto put = [&](int p0, int p1, int p2, int p3) {
+        const uint2 r = coded ? *px : make_uint2(0u, 0u);
+        *px = make_uint2(add_clip2(__byte_perm((uint32_t)p0, (uint32_t)p1, 0x5410), r.x, max_v),
+                         add_clip2(__byte_perm((uint32_t)p2, (uint32_t)p3, 0x5410), r.y, max_v));
         px += step;
     };
     __syncwarp();
     if (angular) {
         // Sample (x, y) blends references idx and idx + 1 by frac, idx * 32 +
         // frac = 32 b + (a + 1) angle, b along the edge and a away from it.
-        int pos = vertical ? 32 * x + ((lane >> hl) + 1) * angle : 32 * (lane >> hl) + (x + 1) * angle;
-        const int dx = vertical ? 32 : angle, dy = vertical ? ys * angle : ys * 32;
-        pos += 32 * (1 - k0);
-        const bool filter0 = edge && angle == 0;  // modes 10 and 26: their first row / column
-        auto blend = [&](int at) {  // ((32 - f) r[k] + f r[k + 1] + 16) >> 5
-            return __dp2a_lo((int)ws.pairs[at >> 5], 32 + (at & 31) * 255, 16) >> 5;
-        };
+        auto blend = [](uint32_t pair, int weights) { return __dp2a_lo((int)pair, weights, 16) >> 5; };
+        auto weights = [](int pos) { return 32 + (pos & 31) * 255; };  // 32 - f | f << 8
+        const uint32_t* const refs = ws.pairs + 1 - k0;
+        if (edge && angle == 0) {  // modes 10 and 26: the first row / column is filtered
+            const int c0 = raw(n2), a0 = raw(vertical ? n2 + 1 : n2 - 1);
 #pragma unroll 1
-        for (int y = lane >> hl; y < n; y += ys, pos += dy) {
-            int p0 = blend(pos), p1 = blend(pos + dx);
-            if (filter0 && (vertical ? x == 0 : y == 0)) {
-                const int c0 = raw(n2), a0 = raw(vertical ? n2 + 1 : n2 - 1);
-                p0 = clamp3i(a0 + ((raw(vertical ? n2 - (y + 1) : n2 + x + 1) - c0) >> 1), 0, max_v);
-                if (!vertical) p1 = clamp3i(a0 + ((raw(n2 + x + 2) - c0) >> 1), 0, max_v);
+            for (int y = y0; y < n; y += ys) {
+                int p[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const bool first = vertical ? x + u == 0 : y == 0;
+                    p[u] = (int)(refs[vertical ? x + u : y] & 0xffffu);
+                    if (first) p[u] = clamp3i(a0 + ((raw(vertical ? n2 - (y + 1) : n2 + x + u + 1) - c0) >> 1), 0, max_v);
+                }
+                put(p[0], p[1], p[2], p[3]);
             }
-            put(p0, p1);
+        } else if (vertical) {
+            int pos = (y0 + 1) * angle;
+#pragma unroll 1
+            for (int y = y0; y < n; y += ys, pos += ys * angle) {
+                const uint32_t* r = refs + x + (pos >> 5);
+                const int w = weights(pos);
+                put(blend(r[0], w), blend(r[1], w), blend(r[2], w), blend(r[3], w));
+            }
+        } else {
+            const int pa = (x + 1) * angle, pb = pa + angle, pc = pb + angle, pd = pc + angle;
+            const int wa = weights(pa), wb = weights(pb), wc = weights(pc), wd = weights(pd);
+            const uint32_t* r = refs + y0;
+            const int ia = pa >> 5, ib = pb >> 5, ic = pc >> 5, id = pd >> 5;
+#pragma unroll 1
+            for (int y = y0; y < n; y += ys, r += ys) put(blend(r[ia], wa), blend(r[ib], wb), blend(r[ic], wc), blend(r[id], wd));
         }
     } else {
         // ws.f: below-left, left column upwards, corner, row above, above-right
         const uint16_t* const left = ws.f + n;       // left[-y]
         const uint16_t* const above = ws.f + n + 2;  // above[x]
-        const int dc = mode == 1 ? (int)(__reduce_add_sync(kFull, lane < n ? (unsigned)above[lane] + left[-lane] : 0u) + n) >> (hl + 2)
+        const int dc = mode == 1 ? (int)(__reduce_add_sync(kFull, lane < n ? (unsigned)above[lane] + left[-lane] : 0u) + n) >> (hl + 3)
                                  : 0;
-        const int ab0 = above[x], ab1 = above[x + 1], rt = above[n], lb = left[-n];
+        const int rt = above[n], lb = left[-n];
+        int ab[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) ab[u] = above[x + u];
 #pragma unroll 1
-        for (int y = lane >> hl; y < n; y += ys) {
+        for (int y = y0; y < n; y += ys) {
             const int lf = left[-y];
-            int p0 = dc, p1 = dc;
+            int q[4] = {dc, dc, dc, dc};
             if (mode == 0) {  // planar
                 const int vb = (y + 1) * lb + n, up = n - 1 - y;
-                p0 = ((n - 1 - x) * lf + (x + 1) * rt + up * ab0 + vb) >> (hl + 2);
-                p1 = ((n - 2 - x) * lf + (x + 2) * rt + up * ab1 + vb) >> (hl + 2);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) q[u] = ((n - 1 - x - u) * lf + (x + u + 1) * rt + up * ab[u] + vb) >> (hl + 3);
             } else if (edge) {
                 if (y == 0) {
-                    p0 = x == 0 ? (lf + 2 * dc + ab0 + 2) >> 2 : (ab0 + 3 * dc + 2) >> 2;
-                    p1 = (ab1 + 3 * dc + 2) >> 2;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) q[u] = (ab[u] + 3 * dc + 2) >> 2;
+                    if (x == 0) q[0] = (lf + 2 * dc + ab[0] + 2) >> 2;
                 } else if (x == 0) {
-                    p0 = (lf + 3 * dc + 2) >> 2;
+                    q[0] = (lf + 3 * dc + 2) >> 2;
                 }
             }
-            put(p0, p1);
+            put(q[0], q[1], q[2], q[3]);
         }
     }
     __syncwarp();
@@ -2141,10 +2164,10 @@ __host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 // availability, coded and PCM tests compile to the plain form.  fine: a TB
 // waits for the edge words it reads; otherwise a CTU waits for all of its
 // neighbours' words before its walk.
-// How the walk takes the TB at an entry: it and the next one are plain 4x4
-// TBs, it is a plain 8x8 TB, it (or the pair) reads neighbour CTUs / covers
-// edge words.
-constexpr uint32_t kWalkPair = 1u, kWalkPlain8 = 2u, kWalkEdge = 4u, kWalkPub = 8u;
+// How the walk takes the TB at an entry: it is a plain 4x4 TB (kWalkTwo: the
+// next one too), a plain 8x8 TB; it (or the pair) reads neighbour CTUs /
+// covers edge words.
+constexpr uint32_t kWalkPlain4 = 1u, kWalkPlain8 = 2u, kWalkEdge = 4u, kWalkPub = 8u, kWalkTwo = 16u;
 
 template <int kCW, bool kFeat>
 __global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 5 : 4)
@@ -2389,13 +2412,19 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 const int S = c ? Scw : ctb, Sh = c ? Sch : ctb, ox = c ? ocx : oxl, oy = c ? ocy : oyl;
                 const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
                 uint16_t* can = can_of(c);
-                const int ls = 31 - __clz(S);
-                for (int i = tid; i < S * Sh; i += kThreads) {
-                    const int y = i >> ls, x = i & (S - 1);
+                const int lq = 28 - __clz(S);  // 8-sample chunks of a row; plane widths are multiples of four
+                for (int i = tid; i < Sh << lq; i += kThreads) {
+                    const int y = i >> lq, x = 8 * (i & ((1 << lq) - 1));
                     const int ax = ox + x, ay = oy + y;
-                    int v = 0;
-                    if (ax < pw && ay < ph) v = load_sample(P.rec[c], P.bps, (size_t)ay * pw + ax);
-                    can[can_in(S, x, y)] = (uint16_t)v;
+                    int v[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+                    if (ay < ph) {
+                        const size_t at = (size_t)ay * pw + ax;
+                        if (ax < pw) ld_row4(P.rec[c], P.bps, at, v[0]);
+                        if (ax + 4 < pw) ld_row4(P.rec[c], P.bps, at + 4, v[1]);
+                    }
+                    *(uint4*)(can + can_in(S, x, y)) =
+                        make_uint4((uint32_t)(v[0][0] | (v[0][1] << 16)), (uint32_t)(v[0][2] | (v[0][3] << 16)),
+                                   (uint32_t)(v[1][0] | (v[1][1] << 16)), (uint32_t)(v[1][2] | (v[1][3] << 16)));
                 }
             }
         }
@@ -2470,7 +2499,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 if (l15 == 0) {
                     const bool pair = e + 1 < cnt && plain && four && (F.flags() & kTbPlain) && F.n2() == 8;
                     const uint32_t g = pair ? f | F.flags() : f;
-                    wf[e] = (uint8_t)((pair ? kWalkPair : (plain && !four ? kWalkPlain8 : 0u)) |
+                    wf[e] = (uint8_t)((plain ? (four ? kWalkPlain4 : kWalkPlain8) : 0u) | (pair ? kWalkTwo : 0u) |
                                       (g & kTbEdge ? kWalkEdge : 0u) | (g & kTbPub ? kWalkPub : 0u));
                 }
                 if (plain) {
@@ -2546,20 +2575,25 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 how = wf[0];
             }
             for (uint32_t e = 0; e < cnt;) {
-                if (how & kWalkPair) {
-                    if (how & kWalkEdge) await(TbEntry{list[e + half]});
+                if (how & kWalkPlain4) {
+                    const bool two = (how & kWalkTwo) != 0u;
+                    const uint32_t next = e + (two ? 2u : 1u);
+                    if (how & kWalkEdge) await(TbEntry{list[two ? e + half : e]});
                     uint16_t* const px = can + org + px4;
+                    // (without a second TB lanes 16..31 hold another kind of TB's word: table offset 0, read only)
                     const int rv = (bw & 1u) ? (int)(int16_t)*px : 0;
                     int s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);
                     if (half == 0) *px = (uint16_t)s;
-                    const uint2 h = fetch(e + 2);
-                    const uint32_t hn = wf[min(e + 2, last)];
+                    const uint2 h = fetch(next);
+                    const uint32_t hn = wf[min(next, last)];
                     __syncwarp();
-                    s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
-                    if (half) *px = (uint16_t)s;
+                    if (two) {
+                        s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
+                        if (half) *px = (uint16_t)s;
+                    }
                     org = (int)(h.x & 0xffffu);
                     bw = tab[(h.y >> 16) + l15];
-                    if (how & kWalkPub) {  // samples on the CTU's right column / bottom row
+                    if ((how & kWalkPub) && (two || half == 0)) {  // samples on the CTU's right column / bottom row
                         const TbEntry E{list[e + half]};
                         uint16_t* const w16 = (uint16_t*)words;
                         const int x = E.x() + (lane & 3), y = E.y() + (l15 >> 2);
@@ -2568,10 +2602,12 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                         if (y == k.Sh - 1) st_edge16(w16 + k.Sh + x, t);
                     }
                     how = hn;
-                    e += 2;
+                    e = next;
                     __syncwarp();
                     continue;
                 }
+                const uint2 h = fetch(e + 1);
+                const uint32_t hn = wf[min(e + 1, last)];
                 TbEntry E{list[e]};
                 if (how & kWalkEdge) await(E);
                 const int n2 = E.n2();
@@ -2594,8 +2630,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                         pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
                     } else if (n2 == 8) {
                         // positions past the line clamp to its last one
-                        walk_tb4(can + E.org() + px4, mode, coded, luma, max_v, can[L.at(lane)],
-                                 g_angular.t4[max(mode - 2, 0)][l15], lane);
+                        walk_tb4(can + E.org() + px4, mode, coded, luma, max_v, can[L.at(lane)], lane);
                     } else if (n2 == 16) {
                         const bool hi_ok = (f & kTbHi32) != 0u;
                         walk_tb8((uint32_t*)(can + E.org() + px8), mode, coded, filt, luma, max_v, can[L.at(lane)],
@@ -2607,8 +2642,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 }
                 const uint32_t was = how;
                 ++e;
-                const uint2 h = fetch(e);
-                how = wf[min(e, last)];
+                how = hn;
                 org = (int)(h.x & 0xffffu);
                 bw = tab[(h.y >> 16) + l15];
                 if (was & kWalkPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
