@@ -258,6 +258,166 @@ __device__ void chroma_segment(const DevPic& P, bool vertical, int edge, int sca
     }
 }
 
+// ---- the same segments of a staged tile (SPlane), in registers: a segment's
+// samples are its own within a pass, so all of them are loaded and stored as
+// four-sample vectors (one thread, 4 lines x 8 taps of luma, 4 x 4 of chroma)
+// instead of one shared-memory access per tap and line. ----
+
+// tap k (0..7: p3 .. p0, q0 .. q3) of line l from the vectors of a segment
+template <bool kVertical>
+__device__ __forceinline__ int seg_get(const uint2 (&v)[8], int l, int k) {
+    const uint2 w = kVertical ? v[2 * l + (k >> 2)] : v[k];
+    const int h = kVertical ? k & 3 : l;
+    const uint32_t x = h < 2 ? w.x : w.y;
+    return (int)(h & 1 ? x >> 16 : x & 0xffffu);
+}
+template <bool kVertical>
+__device__ __forceinline__ void seg_set(uint2 (&v)[8], int l, int k, int val) {
+    uint2& w = kVertical ? v[2 * l + (k >> 2)] : v[k];
+    const int h = kVertical ? k & 3 : l;
+    uint32_t& x = h < 2 ? w.x : w.y;
+    x = h & 1 ? __byte_perm(x, (uint32_t)val, 0x5410) : __byte_perm(x, (uint32_t)val, 0x3254);
+}
+
+template <bool kVertical, class Cl>
+__device__ __forceinline__ void luma_segment_tile(const DevPic& P, int edge, int scan, const SPlane& pl, const Cl& cl,
+                                                  bool any_exempt) {
+    const int mid = scan + 1;
+    const hpvcd_cell q = kVertical ? cl.at(edge >> 2, mid >> 2) : cl.at(mid >> 2, edge >> 2);
+    const int bs = kVertical ? q.bs_v : q.bs_h;
+    if (bs == 0) return;
+    const int qp_p = kVertical ? qp_of(P, cl, edge - 1, mid) : qp_of(P, cl, mid, edge - 1);
+    const int avg = (qp_p + q.qp_y + 1) >> 1;
+    const int sh = P.bd - 8;
+    int bo, to;
+    slice_offsets(P, kVertical ? edge : mid, kVertical ? mid : edge, &bo, &to);
+    const int beta = c_beta[clamp3i(avg + 2 * bo, 0, 51)] << sh;
+    const int tc = c_tc[clamp3i(avg + 2 * (bs - 1) + 2 * to, 0, 53)] << sh;
+    if (tc == 0) return;
+    uint16_t* const base = pl.s + (kVertical ? (scan - pl.y0) * pl.rw + edge - 4 - pl.x0 : (edge - 4 - pl.y0) * pl.rw + scan - pl.x0);
+    uint2 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        v[i] = *(const uint2*)(base + (kVertical ? (i >> 1) * pl.rw + 4 * (i & 1) : i * pl.rw));
+    // deblock.rs:216-238 luma_decision (lines 0 and 3)
+    int dp[2], dq[2];
+    bool sam[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int l = 3 * k;
+        const int p3 = seg_get<kVertical>(v, l, 0), p2 = seg_get<kVertical>(v, l, 1), p1 = seg_get<kVertical>(v, l, 2),
+                  p0 = seg_get<kVertical>(v, l, 3), q0 = seg_get<kVertical>(v, l, 4), q1 = seg_get<kVertical>(v, l, 5),
+                  q2 = seg_get<kVertical>(v, l, 6), q3 = seg_get<kVertical>(v, l, 7);
+        dp[k] = abs(p2 - 2 * p1 + p0);
+        dq[k] = abs(q2 - 2 * q1 + q0);
+        sam[k] = 2 * (dp[k] + dq[k]) < (beta >> 2) && abs(p3 - p0) + abs(q0 - q3) < (beta >> 3) &&
+                 abs(p0 - q0) < ((5 * tc + 1) >> 1);
+    }
+    if (dp[0] + dp[1] + dq[0] + dq[1] >= beta) return;
+    const bool strong = sam[0] && sam[1];
+    const int side_thr = (beta + (beta >> 1)) >> 3;
+    const bool do_p1 = dp[0] + dp[1] < side_thr, do_q1 = dq[0] + dq[1] < side_thr;
+    const int maxv = (1 << P.bd) - 1;
+    // exemption of the P / Q side (whole 4x4 cells)
+    const bool ex_p = any_exempt && (kVertical ? exempt_of(cl, edge - 1, mid) : exempt_of(cl, mid, edge - 1));
+    const bool ex_q = (q.flags & HPVCD_CELL_EXEMPT) != 0;
+    const int tc2 = tc >> 1;
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+        const int p2 = seg_get<kVertical>(v, l, 1), p1 = seg_get<kVertical>(v, l, 2), p0 = seg_get<kVertical>(v, l, 3);
+        const int q0 = seg_get<kVertical>(v, l, 4), q1 = seg_get<kVertical>(v, l, 5), q2 = seg_get<kVertical>(v, l, 6);
+        if (strong) {  // deblock.rs:605-616
+            const int p3 = seg_get<kVertical>(v, l, 0), q3 = seg_get<kVertical>(v, l, 7);
+            auto c = [&](int o, int x) { return clamp3i(clamp3i(x, o - 2 * tc, o + 2 * tc), 0, maxv); };
+            if (!ex_p) {
+                seg_set<kVertical>(v, l, 3, c(p0, (p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3));
+                seg_set<kVertical>(v, l, 2, c(p1, (p2 + p1 + p0 + q0 + 2) >> 2));
+                seg_set<kVertical>(v, l, 1, c(p2, (2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3));
+            }
+            if (!ex_q) {
+                seg_set<kVertical>(v, l, 4, c(q0, (p1 + 2 * p0 + 2 * q0 + 2 * q1 + q2 + 4) >> 3));
+                seg_set<kVertical>(v, l, 5, c(q1, (p0 + q0 + q1 + q2 + 2) >> 2));
+                seg_set<kVertical>(v, l, 6, c(q2, (p0 + q0 + q1 + 3 * q2 + 2 * q3 + 4) >> 3));
+            }
+        } else {  // deblock.rs:617-631
+            const int delta0 = (9 * (q0 - p0) - 3 * (q1 - p1) + 8) >> 4;
+            if (abs(delta0) < tc * 10) {
+                const int delta = clamp3i(delta0, -tc, tc);
+                if (!ex_p) {
+                    seg_set<kVertical>(v, l, 3, clamp3i(p0 + delta, 0, maxv));
+                    if (do_p1)
+                        seg_set<kVertical>(v, l, 2, clamp3i(p1 + clamp3i((((p2 + p0 + 1) >> 1) - p1 + delta) >> 1, -tc2, tc2), 0, maxv));
+                }
+                if (!ex_q) {
+                    seg_set<kVertical>(v, l, 4, clamp3i(q0 - delta, 0, maxv));
+                    if (do_q1)
+                        seg_set<kVertical>(v, l, 5, clamp3i(q1 + clamp3i((((q2 + q0 + 1) >> 1) - q1 - delta) >> 1, -tc2, tc2), 0, maxv));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = kVertical ? 0 : 1; i < (kVertical ? 8 : 7); ++i)  // taps p3 and q3 never change
+        *(uint2*)(base + (kVertical ? (i >> 1) * pl.rw + 4 * (i & 1) : i * pl.rw)) = v[i];
+}
+
+// Chroma (decode.rs:2036-2137): taps p1, p0, q0, q1 of 4 lines, both planes.
+template <bool kVertical, class Cl>
+__device__ __forceinline__ void chroma_segment_tile(const DevPic& P, int edge, int scan, const SPlane& cb, const SPlane& cr,
+                                                    const Cl& cl, bool any_exempt) {
+    const int mid = scan + 1;
+    const int lex = kVertical ? edge * P.sub_w : mid * P.sub_w;
+    const int ley = kVertical ? mid * P.sub_h : edge * P.sub_h;
+    if (lex >= P.w || ley >= P.h) return;
+    const hpvcd_cell q = cl.at(lex >> 2, ley >> 2);
+    if ((kVertical ? q.bs_v : q.bs_h) < 2) return;
+    const int lqx = min(lex, P.w - 1), lqy = min(ley, P.h - 1);
+    const int ppx = kVertical ? min(max(lex - 1, 0), P.w - 1) : lqx, ppy = kVertical ? lqy : min(max(ley - 1, 0), P.h - 1);
+    const int avg = (qp_of(P, cl, ppx, ppy) + qp_of(P, cl, lqx, lqy) + 1) >> 1;
+    int bo, to;
+    slice_offsets(P, lqx, lqy, &bo, &to);
+    (void)bo;
+    const int sh = P.bd_c - 8;
+    const int maxv = (1 << P.bd_c) - 1;
+    const int lines = min((kVertical ? P.ch : P.cw) - scan, 4);
+    // bit l / 4 + l: the P / Q sample of line l is in an exempt cell
+    uint32_t ex = 0;
+    if (any_exempt)
+        for (int l = 0; l < lines; ++l) {
+            const int s = scan + l;
+            if (exempt_of(cl, (kVertical ? edge - 1 : s) * P.sub_w, (kVertical ? s : edge - 1) * P.sub_h)) ex |= 1u << l;
+            if (exempt_of(cl, (kVertical ? edge : s) * P.sub_w, (kVertical ? s : edge) * P.sub_h)) ex |= 16u << l;
+        }
+#pragma unroll 1
+    for (int plane = 0; plane < 2; ++plane) {
+        const int off = plane == 0 ? P.pps_cb_qp_offset : P.pps_cr_qp_offset;
+        const int qc = qpc_map(avg + off, P.idc, P.bd_c);
+        const int tc = c_tc[clamp3i(qc + 2 + 2 * to, 0, 53)] << sh;
+        if (tc == 0) continue;
+        const SPlane& pl = plane == 0 ? cb : cr;
+        uint16_t* const base = pl.s + (kVertical ? (scan - pl.y0) * pl.rw + edge - 4 - pl.x0 : (edge - 4 - pl.y0) * pl.rw + scan - pl.x0);
+        uint2 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (kVertical || (i >= 2 && i < 6))
+                v[i] = *(const uint2*)(base + (kVertical ? (i >> 1) * pl.rw + 4 * (i & 1) : i * pl.rw));
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            const int p1 = seg_get<kVertical>(v, l, 2), p0 = seg_get<kVertical>(v, l, 3), q0 = seg_get<kVertical>(v, l, 4),
+                      q1 = seg_get<kVertical>(v, l, 5);
+            const int delta = clamp3i((((q0 - p0) * 4 + p1 - q1 + 4) >> 3), -tc, tc);
+            if (l < lines) {
+                if (!(ex >> l & 1u)) seg_set<kVertical>(v, l, 3, clamp3i(p0 + delta, 0, maxv));
+                if (!(ex >> l & 16u)) seg_set<kVertical>(v, l, 4, clamp3i(q0 - delta, 0, maxv));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (kVertical || i == 3 || i == 4)
+                *(uint2*)(base + (kVertical ? (i >> 1) * pl.rw + 4 * (i & 1) : i * pl.rw)) = v[i];
+    }
+}
+
 // blockIdx.y = picture, blockIdx.z = 0 luma / 1 chroma.
 __global__ void k_deblock(const DevPic* __restrict__ pics, int vertical) {
     const DevPic& P = pics[blockIdx.y];
@@ -493,6 +653,34 @@ __device__ __forceinline__ uint32_t rgb_px(const RgbCoef& k, int idc, int luma, 
     g = clamp3i(g, 0, k.cmax) >> k.sh;
     b = clamp3i(b, 0, k.cmax) >> k.sh;
     return (uint32_t)r | ((uint32_t)g << 8) | ((uint32_t)b << 16);
+}
+
+// Four pixels of the Q13 matrix (rgb_px for 4:0:0 and every matrix but
+// identity and YCgCo) as the three words of their RGB8 bytes.  The luma
+// factor is common and everything constant is in the chroma terms; two
+// shifts and a clip to the sample range are one shift and a clip to a byte,
+// which the packing conversion does.
+__device__ __forceinline__ uint32_t pack_u8(int b0, int b1, int b2, int b3) {
+    uint32_t t, d;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(b3), "r"(b2), "r"(0));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(b1), "r"(b0), "r"(t));
+    return d;
+}
+__device__ __forceinline__ void rgb_quad(const RgbCoef& k, const int (&luma)[4], const int (&cb)[4], const int (&cr)[4],
+                                         bool mono, uint32_t (&w)[3]) {
+    const int sh = 13 + k.sh, bias = (1 << 12) - k.k_y * k.y_black;
+    int r[4], g[4], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int u = mono ? 0 : cb[i] - k.neutral, v = mono ? 0 : cr[i] - k.neutral;
+        const int yv = k.k_y * luma[i] + bias;
+        r[i] = (yv + k.cr_to_r * v) >> sh;
+        g[i] = (yv + k.cb_to_g * u + k.cr_to_g * v) >> sh;
+        b[i] = (yv + k.cb_to_b * u) >> sh;
+    }
+    w[0] = pack_u8(r[0], g[0], b[0], r[1]);
+    w[1] = pack_u8(g[1], b[1], r[2], g[2]);
+    w[2] = pack_u8(b[2], r[3], g[3], b[3]);
 }
 
 // Index in the oriented W x H image (stored layout) of stored sample (x, y)
@@ -776,68 +964,103 @@ __device__ __forceinline__ void sao_quad(const DevPic& P, int c, const TileComp&
     }
 }
 
+// 16-bit halves of two words.
+__device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// The entries idx (0..7, one per half) of an eight-byte table of signed
+// offsets, as two int16: a byte permute whose selector takes each byte and
+// its replicated sign.
+__device__ __forceinline__ uint32_t offset_pair(uint32_t lo, uint32_t hi, uint32_t idx) {
+    const uint32_t t = (idx | (idx >> 8)) & 0x0707u;
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(lo), "r"(hi), "r"(t | (t << 4) | 0x8080u));
+    return d;
+}
+// Parameters sao_fixed takes: offsets of one byte, a band position whose bands
+// do not wrap around the byte the reference compares in.
+__device__ __forceinline__ bool offsets_fit(const hpvcd_sao_comp& sc) {
+    bool fit = sc.band_pos <= 252;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) fit = fit && sc.offsets[i] >= -128 && sc.offsets[i] <= 127;
+    return fit;
+}
+
 // SAO of one tile component whose samples all lie in one CTB (CTB 64),
-// without exempt cells or region limits: the CTB's parameters, read once,
-// hold for every quad.  kSel: 0..3 edge offset of that class, 4 band
-// offset, 5 off (a copy).  Same arithmetic as sao_quad (sao.rs:179-330).
+// without exempt cells or region limits and with offsets of one byte: the
+// CTB's parameters, read once, hold for every quad.  kSel: 0..3 edge offset
+// of that class, 4 band offset, 5 off (a copy).  Same values as sao_quad
+// (sao.rs:179-330), two samples at a time in 16-bit halves: with every sample
+// below 2^15 a word difference biased by 0x8000 per half never borrows.
 template <int kSel>
 __device__ __forceinline__ void sao_fixed(const TileComp& k, uint16_t* to, const hpvcd_sao_comp sc, int bd, int tid) {
     const int qsh = k.tw == 64 ? 4 : 3;  // quads per row: 16 or 8
     const int nq = k.th << qsh, rw = k.rw();
-    const int mx = (1 << bd) - 1;
-    const int o0 = sc.offsets[0], o1 = sc.offsets[1], o2 = sc.offsets[2], o3 = sc.offsets[3];
+    const uint32_t mx = ((1u << bd) - 1u) * 0x10001u;
+    const uint32_t o0 = (uint8_t)sc.offsets[0], o1 = (uint8_t)sc.offsets[1], o2 = (uint8_t)sc.offsets[2],
+                   o3 = (uint8_t)sc.offsets[3];
+    // edge offset: index 0..4 = 2 + the two signs, nothing at 2; band offset:
+    // index = band - band_pos, nothing from 4 on
+    const uint32_t tab_lo = kSel == 4 ? o0 | (o1 << 8) | (o2 << 16) | (o3 << 24) : o0 | (o1 << 8) | (o2 << 24);
+    const uint32_t tab_hi = kSel == 4 ? 0u : o3;
+    constexpr uint32_t kBias = 0x80008000u;
+#pragma unroll 2
     for (int i = tid; i < nq; i += kTileThreads) {
         const int xq = 4 * (i & ((1 << qsh) - 1)), yq = i >> qsh;
         const int x0 = k.tx + xq, y = k.ty + yq;
         if (x0 >= k.pw || y >= k.ph) continue;
         const uint16_t* row = k.sp.s + (yq + 4) * rw + (xq + 8);  // sample (x0, y) of the staged region
         const uint2 c2 = *(const uint2*)row;
-        int out[4] = {(int)(c2.x & 0xffff), (int)(c2.x >> 16), (int)(c2.y & 0xffff), (int)(c2.y >> 16)};
+        const uint32_t c[2] = {c2.x, c2.y};
+        uint32_t out[2] = {c2.x, c2.y};
         if (kSel == 4) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint8_t rel = (uint8_t)((uint8_t)(out[u] >> (bd - 5)) - sc.band_pos);
-                const int o = rel == 0 ? o0 : (rel == 1 ? o1 : (rel == 2 ? o2 : o3));
-                if (rel < 4) out[u] = clamp3i(out[u] + o, 0, mx);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t band = (c[h] >> (bd - 5)) & 0x001f001fu;
+                const uint32_t rel = ((band | kBias) - sc.band_pos * 0x10001u) ^ kBias;  // large below band_pos
+                out[h] = __viaddmin_s16x2_relu(c[h], offset_pair(tab_lo, tab_hi, min_u16x2(rel, 0x00040004u)), mx);
             }
         } else if (kSel < 4) {
             constexpr int dx = kSel == 1 ? 0 : 1;
             constexpr int dy = kSel == 0 ? 0 : (kSel == 3 ? -1 : 1);
-            // n1 = (x + dx, y + dy), n2 = (x - dx, y - dy)
-            int n1[4], n2[4];
-            auto six = [&](const uint16_t* q, int w[6]) {  // samples x0 - 1 .. x0 + 4 of a staged row
-                const uint2 v = *(const uint2*)q;
-                w[0] = q[-1];
-                w[1] = v.x & 0xffff; w[2] = v.x >> 16; w[3] = v.y & 0xffff; w[4] = v.y >> 16;
-                w[5] = q[4];
-            };
-            if (kSel == 1) {
-                const uint2 a = *(const uint2*)(row + rw), b = *(const uint2*)(row - rw);
-                n1[0] = a.x & 0xffff; n1[1] = a.x >> 16; n1[2] = a.y & 0xffff; n1[3] = a.y >> 16;
-                n2[0] = b.x & 0xffff; n2[1] = b.x >> 16; n2[2] = b.y & 0xffff; n2[3] = b.y >> 16;
-            } else {
-                int wa[6], wb[6];
-                six(row + dy * rw, wa);
-                if (dy != 0) six(row - dy * rw, wb);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    n1[u] = wa[u + 2];
-                    n2[u] = dy != 0 ? wb[u] : wa[u];
-                }
+            if (!(y - dy >= 0 && y + dy >= 0 && y - dy < k.ph && y + dy < k.ph)) {
+                *(uint2*)(to + yq * k.tw + xq) = c2;  // a neighbour row outside the picture
+                continue;
             }
-            const bool rows_ok = y - dy >= 0 && y + dy >= 0 && y - dy < k.ph && y + dy < k.ph;
+            // n1 = (x + dx, y + dy), n2 = (x - dx, y - dy) as pairs
+            uint32_t n1[2], n2[2];
+            const uint2 a = *(const uint2*)(row + dy * rw), b = *(const uint2*)(row - dy * rw);
+            if (kSel == 1) {
+                n1[0] = a.x, n1[1] = a.y, n2[0] = b.x, n2[1] = b.y;
+            } else {
+                const uint32_t right = row[dy * rw + 4], left = row[-dy * rw - 1];
+                n1[0] = __byte_perm(a.x, a.y, 0x5432);
+                n1[1] = __byte_perm(a.y, right, 0x5432);
+                n2[0] = __byte_perm(left, b.x, 0x5410);
+                n2[1] = __byte_perm(b.x, b.y, 0x5432);
+            }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int x = x0 + u;
-                if (!rows_ok || x - dx < 0 || x + dx >= k.pw) continue;  // a neighbour outside the picture
-                const int s0 = out[u];
-                const int e = ((s0 > n1[u]) - (s0 < n1[u])) + ((s0 > n2[u]) - (s0 < n2[u])) + 2;
-                const int o = e == 0 ? o0 : (e == 1 ? o1 : (e == 3 ? o2 : (e == 4 ? o3 : 0)));
-                if (o) out[u] = clamp3i(s0 + o, 0, mx);
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t cb = c[h] | kBias;  // 0x8000 + c - n clamped to 0x7fff .. 0x8001: the sign
+                const uint32_t s1 = max_u16x2(min_u16x2(cb - n1[h], 0x80018001u), 0x7fff7fffu);
+                const uint32_t s2 = max_u16x2(min_u16x2(cb - n2[h], 0x80018001u), 0x7fff7fffu);
+                const uint32_t e = s1 + s2 - 2u * 0x7fff7fffu;  // 0..4 per half
+                out[h] = __viaddmin_s16x2_relu(c[h], offset_pair(tab_lo, tab_hi, e), mx);
+            }
+            if (dx) {  // a neighbour column outside the picture
+                if (x0 == 0) out[0] = __byte_perm(out[0], c[0], 0x3254);
+                if (x0 + 4 >= k.pw) out[1] = __byte_perm(out[1], c[1], 0x7610);
             }
         }
-        *(uint2*)(to + yq * k.tw + xq) =
-            make_uint2((uint32_t)out[0] | ((uint32_t)out[1] << 16), (uint32_t)out[2] | ((uint32_t)out[3] << 16));
+        *(uint2*)(to + yq * k.tw + xq) = make_uint2(out[0], out[1]);
     }
 }
 
@@ -928,9 +1151,9 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
             }
         for (int c = 0; c < ncomp; ++c) {
             const TileComp k = tcomp(c);
-            const int chunks = k.rw() >> 3;
+            const int chunks = k.rw() >> 3;  // 10 or 6
             for (int i = tid; i < k.rh() * chunks; i += kTileThreads) {
-                const int r = i / chunks, q = i - r * chunks;
+                const int r = chunks == 10 ? i / 10 : i / 6, q = i - r * chunks;
                 *(uint4*)(k.sp.s + r * k.rw() + 8 * q) =
                     load8(P.rec[c], P.bps, k.pw, k.ph, k.sp.x0 + 8 * q, k.sp.y0 + r);
             }
@@ -947,8 +1170,8 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
             const SPlane Cr = tcomp(2).sp;
             const int nec_v = Cb.tw / 8 + 1, nsc_v = Cb.rh() / 4;        // chroma V: edges, segments
             const int nec_h = Cb.th / 8 + 1, nsc_h = (Cb.tw + 8) / 4;    // chroma H
-            for (int pass = 0; pass < 2; ++pass) {
-                const bool vertical = pass == 0;
+            auto pass = [&](auto dir) {
+                constexpr bool vertical = decltype(dir)::value;
                 const int n_luma = 9 * 18;
                 const int n_chroma = P.idc ? (vertical ? nec_v * nsc_v : nec_h * nsc_h) : 0;
                 for (int j = tid; j < n_luma + n_chroma; j += kTileThreads) {
@@ -957,7 +1180,7 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
                         const int scan = (vertical ? Y - 4 : X - 4) + 4 * (j / 9);
                         const int emax = vertical ? P.w : P.h, smax = vertical ? P.h : P.w;
                         if (e >= 8 && e <= emax - 4 && scan >= 0 && scan + 4 <= smax)
-                            luma_segment(P, vertical, e, scan, Lc.sp, cl, any_exempt);
+                            luma_segment_tile<vertical>(P, e, scan, Lc.sp, cl, any_exempt);
                     } else {
                         const int jj = j - n_luma;
                         const int ne = vertical ? nec_v : nec_h;
@@ -965,11 +1188,13 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
                         const int scan = (vertical ? Cb.ty - 4 : Cb.tx - 4) + 4 * (jj / ne);
                         const int emax = vertical ? P.cw : P.ch, smax = vertical ? P.ch : P.cw;
                         if (e >= 8 && e <= emax - 2 && scan >= 0 && scan + 4 <= smax)
-                            chroma_segment(P, vertical, e, scan, Cb.sp, Cr, cl, any_exempt);
+                            chroma_segment_tile<vertical>(P, e, scan, Cb.sp, Cr, cl, any_exempt);
                     }
                 }
                 __syncthreads();
-            }
+            };
+            pass(std::true_type{});
+            pass(std::false_type{});
         }
         // ---- 4. SAO from the deblocked samples into the tile's output
         // buffer (a copy for components without SAO) ----
@@ -977,9 +1202,9 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
             const TileComp k = tcomp(c);
             uint16_t* const to = tout_of(c);
             const bool on = sao_on && (P.flags & (c == 0 ? HPVCD_PIC_SAO_LUMA : HPVCD_PIC_SAO_CHROMA));
-            if (!sao_slow && P.log2_ctb >= 6) {  // one CTB covers the tile component
-                hpvcd_sao_comp sc{};
-                if (on) sc = sao.at(X >> P.log2_ctb, Y >> P.log2_ctb, c);
+            hpvcd_sao_comp sc{};
+            if (on && P.log2_ctb >= 6) sc = sao.at(X >> P.log2_ctb, Y >> P.log2_ctb, c);
+            if (!sao_slow && P.log2_ctb >= 6 && offsets_fit(sc)) {  // one CTB covers the tile component
                 const int bd = c ? P.bd_c : P.bd;
                 const int sel = sc.type_idx == 1 ? 4 : (sc.type_idx == 2 ? sc.eo_class : 5);
                 switch (sel) {
@@ -1015,9 +1240,10 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
                 const TileComp k = tcomp(c);
                 const uint16_t* const to = tout_of(c);
                 const int rows = min(k.th, k.ph - k.ty), cols = min(k.tw, k.pw - k.tx);
-                const int chunks = (cols + 7) >> 3;
-                for (int i = tid; i < rows * chunks; i += kTileThreads) {
-                    const int r = i / chunks, q = i - r * chunks;
+                const int lq = k.tw == 64 ? 3 : 2;
+                for (int i = tid; i < rows << lq; i += kTileThreads) {
+                    const int r = i >> lq, q = i & ((1 << lq) - 1);
+                    if (8 * q >= cols) continue;
                     const int x = k.tx + 8 * q, y = k.ty + r;
                     const uint16_t* src = to + r * k.tw + 8 * q;
                     const size_t idx = (size_t)y * k.pw + x;
@@ -1045,6 +1271,8 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
             const int copy_h = min(P.crop_h, max(P.canvas_h - P.dst_y, 0));
             const RgbCoef kc = rgb_coef(P);
             const TileComp B = tcomp(1);
+            const bool q13 = !moves_samples(P.orientation) &&
+                             (P.idc == 0 || (kc.matrix != HPVCD_MATRIX_IDENTITY && kc.matrix != HPVCD_MATRIX_YCGCO));
             const uint16_t* const tl = tout_of(0);
             const uint16_t* const tb = tout_of(1);
             const uint16_t* const tr = tout_of(2);
@@ -1072,6 +1300,16 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
                         cr[0] = r.x & 0xffff; cr[1] = r.x >> 16; cr[2] = r.y & 0xffff; cr[3] = r.y >> 16;
                     }
                 }
+                uint8_t* o = canvas + ((size_t)(P.dst_y + yy) * P.canvas_w + P.dst_x + x0) * 3;
+                if (q13 && cnt == 4 && ((uintptr_t)o & 3) == 0) {
+                    uint32_t w[3];
+                    rgb_quad(kc, luma, cb, cr, P.idc == 0, w);
+                    uint32_t* o32 = (uint32_t*)o;
+                    o32[0] = w[0];
+                    o32[1] = w[1];
+                    o32[2] = w[2];
+                    continue;
+                }
                 uint32_t px[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) px[u] = rgb_px(kc, P.idc, luma[u], cb[u], cr[u]);
@@ -1087,7 +1325,6 @@ k_filter_tile(const DevPic* __restrict__ pics, uint8_t* __restrict__ out, int rg
                     }
                     continue;
                 }
-                uint8_t* o = canvas + ((size_t)(P.dst_y + yy) * P.canvas_w + P.dst_x + x0) * 3;
                 if (cnt == 4 && ((uintptr_t)o & 3) == 0) {
                     uint32_t* o32 = (uint32_t*)o;
                     o32[0] = px[0] | (px[1] << 24);
