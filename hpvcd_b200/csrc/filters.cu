@@ -1408,7 +1408,7 @@ extern "C" cudaError_t hpvcd_launch_yuv_canvas(const hpvcd::DevPic* pics, int n_
 extern "C" cudaError_t hpvcd_launch_filter_tile(const hpvcd::DevPic* pics, int n_pics, int max_tiles, int cfmt,
                                                 int gated, uint8_t* out, cudaStream_t stream) {
     if (n_pics <= 0 || max_tiles <= 0) return cudaSuccess;
-    const int target = 148 * 8;  // resident CTAs of 256 threads on a B200
+    const int target = 148 * 8;  // CTAs of 256 threads, each looping over tiles
     const int per_pic = std::max(1, (target + n_pics - 1) / n_pics);
     dim3 grid(std::min(max_tiles, std::max(per_pic, 1)), n_pics, 1);
     const size_t smem = hpvcd::tile_smem_bytes(cfmt);

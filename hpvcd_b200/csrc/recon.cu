@@ -255,7 +255,9 @@ __host__ __device__ constexpr int tensor_stride(int n) { return n == 32 ? 40 : 2
 // Both stages of an n x n (16 or 32) inverse DCT by one warp: buf holds the
 // dequantised coefficients (row k, column c, stride tensor_stride(n));
 // emit(mt, out) gets, per 16-row tile, out[nt][e] = row mt * 16 + g + 8 *
-// (e / 2), column nt * 8 + 2t + (e & 1), before the storage wrap.  Stage 1's
+// (e / 2), column nt * 8 + 2t + (e & 1), before the storage wrap.  The row
+// tiles are a rolled loop: the kernel's tasks of every size run side by side on
+// an SM, and its warps waited for instructions before anything else.  Stage 1's
 // operand fragments are four rows of one column: two transposed 8x8 loads
 // whose row addresses interleave rows 4t, 4t + 1 and 4t + 2, 4t + 3.
 template <int N, typename Emit>
@@ -263,7 +265,6 @@ __device__ __forceinline__ void idct_tensor(const int16_t* buf, const uint32_t* 
     constexpr int MT = N / 16, NT = N / 8;  // row tiles, column tiles
     constexpr int STR = tensor_stride(N);
     // ---- stage 1: tmp[m][c] = clip((sum_k T[k][m] D[k][c] + 64) >> 7) ----
-    uint32_t tmp[MT][NT][2];  // two int16 per word: columns 2t, 2t + 1 of rows g and g + 8
     const int mat = lane >> 3, li = lane & 7;
     const int row = 4 * (li >> 1) + (li & 1) + 2 * (mat & 1);
     uint32_t bh[NT][N / 16], bl[NT][N / 16];
@@ -283,8 +284,11 @@ __device__ __forceinline__ void idct_tensor(const int16_t* buf, const uint32_t* 
             bh[nt][reg] = __byte_perm(r[2 * h], r[2 * h + 1], 0x7531);
         }
     }
-#pragma unroll
+    const int shift2 = 20 - bd;
+    const int add2 = 1 << (shift2 - 1);
+#pragma unroll 1
     for (int mt = 0; mt < MT; ++mt) {
+        uint32_t tmp[NT][2];  // two int16 per word: columns 2t, 2t + 1 of rows g and g + 8
         uint32_t a[4];
 #pragma unroll
         for (int i = 0; i < (N == 32 ? 4 : 2); ++i)
@@ -302,21 +306,16 @@ __device__ __forceinline__ void idct_tensor(const int16_t* buf, const uint32_t* 
             int v[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = clamp3i((dh[e] * 256 + dl[e] + 64) >> 7, -32768, 32767);
-            tmp[mt][nt][0] = __byte_perm((uint32_t)v[0], (uint32_t)v[1], 0x5410);
-            tmp[mt][nt][1] = __byte_perm((uint32_t)v[2], (uint32_t)v[3], 0x5410);
+            tmp[nt][0] = __byte_perm((uint32_t)v[0], (uint32_t)v[1], 0x5410);
+            tmp[nt][1] = __byte_perm((uint32_t)v[2], (uint32_t)v[3], 0x5410);
         }
-    }
-    // ---- stage 2: out[r][m] = (sum_k tmp[r][k] T[k][m] + add2) >> shift2 ----
-    const int shift2 = 20 - bd;
-    const int add2 = 1 << (shift2 - 1);
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
+        // ---- stage 2: out[r][m] = (sum_k tmp[r][k] T[k][m] + add2) >> shift2 ----
         uint32_t ah[4], al[4];
 #pragma unroll
         for (int half = 0; half < N / 16; ++half)
 #pragma unroll
             for (int rr = 0; rr < 2; ++rr) {
-                const uint32_t p = tmp[mt][2 * half][rr], q = tmp[mt][2 * half + 1][rr];
+                const uint32_t p = tmp[2 * half][rr], q = tmp[2 * half + 1][rr];
                 al[2 * half + rr] = __byte_perm(p, q, 0x6420);
                 ah[2 * half + rr] = __byte_perm(p, q, 0x7531);
             }
@@ -750,10 +749,21 @@ __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
         }
     }
     const Dequant dq(P, t, 2);
-    const uint8_t* sm = scaling_of(P, t, 2);
     const int nx = (t.nx == 0 || t.nx > 4) ? 4 : t.nx;
+    uint32_t m4[4] = {0x10101010u, 0x10101010u, 0x10101010u, 0x10101010u};  // factors of row r
+    if (const uint8_t* sm = scaling_of(P, t, 2)) {
+#pragma unroll 1
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t w = (uint32_t)sm[4 * r] | ((uint32_t)sm[4 * r + 1] << 8) | ((uint32_t)sm[4 * r + 2] << 16) |
+                               ((uint32_t)sm[4 * r + 3] << 24);
+            if (r == 0) m4[0] = w;
+            if (r == 1) m4[1] = w;
+            if (r == 2) m4[2] = w;
+            if (r == 3) m4[3] = w;
+        }
+    }
 #pragma unroll
-    for (int i = 0; i < 16; ++i) d[i] = (i & 3) < nx ? dq(d[i], sm ? sm[i] : 16) : 0;
+    for (int i = 0; i < 16; ++i) d[i] = (i & 3) < nx ? dq(d[i], (int)((m4[i >> 2] >> (8 * (i & 3))) & 0xffu)) : 0;
     const int shift2 = 20 - bd;
     if (c == 0 && (t.flags & HPVCD_TU_INTRA))
         idct4_thread<true>(d, shift2);
@@ -955,29 +965,44 @@ __device__ __forceinline__ void tb_tensor(const DevPic& P, const hpvcd_tu& t, in
     const Dequant dq(P, t, LOG2N);
     const uint8_t* sm = scaling_of(P, t, LOG2N);
     const int nx = (t.nx == 0 || t.nx > N) ? N : t.nx;
+    // factors of the lane's eight columns: the 8x8 list upsampled (its row
+    // changes with the pass), a byte each, two words
+    auto level = [&](const uint4& q, int j) {
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        return c8 ? (int)(int8_t)(w[j >> 2] >> (8 * (j & 3))) : (int)(int16_t)(w[j >> 1] >> (16 * (j & 1)));
+    };
+    const int col = (lane * 8) & (N - 1);
+    if (!sm) {
 #pragma unroll
-    for (int p = 0; p < PASS; ++p) {
-        const int i0 = (p * 32 + lane) * 8, r = i0 >> LOG2N, col = i0 & (N - 1);
-        const uint32_t w[4] = {raw[p].x, raw[p].y, raw[p].z, raw[p].w};
-        uint32_t o[4];
+        for (int p = 0; p < PASS; ++p) {
+            const int r = ((p * 32 + lane) * 8) >> LOG2N;
+            uint32_t o[4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-            int d[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const int j = 2 * h + u;
-                const int l = c8 ? (int)(int8_t)(w[j >> 2] >> (8 * (j & 3))) : (int)(int16_t)(w[j >> 1] >> (16 * (j & 1)));
-                int m = 16;
-                if (sm) {  // the 8x8 list upsampled, with its DC entry
-                    m = sm[(r >> (LOG2N - 3)) * 8 + ((col + j) >> (LOG2N - 3))];
-                    if (i0 + j == 0)
-                        m = P.scaling->dc[LOG2N - 2][min(c, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
-                }
-                d[u] = col + j < nx ? dq(l, m) : 0;
+            for (int h = 0; h < 4; ++h) {
+                const int d0 = col + 2 * h < nx ? dq(level(raw[p], 2 * h), 16) : 0;
+                const int d1 = col + 2 * h + 1 < nx ? dq(level(raw[p], 2 * h + 1), 16) : 0;
+                o[h] = __byte_perm((uint32_t)d0, (uint32_t)d1, 0x5410);
             }
-            o[h] = __byte_perm((uint32_t)d[0], (uint32_t)d[1], 0x5410);
+            *(uint4*)(buf + r * STR + col) = make_uint4(o[0], o[1], o[2], o[3]);
         }
-        *(uint4*)(buf + r * STR + col) = make_uint4(o[0], o[1], o[2], o[3]);
+    } else {
+        const int dc = P.scaling->dc[LOG2N - 2][min(c, 2) + ((t.flags & HPVCD_TU_INTRA) ? 0 : 3)];
+#pragma unroll
+        for (int p = 0; p < PASS; ++p) *(uint4*)(buf + (((p * 32 + lane) * 8) >> LOG2N) * STR + col) = raw[p];
+        __syncwarp();
+#pragma unroll 1
+        for (int p = 0; p < PASS; ++p) {
+            const int i0 = (p * 32 + lane) * 8, r = i0 >> LOG2N;
+            int16_t* q = buf + r * STR + col;
+            const uint4 w = *(const uint4*)q;  // this lane's levels
+#pragma unroll 1
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t pair = c8 ? (j < 4 ? w.x : w.y) : (j < 2 ? w.x : (j < 4 ? w.y : (j < 6 ? w.z : w.w)));
+                const int l = c8 ? (int)(int8_t)(pair >> (8 * (j & 3))) : (int)(int16_t)(pair >> (16 * (j & 1)));
+                const int m = i0 + j == 0 ? dc : sm[(r >> (LOG2N - 3)) * 8 + ((col + j) >> (LOG2N - 3))];
+                q[j] = (int16_t)(col + j < nx ? dq(l, m) : 0);
+            }
+        }
     }
     __syncwarp();
     const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
@@ -1315,7 +1340,7 @@ struct ReconLayout {
     int cs_w, cs_h;  // chroma canvas width and height (CTU interior)
     int rec_cap;     // staged records
     int list_c;      // intra TBs per chroma component
-    size_t off_can_y, off_can_c, off_ws, off_ents, off_tab, off_stamp, off_wf, off_misc, total;
+    size_t off_can_y, off_can_c, off_ws, off_ents, off_tab, off_stamp, off_misc, total;
     __host__ __device__ ReconLayout(int cfmt, int walkers) {
         cs_w = cfmt == kFmt444 ? 64 : 32;
         cs_h = cfmt == kFmt420 ? 32 : 64;
@@ -1328,16 +1353,14 @@ struct ReconLayout {
         o = (o + 15) & ~(size_t)15;
         off_ws = o;    o += (size_t)walkers * kWsBytes;
         off_ents = o;  o += (size_t)(kListCap + 2 * list_c) * sizeof(uint4);
-        off_tab = o;   o += (size_t)(64 * 64 + 2 * cs_w * cs_h) * sizeof(uint32_t);
+        off_tab = o;   o += (size_t)(64 * 64 + cs_w * cs_h) * sizeof(uint32_t);
         off_stamp = o; o += 256 * sizeof(uint32_t);
-        off_wf = o;    o += (size_t)(kListCap + 2 * list_c);
-        o = (o + 15) & ~(size_t)15;
         off_misc = o;  o += 128;  // claimed item, have bits, covered words, done flags, TB counts
         total = o;
     }
     __host__ __device__ int ent_off(int c) const { return c == 0 ? 0 : kListCap + (c - 1) * list_c; }
     __host__ __device__ int ent_cap(int c) const { return c == 0 ? kListCap : list_c; }
-    __host__ __device__ int tab_off(int c) const { return c == 0 ? 0 : 64 * 64 + (c - 1) * cs_w * cs_h; }
+    __host__ __device__ int tab_off(int c) const { return c == 0 ? 0 : 64 * 64; }
 };
 // The CTU's records are staged in the canvases: they are done with (turned
 // into walk entries) before any sample or residual is put there.
@@ -1680,14 +1703,15 @@ __device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need
 // are not one run (possible at slice boundaries and under constrained intra
 // prediction), or that has none, is flagged kTbGather and its line is gathered
 // sample by sample first.
-//   x: canvas offset of the TB | of line position 0 << 16
+//   x: canvas offset of the TB | of line position 0 << 16 | coded << 31
 //   y: canvas offset of the corner | blend table offset of a plain TB << 16
-//   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbCoded | kTbFilt
-//   w: x | y << 8 (in the CTU) | record index (< 1024) << 16 | kTb* flags << 26
+//   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbFilt
+//   w: x (6 bits) | kHow* << 6 | y << 8 (in the CTU) | kHow* << 14 |
+//      record index (< 1024) << 16 | kTb* flags << 26
 // Measured when the entries came in (4032x3024 grid, 70 luma TBs a CTU): the
 // walk's chain went from ~87k to ~46k cycles a CTU (4x4 700 -> 500, 16x16 5100
 // -> 1650, 32x32 10700 -> 3300 cycles); 512x512 tile 1004 -> 649 us.
-constexpr uint32_t kTbCoded = 1u << 30, kTbFilt = 1u << 31;
+constexpr uint32_t kTbCoded = 1u << 31 /* of x */, kTbFilt = 1u << 31 /* of z */;
 // the TB reads neighbour CTUs, its line must be gathered, it is an I_PCM
 // block, it covers edge words, line position 32 is available, it is a 4x4 or
 // 8x8 TB of an angular mode without line or edge filter and with one run of
@@ -1697,15 +1721,16 @@ constexpr uint32_t kTbEdge = 1u, kTbGather = 2u, kTbPcm = 4u, kTbPub = 8u, kTbHi
 struct TbEntry {
     uint4 w;
     __device__ __forceinline__ int org() const { return (int)(w.x & 0xffffu); }
-    __device__ __forceinline__ int line0() const { return (int)(w.x >> 16); }
+    __device__ __forceinline__ int line0() const { return (int)((w.x >> 16) & 0x7fffu); }
+    __device__ __forceinline__ bool coded() const { return (w.x & kTbCoded) != 0u; }
     __device__ __forceinline__ int corner() const { return (int)(w.y & 0xffffu); }
     __device__ __forceinline__ uint32_t tab() const { return w.y >> 16; }
     __device__ __forceinline__ int lo() const { return (int)(w.z & 0xffu); }
     __device__ __forceinline__ int hi() const { return (int)((w.z >> 8) & 0xffu); }
     __device__ __forceinline__ int n2() const { return (int)((w.z >> 16) & 0xffu); }
     __device__ __forceinline__ int mode() const { return (int)((w.z >> 24) & 0x3fu); }
-    __device__ __forceinline__ int x() const { return (int)(w.w & 0xffu); }
-    __device__ __forceinline__ int y() const { return (int)((w.w >> 8) & 0xffu); }
+    __device__ __forceinline__ int x() const { return (int)(w.w & 0x3fu); }
+    __device__ __forceinline__ int y() const { return (int)((w.w >> 8) & 0x3fu); }
     __device__ __forceinline__ uint32_t jrec() const { return (w.w >> 16) & 0x3ffu; }
     __device__ __forceinline__ uint32_t flags() const { return w.w >> 26; }
 };
@@ -1790,7 +1815,7 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
     w.x = (uint32_t)cin(k, x0, y0) | ((uint32_t)cin(k, x0 - 1, y0 + n2 - 1) << 16);
     w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (tab << 16);
     w.z = (uint32_t)lo | ((uint32_t)hi << 8) | ((uint32_t)n2 << 16) | ((uint32_t)t.mode << 24);
-    if (coded) w.z |= kTbCoded;
+    if (coded) w.x |= kTbCoded;
     if (filt) w.z |= kTbFilt;
     w.w = (uint32_t)x0 | ((uint32_t)y0 << 8) | (jrec << 16) | (flags << 26);
     return w;
@@ -1856,14 +1881,14 @@ struct Line {
 };
 
 // Blend table of a CTU component: one word per sample of its plain TBs, by
-// 4x4 blocks in raster order: coded | canvas byte offsets of the two line
-// samples (even, < 2^14) << 0 and << 13 | weight of the second (of 32) << 27.
+// 4x4 blocks in raster order: canvas byte offsets of the two line samples
+// (even, < 2^14) << 0 and << 13 | weight of the second (of 32) << 27.
 // With it the walk neither looks anything up nor clamps: it was 270 cycles a
 // 4x4 TB and 850 an 8x8 one with the table of modes and the line in the loop.
 constexpr uint32_t kBlendAdr = 0x3ffeu;
 static_assert(2 * can_size(64, 64) < 0x4000, "canvas byte offsets fit the blend words");
-__device__ __forceinline__ uint32_t blend_word(const Line& L, uint32_t ang, bool coded) {
-    return (coded ? 1u : 0u) | (uint32_t)(2 * L.at((int)(ang & 0xffu))) | ((uint32_t)(2 * L.at((int)((ang >> 8) & 0xffu))) << 13) |
+__device__ __forceinline__ uint32_t blend_word(const Line& L, uint32_t ang) {
+    return (uint32_t)(2 * L.at((int)(ang & 0xffu))) | ((uint32_t)(2 * L.at((int)((ang >> 8) & 0xffu))) << 13) |
            ((ang & 0x1f0000u) << 11);
 }
 __device__ __forceinline__ int blend_of(const uint16_t* can, uint32_t w) {
@@ -1982,8 +2007,8 @@ __device__ __forceinline__ void walk_tb8(uint32_t* px, int mode, bool coded, boo
 }
 
 // Two horizontally adjacent samples of a plain 8x8 TB per lane.
-__device__ __forceinline__ void walk_plain8(const uint16_t* can, uint32_t* px, uint2 w, int max_v) {
-    const uint32_t rv = (w.x & 1u) ? *px : 0u;
+__device__ __forceinline__ void walk_plain8(const uint16_t* can, uint32_t* px, uint2 w, bool coded, int max_v) {
+    const uint32_t rv = coded ? *px : 0u;
     const uint32_t p0 = (uint32_t)blend_of(can, w.x), p1 = (uint32_t)blend_of(can, w.y);
     *px = add_clip2(p0 | (p1 << 16), rv, max_v);
     __syncwarp();
@@ -2164,10 +2189,11 @@ __host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 // availability, coded and PCM tests compile to the plain form.  fine: a TB
 // waits for the edge words it reads; otherwise a CTU waits for all of its
 // neighbours' words before its walk.
-// How the walk takes the TB at an entry: it is a plain 4x4 TB (kWalkTwo: the
-// next one too), a plain 8x8 TB; it (or the pair) reads neighbour CTUs /
+// How the walk takes the TB at an entry (bits of its word w): it is a plain
+// 4x4 TB (kHowTwo: the next one too), it (or the pair) reads neighbour CTUs /
 // covers edge words.
-constexpr uint32_t kWalkPlain4 = 1u, kWalkPlain8 = 2u, kWalkEdge = 4u, kWalkPub = 8u, kWalkTwo = 16u;
+constexpr uint32_t kHowTwo = 1u << 6, kHowEdge = 1u << 7, kHowPub = 1u << 14, kHowPlain4 = 1u << 15;
+constexpr uint32_t kHowPlain = kTbPlain << 26;
 
 template <int kCW, bool kFeat>
 __global__ void __launch_bounds__(32 * recon_warps(kCW), kCW == 1 ? 5 : 4)
@@ -2213,7 +2239,8 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         uint32_t* s_have = (uint32_t*)(smem + lay.off_misc) + 1;  // have bits, two words per component
         uint32_t* s_cov = s_have + 6;                             // edge words covered by intra TBs
         uint32_t* s_done = s_cov + 3;                             // walking warps that are done
-        uint32_t* s_wcnt = s_done + 3;                            // TBs found per warp and component
+        uint32_t* s_diff = s_done + 3;                            // the Cb and Cr TBs differ in more than their residual
+        uint32_t* s_wcnt = s_diff + 1;                            // TBs found per warp and component
         auto can_of = [&](int c) -> uint16_t* {
             return c == 0 ? (uint16_t*)(smem + lay.off_can_y)
                           : (uint16_t*)(smem + lay.off_can_c) + (size_t)(c - 1) * can_size(lay.cs_w, lay.cs_h);
@@ -2223,6 +2250,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         asm volatile("cp.async.commit_group;" ::: "memory");
         for (int i = tid; i < 256; i += kThreads) stamp[i] = kNoStamp;
         if (tid < 3) s_cov[tid] = s_done[tid] = 0u;
+        if (tid == 3) *s_diff = 0u;
         if (warp == kWalkers)  // words outside the picture count as present
             for (int c = 0; c < ncomp; ++c) {
                 const EdgeGeo e = edge_geo(P, c, it.cx, it.cy);
@@ -2456,23 +2484,26 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 for (uint32_t e = lane; e < cnt; e += 32) {
                     TbEntry E;
                     E.w = list[e];
-                    if ((E.w.z & kTbCoded) && !(E.flags() & kTbPcm))
+                    if (E.coded() && !(E.flags() & kTbPcm))
                         stage_residual(k, 31 - __clz(E.n2()) - 1, E.x(), E.y());
                 }
             }
         }
         // ---- how the walk takes each entry, and the blend table: by all warps,
-        // two TBs at a time ----
+        // two TBs at a time.  Cb and Cr share one table: their TBs have the
+        // same places, modes and available lines (a CTU where they do not walks
+        // its Cr without the table) ----
+        if (tid == 0 && listed[1] != listed[2]) *s_diff = 1u;
         const int half = lane >> 4, l15 = lane & 15;
         for (int c = 0; c < ncomp; ++c) {
             const int S = c ? Scw : ctb, row = can_row(S);
             uint32_t* tab = (uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
-            const uint4* list = ents + lay.ent_off(c);
-            uint8_t* wf = smem + lay.off_wf + lay.ent_off(c);
+            uint4* list = ents + lay.ent_off(c);
+            const uint4* cb_list = ents + lay.ent_off(1);
             const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
             // the angular words of the next TB are on their way while one is done
             auto angles = [&](const TbEntry& E, uint32_t (&ang)[4]) {
-                if (!(E.flags() & kTbPlain)) return;
+                if (c == 2 || !(E.flags() & kTbPlain)) return;
                 const bool four = E.n2() == 8;
                 const uint32_t* a = (four ? g_angular.t4[E.mode() - 2] : g_angular.t8[E.mode() - 2]) + l15;
                 ang[0] = a[0];
@@ -2499,20 +2530,23 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 if (l15 == 0) {
                     const bool pair = e + 1 < cnt && plain && four && (F.flags() & kTbPlain) && F.n2() == 8;
                     const uint32_t g = pair ? f | F.flags() : f;
-                    wf[e] = (uint8_t)((plain ? (four ? kWalkPlain4 : kWalkPlain8) : 0u) | (pair ? kWalkTwo : 0u) |
-                                      (g & kTbEdge ? kWalkEdge : 0u) | (g & kTbPub ? kWalkPub : 0u));
+                    list[e].w = (E.w.w & 0xffff3f3fu) | (plain && four ? kHowPlain4 : 0u) | (pair ? kHowTwo : 0u) |
+                                (g & kTbEdge ? kHowEdge : 0u) | (g & kTbPub ? kHowPub : 0u);
+                    if (c == 2) {
+                        const uint4 b = cb_list[min(e, listed[1] ? listed[1] - 1 : 0u)];
+                        if (((b.x ^ E.w.x) & 0x7fffffffu) | (b.y ^ E.w.y) | (b.z ^ E.w.z) | ((b.w ^ E.w.w) & kHowPlain)) *s_diff = 1u;
+                    }
                 }
-                if (plain) {
+                if (plain && c < 2) {
                     const Line L(E, row);
-                    const bool coded = (E.w.z & kTbCoded) != 0u;
                     uint32_t* t = tab + E.tab();
                     if (four) {
-                        t[l15] = blend_word(L, ang[0], coded);
+                        t[l15] = blend_word(L, ang[0]);
                     } else {
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             const int x = l15 & 7, y = 2 * u + (l15 >> 3);
-                            t[((y >> 2) * (S >> 2) + (x >> 2)) * 16 + (y & 3) * 4 + (x & 3)] = blend_word(L, ang[u], coded);
+                            t[((y >> 2) * (S >> 2) + (x >> 2)) * 16 + (y & 3) * 4 + (x & 3)] = blend_word(L, ang[u]);
                         }
                     }
                 }
@@ -2532,7 +2566,8 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             const Comp k = comp_of(c);
             const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]), last = cnt ? cnt - 1 : 0u;
             const uint4* list = ents + lay.ent_off(c);
-            const uint8_t* wf = smem + lay.off_wf + lay.ent_off(c);
+            // (a walk without the table takes every TB by its line)
+            const uint32_t how_mask = c == 2 && *s_diff ? ~(kHowPlain | kHowPlain4 | kHowTwo) : 0xffffffffu;
             const uint32_t* tab = (const uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
             uint16_t* const can = k.can;
             const int row = can_row(k.S), max_v = k.max_v;
@@ -2565,35 +2600,35 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             // Plain 4x4 TBs are taken in pairs: lanes 0..15 hold TB e, lanes
             // 16..31 TB e + 1, predicted after TB e is stored.  The pair's
             // blend words and place are loaded an iteration ahead.
-            uint32_t how = 0, bw = 0;
-            int org = 0;
+            uint32_t how = 0, bw = 0, place = 0;  // flags, blend word, word x of the entry
             auto fetch = [&](uint32_t e) { return *(const uint2*)&list[min(e + half, last)]; };
+            auto how_of = [&](uint32_t e) { return list[min(e, last)].w & how_mask; };
             if (cnt) {
                 const uint2 h = fetch(0);
-                org = (int)(h.x & 0xffffu);
+                place = h.x;
                 bw = tab[(h.y >> 16) + l15];
-                how = wf[0];
+                how = how_of(0);
             }
             for (uint32_t e = 0; e < cnt;) {
-                if (how & kWalkPlain4) {
-                    const bool two = (how & kWalkTwo) != 0u;
+                if (how & kHowPlain4) {
+                    const bool two = (how & kHowTwo) != 0u;
                     const uint32_t next = e + (two ? 2u : 1u);
-                    if (how & kWalkEdge) await(TbEntry{list[two ? e + half : e]});
-                    uint16_t* const px = can + org + px4;
+                    if (how & kHowEdge) await(TbEntry{list[two ? e + half : e]});
+                    uint16_t* const px = can + (place & 0xffffu) + px4;
                     // (without a second TB lanes 16..31 hold another kind of TB's word: table offset 0, read only)
-                    const int rv = (bw & 1u) ? (int)(int16_t)*px : 0;
+                    const int rv = (place & kTbCoded) ? (int)(int16_t)*px : 0;
                     int s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);
                     if (half == 0) *px = (uint16_t)s;
                     const uint2 h = fetch(next);
-                    const uint32_t hn = wf[min(next, last)];
+                    const uint32_t hn = how_of(next);
                     __syncwarp();
                     if (two) {
                         s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
                         if (half) *px = (uint16_t)s;
                     }
-                    org = (int)(h.x & 0xffffu);
+                    place = h.x;
                     bw = tab[(h.y >> 16) + l15];
-                    if ((how & kWalkPub) && (two || half == 0)) {  // samples on the CTU's right column / bottom row
+                    if ((how & kHowPub) && (two || half == 0)) {  // samples on the CTU's right column / bottom row
                         const TbEntry E{list[e + half]};
                         uint16_t* const w16 = (uint16_t*)words;
                         const int x = E.x() + (lane & 3), y = E.y() + (l15 >> 2);
@@ -2607,12 +2642,13 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                     continue;
                 }
                 const uint2 h = fetch(e + 1);
-                const uint32_t hn = wf[min(e + 1, last)];
+                const uint32_t hn = how_of(e + 1);
                 TbEntry E{list[e]};
-                if (how & kWalkEdge) await(E);
+                if (how & kHowEdge) await(E);
                 const int n2 = E.n2();
-                if (how & kWalkPlain8) {
-                    walk_plain8(can, (uint32_t*)(can + E.org() + px8), *(const uint2*)(tab + E.tab() + tab8), max_v);
+                if (how & kHowPlain) {
+                    walk_plain8(can, (uint32_t*)(can + E.org() + px8), *(const uint2*)(tab + E.tab() + tab8), E.coded(),
+                                max_v);
                 } else {
                     const uint32_t f = E.flags();
                     const int mode = E.mode();
@@ -2620,12 +2656,12 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                     if (f & kTbGather) {
                         gather_line(k, 31 - __clz(n2) - 1, E.x(), E.y(), stamp, E.jrec(), ws, lane);
                         const uint32_t at = (uint32_t)(ws.s - can);  // position i at canvas offset at + i
-                        E.w.x = (E.w.x & 0xffffu) | (at << 16);
+                        E.w.x = (E.w.x & (0xffffu | kTbCoded)) | (at << 16);
                         E.w.y = (E.w.y & 0xffff0000u) | (at + (uint32_t)n2);
                         stride = -1;
                     }
                     const Line L(E, stride);
-                    const bool coded = (E.w.z & kTbCoded) != 0u, filt = (E.w.z & kTbFilt) != 0u;
+                    const bool coded = E.coded(), filt = (E.w.z & kTbFilt) != 0u;
                     if (kFeat && (f & kTbPcm)) {
                         pcm_tb(k, 31 - __clz(n2) - 1, E.x(), E.y(), lane);
                     } else if (n2 == 8) {
@@ -2643,9 +2679,9 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 const uint32_t was = how;
                 ++e;
                 how = hn;
-                org = (int)(h.x & 0xffffu);
+                place = h.x;
                 bw = tab[(h.y >> 16) + l15];
-                if (was & kWalkPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
+                if (was & kHowPub) publish_tb(can, row, k.S, k.Sh, E.x(), E.y(), n2 >> 1, words, lane);
             }
         }
         if (warp < kWalkers && lane == 0) *(volatile uint32_t*)&s_done[warp] = 1u;

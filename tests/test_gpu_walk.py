@@ -68,3 +68,18 @@ def test_sizes(mix, cbf, depth):
         c.tu_mix[i] = m
     s.add(c)
     check(s.pictures())
+
+
+# Cr TBs whose modes differ from Cb's: the two components share no table then
+@pytest.mark.parametrize("idc", [1, 2, 3])
+@pytest.mark.parametrize("share", [1.0, 0.02])
+def test_cr_modes_of_their_own(idc, share):
+    s = synth.SynthSet()
+    s.add(synth.intra_cfg(31 + idc, 320, 192, bit_depth=10, chroma_idc=idc))
+    p = s.picture(0)
+    rng = np.random.default_rng(idc)
+    tus = synth.tus_of(p).copy()
+    cr = (tus["comp"] == 2) & (rng.random(tus.size) < share)
+    tus["mode"][cr] = rng.integers(0, 35, int(cr.sum()))
+    p.tus = tus.ctypes.data
+    check([p])
