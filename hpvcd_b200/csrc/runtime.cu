@@ -220,17 +220,25 @@ struct hpvcd_plan {
         int cfmt;
         uint32_t item_off, n_items, n_full;
         uint32_t ready;
+        bool inter;  // some of its pictures predict from others
     };
     std::vector<Wave> waves;
     // k_recon CTAs per SM by class and build (1 two warps, 2 three warps,
     // 3 three warps register-capped; index build - 1)
     int occ[3][3] = {{1, 1, 1}, {1, 1, 1}, {1, 1, 1}};
-    // Build of a wave's wavefront kernel (hpvcd_sched.chroma_warps): 0 picks
-    // one warp for both chroma components at 4:2:0 and 4:0:0, where their
-    // walks together are shorter than the luma walk, else one warp each.
-    int build_of(const Wave& wv) const {
-        const uint32_t cw = sched.chroma_warps;
-        return cw >= 1 && cw <= 3 ? (int)cw : (wv.cfmt == 0 ? 1 : 2);
+    // Build of a wave's wavefront kernel (hpvcd_sched.chroma_warps; 0, the
+    // default, is one warp per chroma component: 24 mixed images 4305 us
+    // against 4597 with one warp for both, single pictures the same).
+    int build_of() const { return sched.chroma_warps >= 1 && sched.chroma_warps <= 3 ? (int)sched.chroma_warps : 2; }
+    // CTAs of a wave's persistent grid, `slots` of them resident.  Intra
+    // pictures walk at most `ready` CTUs at once; three CTAs for each keep the
+    // set-up of the next ones off the chain, and CTAs beyond that (but one per
+    // SM) only wait beside the walking ones (3840x2160: 148 CTAs 1810 us, 592
+    // 1970 us; the 4032x3024 grid, 192 ready: 296 CTAs 608 us, 444 577 us, 592
+    // 581 us).  CTUs of inter pictures mostly wait for nothing.
+    int grid_of(const Wave& wv, int slots, int n_seg) const {
+        if (!wv.inter) slots = std::min(slots, std::max(3 * (int)wv.ready, std::max(1, sms / std::max(1, n_seg))));
+        return std::max(1, std::min(slots, (int)wv.n_items));
     }
     int occ_of(int cfmt, int build) const { return occ[cfmt][build - 1]; }
     int sms = 148;
@@ -591,9 +599,11 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
         for (int cls = 0; cls < 3; ++cls) {
             const uint32_t off = (uint32_t)P->items.size();
             uint32_t ready = 0;
+            bool inter = false;
             for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics; ++i) {
                 const hpvcd_picture& p = pics[i];
                 if ((p.flags & HPVCD_PIC_PRED_IN_PLANE) || recon_class(p) != cls) continue;
+                inter |= (p.flags & HPVCD_PIC_INTER) != 0;
                 const Geo g = geo_of(p);
                 ready += (uint32_t)std::min(g.ctb_rows, (g.ctb_cols + 1) / 2);
             }
@@ -609,7 +619,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
                     }
                 }
             const uint32_t cnt = (uint32_t)P->items.size() - off;
-            if (cnt) P->waves.push_back(hpvcd_plan::Wave{si, cls, off, cnt, cnt, ready});
+            if (cnt) P->waves.push_back(hpvcd_plan::Wave{si, cls, off, cnt, cnt, ready, inter});
         }
         s.n_waves = (uint32_t)P->waves.size() - s.wave_first;
     }
@@ -874,12 +884,12 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
             // its own layout and work counter
             for (uint32_t w = s.wave_first; w < s.wave_first + s.n_waves; ++w) {
                 const hpvcd_plan::Wave& wv = P->waves[w];
-                const int build = P->build_of(wv);
+                const int build = P->build_of();
                 int occ = P->occ_of(wv.cfmt, build);
                 if (P->sched.recon_ctas_per_sm > 0) occ = std::min<int>(occ, (int)P->sched.recon_ctas_per_sm);
                 // concurrent segments share the SMs: each gets its share of the CTAs
                 const int share = P->concurrent ? std::max(1, P->sms * occ / (int)n_seg) : P->sms * occ;
-                const int grid = std::max(1, std::min<int>(share, (int)wv.n_items));
+                const int grid = P->grid_of(wv, share, P->concurrent ? (int)n_seg : 1);
                 e = hpvcd_launch_recon(P->d_pics, P->d_items + wv.item_off, wv.n_items, P->d_scratch + w, d_err,
                                        wv.cfmt, grid, build, P->recon_feat ? 1 : 0,
                                        P->sched.wave ? 0 : 1, P->spin_limit, st);
@@ -1983,7 +1993,7 @@ hpvcd_status noalloc_setup(int dev, NoAllocDevice** out) {
         d.edges = (unsigned char*)q;
         e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return cuda_status(e);
-        for (int f = 0; f < 3; ++f) d.occ[f] = std::max(1, hpvcd_recon_occupancy(f, 1));
+        for (int f = 0; f < 3; ++f) d.occ[f] = std::max(1, hpvcd_recon_occupancy(f, 2));
         e = cudaGetLastError();
         if (e != cudaSuccess) return cuda_status(e);
         d.base = (unsigned char*)p;
@@ -2139,8 +2149,10 @@ HPVCD_API hpvcd_status hpvcd_decode_noalloc(const hpvcd_picture* dev_pic, void* 
     if (e != cudaSuccess) return cuda_status(e);
     if (d.needs_wavefront) {
         const int cfmt = p.chroma_idc == 3 ? 1 : (p.chroma_idc == 2 ? 2 : 0);
-        const int grid = std::max(1, std::min<int>(nd->sms * nd->occ[cfmt], (int)n_ctu));
-        e = hpvcd_launch_recon(dp, (const CtuItem*)(base + L.items), n_ctu, work_counter, d_err, cfmt, grid, 1,
+        // three CTAs per CTU that can be walked at once, one per SM at least
+        const int ready = std::min(g.ctb_rows, (g.ctb_cols + 1) / 2);
+        const int grid = std::max(1, std::min<int>(std::min(nd->sms * nd->occ[cfmt], std::max(3 * ready, nd->sms)), (int)n_ctu));
+        e = hpvcd_launch_recon(dp, (const CtuItem*)(base + L.items), n_ctu, work_counter, d_err, cfmt, grid, 2,
                                (p.ctb_region || (p.flags & (HPVCD_PIC_CONSTRAINED_INTRA | HPVCD_PIC_CROSS_COMPONENT |
                                                            HPVCD_PIC_PCM))) ? 1 : 0,
                                1, 0, st);
