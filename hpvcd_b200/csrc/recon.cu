@@ -2489,21 +2489,38 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 }
             }
         }
-        // ---- how the walk takes each entry, and the blend table: by all warps,
-        // two TBs at a time.  Cb and Cr share one table: their TBs have the
-        // same places, modes and available lines (a CTU where they do not walks
-        // its Cr without the table) ----
+        // ---- how the walk takes each entry, one thread each.  Cb and Cr share a
+        // blend table: their TBs have the same places, modes and available
+        // lines (a CTU where they do not walks its Cr without the table) ----
         if (tid == 0 && listed[1] != listed[2]) *s_diff = 1u;
-        const int half = lane >> 4, l15 = lane & 15;
         for (int c = 0; c < ncomp; ++c) {
-            const int S = c ? Scw : ctb, row = can_row(S);
-            uint32_t* tab = (uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
             uint4* list = ents + lay.ent_off(c);
             const uint4* cb_list = ents + lay.ent_off(1);
             const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
+            for (uint32_t e = tid; e < cnt; e += kThreads) {
+                const TbEntry E{list[e]}, F{list[min(e + 1, cnt - 1)]};
+                const uint32_t f = E.flags();
+                const bool four = (f & kTbPlain) && E.n2() == 8;
+                const bool pair = e + 1 < cnt && four && (F.flags() & kTbPlain) && F.n2() == 8;
+                const uint32_t g = pair ? f | F.flags() : f;
+                list[e].w = (E.w.w & 0xffff3f3fu) | (four ? kHowPlain4 : 0u) | (pair ? kHowTwo : 0u) |
+                            (g & kTbEdge ? kHowEdge : 0u) | (g & kTbPub ? kHowPub : 0u);
+                if (c == 2) {
+                    const uint4 b = cb_list[min(e, listed[1] ? listed[1] - 1 : 0u)];
+                    if (((b.x ^ E.w.x) & 0x7fffffffu) | (b.y ^ E.w.y) | (b.z ^ E.w.z) | ((b.w ^ E.w.w) & kHowPlain)) *s_diff = 1u;
+                }
+            }
+        }
+        // ---- the blend tables, by all warps, two TBs at a time ----
+        const int half = lane >> 4, l15 = lane & 15;
+        for (int c = 0; c < min(ncomp, 2); ++c) {
+            const int S = c ? Scw : ctb, row = can_row(S);
+            uint32_t* tab = (uint32_t*)(smem + lay.off_tab) + lay.tab_off(c);
+            const uint4* list = ents + lay.ent_off(c);
+            const uint32_t cnt = c == 0 ? listed[0] : listed[1];
             // the angular words of the next TB are on their way while one is done
             auto angles = [&](const TbEntry& E, uint32_t (&ang)[4]) {
-                if (c == 2 || !(E.flags() & kTbPlain)) return;
+                if (!(E.flags() & kTbPlain)) return;
                 const bool four = E.n2() == 8;
                 const uint32_t* a = (four ? g_angular.t4[E.mode() - 2] : g_angular.t8[E.mode() - 2]) + l15;
                 ang[0] = a[0];
@@ -2517,7 +2534,6 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 angles(E, ang);
             }
             while (e < cnt) {
-                const TbEntry F{list[min(e + 1, cnt - 1)]};
                 const uint32_t en = e + 2 * kWarps;
                 TbEntry N{};
                 uint32_t ang_n[4] = {0u, 0u, 0u, 0u};
@@ -2525,22 +2541,10 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                     N.w = list[en];
                     angles(N, ang_n);
                 }
-                const uint32_t f = E.flags();
-                const bool plain = (f & kTbPlain) != 0u, four = E.n2() == 8;
-                if (l15 == 0) {
-                    const bool pair = e + 1 < cnt && plain && four && (F.flags() & kTbPlain) && F.n2() == 8;
-                    const uint32_t g = pair ? f | F.flags() : f;
-                    list[e].w = (E.w.w & 0xffff3f3fu) | (plain && four ? kHowPlain4 : 0u) | (pair ? kHowTwo : 0u) |
-                                (g & kTbEdge ? kHowEdge : 0u) | (g & kTbPub ? kHowPub : 0u);
-                    if (c == 2) {
-                        const uint4 b = cb_list[min(e, listed[1] ? listed[1] - 1 : 0u)];
-                        if (((b.x ^ E.w.x) & 0x7fffffffu) | (b.y ^ E.w.y) | (b.z ^ E.w.z) | ((b.w ^ E.w.w) & kHowPlain)) *s_diff = 1u;
-                    }
-                }
-                if (plain && c < 2) {
+                if (E.flags() & kTbPlain) {
                     const Line L(E, row);
                     uint32_t* t = tab + E.tab();
-                    if (four) {
+                    if (E.n2() == 8) {
                         t[l15] = blend_word(L, ang[0]);
                     } else {
 #pragma unroll
