@@ -7,8 +7,8 @@
 // outputs it reaches vertically, so a tile needs 15 horizontal sums a column
 // instead of 64 and every sum is two (8-bit) or four (above) packed dot
 // products over words loaded once.  Then the uni / bi / explicitly weighted
-// combination with clipping (mc.rs:538-736), written into the current
-// picture's plane.  The work is bound by instruction issue and L1 lookups: a
+// combination with clipping (mc.rs:538-736), plus the residual, written into
+// the current picture's plane.  The work is bound by instruction issue and L1 lookups: a
 // 1920x1080 frame of the synthetic GOP took 135 us with one thread per output
 // sample filtering 64 loads.
 #include "common.cuh"
@@ -120,8 +120,8 @@ __device__ __forceinline__ void interp_column(const void* plane, int pw, int ph,
 // One column of a tile of component c: ROWS samples from (x, y) of the plane,
 // of which `rows` are written.
 template <int TAPS, int ROWS, int BPS>
-__device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, int pic_index, const hpvcd_pu& u, int c, int x,
-                                          int y, int rows) {
+__device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, const void* const (*refs)[3], int c, int x, int y,
+                                          int rows) {
     const bool luma = TAPS == 8;
     const int pw = luma ? P.w : P.cw, ph = luma ? P.h : P.ch;
     const int bd = luma ? P.bd : P.bd_c;
@@ -129,14 +129,9 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
     int a[ROWS], b[ROWS];  // the lists found, in turn
     int have = 0;
 #pragma unroll 1
-    for (int l = 0; l < 2; ++l) {  // reference views per list (decode.rs:7040-7120 ref_frame_for_lists)
-        if (!(u.flags & (l ? HPVCD_PU_L1 : HPVCD_PU_L0))) continue;
-        const int ri = u.ref_idx[l];
-        if (ri < 0 || ri >= HPVCD_MAX_REFS) continue;
-        // the host maps references to earlier pictures of the batch (< pic_index)
-        // or to DPB pictures appended after the batch's own; -1 is none
-        const int rp = P.ref_pic[l][ri];
-        if (rp < 0 || rp == pic_index) continue;
+    for (int l = 0; l < 2; ++l) {
+        const void* const ref = refs[l][c];
+        if (!ref) continue;
         have |= 1 << l;
         int ix, iy, fx, fy;
         if (luma) {
@@ -148,7 +143,7 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
             fx = mvcx & 7, fy = mvcy & 7;
         }
         int t[ROWS];
-        interp_column<TAPS, ROWS, BPS>(pics[rp].fin[c], pw, ph, x + ix, y + iy, fx, fy, bd, t);
+        interp_column<TAPS, ROWS, BPS>(ref, pw, ph, x + ix, y + iy, fx, fy, bd, t);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             b[r] = t[r];
@@ -202,21 +197,26 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const DevPic* pics, i
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) v[r] = 1 << (bd - 1);
     }
+    // the residual (k_residual; zero without one) is added here, reconstruct.rs:214-251
     void* dst = P.rec[c];
+    const int rs = P.res_stride[c];
+    const int16_t* res = P.res[c] + (size_t)y * rs + x;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) a[r] = r < rows ? (int)res[(size_t)r * rs] : 0;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
-        if (r < rows) store_sample(dst, BPS, (size_t)(y + r) * pw + x, v[r]);
+        if (r < rows) store_sample(dst, BPS, (size_t)(y + r) * pw + x, clamp3i(v[r] + a[r], 0, mx));
 }
 
 // A CTA takes kMcPus consecutive PUs; blockIdx.y = its share of their tiles
 // (kMcSplit CTAs interleave, so that a run of large PUs does not end up on one
 // SM).  A warp takes four tiles of luma, or of both chroma components, at a
 // time.
-constexpr int kMcPus = 32, kMcSplit = 8, kMcWarps = 8;
+constexpr int kMcPus = 32, kMcSplit = 12, kMcWarps = 8;
 
 template <int BPS>
-__device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, const hpvcd_pu* s_pu, const uint32_t* s_pre) {
-    const DevPic& P = pics[pic_index];
+__device__ __forceinline__ void mc_tiles(const DevPic& P, const hpvcd_pu* s_pu, const uint32_t* s_pre,
+                                         const void* const (*s_ref)[2][3]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, l = lane & 7;
     const uint32_t tiles = s_pre[kMcPus], groups = (tiles + 3) / 4;
     const uint32_t tasks = P.idc ? 2 * groups : groups;
@@ -234,7 +234,7 @@ __device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, cons
         if (luma) {
             const int x = u.x + 8 * tx + l, y = u.y + 8 * ty;
             const int rows = min(min((int)u.h - 8 * ty, 8), P.h - y);
-            if (8 * tx + l < u.w && x < P.w && rows > 0) mc_column<8, 8, BPS>(P, pics, pic_index, u, 0, x, y, rows);
+            if (8 * tx + l < u.w && x < P.w && rows > 0) mc_column<8, 8, BPS>(P, u, s_ref[j], 0, x, y, rows);
         } else {
             const int sw = P.sub_w, sh = P.sub_h, cols = 8 / sw;
             const int ox = cols * tx + (l & (cols - 1)), oy = 8 / sh * ty;
@@ -242,11 +242,11 @@ __device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, cons
             const int rows = min(min(u.h / sh - oy, 8 / sh), P.ch - y);
             if (ox < u.w / sw && x < P.cw && rows > 0) {
                 if (sw == 1) {  // 4:4:4: both components by every lane
-                    for (int c = 1; c < 3; ++c) mc_column<4, 8, BPS>(P, pics, pic_index, u, c, x, y, rows);
+                    for (int c = 1; c < 3; ++c) mc_column<4, 8, BPS>(P, u, s_ref[j], c, x, y, rows);
                 } else if (sh == 1) {
-                    mc_column<4, 8, BPS>(P, pics, pic_index, u, 1 + (l >> 2), x, y, rows);
+                    mc_column<4, 8, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows);
                 } else {
-                    mc_column<4, 4, BPS>(P, pics, pic_index, u, 1 + (l >> 2), x, y, rows);
+                    mc_column<4, 4, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows);
                 }
             }
         }
@@ -256,6 +256,11 @@ __device__ __forceinline__ void mc_tiles(const DevPic* pics, int pic_index, cons
 __global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restrict__ pics, int pic_index) {
     __shared__ hpvcd_pu s_pu[kMcPus];
     __shared__ uint32_t s_pre[kMcPus + 1];  // tiles of the PUs before
+    // reference planes of the PUs by list and component, NULL where there is
+    // none (looked up here once: in the tasks it was two dependent loads before
+    // the first sample)
+    __shared__ const void* s_ref[kMcPus][2][3];
+    static_assert(kMcPus == 32, "one PU per lane");
     const DevPic& P = pics[pic_index];
     const uint32_t first = blockIdx.x * kMcPus;
     if (threadIdx.x < 32) {
@@ -264,6 +269,17 @@ __global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restric
             const hpvcd_pu u = P.pus[first + threadIdx.x];
             s_pu[threadIdx.x] = u;
             n = ((u.w + 7u) >> 3) * ((u.h + 7u) >> 3);
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {  // reference views per list (decode.rs:7040-7120 ref_frame_for_lists)
+                const int ri = u.ref_idx[l];
+                int rp = -1;
+                if ((u.flags & (l ? HPVCD_PU_L1 : HPVCD_PU_L0)) && ri >= 0 && ri < HPVCD_MAX_REFS) rp = P.ref_pic[l][ri];
+                // the host maps references to earlier pictures of the batch (< pic_index)
+                // or to DPB pictures appended after the batch's own; -1 is none
+                if (rp == pic_index) rp = -1;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) s_ref[threadIdx.x][l][c] = rp >= 0 ? pics[rp].fin[c] : nullptr;
+            }
         }
         for (int d = 1; d < kMcPus; d <<= 1) {
             const uint32_t o = __shfl_up_sync(0xffffffffu, n, d);
@@ -274,9 +290,9 @@ __global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restric
     }
     __syncthreads();
     if (P.bps == 1)
-        mc_tiles<1>(pics, pic_index, s_pu, s_pre);
+        mc_tiles<1>(P, s_pu, s_pre, s_ref);
     else
-        mc_tiles<2>(pics, pic_index, s_pu, s_pre);
+        mc_tiles<2>(P, s_pu, s_pre, s_ref);
 }
 
 }  // namespace hpvcd

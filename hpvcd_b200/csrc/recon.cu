@@ -6,9 +6,11 @@
 // Two kernels:
 //
 //  k_residual -- every coded TB of every picture, fully parallel (a lane, eight
-//     lanes or a warp per TB by its size).  TBs whose prediction is already in the plane (inter TBs,
-//     prediction-in-plane pictures) are added and clipped into the plane
-//     right away; intra TBs leave an int16 residual in a residual plane.
+//     lanes or a warp per TB by its size).  The TBs of prediction-in-plane
+//     pictures are added and clipped into the plane right away; all others
+//     leave an int16 residual in a residual plane, which k_recon adds to intra
+//     and motion compensation to inter samples (so the residuals of a sequence
+//     wait for nothing and stay off its frame-to-frame chain).
 //     (for 8-bit the reference itself truncates to i16, transform.rs:55-63;
 //     then every residual is clamped to +-(2^bd - 1), which the clip of the
 //     sum to [0, 2^bd - 1] cannot tell from the full value.)
@@ -697,23 +699,21 @@ __device__ __forceinline__ bool tb_plain(const DevPic& P, const hpvcd_tu& t) {
     return (int)t.x < pw && (int)t.y < ph && (uint64_t)t.coeff_off + (1u << (2 * t.log2n)) <= P.n_coeffs;
 }
 
-// TBs whose prediction is already in the plane (inter TBs and
-// prediction-in-plane pictures); the others leave their residual in the int16
-// residual plane.
-__device__ __forceinline__ bool tb_in_plane(const DevPic& P, const hpvcd_tu& t) {
-    return (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
-}
+// Whether a picture's prediction is already in its planes: its TBs are added
+// there.  Every other TB leaves its residual in the int16 residual plane,
+// which motion compensation (inter TBs) or k_recon (intra TBs) adds.
+__device__ __forceinline__ bool in_plane_of(const DevPic& P) { return (P.flags & HPVCD_PIC_PRED_IN_PLANE) != 0; }
 
 // Residual of one plain 4x4 TB by one thread (the 4x4 case of
 // tb_residual_warp), stored where the warp path stores it: added to the plane
-// and clipped for TBs predicted in the plane, else into the int16 residual
+// and clipped where the prediction is in it, else into the int16 residual
 // plane.
 __device__ void tb4_thread(const DevPic& P, const hpvcd_tu& t) {
     const int c = t.comp;
     const int bd = c ? P.bd_c : P.bd;
     const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
     const int x0 = t.x, y0 = t.y;
-    const bool in_plane = tb_in_plane(P, t);
+    const bool in_plane = in_plane_of(P);
     // the plane's rows are read up front, beside the levels
     int pv[4][4];
     void* pl = P.rec[c];
@@ -867,7 +867,7 @@ __device__ __forceinline__ void tb8_rows(const DevPic& P, const hpvcd_tu& t, int
     const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
     const int x0 = t.x, y = t.y + q;
     if (y >= ph) return;
-    const bool in_plane = tb_in_plane(P, t);
+    const bool in_plane = in_plane_of(P);
     void* pl = P.rec[c];
     const size_t p0 = (size_t)y * pw + x0;
     const bool pvec = in_plane && x0 + 8 <= pw && (p0 & 3) == 0;
@@ -1008,7 +1008,7 @@ __device__ __forceinline__ void tb_tensor(const DevPic& P, const hpvcd_tu& t, in
     const int pw = c ? P.cw : P.w, ph = c ? P.ch : P.h;
     const int x0 = t.x, y0 = t.y;
     const int g = lane >> 2, tq = lane & 3;
-    const bool in_plane = tb_in_plane(P, t);
+    const bool in_plane = in_plane_of(P);
     const bool i16s = bd <= 8;
     const int mx = (1 << bd) - 1, bps = P.bps;
     void* pl = P.rec[c];
@@ -1081,7 +1081,7 @@ __device__ __noinline__ void tb_general(const DevPic& P, const hpvcd_tu& t, cons
         return;
     }
     const int x0 = t.x, y0 = t.y;
-    if (tb_in_plane(P, t)) {  // prediction already in the plane: add + clip (reconstruct.rs:214-251)
+    if (in_plane_of(P)) {  // prediction already in the plane: add + clip (reconstruct.rs:214-251)
         void* pl = P.rec[c];
         const int mx = (1 << (c ? P.bd_c : P.bd)) - 1;
         const int keep = (t.flags & HPVCD_TU_PCM) ? 0 : 1;  // I_PCM samples replace the plane's
@@ -1265,7 +1265,7 @@ k_ccp(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, 
         __syncwarp();
         const int c = t.comp, x0 = t.x, y0 = t.y, pw = P.cw, ph = P.ch;
         const int bdy = P.bd, bdc = P.bd_c, rs = t.res_scale;
-        const bool in_plane = (P.flags & HPVCD_PIC_PRED_IN_PLANE) || !(t.flags & HPVCD_TU_INTRA);
+        const bool in_plane = in_plane_of(P);
         const int mx = (1 << bdc) - 1;
         auto out = [&](int r, int m, long long v) {
             const long long sy = ((long long)ry[r * n + m] << bdc) >> bdy;

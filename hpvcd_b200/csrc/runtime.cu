@@ -258,6 +258,9 @@ struct hpvcd_plan {
     // concurrent segments (independent pictures): one stream per segment,
     // forked from and joined back into the launching stream
     bool concurrent = false;
+    // a sequence (one segment per picture): the residuals of every picture
+    // but the first are computed beside the first one's wavefront
+    bool sequence = false;
     GroupStreams own;                  // used when the plan is not lent a set
     const GroupStreams* gs = nullptr;  // the set the launches use
 
@@ -274,13 +277,20 @@ struct hpvcd_plan {
             if ((src[i].flags & HPVCD_PIC_CROSS_COMPONENT) && src[i].n_tus) return true;
         return false;
     }
+    // whether a picture after the first segment has
+    bool rest_ccp() const {
+        for (size_t i = 1; i < segs.size(); ++i)
+            if (seg_ccp(segs[i])) return true;
+        return false;
+    }
     uint32_t launches_for(uint32_t stages) const {
         uint32_t L = 0;
         for (const auto& s : segs) {
             if (stages & HPVCD_STAGE_RECON) {
                 for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics; ++i)
                     if ((src[i].flags & HPVCD_PIC_INTER) && src[i].n_pus) ++L;
-                if (rec_prefix[s.first_pic + s.n_pics] > rec_prefix[s.first_pic]) L += 1 + seg_ccp(s);
+                const uint32_t last = sequence ? (&s == &segs[0] ? s.first_pic + s.n_pics : 0u) : s.first_pic + s.n_pics;
+                if (last && rec_prefix[last] > rec_prefix[s.first_pic]) L += 1 + seg_ccp(s);
                 for (uint32_t w = s.wave_first; w < s.wave_first + s.n_waves; ++w) L += waves[w].n_items > 0;
             }
             if ((stages & kFilterStages) == kFilterStages) {
@@ -292,6 +302,10 @@ struct hpvcd_plan {
             if ((stages & HPVCD_STAGE_SAO) && s.max_sao > 0) ++L;
             if (concurrent && (stages & HPVCD_STAGE_OUTPUT) && canvas_kind(out.kind) && s.max_rgb > 0)
                 L += (uint32_t)any_rgb_canvas + (uint32_t)any_native_canvas;
+        }
+        if (sequence && (stages & HPVCD_STAGE_RECON)) {
+            const uint32_t first = segs[0].first_pic + segs[0].n_pics;
+            if (rec_prefix[src.size()] > rec_prefix[first]) L += 1 + rest_ccp();
         }
         if (!concurrent && (stages & HPVCD_STAGE_OUTPUT) && canvas_kind(out.kind) && max_rgb > 0)
             L += (stages & kFilterStages) == kFilterStages
@@ -586,6 +600,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
             P->concurrent = P->segs.size() > 1;
         }
     }
+    P->sequence = any_inter && P->segs.size() > 1;
     // ---- wavefront schedule per segment and format class: CTUs sorted by
     // (x + 2y, picture, y) ----
     for (uint32_t si = 0; si < P->segs.size(); ++si) {
@@ -816,7 +831,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
             return cuda_status(fe);
         }
     }
-    if (P->concurrent) {
+    if (P->concurrent || P->sequence) {
         GroupStreams* set = lend ? lend : &P->own;
         const cudaError_t ce = set->create();
         if (ce != cudaSuccess) {
@@ -857,6 +872,32 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
         }
     }
     const cudaStream_t origin = st;
+    // Residual planes of inter pictures start at zero: motion compensation adds
+    // them to every sample, coded or not.
+    auto clear_residual = [&](uint32_t i, cudaStream_t s) -> cudaError_t {
+        if (!(P->src[i].flags & HPVCD_PIC_INTER) || !P->src[i].n_pus) return cudaSuccess;
+        return cudaMemsetAsync(P->pics[i].res[0], 0, res_plane_bytes(geo_of(P->src[i])), s);
+    };
+    auto residuals = [&](uint32_t first, uint32_t end, bool ccp, cudaStream_t s) -> cudaError_t {
+        const uint32_t nrec = P->rec_prefix[end] - P->rec_prefix[first];
+        cudaError_t r = cudaSuccess;
+        for (uint32_t i = first; i < end && r == cudaSuccess; ++i) r = clear_residual(i, s);
+        if (r == cudaSuccess)
+            r = hpvcd_launch_residual(P->d_pics + first, P->d_prefix + first, end - first, nrec, d_err, P->sms,
+                                      (int)P->sched.idct, s);
+        if (r == cudaSuccess && nrec && ccp)
+            r = hpvcd_launch_ccp(P->d_pics + first, P->d_prefix + first, end - first, nrec, d_err, P->sms, s);
+        return r;
+    };
+    const bool beside = P->sequence && (stages & HPVCD_STAGE_RECON);
+    if (beside) {  // the later pictures' residuals beside the first picture
+        const uint32_t first = P->segs[0].first_pic + P->segs[0].n_pics;
+        e = cudaEventRecord(P->gs->ev_fork, origin);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(P->gs->aux[0], P->gs->ev_fork, 0);
+        if (e == cudaSuccess) e = residuals(first, (uint32_t)P->src.size(), P->rest_ccp(), P->gs->aux[0]);
+        if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_join[0], P->gs->aux[0]);
+        if (e != cudaSuccess) return cuda_status(e);
+    }
     if (P->concurrent) {  // fork: every segment's stream starts after the work above
         e = cudaEventRecord(P->gs->ev_fork, origin);
         for (uint32_t si = 0; si < n_seg && e == cudaSuccess; ++si)
@@ -868,17 +909,13 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
         const DevPic* dp = P->d_pics + s.first_pic;
         if (P->concurrent) st = P->gs->aux[si];
         if (stages & HPVCD_STAGE_RECON) {
-            for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics; ++i)
-                if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus) {
+            if (beside && si == 1)
+                e = cudaStreamWaitEvent(origin, P->gs->ev_join[0], 0);
+            else if (!beside || si == 0)
+                e = residuals(s.first_pic, s.first_pic + s.n_pics, P->seg_ccp(s), st);
+            for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics && e == cudaSuccess; ++i)
+                if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus)
                     e = hpvcd_launch_mc(P->d_pics, (int)i, (int)P->src[i].n_pus, P->src[i].chroma_idc ? 3 : 1, st);
-                    if (e != cudaSuccess) return cuda_status(e);
-                }
-            const uint32_t nrec = P->rec_prefix[s.first_pic + s.n_pics] - P->rec_prefix[s.first_pic];
-            e = hpvcd_launch_residual(P->d_pics + s.first_pic, P->d_prefix + s.first_pic, s.n_pics, nrec, d_err,
-                                      P->sms, (int)P->sched.idct, st);
-            if (e == cudaSuccess && nrec && P->seg_ccp(s))
-                e = hpvcd_launch_ccp(P->d_pics + s.first_pic, P->d_prefix + s.first_pic, s.n_pics, nrec, d_err,
-                                     P->sms, st);
             if (e != cudaSuccess) return cuda_status(e);
             // the segment's format classes one after another, each wave with
             // its own layout and work counter
