@@ -1481,26 +1481,26 @@ __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
 }
 
 // Stages the visible part of a coded n x n TB's residual (written by
-// k_residual) into the TB's own canvas area with asynchronous copies issued
-// by one lane: 16 bytes per copy, 8 for 4x4 TBs.  Every coded TB of a CTU is
-// staged before its walk starts (the lanes of the walking warp take the
-// list entries in turn).  The area of a TB not yet reconstructed is never an
-// available reference sample of an earlier TB (its stamp is later), so the
-// staged values are never read as samples; each lane predicting a sample
-// reads its residual in place.
-__device__ __forceinline__ void stage_residual(const Comp& k, int log2n, int x0, int y0) {
-    const int n = 1 << log2n;
+// k_residual) into the TB's own canvas area with asynchronous copies, the
+// lanes of a warp side by side: 16 bytes per copy, 8 for 4x4 TBs.  Every coded
+// TB of a CTU is staged before its walk starts.  The area of a TB not yet
+// reconstructed is never an available reference sample of an earlier TB (its
+// stamp is later), so the staged values are never read as samples; each lane
+// predicting a sample reads its residual in place.
+__device__ __forceinline__ void stage_residual(const Comp& k, int n, int x0, int y0, int lane) {
     const int vw = min(n, k.pw - (k.ox + x0)), vh = min(n, k.ph - (k.oy + y0));
     const int16_t* src = k.res + (size_t)y0 * k.rs + x0;
     uint16_t* dst = k.can + cin(k, x0, y0);
     const int cr = can_row(k.S);
     if (n == 4) {
-        for (int r = 0; r < vh; ++r) cp_async8(dst + r * cr, src + (size_t)r * k.rs);
+        if (lane < vh) cp_async8(dst + lane * cr, src + (size_t)lane * k.rs);
         return;
     }
-    const int chunks = (vw + 7) >> 3;
-    for (int r = 0; r < vh; ++r)
-        for (int q = 0; q < chunks; ++q) cp_async16(dst + r * cr + 8 * q, src + (size_t)r * k.rs + 8 * q);
+    const int lq = 28 - __clz(n);  // 8-sample chunks of a row
+    for (int i = lane; i < vh << lq; i += 32) {
+        const int r = i >> lq, q = 8 * (i & ((1 << lq) - 1));
+        if (q < vw) cp_async16(dst + r * cr + q, src + (size_t)r * k.rs + q);
+    }
 }
 
 // ---- edges between neighbouring CTUs ----
@@ -2461,8 +2461,8 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
         // every sample of the CTU comes from the walk, so the whole visible
         // residual block of each component is copied by all threads (the areas
         // of uncoded TBs are never read); in an inter picture the canvas holds
-        // inter samples, so only the areas of coded intra TBs are staged (one
-        // lane of the walking warp each) ----
+        // inter samples, so only the areas of coded intra TBs are staged (a warp
+        // each) ----
         if (!(P.flags & HPVCD_PIC_INTER)) {
             for (int c = 0; c < ncomp; ++c) {
                 const int S = c ? Scw : ctb, Sh = c ? Sch : ctb, ox = c ? ocx : oxl, oy = c ? ocy : oyl;
@@ -2477,15 +2477,13 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 }
             }
         } else {
-            for (int c = c_lo; c <= c_hi && c < ncomp; ++c) {
+            for (int c = 0; c < ncomp; ++c) {
                 const Comp k = comp_of(c);
                 const uint4* list = ents + lay.ent_off(c);
                 const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
-                for (uint32_t e = lane; e < cnt; e += 32) {
-                    TbEntry E;
-                    E.w = list[e];
-                    if (E.coded() && !(E.flags() & kTbPcm))
-                        stage_residual(k, 31 - __clz(E.n2()) - 1, E.x(), E.y());
+                for (uint32_t e = warp; e < cnt; e += kWarps) {
+                    const TbEntry E{list[e]};
+                    if (E.coded() && !(E.flags() & kTbPcm)) stage_residual(k, E.n2() >> 1, E.x(), E.y(), lane);
                 }
             }
         }
