@@ -2611,35 +2611,33 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 bw = tab[(h.y >> 16) + l15];
                 how = how_of(0);
             }
+            // Samples s of the half-warps' 4x4 TBs that lie on the CTU's right
+            // column or bottom row.
+            auto publish4 = [&](int s, uint32_t entry) {
+                const TbEntry E{list[entry]};
+                uint16_t* const w16 = (uint16_t*)words;
+                const int x = E.x() + (lane & 3), y = E.y() + (l15 >> 2);
+                const uint16_t t = (uint16_t)(s | 0x8000);
+                if (x == k.S - 1) st_edge16(w16 + y, t);
+                if (y == k.Sh - 1) st_edge16(w16 + k.Sh + x, t);
+            };
             for (uint32_t e = 0; e < cnt;) {
-                if (how & kHowPlain4) {
-                    const bool two = (how & kHowTwo) != 0u;
-                    const uint32_t next = e + (two ? 2u : 1u);
-                    if (how & kHowEdge) await(TbEntry{list[two ? e + half : e]});
+                if (how & kHowTwo) {
+                    if (how & kHowEdge) await(TbEntry{list[e + half]});
                     uint16_t* const px = can + (place & 0xffffu) + px4;
-                    // (without a second TB lanes 16..31 hold another kind of TB's word: table offset 0, read only)
                     const int rv = (place & kTbCoded) ? (int)(int16_t)*px : 0;
                     int s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);
                     if (half == 0) *px = (uint16_t)s;
-                    const uint2 h = fetch(next);
-                    const uint32_t hn = how_of(next);
+                    const uint2 h = fetch(e + 2);
+                    const uint32_t hn = how_of(e + 2);
                     __syncwarp();
-                    if (two) {
-                        s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
-                        if (half) *px = (uint16_t)s;
-                    }
+                    s = __viaddmin_s32_relu(blend_of(can, bw), rv, max_v);  // (the first TB's lanes: the same again)
+                    if (half) *px = (uint16_t)s;
                     place = h.x;
                     bw = tab[(h.y >> 16) + l15];
-                    if ((how & kHowPub) && (two || half == 0)) {  // samples on the CTU's right column / bottom row
-                        const TbEntry E{list[e + half]};
-                        uint16_t* const w16 = (uint16_t*)words;
-                        const int x = E.x() + (lane & 3), y = E.y() + (l15 >> 2);
-                        const uint16_t t = (uint16_t)(s | 0x8000);
-                        if (x == k.S - 1) st_edge16(w16 + y, t);
-                        if (y == k.Sh - 1) st_edge16(w16 + k.Sh + x, t);
-                    }
+                    if (how & kHowPub) publish4(s, e + half);
                     how = hn;
-                    e = next;
+                    e += 2;
                     __syncwarp();
                     continue;
                 }
@@ -2648,7 +2646,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 TbEntry E{list[e]};
                 if (how & kHowEdge) await(E);
                 const int n2 = E.n2();
-                if (how & kHowPlain) {
+                if ((how & kHowPlain) && !(how & kHowPlain4)) {
                     walk_plain8(can, (uint32_t*)(can + E.org() + px8), *(const uint2*)(tab + E.tab() + tab8), E.coded(),
                                 max_v);
                 } else {
