@@ -6,6 +6,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <new>
 #include <thread>
@@ -223,8 +224,8 @@ struct hpvcd_plan {
         bool inter;  // some of its pictures predict from others
     };
     std::vector<Wave> waves;
-    // k_recon CTAs per SM by class and build (1 two warps, 2 three warps,
-    // 3 three warps register-capped; index build - 1)
+    // k_recon CTAs per SM by class and build (1 one walking warp for both
+    // chroma components, 2 and 3 one each; index build - 1)
     int occ[3][3] = {{1, 1, 1}, {1, 1, 1}, {1, 1, 1}};
     // Build of a wave's wavefront kernel (hpvcd_sched.chroma_warps; 0, the
     // default, is one warp per chroma component: 24 mixed images 4305 us
@@ -846,7 +847,14 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
     return HPVCD_OK;
 }
 
-hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
+// What a caller enqueues on the launching stream around the concurrent
+// segments of a launch: `inputs` before a segment starts (its stream waits for
+// it), `outputs` once it has joined back, in segment order.
+struct SegmentHooks {
+    std::function<cudaError_t(uint32_t)> inputs, outputs;
+};
+
+hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const SegmentHooks* hooks = nullptr) {
     cudaError_t e = cudaSuccess;
     // Work counters, the device error word and the wavefront edge words are
     // reset by every launch that reconstructs.
@@ -898,16 +906,16 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
         if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_join[0], P->gs->aux[0]);
         if (e != cudaSuccess) return cuda_status(e);
     }
-    if (P->concurrent) {  // fork: every segment's stream starts after the work above
-        e = cudaEventRecord(P->gs->ev_fork, origin);
-        for (uint32_t si = 0; si < n_seg && e == cudaSuccess; ++si)
-            e = cudaStreamWaitEvent(P->gs->aux[si], P->gs->ev_fork, 0);
-        if (e != cudaSuccess) return cuda_status(e);
-    }
     for (uint32_t si = 0; si < n_seg; ++si) {
         const Segment& s = P->segs[si];
         const DevPic* dp = P->d_pics + s.first_pic;
-        if (P->concurrent) st = P->gs->aux[si];
+        if (P->concurrent) {  // fork: the segment's stream starts after the work above and its inputs
+            if (hooks && hooks->inputs) e = hooks->inputs(si);
+            if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_fork, origin);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(P->gs->aux[si], P->gs->ev_fork, 0);
+            if (e != cudaSuccess) return cuda_status(e);
+            st = P->gs->aux[si];
+        }
         if (stages & HPVCD_STAGE_RECON) {
             if (beside && si == 1)
                 e = cudaStreamWaitEvent(origin, P->gs->ev_join[0], 0);
@@ -955,12 +963,16 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st) {
                     e = hpvcd_launch_yuv_canvas(dp, (int)s.n_pics, s.max_rgb, P->d_canvas, st);
                 if (e != cudaSuccess) return cuda_status(e);
             }
-            e = cudaEventRecord(P->gs->ev_join[si], st);  // join back into the launching stream
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(origin, P->gs->ev_join[si], 0);
+            e = cudaEventRecord(P->gs->ev_join[si], st);
             if (e != cudaSuccess) return cuda_status(e);
         }
     }
     st = origin;
+    for (uint32_t si = 0; P->concurrent && si < n_seg; ++si) {  // join back into the launching stream
+        e = cudaStreamWaitEvent(origin, P->gs->ev_join[si], 0);
+        if (e == cudaSuccess && hooks && hooks->outputs) e = hooks->outputs(si);
+        if (e != cudaSuccess) return cuda_status(e);
+    }
     if (!P->concurrent && (stages & HPVCD_STAGE_OUTPUT) && canvas_kind(P->out.kind)) {
         if (P->any_rgb_canvas && !fused)
             e = hpvcd_launch_rgb(P->d_pics, (int)P->src.size(), P->max_rgb, P->d_canvas, st);
@@ -1712,20 +1724,26 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     if (st == HPVCD_OK && !direct_out) st = grow_pinned(&slot->h_out, &slot->h_out_cap, out_bytes);
     if (st != HPVCD_OK) return st;
     cudaError_t e = cudaSuccess;
-    if (all_pinned) {
-        for (const Run& r : runs) {
-            e = cudaMemcpyAsync(slot->d_in + r.off, r.src, r.bytes, cudaMemcpyHostToDevice, slot->stream);
-            if (e != cudaSuccess) break;
+    // Enqueues the upload of arena bytes [b0, b1) (ranges in ascending order).
+    std::vector<hpvcd_host::CopyTask> tasks;
+    size_t pi = 0, part_done = 0;
+    auto upload = [&](size_t b0, size_t b1) -> cudaError_t {
+        cudaError_t r = cudaSuccess;
+        if (all_pinned) {
+            for (const Run& run : runs) {
+                const size_t a = std::max(b0, run.off), b = std::min(b1, run.off + run.bytes);
+                if (a >= b) continue;
+                r = cudaMemcpyAsync(slot->d_in + a, run.src + (a - run.off), b - a, cudaMemcpyHostToDevice, slot->stream);
+                if (r != cudaSuccess) break;
+            }
+            return r;
         }
-    } else {
         // Staged through the slot's page-locked buffer in windows of
         // kStageWindow bytes: the copy pool fills window k + 1 while window
         // k's DMA runs.  Parts are laid out in ascending offsets.
         constexpr size_t kStageWindow = 8u << 20;
-        std::vector<hpvcd_host::CopyTask> tasks;
-        size_t w0 = 0, pi = 0, part_done = 0;
-        while (w0 < total && e == cudaSuccess) {
-            const size_t w1 = std::min(total, w0 + kStageWindow);
+        for (size_t w0 = b0; w0 < b1 && r == cudaSuccess;) {
+            const size_t w1 = std::min(b1, w0 + kStageWindow);
             tasks.clear();
             while (pi < parts.size() && parts[pi].off + part_done < w1) {
                 const InputPart& pt = parts[pi];
@@ -1739,10 +1757,20 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
                 }
             }
             hpvcd_host::parallel_copy(tasks.data(), tasks.size());
-            e = cudaMemcpyAsync(slot->d_in + w0, slot->h_in + w0, w1 - w0, cudaMemcpyHostToDevice, slot->stream);
+            r = cudaMemcpyAsync(slot->d_in + w0, slot->h_in + w0, w1 - w0, cudaMemcpyHostToDevice, slot->stream);
             w0 = w1;
         }
-    }
+        return r;
+    };
+    // A batch of the layout before whose segments run concurrently uploads its
+    // inputs segment by segment, each segment starting as soon as its own are
+    // there (4032x3024 grid from page-locked memory and back: 1838 us with
+    // every copy before and after the decode).  The segments are those of
+    // the plan; a prediction copied into the planes, or features computed on
+    // the device, need every input first.
+    bool by_segment = reuse && slot->plan->concurrent && !g->sel;
+    for (uint32_t i = 0; i < n; ++i) by_segment = by_segment && !(pics[i].flags & HPVCD_PIC_PRED_IN_PLANE);
+    if (!by_segment) e = upload(0, total);
     if (e != cudaSuccess) return cuda_status(e);
     for (const InputPart& pt : parts) point_at(dev[pt.pic], pt.kind, slot->d_in + pt.off);
     slot->wp.assign(n, hpvcd_wp_table{});
@@ -1811,19 +1839,12 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     // wait for their neighbour CTUs in place, holding slots the other
     // tickets' kernels need).  At three tickets in flight on the 4032x3024
     // grid the share is worth about 15 % of throughput; a ticket alone keeps
-    // the full grid.  Sharing, the default build is the register-capped one:
-    // eight CTAs per SM split between the tickets instead of five (at four
-    // tickets in flight one CTA per SM each with the plain build, a quarter
-    // of that per group of the grid, fewer than the group's ready CTUs).
-    // With two CTAs per SM per ticket the quadrant-level wavefront also pays
-    // while sharing (four grids in flight: 1.19 against 1.29 ms per image
-    // with whole-CTU waits, same box).
+    // the full grid.
     {
         if (others > 0) {
             hpvcd_sched s2 = slot->plan->sched;
             const hpvcd_plan* pl = slot->plan;
-            if (s2.chroma_warps == 0) s2.chroma_warps = 3;
-            const int occ = std::max(1, pl->occ_of(pl->waves.empty() ? 0 : pl->waves[0].cfmt, (int)s2.chroma_warps));
+            const int occ = std::max(1, pl->occ_of(pl->waves.empty() ? 0 : pl->waves[0].cfmt, pl->build_of()));
             const int share = std::max(1, occ / (others + 1));
             const int cur = s2.recon_ctas_per_sm ? (int)s2.recon_ctas_per_sm : occ;
             s2.recon_ctas_per_sm = (uint32_t)std::min(cur, share);
@@ -1840,31 +1861,70 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
             if (we != cudaSuccess) return cuda_status(we);
         }
     }
-    st = plan_launch(slot->plan, HPVCD_STAGE_ALL, slot->stream);
-    if (st != HPVCD_OK) return st;
-    st = dpb_after_launch(g, slot, slot_idx, pics, n);
-    if (st != HPVCD_OK) return st;
-    // ---- output copy back ----
+    // ---- launch and output copy back; the output of concurrent segments goes
+    // back as they finish: the bytes before the first one a later segment writes ----
     hpvcd_plan* P = slot->plan;
     unsigned char* host_out = direct_out && !per_canvas_out ? (unsigned char*)out->host_dst : slot->h_out;
     slot->direct_out = direct_out ? (per_canvas_out ? (void*)1 : out->host_dst) : nullptr;
-    if (per_canvas_out) {  // each canvas straight into its own buffer
-        for (size_t k = 0; k < P->canvases.size() && e == cudaSuccess; ++k)
-            e = cudaMemcpyAsync(out->canvas_dst[k], P->d_canvas + P->canvas_offs[k], P->canvas_sizes[k],
-                                cudaMemcpyDeviceToHost, slot->stream);
-    } else if (canvas_kind(P->out.kind)) {
-        e = cudaMemcpyAsync(host_out, P->d_canvas, P->canvas_bytes, cudaMemcpyDeviceToHost, slot->stream);
-    } else {
-        size_t o = 0;
-        for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) {
-            const Geo geo = geo_of(pics[i]);
-            for (int c = 0; c < (pics[i].chroma_idc ? 3 : 1) && e == cudaSuccess; ++c) {
+    size_t copied = 0;        // canvas bytes, or pictures, copied so far
+    size_t plane_bytes = 0;   // plane bytes of the pictures copied so far
+    auto copy_canvas = [&](size_t upto) -> cudaError_t {
+        cudaError_t r = cudaSuccess;
+        if (per_canvas_out) {  // each canvas straight into its own buffer
+            for (size_t k = 0; k < P->canvases.size() && r == cudaSuccess; ++k) {
+                const size_t a = std::max<size_t>(copied, P->canvas_offs[k]),
+                             b = std::min<size_t>(upto, P->canvas_offs[k] + P->canvas_sizes[k]);
+                if (a < b)
+                    r = cudaMemcpyAsync((unsigned char*)out->canvas_dst[k] + (a - P->canvas_offs[k]), P->d_canvas + a, b - a,
+                                        cudaMemcpyDeviceToHost, slot->stream);
+            }
+        } else if (copied < upto) {
+            r = cudaMemcpyAsync(host_out + copied, P->d_canvas + copied, upto - copied, cudaMemcpyDeviceToHost, slot->stream);
+        }
+        copied = std::max(copied, upto);
+        return r;
+    };
+    auto copy_planes = [&](size_t upto) -> cudaError_t {
+        cudaError_t r = cudaSuccess;
+        for (; copied < upto && r == cudaSuccess; ++copied) {
+            const Geo geo = geo_of(pics[copied]);
+            for (int c = 0; c < (pics[copied].chroma_idc ? 3 : 1) && r == cudaSuccess; ++c) {
                 const size_t b = c ? geo.chroma_bytes : geo.luma_bytes;
-                e = cudaMemcpyAsync(host_out + o, P->pics[i].fin[c], b, cudaMemcpyDeviceToHost, slot->stream);
-                o += b;
+                r = cudaMemcpyAsync(host_out + plane_bytes, P->pics[copied].fin[c], b, cudaMemcpyDeviceToHost, slot->stream);
+                plane_bytes += b;
             }
         }
-    }
+        return r;
+    };
+    const bool to_canvas = canvas_kind(P->out.kind);
+    SegmentHooks hooks;
+    if (by_segment)
+        hooks.inputs = [&](uint32_t si) -> cudaError_t {
+            const uint32_t first = P->segs[si].first_pic, end = first + P->segs[si].n_pics;
+            size_t b0 = total, b1 = total;  // the first byte of the segment's parts and of the next one's
+            for (const InputPart& pt : parts) {
+                if (pt.pic >= first) b0 = std::min(b0, pt.off);
+                if (pt.pic >= end) b1 = std::min(b1, pt.off);
+            }
+            return upload(b0, b1);
+        };
+    hooks.outputs = [&](uint32_t si) -> cudaError_t {
+        const uint32_t end = P->segs[si].first_pic + P->segs[si].n_pics;
+        if (!to_canvas) return copy_planes(end);
+        size_t upto = P->canvas_bytes;
+        for (uint32_t i = end; i < n; ++i) {
+            const DevPic& d = P->pics[i];
+            const bool moved = d.orientation > (int)HPVCD_ORIENT_NORMAL;
+            const size_t sample = d.matrix == (int)HPVCD_CANVAS_NATIVE ? (size_t)d.bps : 3;
+            upto = std::min(upto, (size_t)d.canvas_off + (moved ? 0 : (size_t)d.dst_y * d.canvas_w * sample));
+        }
+        return copy_canvas(upto);
+    };
+    st = plan_launch(P, HPVCD_STAGE_ALL, slot->stream, &hooks);
+    if (st != HPVCD_OK) return st;
+    st = dpb_after_launch(g, slot, slot_idx, pics, n);
+    if (st != HPVCD_OK) return st;
+    e = to_canvas ? copy_canvas(P->canvas_bytes) : copy_planes(n);
     if (e == cudaSuccess) e = cudaEventRecord(slot->done, slot->stream);
     if (e != cudaSuccess) return cuda_status(e);
     slot->busy = true;
