@@ -1106,29 +1106,32 @@ __device__ __noinline__ void tb_general(const DevPic& P, const hpvcd_tu& t, cons
 // Classes of coded records, in the order their warp tasks are taken: the
 // longest first, so that the last tasks of a CTA are short.
 constexpr int kCls32 = 0, kCls16 = 1, kClsGeneral = 2, kCls8 = 3, kCls4 = 4, kClasses = 5;
-constexpr uint32_t kResMaxChunk = 256;  // records of a CTA step (one per thread)
+constexpr uint32_t kResMaxChunk = 1024;  // records of a CTA step
 
-// One CTA takes `chunk` consecutive records at a time: every thread loads one,
-// finds its picture (one search per CTA, then a short walk) and files it
-// under its class; the warps then take tasks off the class lists: one 32x32,
-// 16x16 or general TB, four 8x8 (eight lanes each) or thirty-two 4x4 (one
-// lane each).  What bounds a launch is the latency of its longest chain of
-// tasks, so the chunk is chosen by the record count (hpvcd_launch_residual)
-// to spread small pictures over all SMs.  One warp taking 32 consecutive
-// records one after another, one sample per lane and step, took 150 us on
-// any picture of 512x512 and up; the whole call on a residual-only 512x512
-// picture went from 191 to 38.5 us, the 4032x3024 grid from 1522 to 1373 us.
+// One CTA takes `chunk` consecutive records at a time and sorts them by class
+// (the picture of the first by one search, of the others by a short walk from
+// it); the warps then take tasks off the sorted list: one 32x32, 16x16 or
+// general TB, four 8x8 (eight lanes each) or thirty-two 4x4 (one lane each).
+// What bounds a launch on a small picture is the latency of its longest chain
+// of tasks, so the chunk is chosen by the record count (hpvcd_launch_residual)
+// to spread it over all SMs; on a large one the warps wait for instructions
+// first (the stall before any other at 256 records a step), and a long sorted
+// list keeps the warps of an SM in the same code: up to 1024 records a step
+// instead of 256 took the whole call on 24 mixed pictures from 4115 to 3940 us
+// and the 1920x1080 sequence from 2480 to 2421, and left the residual-only
+// 512x512 picture at 41 (40 before: one phase more).  One warp taking 32
+// consecutive records one after another, one sample per lane and step, took
+// 150 us on any picture of 512x512 and up (whole call 185 us).
 template <int kIdct>
 __global__ void __launch_bounds__(kResWarps * 32, 4)
 k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_prefix, uint32_t n_pics,
            uint32_t* dev_err, uint32_t chunk) {
     __shared__ __align__(16) BasisTables basis;
     __shared__ __align__(16) int16_t scr[kResWarps][2 * 32 * kScr];  // per warp
-    __shared__ __align__(16) uint4 s_rec[kResMaxChunk];
-    __shared__ uint32_t s_pic[kResMaxChunk];
-    __shared__ uint8_t s_list[kClasses][kResMaxChunk];
+    __shared__ uint32_t s_pic[kResMaxChunk];   // picture of a record
+    __shared__ uint16_t s_list[kResMaxChunk];  // records by class
     __shared__ uint32_t s_cnt[kClasses], s_next;
-    static_assert(kResMaxChunk <= kResWarps * 32, "one record per thread");
+    constexpr int kPerThread = kResMaxChunk / (kResWarps * 32);
     static_assert(tensor_stride(32) * 32 <= 2 * 32 * kScr, "the tensor path's block fits the scratch");
     stage_table(&basis, &g_basis, (int)sizeof(basis));
     constexpr unsigned kAll = 0xffffffffu;
@@ -1139,35 +1142,52 @@ k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_pre
         if (threadIdx.x < kClasses) s_cnt[threadIdx.x] = 0u;
         if (threadIdx.x == kClasses) s_next = 0u;
         __syncthreads();
-        const uint32_t gl = g0 + threadIdx.x;
-        if (threadIdx.x < chunk && gl < total) {
-            uint32_t pic = 0, hi = n_pics;
-            while (hi - pic > 1) {  // the picture of the step's first record (uniform)
-                const uint32_t mid = (pic + hi) >> 1;
-                if (rec_prefix[mid] <= g0) pic = mid; else hi = mid;
-            }
+        uint32_t pic = 0;
+        for (uint32_t hi = n_pics; hi - pic > 1;) {  // the picture of the step's first record (uniform)
+            const uint32_t mid = (pic + hi) >> 1;
+            if (rec_prefix[mid] <= g0) pic = mid; else hi = mid;
+        }
+        uint32_t cls[kPerThread], place[kPerThread];  // a record's class and its place there
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u) {
+            const uint32_t i = u * (kResWarps * 32) + threadIdx.x, gl = g0 + i;
+            cls[u] = kClasses;
+            if (i >= chunk || gl >= total) continue;
             while (rec_prefix[pic + 1] <= gl) ++pic;
             const DevPic& P = pics[pic];
             const uint4 r4 = *(const uint4*)(P.tus + (gl - rec_prefix[pic]));  // records are 16-byte aligned
             hpvcd_tu t;
             memcpy(&t, &r4, sizeof(t));
-            if (t.flags & HPVCD_TU_CBF) {
-                int cls = kClsGeneral;
-                if (tb_plain(P, t)) {
-                    if (t.log2n <= 3)
-                        cls = t.log2n == 2 ? kCls4 : kCls8;
-                    else if (kIdct == kIdctTensor && (t.x & 1) == 0)
-                        cls = t.log2n == 4 ? kCls16 : kCls32;
-                }
-                s_rec[threadIdx.x] = r4;
-                s_pic[threadIdx.x] = pic;
-                s_list[cls][atomicAdd(&s_cnt[cls], 1u)] = (uint8_t)threadIdx.x;
+            if (!(t.flags & HPVCD_TU_CBF)) continue;
+            cls[u] = kClsGeneral;
+            if (tb_plain(P, t)) {
+                if (t.log2n <= 3)
+                    cls[u] = t.log2n == 2 ? kCls4 : kCls8;
+                else if (kIdct == kIdctTensor && (t.x & 1) == 0)
+                    cls[u] = t.log2n == 4 ? kCls16 : kCls32;
             }
+            s_pic[i] = pic;
+            place[u] = atomicAdd(&s_cnt[cls[u]], 1u);
         }
         __syncthreads();
         const uint32_t e32 = s_cnt[kCls32], e16 = e32 + s_cnt[kCls16], eg = e16 + s_cnt[kClsGeneral];
         const uint32_t n8 = s_cnt[kCls8], n4 = s_cnt[kCls4];
         const uint32_t e8 = eg + (n8 + 3) / 4, e4 = e8 + (n4 + 31) / 32;
+#pragma unroll
+        for (int u = 0; u < kPerThread; ++u) {
+            if (cls[u] == kClasses) continue;
+            place[u] += cls[u] == kCls32 ? 0u : cls[u] == kCls16 ? e32 : cls[u] == kClsGeneral ? e16 : cls[u] == kCls8 ? eg : eg + n8;
+            s_list[place[u]] = (uint16_t)(u * (kResWarps * 32) + threadIdx.x);
+        }
+        __syncthreads();
+        // the record at place k of the sorted list, and its picture
+        auto record = [&](uint32_t k, hpvcd_tu& t) -> const DevPic& {
+            const uint32_t i = s_list[k], pi = s_pic[i];
+            const DevPic& P = pics[pi];
+            const uint4 r4 = *(const uint4*)(P.tus + (g0 + i - rec_prefix[pi]));
+            memcpy(&t, &r4, sizeof(t));
+            return P;
+        };
         for (;;) {
             uint32_t task = 0;
             if (lane == 0) task = atomicAdd(&s_next, 1u);
@@ -1175,13 +1195,10 @@ k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_pre
             if (task >= e4) break;
             hpvcd_tu t;
             if (task < eg) {
-                const int cls = task < e32 ? kCls32 : (task < e16 ? kCls16 : kClsGeneral);
-                const uint32_t j = s_list[cls][task - (cls == kCls32 ? 0u : (cls == kCls16 ? e32 : e16))];
-                memcpy(&t, &s_rec[j], sizeof(t));
-                const DevPic& P = pics[s_pic[j]];
-                if (kIdct == kIdctTensor && cls == kCls32)
+                const DevPic& P = record(task, t);
+                if (kIdct == kIdctTensor && task < e32)
                     tb_tensor<32>(P, t, scr[warp], basis.frags, lane);
-                else if (kIdct == kIdctTensor && cls == kCls16)
+                else if (kIdct == kIdctTensor && task < e16)
                     tb_tensor<16>(P, t, scr[warp], basis.frags, lane);
                 else
                     tb_general<kIdct == kIdctButterfly ? kIdctButterfly : kIdctMatrix>(P, t, basis.dct, scr[warp],
@@ -1189,9 +1206,7 @@ k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_pre
             } else if (task < e8) {
                 const uint32_t k = (task - eg) * 4 + (lane >> 3);
                 const int q = lane & 7;
-                const uint32_t j = k < n8 ? s_list[kCls8][k] : s_list[kCls8][0];
-                memcpy(&t, &s_rec[j], sizeof(t));
-                const DevPic& P = pics[s_pic[j]];
+                const DevPic& P = record(eg + min(k, n8 - 1), t);
                 int16_t* S = scr[warp] + (lane >> 3) * 72;
                 if (k < n8) tb8_cols(P, t, q, S);
                 __syncwarp();
@@ -1200,9 +1215,8 @@ k_residual(const DevPic* __restrict__ pics, const uint32_t* __restrict__ rec_pre
             } else {
                 const uint32_t k = (task - e8) * 32 + lane;
                 if (k < n4) {
-                    const uint32_t j = s_list[kCls4][k];
-                    memcpy(&t, &s_rec[j], sizeof(t));
-                    tb4_thread(pics[s_pic[j]], t);
+                    const DevPic& P = record(eg + n8 + k, t);
+                    tb4_thread(P, t);
                 }
                 __syncwarp();
             }
@@ -2731,12 +2745,14 @@ extern "C" cudaError_t hpvcd_launch_residual(const hpvcd::DevPic* pics, const ui
                                              int sms, int idct, cudaStream_t stream) {
     if (total_records == 0) return cudaSuccess;
     // Records of a CTA step: at least kResMinChunk (a warp's worth), doubled
-    // while twice as many still give every SM two CTAs, so that a small
-    // picture spreads over the whole chip and a large one fills the lanes of
-    // its 4x4 tasks.
+    // while twice as many still give every SM a step, so that a small picture
+    // spreads over the whole chip and a large one fills the lanes of its 4x4
+    // tasks and keeps to one class for long (4032x3024 grid, whole call: 559
+    // us, 571 with two steps per SM and 604 with four; 24 mixed pictures
+    // 3937 to 3951 in all three).
     constexpr uint32_t kResMinChunk = 32;
     uint32_t chunk = kResMinChunk;
-    while (chunk < hpvcd::kResMaxChunk && total_records / (2 * chunk) >= 2u * (uint32_t)sms) chunk *= 2;
+    while (chunk < hpvcd::kResMaxChunk && total_records / (2 * chunk) >= (uint32_t)sms) chunk *= 2;
     const uint32_t steps = (total_records + chunk - 1) / chunk;
     const uint32_t cap = (uint32_t)sms * 4u;  // resident CTAs
     const int grid = (int)(steps < cap ? steps : cap), threads = hpvcd::kResWarps * 32;

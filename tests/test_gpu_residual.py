@@ -99,3 +99,15 @@ def test_added_in_plane(w, h, depth):
     s.add(synth.intra_cfg(1, w, h, bit_depth=depth))
     s.add(synth.inter_cfg(2, w, h, bit_depth=depth, intra_cu_p=0.5))
     check(s.pictures())
+
+
+# a launch large enough for the longest sorted lists, over pictures whose ends
+# fall inside a CTA step and beside others of a few records
+def test_long_lists():
+    s = synth.SynthSet()
+    for i in range(13):
+        s.add(synth.residual_cfg(70 + i, 1016 + 8 * (i % 3), 776, bit_depth=8 + 2 * (i & 1), chroma_idc=3))
+        s.add(synth.residual_cfg(90 + i, 16, 8))
+    pics = s.pictures()
+    assert sum(p.n_tus for p in pics) > 2 * 148 * 1024
+    check(pics)
