@@ -1,16 +1,18 @@
 // mc.cu -- motion compensation (mc.rs + decode.rs:7000-7488 motion_compensate).
 //
 // PUs are cut into 8x8 luma tiles (and the chroma they cover).  Eight lanes
-// take a tile, one column each: a lane filters its column's rows horizontally
-// (8-tap luma quarter-pel, 4-tap chroma eighth-pel, mc.rs:351-530, edge-clamped
-// reference fetch mc.rs:310) and adds each row's 14-bit intermediate to the
-// outputs it reaches vertically, so a tile needs 15 horizontal sums a column
-// instead of 64 and every sum is two (8-bit) or four (above) packed dot
-// products over words loaded once.  Then the uni / bi / explicitly weighted
-// combination with clipping (mc.rs:538-736), plus the residual, written into
-// the current picture's plane.  The work is bound by instruction issue and L1 lookups: a
-// 1920x1080 frame of the synthetic GOP took 135 us with one thread per output
-// sample filtering 64 loads.
+// take a tile: together they copy the reference blocks of both lists to shared
+// memory in 16-byte chunks (asynchronously, so that a tile waits for memory
+// once), then one column each, a lane filters its column's rows horizontally
+// (8-tap luma quarter-pel, 4-tap chroma eighth-pel, mc.rs:351-530) and adds
+// each row's 14-bit intermediate to the outputs it reaches vertically, so a
+// tile needs 15 horizontal sums a column instead of 64 and every sum is two
+// (8-bit) or four (above) packed dot products.  Then the uni / bi / explicitly
+// weighted combination with clipping (mc.rs:538-736), plus the residual,
+// written into the current picture's plane.  Bound by memory latency at 32
+// warps an SM, then by instruction issue (0.52 a cycle).  A 1920x1080 frame of
+// the synthetic GOP: 135 us with one thread per output sample filtering 64
+// loads, 55 with each lane loading its own rows, 43 with the shared blocks.
 #include "common.cuh"
 
 namespace hpvcd {
@@ -40,52 +42,59 @@ __device__ __forceinline__ int dot2hi(uint32_t a, uint32_t b, int c) {
     return d;
 }
 
-// The same words column by column, the picture's first and last column
-// repeated (rare, and kept out of the unrolled rows: the kernel's code already
-// fills the instruction cache).
-template <int TAPS, int BPS>
-__device__ __noinline__ uint4 fetch_clamped(const void* plane, int pw, int x, int y) {
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    const size_t row = (size_t)y * pw;
-#pragma unroll
-    for (int i = 0; i < TAPS; ++i)
-        w[i * BPS / 4] |= (uint32_t)load_sample(plane, BPS, row + clamp3i(x + i, 0, pw - 1)) << (8 * BPS * (i & (4 / BPS - 1)));
-    return make_uint4(w[0], w[1], w[2], w[3]);
-}
+// The reference block of a tile of LANES columns: every row as the 16-byte
+// chunks that hold its LANES + TAPS - 1 samples, kept at their own alignment.
+template <int TAPS, int LANES, int BPS>
+struct Block {
+    static constexpr int kCols = LANES + TAPS - 1, kChunks = (kCols * BPS + 15 - BPS) / 16 + 1;
+    static constexpr int kRowBytes = 16 * kChunks;
+};
+// bytes of an eight-lane group's block of one list (16-bit luma: 15 rows of
+// 48; 16-bit 4:2:2 chroma: two components of 11 rows of 32); the groups of a
+// warp start in different banks
+constexpr int kBlockBytes = 720, kHalfBlock = 352, kMcWarps = 8;
+constexpr int kListBytes = 4 * kMcWarps * kBlockBytes;  // all groups' blocks of one list
 
-// TAPS samples of a row starting at column x, packed in words (four 8-bit or
-// two 16-bit samples each).  Inside the picture by aligned 32-bit loads (rows
-// and planes are multiples of four samples from an aligned start, so a word
-// holding a sample of the plane lies inside it).
-template <int TAPS, int BPS>
-__device__ __forceinline__ void fetch_row(const void* plane, int pw, int x, int y, bool inside,
-                                          uint32_t (&w)[TAPS * BPS / 4]) {
-    constexpr int W = TAPS * BPS / 4;
-    if (inside) {
-        const uintptr_t a = (uintptr_t)plane + ((size_t)y * pw + x) * BPS;
-        const uint32_t* q = (const uint32_t*)(a & ~(uintptr_t)3);
-        const int sh = (int)(a & 3) * 8;
-        uint32_t r[W + 1];
+// Start to fetch the block's rows from (x, y), column 0 of lane 0 with its
+// taps, by its LANES lanes together; outside the picture sample by sample, the
+// first and last row and column repeated (mc.rs:310).
+template <int TAPS, int ROWS, int LANES, int BPS>
+__device__ __forceinline__ void fetch_block(const void* plane, int pw, int ph, int x, int y, char* buf, int q) {
+    using B = Block<TAPS, LANES, BPS>;
+    constexpr int kRows = ROWS + TAPS - 1, kLoads = (kRows * B::kChunks + LANES - 1) / LANES;
+    const uintptr_t col = (uintptr_t)plane + (intptr_t)x * BPS;
+    if (x >= 0 && x + B::kCols <= pw) {
 #pragma unroll
-        for (int i = 0; i < W; ++i) r[i] = q[i];
-        r[W] = sh ? q[W] : 0u;
-#pragma unroll
-        for (int i = 0; i < W; ++i) w[i] = __funnelshift_r(r[i], r[i + 1], sh);
+        for (int k = 0; k < kLoads; ++k) {
+            const int i = q + k * LANES, r = i / B::kChunks, j = i - r * B::kChunks;
+            const uintptr_t a = col + (size_t)clamp3i(y + r, 0, ph - 1) * pw * BPS;
+            // an aligned chunk that holds a sample of the plane lies in its allocation
+            if (r < kRows && 16 * j < (int)(a & 15) + B::kCols * BPS) {
+                const uint32_t d = (uint32_t)__cvta_generic_to_shared(buf + 16 * i);
+                const uintptr_t from = (a & ~(uintptr_t)15) + 16 * j;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(from) : "memory");
+            }
+        }
     } else {
-        const uint4 v = fetch_clamped<TAPS, BPS>(plane, pw, x, y);
-        const uint32_t t[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < W; ++i) w[i] = t[i];
+#pragma unroll 1
+        for (int i = q; i < kRows * B::kCols; i += LANES) {
+            const int r = i / B::kCols, c = i - r * B::kCols;
+            const size_t row = (size_t)clamp3i(y + r, 0, ph - 1) * pw;
+            char* d = buf + r * B::kRowBytes + (int)((col + row * BPS) & 15) + c * BPS;
+            const int smp = load_sample(plane, BPS, row + clamp3i(x + c, 0, pw - 1));
+            if (BPS == 1) *(uint8_t*)d = (uint8_t)smp; else *(uint16_t*)d = (uint16_t)smp;
+        }
     }
 }
 
-// The 14-bit intermediates (int16) of ROWS vertically adjacent samples whose
-// first reference sample is (x, y).  A zero fraction is the tap 64 alone,
-// which gives the reference's unfiltered cases exactly: (64 r) >> (bd - 8) loses
-// no bit for bd <= 14, and (64 h) >> 6 = h.
-template <int TAPS, int ROWS, int BPS>
+// The 14-bit intermediates (int16) of ROWS vertically adjacent samples of lane
+// q's column; (x, y) is the reference sample of lane 0's first.  A zero
+// fraction is the tap 64 alone, which gives the reference's unfiltered cases
+// exactly: (64 r) >> (bd - 8) loses no bit for bd <= 14, and (64 h) >> 6 = h.
+template <int TAPS, int ROWS, int LANES, int BPS>
 __device__ __forceinline__ void interp_column(const void* plane, int pw, int ph, int x, int y, int fx, int fy, int bd,
-                                              int (&out)[ROWS]) {
+                                              const char* buf, int q, int (&out)[ROWS]) {
+    using B = Block<TAPS, LANES, BPS>;
     constexpr int back = TAPS / 2 - 1, W = TAPS * BPS / 4;
     const int s1 = bd - 8;
     const uint32_t h0 = TAPS == 8 ? c_luma_filter[fx][0] : c_chroma_filter[fx], h1 = TAPS == 8 ? c_luma_filter[fx][1] : 0u;
@@ -95,11 +104,16 @@ __device__ __forceinline__ void interp_column(const void* plane, int pw, int ph,
     for (int t = 0; t < TAPS; ++t) vt[t] = t < 4 ? tap(v0, t) : tap(v1, t & 3);
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) out[r] = 0;
-    const bool inside = x - back >= 0 && x - back + TAPS <= pw;
+    const uint32_t col = (uint32_t)(uintptr_t)plane + (uint32_t)((x - back) * BPS), pitch = (uint32_t)(pw * BPS);
 #pragma unroll
     for (int r = 0; r < ROWS + TAPS - 1; ++r) {
-        uint32_t w[W];
-        fetch_row<TAPS, BPS>(plane, pw, x - back, clamp3i(y - back + r, 0, ph - 1), inside, w);
+        const uint32_t at = ((col + (uint32_t)clamp3i(y - back + r, 0, ph - 1) * pitch) & 15u) + q * BPS;
+        const uint32_t* src = (const uint32_t*)(buf + r * B::kRowBytes) + (at >> 2);
+        uint32_t w[W + 1];
+#pragma unroll
+        for (int i = 0; i <= W; ++i) w[i] = src[i];
+#pragma unroll
+        for (int i = 0; i < W; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], 8 * (at & 3));
         int h;
         if constexpr (BPS == 1) {
             h = dot4(w[0], h0, 0);
@@ -117,23 +131,22 @@ __device__ __forceinline__ void interp_column(const void* plane, int pw, int ph,
     for (int r = 0; r < ROWS; ++r) out[r] = (int)(int16_t)(out[r] >> 6);
 }
 
-// One column of a tile of component c: ROWS samples from (x, y) of the plane,
-// of which `rows` are written.
-template <int TAPS, int ROWS, int BPS>
+// Lane q's column of a tile of component c whose first sample is (x, y): ROWS
+// samples, of which `rows` are written (none by a lane outside the PU).  The
+// tile's LANES lanes come here together.
+template <int TAPS, int ROWS, int LANES, int BPS>
 __device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, const void* const (*refs)[3], int c, int x, int y,
-                                          int rows) {
-    const bool luma = TAPS == 8;
+                                          int rows, char* buf) {
+    const int q = threadIdx.x & (LANES - 1);
+    const unsigned group = ((1u << LANES) - 1) << (threadIdx.x & 31 & ~(LANES - 1));
+    static_assert((ROWS + TAPS - 1) * Block<TAPS, LANES, BPS>::kRowBytes <= (LANES == 8 ? kBlockBytes : kHalfBlock),
+                  "the block fits its group's bytes");
+    constexpr bool luma = TAPS == 8;
+    constexpr int back = TAPS / 2 - 1;
     const int pw = luma ? P.w : P.cw, ph = luma ? P.h : P.ch;
     const int bd = luma ? P.bd : P.bd_c;
     const int mx = (1 << bd) - 1;
-    int a[ROWS], b[ROWS];  // the lists found, in turn
-    int have = 0;
-#pragma unroll 1
-    for (int l = 0; l < 2; ++l) {
-        const void* const ref = refs[l][c];
-        if (!ref) continue;
-        have |= 1 << l;
-        int ix, iy, fx, fy;
+    auto vector = [&](int l, int& ix, int& iy, int& fx, int& fy) {
         if (luma) {
             ix = u.mv[l][0] >> 2, iy = u.mv[l][1] >> 2;
             fx = u.mv[l][0] & 3, fy = u.mv[l][1] & 3;
@@ -142,8 +155,29 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, co
             ix = mvcx >> 3, iy = mvcy >> 3;
             fx = mvcx & 7, fy = mvcy & 7;
         }
+    };
+    __syncwarp(group);  // the blocks before are read
+#pragma unroll 1
+    for (int l = 0; l < 2; ++l) {
+        const void* const ref = refs[l][c];
+        if (!ref) continue;
+        int ix, iy, fx, fy;
+        vector(l, ix, iy, fx, fy);
+        fetch_block<TAPS, ROWS, LANES, BPS>(ref, pw, ph, x + ix - back, y + iy - back, buf + l * kListBytes, q);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp(group);
+    int a[ROWS], b[ROWS];  // the lists found, in turn
+    int have = 0;
+#pragma unroll 1
+    for (int l = 0; l < 2; ++l) {
+        const void* const ref = refs[l][c];
+        if (!ref) continue;
+        have |= 1 << l;
+        int ix, iy, fx, fy;
+        vector(l, ix, iy, fx, fy);
         int t[ROWS];
-        interp_column<TAPS, ROWS, BPS>(ref, pw, ph, x + ix, y + iy, fx, fy, bd, t);
+        interp_column<TAPS, ROWS, LANES, BPS>(ref, pw, ph, x + ix, y + iy, fx, fy, bd, buf + l * kListBytes, q, t);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             b[r] = t[r];
@@ -200,26 +234,27 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, co
     // the residual (k_residual; zero without one) is added here, reconstruct.rs:214-251
     void* dst = P.rec[c];
     const int rs = P.res_stride[c];
-    const int16_t* res = P.res[c] + (size_t)y * rs + x;
+    const int16_t* res = P.res[c] + (size_t)y * rs + x + q;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) a[r] = r < rows ? (int)res[(size_t)r * rs] : 0;
 #pragma unroll
     for (int r = 0; r < ROWS; ++r)
-        if (r < rows) store_sample(dst, BPS, (size_t)(y + r) * pw + x, clamp3i(v[r] + a[r], 0, mx));
+        if (r < rows) store_sample(dst, BPS, (size_t)(y + r) * pw + x + q, clamp3i(v[r] + a[r], 0, mx));
 }
 
 // A CTA takes kMcPus consecutive PUs; blockIdx.y = its share of their tiles
 // (kMcSplit CTAs interleave, so that a run of large PUs does not end up on one
 // SM).  A warp takes four tiles of luma, or of both chroma components, at a
 // time.
-constexpr int kMcPus = 32, kMcSplit = 12, kMcWarps = 8;
+constexpr int kMcPus = 32, kMcSplit = 12;
 
 template <int BPS>
 __device__ __forceinline__ void mc_tiles(const DevPic& P, const hpvcd_pu* s_pu, const uint32_t* s_pre,
-                                         const void* const (*s_ref)[2][3]) {
+                                         const void* const (*s_ref)[2][3], char* block) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, l = lane & 7;
     const uint32_t tiles = s_pre[kMcPus], groups = (tiles + 3) / 4;
     const uint32_t tasks = P.idc ? 2 * groups : groups;
+    char* buf = block + (threadIdx.x >> 3) * kBlockBytes;
     for (uint32_t t = blockIdx.y * kMcWarps + warp; t < tasks; t += kMcSplit * kMcWarps) {
         const bool luma = t < groups;
         const uint32_t tile = (luma ? t : t - groups) * 4 + g;
@@ -232,28 +267,28 @@ __device__ __forceinline__ void mc_tiles(const DevPic& P, const hpvcd_pu* s_pu, 
         const int k = (int)(tile - s_pre[j]), tw = (u.w + 7) >> 3;
         const int ty = k / tw, tx = k - ty * tw;
         if (luma) {
-            const int x = u.x + 8 * tx + l, y = u.y + 8 * ty;
-            const int rows = min(min((int)u.h - 8 * ty, 8), P.h - y);
-            if (8 * tx + l < u.w && x < P.w && rows > 0) mc_column<8, 8, BPS>(P, u, s_ref[j], 0, x, y, rows);
+            const int x = u.x + 8 * tx, y = u.y + 8 * ty;
+            const int rows = 8 * tx + l < u.w && x + l < P.w ? min(min((int)u.h - 8 * ty, 8), P.h - y) : 0;
+            mc_column<8, 8, 8, BPS>(P, u, s_ref[j], 0, x, y, rows, buf);
         } else {
-            const int sw = P.sub_w, sh = P.sub_h, cols = 8 / sw;
-            const int ox = cols * tx + (l & (cols - 1)), oy = 8 / sh * ty;
+            const int sw = P.sub_w, sh = P.sub_h, cols = 8 / sw, q = l & (cols - 1);
+            const int ox = cols * tx, oy = 8 / sh * ty;
             const int x = u.x / sw + ox, y = u.y / sh + oy;
-            const int rows = min(min(u.h / sh - oy, 8 / sh), P.ch - y);
-            if (ox < u.w / sw && x < P.cw && rows > 0) {
-                if (sw == 1) {  // 4:4:4: both components by every lane
-                    for (int c = 1; c < 3; ++c) mc_column<4, 8, BPS>(P, u, s_ref[j], c, x, y, rows);
-                } else if (sh == 1) {
-                    mc_column<4, 8, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows);
-                } else {
-                    mc_column<4, 4, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows);
-                }
+            const int rows = ox + q < u.w / sw && x + q < P.cw ? min(min(u.h / sh - oy, 8 / sh), P.ch - y) : 0;
+            char* half = buf + (l >> 2) * kHalfBlock;
+            if (sw == 1) {  // 4:4:4: both components by every lane
+                for (int c = 1; c < 3; ++c) mc_column<4, 8, 8, BPS>(P, u, s_ref[j], c, x, y, rows, buf);
+            } else if (sh == 1) {
+                mc_column<4, 8, 4, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows, half);
+            } else {
+                mc_column<4, 4, 4, BPS>(P, u, s_ref[j], 1 + (l >> 2), x, y, rows, half);
             }
         }
     }
 }
 
 __global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restrict__ pics, int pic_index) {
+    __shared__ __align__(16) char block[2 * kListBytes];
     __shared__ hpvcd_pu s_pu[kMcPus];
     __shared__ uint32_t s_pre[kMcPus + 1];  // tiles of the PUs before
     // reference planes of the PUs by list and component, NULL where there is
@@ -290,17 +325,15 @@ __global__ void __launch_bounds__(32 * kMcWarps, 4) k_mc(const DevPic* __restric
     }
     __syncthreads();
     if (P.bps == 1)
-        mc_tiles<1>(P, s_pu, s_pre, s_ref);
+        mc_tiles<1>(P, s_pu, s_pre, s_ref, block);
     else
-        mc_tiles<2>(P, s_pu, s_pre, s_ref);
+        mc_tiles<2>(P, s_pu, s_pre, s_ref, block);
 }
 
 }  // namespace hpvcd
 
-extern "C" cudaError_t hpvcd_launch_mc(const hpvcd::DevPic* pics, int pic_index, int n_pus, int n_comp,
-                                       cudaStream_t stream) {
+extern "C" cudaError_t hpvcd_launch_mc(const hpvcd::DevPic* pics, int pic_index, int n_pus, cudaStream_t stream) {
     if (n_pus <= 0) return cudaSuccess;
-    (void)n_comp;
     dim3 grid((n_pus + hpvcd::kMcPus - 1) / hpvcd::kMcPus, hpvcd::kMcSplit);
     hpvcd::k_mc<<<grid, 32 * hpvcd::kMcWarps, 0, stream>>>(pics, pic_index);
     hpvcd_note_launches(1);

@@ -37,7 +37,7 @@ extern "C" cudaError_t hpvcd_launch_rgb(const DevPic*, int, int, uint8_t*, cudaS
 extern "C" cudaError_t hpvcd_launch_yuv_canvas(const DevPic*, int, int, uint8_t*, cudaStream_t);
 extern "C" cudaError_t hpvcd_launch_filter_tile(const DevPic*, int, int, int, int, uint8_t*, cudaStream_t);
 extern "C" cudaError_t hpvcd_filter_tile_setup();
-extern "C" cudaError_t hpvcd_launch_mc(const DevPic*, int, int, int, cudaStream_t);
+extern "C" cudaError_t hpvcd_launch_mc(const DevPic*, int, int, cudaStream_t);
 extern "C" hpvcd_status hpvcd_mlp_pick(hpvcd_mlp*, const float*, uint32_t, void*, uint32_t*);
 extern "C" uint32_t hpvcd_mlp_variants(const hpvcd_mlp*);
 extern "C" cudaError_t hpvcd_launch_features(const DevPic*, uint32_t, uint32_t, unsigned long long*, float*, int,
@@ -923,7 +923,7 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
                 e = residuals(s.first_pic, s.first_pic + s.n_pics, P->seg_ccp(s), st);
             for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics && e == cudaSuccess; ++i)
                 if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus)
-                    e = hpvcd_launch_mc(P->d_pics, (int)i, (int)P->src[i].n_pus, P->src[i].chroma_idc ? 3 : 1, st);
+                    e = hpvcd_launch_mc(P->d_pics, (int)i, (int)P->src[i].n_pus, st);
             if (e != cudaSuccess) return cuda_status(e);
             // the segment's format classes one after another, each wave with
             // its own layout and work counter
