@@ -37,7 +37,7 @@ struct DevPic {
     // final picture after SAO (equal to `rec` when SAO does not run).
     void* rec[3];
     void* fin[3];
-    int16_t* res[3];        // int16 residual planes of intra TBs (k_residual -> k_recon)
+    int16_t* res[3];        // int16 residual planes (k_residual -> k_recon, k_mc)
     int32_t res_stride[3];  // row stride of res[c] in samples (multiple of 16)
     unsigned long long* edges;  // wavefront: edge words of every CTU (edge_words_per_ctu), zero at launch
     // output placement on its RGB canvas

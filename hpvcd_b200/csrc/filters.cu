@@ -109,21 +109,6 @@ struct GLines {
     __device__ int ld(int line, int tap) const { return load_sample(p, bps, (size_t)(base + line * ls + tap * ts)); }
     __device__ void st(int line, int tap, int v) const { store_sample(p, bps, (size_t)(base + line * ls + tap * ts), v); }
 };
-struct SLines {
-    uint16_t* p;
-    int ls, ts;
-    __device__ SLines(const SPlane& r, bool vertical, int edge, int scan)
-        : p(r.s + (vertical ? (scan - r.y0) * r.rw + (edge - r.x0) : (edge - r.y0) * r.rw + (scan - r.x0))),
-          ls(vertical ? r.rw : 1), ts(vertical ? 1 : r.rw) {}
-    __device__ int ld(int line, int tap) const { return p[line * ls + tap * ts]; }
-    __device__ void st(int line, int tap, int v) const { p[line * ls + tap * ts] = (uint16_t)v; }
-};
-__device__ __forceinline__ GLines lines_of(const GPlane& g, bool vertical, int edge, int scan) {
-    return GLines(g, vertical, edge, scan);
-}
-__device__ __forceinline__ SLines lines_of(const SPlane& r, bool vertical, int edge, int scan) {
-    return SLines(r, vertical, edge, scan);
-}
 
 // Luma segment: 8 taps x 4 lines around the edge (tap -4..3 = p3..p0,
 // q0..q3).  The decision reads lines 0 and 3; each line is then loaded,
@@ -144,7 +129,7 @@ __device__ __forceinline__ void luma_segment(const DevPic& P, bool vertical, int
     const int beta = c_beta[clamp3i(avg + 2 * bo, 0, 51)] << sh;
     const int tc = c_tc[clamp3i(avg + 2 * (bs - 1) + 2 * to, 0, 53)] << sh;
     if (tc == 0) return;
-    const auto L = lines_of(pl, vertical, edge, scan);
+    const GLines L(pl, vertical, edge, scan);
     // deblock.rs:216-238 luma_decision (lines 0 and 3)
     int dp[2], dq[2], far[2], near_[2];
 #pragma unroll
@@ -241,7 +226,7 @@ __device__ void chroma_segment(const DevPic& P, bool vertical, int edge, int sca
         const int qc = qpc_map(avg + off, P.idc, P.bd_c);
         const int tc = c_tc[clamp3i(qc + 2 + 2 * to, 0, 53)] << sh;
         if (tc == 0) continue;
-        const auto L = lines_of(plane == 0 ? cb : cr, vertical, edge, scan);
+        const GLines L(plane == 0 ? cb : cr, vertical, edge, scan);
         for (int s = scan; s < scan + 4; ++s) {
             if (s >= scan_max) continue;
             const int l = s - scan;

@@ -2852,8 +2852,8 @@ int g_attr_occ[kAttrDevices][3][3];
 }  // namespace
 
 // CTAs per SM of the wavefront kernel with the layout of `cfmt` in build
-// `chroma_warps` (1 two warps, 2 three warps, 3 three warps register-capped;
-// 0 counts as 2); the first call on a device sets the attributes of every
+// `chroma_warps` (1 one walking warp for both chroma components, 2 and 3 one
+// each; 0 counts as 2); the first call on a device sets the attributes of every
 // instantiation (recon_attrs) and of the residual kernel.
 extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
     const int build = chroma_warps >= 1 && chroma_warps <= 3 ? chroma_warps : 2;

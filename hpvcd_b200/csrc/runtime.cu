@@ -1764,8 +1764,8 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     };
     // A batch of the layout before whose segments run concurrently uploads its
     // inputs segment by segment, each segment starting as soon as its own are
-    // there (4032x3024 grid from page-locked memory and back: 1838 us with
-    // every copy before and after the decode).  The segments are those of
+    // there (4032x3024 grid from page-locked memory and back: 1500 us, 1838
+    // with every copy before or after the decode).  The segments are those of
     // the plan; a prediction copied into the planes, or features computed on
     // the device, need every input first.
     bool by_segment = reuse && slot->plan->concurrent && !g->sel;

@@ -458,7 +458,7 @@ hpvcd_status hpvcd_gpu_set_dpb(hpvcd_gpu* ctx, hpvcd_dpb* dpb);
 /* ------------------------------------------------------------------------ */
 /* Device-buffer API (plans).  The picture descriptors point at device      */
 /* memory that stays valid while the plan lives.  A plan owns its own        */
-/* device scratch (work queues, wavefront progress words, ping-pong        */
+/* device scratch (work queues, wavefront edge words, ping-pong            */
 /* planes) and output.                                                     */
 /* hpvcd_plan_launch only enqueues kernels on `stream` (no allocation, no    */
 /* synchronisation), so it can be captured into a CUDA graph.               */
@@ -482,17 +482,14 @@ typedef struct hpvcd_sched {
                                    tensor-core products (int16 operands split exactly into int8
                                    halves), 1 even-odd butterflies, 2 matrix product with all-zero
                                    rows / columns skipped */
-    uint32_t chroma_warps;      /* build of the wavefront kernel: 2 one warp per chroma component
-                                   (three warps per CTA), 1 one warp for Cb, then Cr (two warps
-                                   per CTA: more CTAs per SM), 3 three warps with at most 80
-                                   registers per thread (8 CTAs per SM instead of 5: for batches
-                                   with thousands of CTUs ready at once), 0 three warps, the
-                                   register-capped build for a wave with more CTUs ready at once
-                                   than the plain build's CTAs hold */
+    uint32_t chroma_warps;      /* build of the wavefront kernel: 2 (and 3, and the default 0) one
+                                   walking warp per chroma component (four warps per CTA with luma
+                                   and edges), 1 one for Cb, then Cr (three warps per CTA: more CTAs
+                                   per SM) */
     uint32_t recon_ctas_per_sm; /* persistent wavefront CTAs per SM (0 -> occupancy max) */
-    uint32_t wave;              /* wavefront synchronisation: 0 per quadrant (a CTU is walked while
-                                   its left / above-right neighbours still are), 1 whole CTUs (one
-                                   wait per CTU: fewer polls when tickets share the SMs) */
+    uint32_t wave;              /* wavefront synchronisation: 0 per TB (a CTU is walked while its
+                                   neighbours still are), 1 whole CTUs (every edge sample before the
+                                   first TB) */
 } hpvcd_sched;
 
 hpvcd_status hpvcd_plan_create(const hpvcd_picture* dev_pics, uint32_t n,
@@ -609,7 +606,8 @@ hpvcd_status hpvcd_plan_select(hpvcd_plan* plan, hpvcd_mlp* mlp, const hpvcd_sch
 /* the decoder a fixed share of HBM, or a frame loop in which a cudaMalloc / */
 /* cudaFree (which synchronise the device) would stall other streams.       */
 /* ------------------------------------------------------------------------ */
-/* Bytes of the fixed scratch array each device holds for this entry point:
+/* Bytes of the fixed scratch array each device holds for this entry point
+ * (the wavefront's edge words have a fixed array of their own):
  * enough for every picture up to 1024x1024 luma samples (any chroma format,
  * bit depth, deblocking and SAO). */
 #define HPVCD_NOALLOC_SCRATCH_BYTES (12u * 1024u * 1024u + 256u * 1024u)
@@ -619,10 +617,10 @@ hpvcd_status hpvcd_plan_select(hpvcd_plan* plan, hpvcd_mlp* mlp, const hpvcd_sch
  * unused for 4:0:0), each 256-byte aligned, unpadded (luma stride = width *
  * bytes per sample, as hpvcd_plan_planes).  Enqueues its kernels on `stream`
  * and returns; allocates no memory of any kind.  Its scratch (work counter,
- * error word, wavefront progress words, picture record, CTU list, residual and
- * pre-SAO planes) is one fixed array in the library's device memory; the
- * call itself zeroes the counter, error word and progress words on `stream`
- * before use, and nothing else needs to start at zero.
+ * error word, picture record, CTU list, residual and pre-SAO planes, and
+ * beside them the wavefront's edge words, 2.5 MiB) is fixed arrays in the
+ * library's device memory; the call itself zeroes the counter, error word and
+ * edge words on `stream` before use, and nothing else needs to start at zero.
  *   - The first call on a device does the set-up (looks up the array's
  *     address, sets the kernel's shared-memory limit) with that device
  *     current; make it before any stream capture.
