@@ -133,12 +133,14 @@ __device__ __forceinline__ void interp_column(const void* plane, int pw, int ph,
 
 // Lane q's column of a tile of component c whose first sample is (x, y): ROWS
 // samples, of which `rows` are written (none by a lane outside the PU).  The
-// tile's LANES lanes come here together.
+// eight lanes of a group come here together, one tile of eight lanes or two of
+// four.
 template <int TAPS, int ROWS, int LANES, int BPS>
 __device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, const void* const (*refs)[3], int c, int x, int y,
                                           int rows, char* buf) {
     const int q = threadIdx.x & (LANES - 1);
     const unsigned group = ((1u << LANES) - 1) << (threadIdx.x & 31 & ~(LANES - 1));
+    const unsigned owners = 0xffu << (threadIdx.x & 24);  // the eight lanes whose tiles share buf
     static_assert((ROWS + TAPS - 1) * Block<TAPS, LANES, BPS>::kRowBytes <= (LANES == 8 ? kBlockBytes : kHalfBlock),
                   "the block fits its group's bytes");
     constexpr bool luma = TAPS == 8;
@@ -156,7 +158,9 @@ __device__ __forceinline__ void mc_column(const DevPic& P, const hpvcd_pu& u, co
             fx = mvcx & 7, fy = mvcy & 7;
         }
     };
-    __syncwarp(group);  // the blocks before are read
+    // The blocks before are read, by every lane that shares the bytes: a chroma
+    // tile's four lanes write where all eight read a luma block.
+    __syncwarp(owners);
 #pragma unroll 1
     for (int l = 0; l < 2; ++l) {
         const void* const ref = refs[l][c];
