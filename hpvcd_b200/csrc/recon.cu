@@ -2380,7 +2380,11 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 memcpy(&t, &recs[i], sizeof(t));
                 int x, y;
                 if ((t.flags & HPVCD_TU_INTRA) && intra_pred_ok && rec_check(t, x, y) == 1) {
-                    if (t.mode > 34 || t.log2n > 5) {
+                    // The walk stages, reads and writes a TB's samples in words
+                    // of up to 16 bytes, and its edge words four samples at a
+                    // time: only a TB at a multiple of its size (the only places
+                    // a coding quadtree has) is listed.
+                    if (t.mode > 34 || t.log2n > 5 || ((x | y) & ((1 << t.log2n) - 1))) {
                         atomicOr(dev_err, DEV_ERR_BITSTREAM);
                     } else {
                         tc = t.comp;

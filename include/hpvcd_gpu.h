@@ -90,7 +90,8 @@ typedef enum hpvcd_status {
  *   is how the end of an inter CU is signalled (decode.rs:6546-6548).  Such a
  *   record may have log2n up to 6.
  *
- * x, y are in samples of the component plane.  For 4:2:0, a group of four 4x4
+ * x, y are in samples of the component plane; an intra TB lies at a multiple of
+ * its size (others are HPVCD_ERR_BITSTREAM).  For 4:2:0, a group of four 4x4
  * luma TBs is followed by one 4x4 chroma TB per chroma component at the
  * parent's position (decode.rs:3601-3609).  For 4:2:2 every chroma TB of the
  * 4:2:0 layout is two square TBs stacked vertically, the upper one first,
