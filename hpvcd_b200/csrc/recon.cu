@@ -1382,6 +1382,8 @@ static_assert(kRecCap420 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(
                   kRecCap422 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(32, 64)) * sizeof(uint16_t) &&
                   kRecCap444 * sizeof(hpvcd_tu) <= (can_size(64, 64) + 2 * can_size(64, 64)) * sizeof(uint16_t),
               "records fit the canvases");
+// (a gathered line is addressed from its component's canvas on)
+static_assert(3 * can_size(64, 64) + 3 * kWsBytes / sizeof(uint16_t) < 0x4000, "line positions fit the walk entries");
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1717,7 +1719,8 @@ __device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need
 // are not one run (possible at slice boundaries and under constrained intra
 // prediction), or that has none, is flagged kTbGather and its line is gathered
 // sample by sample first.
-//   x: canvas offset of the TB | of line position 0 << 16 | coded << 31
+//   x: canvas offset of the TB | of line position 0 << 16 | plain << 30 |
+//      coded << 31
 //   y: canvas offset of the corner | blend table offset of a plain TB << 16
 //   z: lo | hi << 8 | 2n << 16 | mode << 24 | kTbFilt
 //   w: x (6 bits) | kHow* << 6 | y << 8 (in the CTU) | kHow* << 14 |
@@ -1725,7 +1728,7 @@ __device__ __noinline__ Have wait_edges(Have h, uint32_t need_top, uint32_t need
 // Measured when the entries came in (4032x3024 grid, 70 luma TBs a CTU): the
 // walk's chain went from ~87k to ~46k cycles a CTU (4x4 700 -> 500, 16x16 5100
 // -> 1650, 32x32 10700 -> 3300 cycles); 512x512 tile 1004 -> 649 us.
-constexpr uint32_t kTbCoded = 1u << 31 /* of x */, kTbFilt = 1u << 31 /* of z */;
+constexpr uint32_t kTbCoded = 1u << 31, kTbPlainX = 1u << 30 /* of x */, kTbFilt = 1u << 31 /* of z */;
 // the TB reads neighbour CTUs, its line must be gathered, it is an I_PCM
 // block, it covers edge words, line position 32 is available, it is a 4x4 or
 // 8x8 TB of an angular mode without line or edge filter and with one run of
@@ -1735,8 +1738,9 @@ constexpr uint32_t kTbEdge = 1u, kTbGather = 2u, kTbPcm = 4u, kTbPub = 8u, kTbHi
 struct TbEntry {
     uint4 w;
     __device__ __forceinline__ int org() const { return (int)(w.x & 0xffffu); }
-    __device__ __forceinline__ int line0() const { return (int)((w.x >> 16) & 0x7fffu); }
+    __device__ __forceinline__ int line0() const { return (int)((w.x >> 16) & 0x3fffu); }
     __device__ __forceinline__ bool coded() const { return (w.x & kTbCoded) != 0u; }
+    __device__ __forceinline__ bool plain() const { return (w.x & kTbPlainX) != 0u; }
     __device__ __forceinline__ int corner() const { return (int)(w.y & 0xffffu); }
     __device__ __forceinline__ uint32_t tab() const { return w.y >> 16; }
     __device__ __forceinline__ int lo() const { return (int)(w.z & 0xffu); }
@@ -1748,6 +1752,22 @@ struct TbEntry {
     __device__ __forceinline__ uint32_t jrec() const { return (w.w >> 16) & 0x3ffu; }
     __device__ __forceinline__ uint32_t flags() const { return w.w >> 26; }
 };
+
+// An entry whose owner may be adding the walk's kHow* bits to word w at the
+// same time: w is read (and written by set_how) by strong accesses of its own,
+// not as a part of the vector; the bits that are read never change.  (Two
+// barriers around the additions instead: 24 mixed pictures 4146 us for 3946,
+// 4032x3024 grid 579 for 557.)
+__device__ __forceinline__ TbEntry shared_entry(const uint4* e) {
+    const uint2 xy = *(const uint2*)e;
+    return TbEntry{make_uint4(xy.x, xy.y, e->z, *(const volatile uint32_t*)&e->w)};
+}
+// The same without w.
+__device__ __forceinline__ TbEntry line_entry(const uint4* e) {
+    const uint2 xy = *(const uint2*)e;
+    return TbEntry{make_uint4(xy.x, xy.y, e->z, 0u)};
+}
+__device__ __forceinline__ void set_how(uint4* e, uint32_t w) { *(volatile uint32_t*)&e->w = w; }
 
 // The walk entry of intra record j (t, at (x0, y0) of the CTU); `flags` gives
 // kTbPcm and kTbPub, the others are added here.
@@ -1830,6 +1850,7 @@ __device__ __forceinline__ uint4 make_entry(const Comp& k, const hpvcd_tu& t, in
     w.y = (uint32_t)cidx(k, x0 - 1, y0 - 1) | (tab << 16);
     w.z = (uint32_t)lo | ((uint32_t)hi << 8) | ((uint32_t)n2 << 16) | ((uint32_t)t.mode << 24);
     if (coded) w.x |= kTbCoded;
+    if (flags & kTbPlain) w.x |= kTbPlainX;
     if (filt) w.z |= kTbFilt;
     w.w = (uint32_t)x0 | ((uint32_t)y0 << 8) | (jrec << 16) | (flags << 26);
     return w;
@@ -2500,7 +2521,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 const uint4* list = ents + lay.ent_off(c);
                 const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
                 for (uint32_t e = warp; e < cnt; e += kWarps) {
-                    const TbEntry E{list[e]};
+                    const TbEntry E = shared_entry(&list[e]);
                     if (E.coded() && !(E.flags() & kTbPcm)) stage_residual(k, E.n2() >> 1, E.x(), E.y(), lane);
                 }
             }
@@ -2514,16 +2535,16 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             const uint4* cb_list = ents + lay.ent_off(1);
             const uint32_t cnt = c == 0 ? listed[0] : (c == 1 ? listed[1] : listed[2]);
             for (uint32_t e = tid; e < cnt; e += kThreads) {
-                const TbEntry E{list[e]}, F{list[min(e + 1, cnt - 1)]};
+                const TbEntry E{list[e]}, F = shared_entry(&list[min(e + 1, cnt - 1)]);
                 const uint32_t f = E.flags();
                 const bool four = (f & kTbPlain) && E.n2() == 8;
                 const bool pair = e + 1 < cnt && four && (F.flags() & kTbPlain) && F.n2() == 8;
                 const uint32_t g = pair ? f | F.flags() : f;
-                list[e].w = (E.w.w & 0xffff3f3fu) | (four ? kHowPlain4 : 0u) | (pair ? kHowTwo : 0u) |
-                            (g & kTbEdge ? kHowEdge : 0u) | (g & kTbPub ? kHowPub : 0u);
+                set_how(&list[e], E.w.w | (four ? kHowPlain4 : 0u) | (pair ? kHowTwo : 0u) |
+                                      (g & kTbEdge ? kHowEdge : 0u) | (g & kTbPub ? kHowPub : 0u));
                 if (c == 2) {
-                    const uint4 b = cb_list[min(e, listed[1] ? listed[1] - 1 : 0u)];
-                    if (((b.x ^ E.w.x) & 0x7fffffffu) | (b.y ^ E.w.y) | (b.z ^ E.w.z) | ((b.w ^ E.w.w) & kHowPlain)) *s_diff = 1u;
+                    const uint4 b = line_entry(&cb_list[min(e, listed[1] ? listed[1] - 1 : 0u)]).w;
+                    if (((b.x ^ E.w.x) & ~kTbCoded) | (b.y ^ E.w.y) | (b.z ^ E.w.z)) *s_diff = 1u;
                 }
             }
         }
@@ -2536,7 +2557,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             const uint32_t cnt = c == 0 ? listed[0] : listed[1];
             // the angular words of the next TB are on their way while one is done
             auto angles = [&](const TbEntry& E, uint32_t (&ang)[4]) {
-                if (!(E.flags() & kTbPlain)) return;
+                if (!E.plain()) return;
                 const bool four = E.n2() == 8;
                 const uint32_t* a = (four ? g_angular.t4[E.mode() - 2] : g_angular.t8[E.mode() - 2]) + l15;
                 ang[0] = a[0];
@@ -2546,7 +2567,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
             TbEntry E{};
             uint32_t ang[4] = {0u, 0u, 0u, 0u};
             if (e < cnt) {
-                E.w = list[e];
+                E = line_entry(&list[e]);
                 angles(E, ang);
             }
             while (e < cnt) {
@@ -2554,10 +2575,10 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                 TbEntry N{};
                 uint32_t ang_n[4] = {0u, 0u, 0u, 0u};
                 if (en < cnt) {
-                    N.w = list[en];
+                    N = line_entry(&list[en]);
                     angles(N, ang_n);
                 }
-                if (E.flags() & kTbPlain) {
+                if (E.plain()) {
                     const Line L(E, row);
                     uint32_t* t = tab + E.tab();
                     if (E.n2() == 8) {
