@@ -1542,8 +1542,8 @@ __device__ __forceinline__ unsigned long long* edge_words(const DevPic& P, int c
     return c ? w + edge_words_of(ctb, P.sub_w, P.sub_h, 0) + (c - 1) * edge_words_of(ctb, P.sub_w, P.sub_h, 1) : w;
 }
 constexpr unsigned long long kEdgeTags = 0x8000800080008000ull;
-__device__ __forceinline__ unsigned long long edge_pack(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    return (unsigned long long)(a | (b << 16)) | ((unsigned long long)(c | (d << 16)) << 32) | kEdgeTags;
+__device__ __forceinline__ void put_edge(unsigned long long* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    st_edge(p, a | 0x8000u, b | 0x8000u, c | 0x8000u, d | 0x8000u);
 }
 
 // Publishes the edge words a finished n x n TB at (x0, y0) covers, from the
@@ -1555,7 +1555,7 @@ __device__ __forceinline__ void publish_tb(const uint16_t* can, int row, int S, 
     if (i < (n >> 2) && (bottom ? y0 + n == Sh : x0 + n == S)) {
         const int x = bottom ? x0 + 4 * i : S - 1, y = bottom ? Sh - 1 : y0 + 4 * i, st = bottom ? 1 : row;
         const uint16_t* q = can + can_in(S, x, y);
-        st_edge(words + (bottom ? (Sh >> 2) + (x >> 2) : y >> 2), edge_pack(q[0], q[st], q[2 * st], q[3 * st]));
+        put_edge(words + (bottom ? (Sh >> 2) + (x >> 2) : y >> 2), q[0], q[st], q[2 * st], q[3 * st]);
     }
 }
 
@@ -1606,8 +1606,7 @@ __device__ void edge_service(const DevPic& P, int cx, int cy, int ncomp, CanOf c
             const bool bottom = lane >= 16;
             const int i = lane & 15, st = bottom ? 1 : can_row(e.S);
             const uint16_t* q = can + (bottom ? can_in(e.S, 4 * i, e.Sh - 1) : can_in(e.S, e.S - 1, 4 * i));
-            st_edge(edge_words(P, cx, cy, c) + (bottom ? (e.Sh >> 2) + i : i),
-                    edge_pack(q[0] & 0x7fffu, q[st] & 0x7fffu, q[2 * st] & 0x7fffu, q[3 * st] & 0x7fffu));
+            put_edge(edge_words(P, cx, cy, c) + (bottom ? (e.Sh >> 2) + i : i), q[0], q[st], q[2 * st], q[3 * st]);
         }
         if (edge_top_in(e, lane)) {
             const int w = e.S >> 2;
@@ -2467,7 +2466,7 @@ k_recon(const DevPic* __restrict__ pics, const CtuItem* __restrict__ items, uint
                         const int ay = e.oy + (i < nr ? 4 * i + u : e.Sh - 1);
                         v[u] = ax < e.pw && ay < e.ph ? (uint32_t)load_sample(P.rec[c], P.bps, (size_t)ay * e.pw + ax) : 0u;
                     }
-                    st_edge(words + i, edge_pack(v[0], v[1], v[2], v[3]));
+                    put_edge(words + i, v[0], v[1], v[2], v[3]);
                 }
             }
             continue;
