@@ -101,6 +101,13 @@ bool sao_active(const hpvcd_picture& p) {
     return p.sao && (p.flags & (HPVCD_PIC_SAO_LUMA | HPVCD_PIC_SAO_CHROMA));
 }
 
+// Whether a picture's residuals wait for its motion compensation: they are added
+// to the plane, which holds the prediction (everywhere else motion compensation
+// adds the residual plane).
+bool mc_before_residual(const hpvcd_picture& p) {
+    return (p.flags & HPVCD_PIC_PRED_IN_PLANE) && (p.flags & HPVCD_PIC_INTER) && p.n_pus;
+}
+
 struct Segment {
     uint32_t first_pic, n_pics;
     uint32_t wave_first, n_waves;  // the segment's wavefront launches (hpvcd_plan::waves)
@@ -259,8 +266,9 @@ struct hpvcd_plan {
     // concurrent segments (independent pictures): one stream per segment,
     // forked from and joined back into the launching stream
     bool concurrent = false;
-    // a sequence (one segment per picture): the residuals of every picture
-    // but the first are computed beside the first one's wavefront
+    // a sequence (one segment per picture, every residual independent of the
+    // motion compensation): the residuals of every picture but the first are
+    // computed beside the first one's wavefront
     bool sequence = false;
     GroupStreams own;                  // used when the plan is not lent a set
     const GroupStreams* gs = nullptr;  // the set the launches use
@@ -602,6 +610,8 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
         }
     }
     P->sequence = any_inter && P->segs.size() > 1;
+    for (uint32_t i = 0; i < n; ++i)
+        if (mc_before_residual(pics[i])) P->sequence = false;
     // ---- wavefront schedule per segment and format class: CTUs sorted by
     // (x + 2y, picture, y) ----
     for (uint32_t si = 0; si < P->segs.size(); ++si) {
@@ -882,19 +892,26 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
     const cudaStream_t origin = st;
     // Residual planes of inter pictures start at zero: motion compensation adds
     // them to every sample, coded or not.
-    auto clear_residual = [&](uint32_t i, cudaStream_t s) -> cudaError_t {
-        if (!(P->src[i].flags & HPVCD_PIC_INTER) || !P->src[i].n_pus) return cudaSuccess;
-        return cudaMemsetAsync(P->pics[i].res[0], 0, res_plane_bytes(geo_of(P->src[i])), s);
+    auto clear_residuals = [&](uint32_t first, uint32_t end, cudaStream_t s) -> cudaError_t {
+        cudaError_t r = cudaSuccess;
+        for (uint32_t i = first; i < end && r == cudaSuccess; ++i)
+            if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus)
+                r = cudaMemsetAsync(P->pics[i].res[0], 0, res_plane_bytes(geo_of(P->src[i])), s);
+        return r;
     };
     auto residuals = [&](uint32_t first, uint32_t end, bool ccp, cudaStream_t s) -> cudaError_t {
         const uint32_t nrec = P->rec_prefix[end] - P->rec_prefix[first];
-        cudaError_t r = cudaSuccess;
-        for (uint32_t i = first; i < end && r == cudaSuccess; ++i) r = clear_residual(i, s);
-        if (r == cudaSuccess)
-            r = hpvcd_launch_residual(P->d_pics + first, P->d_prefix + first, end - first, nrec, d_err, P->sms,
-                                      (int)P->sched.idct, s);
+        cudaError_t r = hpvcd_launch_residual(P->d_pics + first, P->d_prefix + first, end - first, nrec, d_err, P->sms,
+                                              (int)P->sched.idct, s);
         if (r == cudaSuccess && nrec && ccp)
             r = hpvcd_launch_ccp(P->d_pics + first, P->d_prefix + first, end - first, nrec, d_err, P->sms, s);
+        return r;
+    };
+    auto motion = [&](uint32_t first, uint32_t end, cudaStream_t s) -> cudaError_t {
+        cudaError_t r = cudaSuccess;
+        for (uint32_t i = first; i < end && r == cudaSuccess; ++i)
+            if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus)
+                r = hpvcd_launch_mc(P->d_pics, (int)i, (int)P->src[i].n_pus, s);
         return r;
     };
     const bool beside = P->sequence && (stages & HPVCD_STAGE_RECON);
@@ -902,6 +919,7 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
         const uint32_t first = P->segs[0].first_pic + P->segs[0].n_pics;
         e = cudaEventRecord(P->gs->ev_fork, origin);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(P->gs->aux[0], P->gs->ev_fork, 0);
+        if (e == cudaSuccess) e = clear_residuals(first, (uint32_t)P->src.size(), P->gs->aux[0]);
         if (e == cudaSuccess) e = residuals(first, (uint32_t)P->src.size(), P->rest_ccp(), P->gs->aux[0]);
         if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_join[0], P->gs->aux[0]);
         if (e != cudaSuccess) return cuda_status(e);
@@ -917,13 +935,16 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
             st = P->gs->aux[si];
         }
         if (stages & HPVCD_STAGE_RECON) {
-            if (beside && si == 1)
+            const uint32_t first = s.first_pic, end = s.first_pic + s.n_pics;
+            const bool own = !beside || si == 0;  // (the others' residuals are computed by the launch above)
+            const bool mc_first = mc_before_residual(P->src[first]);  // a picture with PUs is a segment of its own
+            if (own)
+                e = clear_residuals(first, end, st);
+            else if (si == 1)
                 e = cudaStreamWaitEvent(origin, P->gs->ev_join[0], 0);
-            else if (!beside || si == 0)
-                e = residuals(s.first_pic, s.first_pic + s.n_pics, P->seg_ccp(s), st);
-            for (uint32_t i = s.first_pic; i < s.first_pic + s.n_pics && e == cudaSuccess; ++i)
-                if ((P->src[i].flags & HPVCD_PIC_INTER) && P->src[i].n_pus)
-                    e = hpvcd_launch_mc(P->d_pics, (int)i, (int)P->src[i].n_pus, st);
+            if (e == cudaSuccess && mc_first) e = motion(first, end, st);
+            if (e == cudaSuccess && own) e = residuals(first, end, P->seg_ccp(s), st);
+            if (e == cudaSuccess && !mc_first) e = motion(first, end, st);
             if (e != cudaSuccess) return cuda_status(e);
             // the segment's format classes one after another, each wave with
             // its own layout and work counter
