@@ -435,7 +435,8 @@ size_t plan_footprint(const hpvcd_picture* pics, uint32_t n, const hpvcd_output*
         const size_t one = align_up(g.luma_bytes, 256) + 2 * align_up(g.chroma_bytes, 256);
         bytes += one * (sao_active(pics[i]) ? 2 : 1);
         bytes += res_plane_bytes(g);
-        bytes += (size_t)g.ctb_cols * g.ctb_rows * (4 + sizeof(CtuItem));
+        if (!(pics[i].flags & HPVCD_PIC_PRED_IN_PLANE))  // pictures with a wavefront: edge words and work list
+            bytes += 8 * edge_words_of_picture(pics[i], g) + (size_t)g.ctb_cols * g.ctb_rows * sizeof(CtuItem);
     }
     bytes += n * sizeof(DevPic);
     bytes += output_bytes(pics, n, out);
