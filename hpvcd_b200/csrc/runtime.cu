@@ -427,13 +427,36 @@ size_t output_bytes(const hpvcd_picture* pics, uint32_t n, const hpvcd_output* o
     return b;
 }
 
-// Device bytes a plan for these pictures needs (planes, scratch, canvas).
+// Which pictures keep their final planes: all, unless the output is RGB8
+// canvases only; then those that a later picture predicts from, that a DPB
+// stores, or whose canvas is a native one.
+std::vector<char> kept_final_planes(const hpvcd_picture* pics, uint32_t n, const hpvcd_output* out) {
+    std::vector<char> keep(n, 1);
+    if (!out || out->kind != HPVCD_OUT_RGB8 || !(out->options & HPVCD_OUTPUT_CANVAS_ONLY)) return keep;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t k = out->place[i].canvas;
+        keep[i] = (pics[i].flags & HPVCD_PIC_STORE_MASK) != 0 ||
+                  (k < n_canvases_of(out) && native_canvas(out->kind, canvas_of(out, k)));
+    }
+    for (uint32_t i = 0; i < n; ++i)
+        for (int l = 0; l < 2; ++l)
+            for (int r = 0; r < HPVCD_MAX_REFS; ++r) {
+                const int sv = pics[i].ref_slot[l][r];
+                if (sv >= 0 && (uint32_t)sv < n) keep[(size_t)sv] = 1;
+            }
+    return keep;
+}
+
+// Device bytes a plan for these pictures needs (planes, scratch, canvas; the
+// planes of a plane output count as output).
 size_t plan_footprint(const hpvcd_picture* pics, uint32_t n, const hpvcd_output* out) {
     size_t bytes = 0;
+    const bool to_canvas = out && canvas_kind(out->kind);
+    const std::vector<char> keep_fin = kept_final_planes(pics, n, out);
     for (uint32_t i = 0; i < n; ++i) {
         const Geo g = geo_of(pics[i]);
         const size_t one = align_up(g.luma_bytes, 256) + 2 * align_up(g.chroma_bytes, 256);
-        bytes += one * (sao_active(pics[i]) ? 2 : 1);
+        bytes += one * (sao_active(pics[i]) || (to_canvas && keep_fin[i]) ? 2 : 1);
         bytes += res_plane_bytes(g);
         if (!(pics[i].flags & HPVCD_PIC_PRED_IN_PLANE))  // pictures with a wavefront: edge words and work list
             bytes += 8 * edge_words_of_picture(pics[i], g) + (size_t)g.ctb_cols * g.ctb_rows * sizeof(CtuItem);
@@ -545,21 +568,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
             P->recon_feat = true;
         if (pics[i].flags & HPVCD_PIC_INTER) any_inter = true;
     }
-    // ---- which pictures keep their final planes: all, unless the output is
-    // RGB8 canvases only; then those that a later picture predicts from,
-    // that a DPB stores, or whose canvas is a native one ----
-    std::vector<char> keep_fin(n, 1);
-    if (out && out->kind == HPVCD_OUT_RGB8 && (out->options & HPVCD_OUTPUT_CANVAS_ONLY)) {
-        for (uint32_t i = 0; i < n; ++i)
-            keep_fin[i] = (pics[i].flags & HPVCD_PIC_STORE_MASK) != 0 ||
-                          native_canvas(out->kind, canvas_of(out, out->place[i].canvas));
-        for (uint32_t i = 0; i < n; ++i)
-            for (int l = 0; l < 2; ++l)
-                for (int r = 0; r < HPVCD_MAX_REFS; ++r) {
-                    const int sv = pics[i].ref_slot[l][r];
-                    if (sv >= 0 && (uint32_t)sv < n) keep_fin[(size_t)sv] = 1;
-                }
-    }
+    const std::vector<char> keep_fin = kept_final_planes(pics, n, out);
     // ---- planes + scratch layout ----
     size_t plane_bytes = 0;
     std::vector<size_t> rec_off(n), fin_off(n);

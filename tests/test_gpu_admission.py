@@ -35,10 +35,11 @@ def held_bytes(pics, canvas, separate_final):
     arr = (abi.Picture * len(pics))(*pics)
     arena = abi.lib().hpvcd_gpu_packed_size(arr, len(pics))
     total = up(arena + arena // 4, 1 << 20) + canvas
-    for p in pics:
+    referenced = {r for p in pics for row in p.ref_slot for r in row}
+    for i, p in enumerate(pics):
         g = synth.geometry(p)
         w, h, cw, ch = g["w"], g["h"], g["cw"], g["ch"]
-        total += planes_bytes(w, h, cw, ch, g["bytes_per_sample"]) * (2 if separate_final else 1)
+        total += planes_bytes(w, h, cw, ch, g["bytes_per_sample"]) * (2 if separate_final or i in referenced else 1)
         total += up(up(w, 16) * h * 2, 256) + 2 * up(up(cw, 16) * ch * 2, 256)
         ctb, sw, sh = 1 << p.log2_ctb, 2 if p.chroma_idc in (1, 2) else 1, 2 if p.chroma_idc == 1 else 1
         words = ctb // 2 + (2 * (ctb // sw // 4 + ctb // sh // 4) if p.chroma_idc else 0)
@@ -73,3 +74,11 @@ def batch(idc, log2_ctb, sao):
 def test_edge_words_are_counted(idc, log2_ctb):
     s, out, place = batch(idc, log2_ctb, True)
     check(s.pictures(), out, 1024 * 512 * 3, True)
+
+
+@pytest.mark.parametrize("canvas_only", [False, True])
+@pytest.mark.parametrize("sao", [False, True])
+def test_kept_final_planes_are_counted(canvas_only, sao):
+    s, out, place = batch(1, 6, sao)
+    out.options = abi.OUTPUT_CANVAS_ONLY if canvas_only else 0
+    check(s.pictures(), out, 1024 * 512 * 3, sao or not canvas_only)
