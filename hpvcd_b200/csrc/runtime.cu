@@ -874,7 +874,9 @@ struct SegmentHooks {
     std::function<cudaError_t(uint32_t)> inputs, outputs;
 };
 
-hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const SegmentHooks* hooks = nullptr) {
+// The enqueueing part of plan_launch; `forked` counts the group streams that
+// were given work.
+hpvcd_status plan_enqueue(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const SegmentHooks* hooks, uint32_t* forked) {
     cudaError_t e = cudaSuccess;
     // Work counters, the device error word and the wavefront edge words are
     // reset by every launch that reconstructs.
@@ -929,6 +931,7 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
         const uint32_t first = P->segs[0].first_pic + P->segs[0].n_pics;
         e = cudaEventRecord(P->gs->ev_fork, origin);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(P->gs->aux[0], P->gs->ev_fork, 0);
+        if (e == cudaSuccess) *forked = 1;
         if (e == cudaSuccess) e = clear_residuals(first, (uint32_t)P->src.size(), P->gs->aux[0]);
         if (e == cudaSuccess) e = residuals(first, (uint32_t)P->src.size(), P->rest_ccp(), P->gs->aux[0]);
         if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_join[0], P->gs->aux[0]);
@@ -942,6 +945,7 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
             if (e == cudaSuccess) e = cudaEventRecord(P->gs->ev_fork, origin);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(P->gs->aux[si], P->gs->ev_fork, 0);
             if (e != cudaSuccess) return cuda_status(e);
+            *forked = si + 1;
             st = P->gs->aux[si];
         }
         if (stages & HPVCD_STAGE_RECON) {
@@ -1012,6 +1016,20 @@ hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const 
         if (e != cudaSuccess) return cuda_status(e);
     }
     return HPVCD_OK;
+}
+
+// A launch that fails half way still joins the group streams it forked, so that
+// what the caller enqueues on `st` next (another launch of the plan, the frees
+// of its buffers) follows the work that did start.
+hpvcd_status plan_launch(hpvcd_plan* P, uint32_t stages, cudaStream_t st, const SegmentHooks* hooks = nullptr) {
+    uint32_t forked = 0;
+    const hpvcd_status s = plan_enqueue(P, stages, st, hooks, &forked);
+    if (s == HPVCD_OK) return s;
+    for (uint32_t g = 0; g < forked; ++g)
+        if (cudaEventRecord(P->gs->ev_join[g], P->gs->aux[g]) == cudaSuccess)
+            cudaStreamWaitEvent(st, P->gs->ev_join[g], 0);
+    cudaGetLastError();  // reported; the next launch's check starts clean
+    return s;
 }
 
 // Re-point the input fields of an existing plan at new device buffers of a
@@ -1801,8 +1819,15 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     // the device, need every input first.
     bool by_segment = reuse && slot->plan->concurrent && !g->sel;
     for (uint32_t i = 0; i < n; ++i) by_segment = by_segment && !(pics[i].flags & HPVCD_PIC_PRED_IN_PLANE);
+    // A batch that fails from here on leaves nothing in flight: the slot is free
+    // for the next one, and the caller's buffers are its own again.
+    auto fail = [&](hpvcd_status s) -> hpvcd_status {
+        cudaStreamSynchronize(slot->stream);
+        cudaGetLastError();  // reported; the next launch's check starts clean
+        return s;
+    };
     if (!by_segment) e = upload(0, total);
-    if (e != cudaSuccess) return cuda_status(e);
+    if (e != cudaSuccess) return fail(cuda_status(e));
     for (const InputPart& pt : parts) point_at(dev[pt.pic], pt.kind, slot->d_in + pt.off);
     slot->wp.assign(n, hpvcd_wp_table{});
     bool any_wp = false;
@@ -1827,7 +1852,7 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     }
     g->in_use = g->in_use - held + slot->d_in_cap + slot->plan_bytes;
     slot->held = slot->d_in_cap + slot->plan_bytes;
-    if (st != HPVCD_OK) return st;
+    if (st != HPVCD_OK) return fail(st);
     int others = 0;  // tickets of this context already in flight
     for (const Slot& s : g->slots)
         if (s.busy && &s != slot) ++others;
@@ -1836,7 +1861,7 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
     // batches outside the network's domain).
     if (g->sel && others > 0) {
         st = hpvcd_plan_set_sched(slot->plan, &g->fixed);
-        if (st != HPVCD_OK) return st;
+        if (st != HPVCD_OK) return fail(st);
         ++g->sel_picks[HPVCD_MLP_MAX_VARIANTS];
     } else if (g->sel) {  // the network picks the batch's schedule from its features
         // Up to kHostPickRecords records (a few ms of host work at most) the
@@ -1850,7 +1875,7 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
         if (records <= kHostPickRecords) {
             float fv[HPVCD_FEATURES];
             st = hpvcd_batch_features(pics, n, fv);
-            if (st != HPVCD_OK) return st;
+            if (st != HPVCD_OK) return fail(st);
             pick = hpvcd_mlp_pick_host(g->sel_w.data(), (uint32_t)g->sel_cands.size(), fv, g->sel_lohi,
                                        g->sel_has_domain);
             st = hpvcd_plan_set_sched(slot->plan, pick == HPVCD_MLP_NO_PICK ? &g->fixed : &g->sel_cands[pick]);
@@ -1859,11 +1884,11 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
                                    slot->stream, &pick);
             if (st == HPVCD_OK && pick == HPVCD_MLP_NO_PICK) st = hpvcd_plan_set_sched(slot->plan, &g->fixed);
         }
-        if (st != HPVCD_OK) return st;
+        if (st != HPVCD_OK) return fail(st);
         ++g->sel_picks[pick == HPVCD_MLP_NO_PICK ? HPVCD_MLP_MAX_VARIANTS : pick];
     } else {
         st = hpvcd_plan_set_sched(slot->plan, &g->fixed);
-        if (st != HPVCD_OK) return st;
+        if (st != HPVCD_OK) return fail(st);
     }
     // Tickets already in flight share the SMs with this one: the wavefront
     // kernel's persistent grid keeps to its share of the CTA slots (its CTAs
@@ -1880,7 +1905,7 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
             const int cur = s2.recon_ctas_per_sm ? (int)s2.recon_ctas_per_sm : occ;
             s2.recon_ctas_per_sm = (uint32_t)std::min(cur, share);
             st = hpvcd_plan_set_sched(slot->plan, &s2);
-            if (st != HPVCD_OK) return st;
+            if (st != HPVCD_OK) return fail(st);
         }
     }
     const int slot_idx = (int)(slot - g->slots.data());
@@ -1889,7 +1914,7 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
         hpvcd_dpb::Entry& E = g->dpb->entries[(size_t)en];
         if (E.written) {
             const cudaError_t we = cudaStreamWaitEvent(slot->stream, E.ev_write, 0);
-            if (we != cudaSuccess) return cuda_status(we);
+            if (we != cudaSuccess) return fail(cuda_status(we));
         }
     }
     // ---- launch and output copy back; the output of concurrent segments goes
@@ -1952,12 +1977,12 @@ HPVCD_API hpvcd_status hpvcd_gpu_submit(hpvcd_gpu* g, const hpvcd_picture* pics,
         return copy_canvas(upto);
     };
     st = plan_launch(P, HPVCD_STAGE_ALL, slot->stream, &hooks);
-    if (st != HPVCD_OK) return st;
+    if (st != HPVCD_OK) return fail(st);
     st = dpb_after_launch(g, slot, slot_idx, pics, n);
-    if (st != HPVCD_OK) return st;
+    if (st != HPVCD_OK) return fail(st);
     e = to_canvas ? copy_canvas(P->canvas_bytes) : copy_planes(n);
     if (e == cudaSuccess) e = cudaEventRecord(slot->done, slot->stream);
-    if (e != cudaSuccess) return cuda_status(e);
+    if (e != cudaSuccess) return fail(cuda_status(e));
     slot->busy = true;
     slot->ticket = g->next_ticket++;
     slot->out_bytes = out_bytes;
