@@ -19,17 +19,18 @@
 //     CTUs are claimed from a global queue sorted by wavefront index
 //     (x + 2y) across all pictures, so a CTU is only claimed after every CTU
 //     it depends on (left, above-left, above, above-right) was claimed by a
-//     running CTA: no deadlock for any grid size.  Per CTU the residuals and
-//     records are staged with cp.async, then luma, Cb and Cr are walked by
-//     three warps in parallel (chroma availability only depends on the luma
-//     `decoded` map, which each warp replays from the records), all in
-//     shared memory.  Neighbours synchronise per component and quadrant:
-//     each walking warp releases how many quadrants of its CTU are done once
-//     their right-column / bottom-row samples are in the plane, and reads a
-//     neighbour's edge segment only when a TB on its own top or left edge
-//     needs it (waits bounded), so a CTU starts while its left and
-//     above-right neighbours are still being walked.  Finally the whole CTU
-//     is written out for the filters.
+//     running CTA: no deadlock for any grid size.  Per CTU all warps turn the
+//     records into walk entries, residuals are staged with cp.async and a
+//     blend table is filled, all in shared memory; then luma, Cb and Cr are
+//     walked by warps of their own in parallel (chroma availability only
+//     depends on the luma `decoded` map, which the records give beforehand).
+//     Neighbours synchronise per TB: a walking warp writes the samples of its
+//     CTU's right column and bottom row into edge words as each TB is done,
+//     and the CTA's last warp moves the neighbours' words into shared memory,
+//     where a walking warp looks before a TB on the CTU's top or left edge
+//     (waits bounded).  So a CTU starts while its left and above-right
+//     neighbours are still being walked.  Finally the whole CTU is written out
+//     for the filters.
 #include <mutex>
 #include <climits>
 
@@ -2211,11 +2212,12 @@ __device__ __noinline__ void gather_line(const Comp& k, int log2n, int x0, int y
     __syncwarp();
 }
 
-// Warps of a k_recon CTA: warp 0 walks luma, chroma is walked by warp 1 (Cb,
-// then Cr: kCW = 1) or by warps 1 and 2 (one component each: kCW = 2), and the
-// last warp moves edge words.  At 4:2:0 a CTU's two chroma walks together are
-// shorter than its luma walk, so one warp for both loses nothing; at 4:2:2 and
-// 4:4:4 they would be the longer chain.
+// Warps of a k_recon CTA: warp 0 walks luma, chroma is walked by warps 1 and 2
+// (one component each: kCW = 2, the default) or by warp 1 (Cb, then Cr: kCW =
+// 1), and the last warp moves edge words.  At 4:2:0 a CTU's two chroma walks
+// together are shorter than its luma walk, so a picture alone takes as long
+// either way; 24 mixed pictures took 4305 us with kCW = 2 and 4597 with kCW = 1,
+// and at 4:2:2 and 4:4:4 one warp for both would be the longer chain.
 __host__ __device__ constexpr int recon_warps(int kCW) { return 2 + kCW; }
 
 // kFeat: some picture of the launch has slices / tiles, constrained intra
@@ -2811,9 +2813,7 @@ extern "C" cudaError_t hpvcd_launch_recon(const hpvcd::DevPic* pics, const hpvcd
     // the dynamic shared-memory limit was raised by hpvcd_recon_occupancy()
     // when the plan was built (no non-stream API call here, so launches can
     // be captured into CUDA graphs)
-    // build: 1 one chroma warp (Cb, then Cr), 2 (and 3) one warp per chroma
-    // component
-    const int cw = chroma_warps == 1 ? 1 : 2;
+    const int cw = chroma_warps == 1 ? 1 : 2;  // walking warps for chroma
     const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw) - 1).total;
     const int threads = 32 * hpvcd::recon_warps(cw);
     // default: 2^22 polls of up to 64 ns each bound one wait to a few hundred ms
@@ -2850,9 +2850,8 @@ void recon_attrs(int lim) {
 }
 
 // Occupancy of one build with the layout of `cfmt` (attributes already set).
-int recon_occupancy_of(int cfmt, int chroma_warps) {
+int recon_occupancy_of(int cfmt, int cw) {
     int blocks = 0;
-    const int cw = chroma_warps == 1 ? 1 : 2;
     const size_t smem = hpvcd::ReconLayout(cfmt, hpvcd::recon_warps(cw) - 1).total;
     if (cw == 2)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, hpvcd::k_recon<2, false>, 32 * hpvcd::recon_warps(2),
@@ -2872,15 +2871,15 @@ int recon_occupancy_of(int cfmt, int chroma_warps) {
 constexpr int kAttrDevices = 64;
 std::mutex g_attr_mu;
 bool g_attr_done[kAttrDevices];
-int g_attr_occ[kAttrDevices][3][3];
+int g_attr_occ[kAttrDevices][3][2];
 }  // namespace
 
-// CTAs per SM of the wavefront kernel with the layout of `cfmt` in build
-// `chroma_warps` (1 one walking warp for both chroma components, 2 and 3 one
-// each; 0 counts as 2); the first call on a device sets the attributes of every
-// instantiation (recon_attrs) and of the residual kernel.
+// CTAs per SM of the wavefront kernel with the layout of `cfmt` and
+// `chroma_warps` (1 or 2) walking warps for chroma; the first call on a device
+// sets the attributes of every instantiation (recon_attrs) and of the residual
+// kernel.
 extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
-    const int build = chroma_warps >= 1 && chroma_warps <= 3 ? chroma_warps : 2;
+    const int cw = chroma_warps == 1 ? 1 : 2;
     const int cf = cfmt >= 0 && cfmt <= 2 ? cfmt : 0;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kAttrDevices) {
@@ -2888,7 +2887,7 @@ extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
         dev = -1;
     }
     std::lock_guard<std::mutex> lock(g_attr_mu);
-    if (dev >= 0 && g_attr_done[dev]) return g_attr_occ[dev][cf][build - 1];
+    if (dev >= 0 && g_attr_done[dev]) return g_attr_occ[dev][cf][cw - 1];
     const int lim = (int)hpvcd::ReconLayout(hpvcd::kFmt444, hpvcd::recon_warps(2) - 1).total;
     recon_attrs<1, false>(lim);
     recon_attrs<2, false>(lim);
@@ -2901,9 +2900,9 @@ extern "C" int hpvcd_recon_occupancy(int cfmt, int chroma_warps) {
                          (int)cudaSharedmemCarveoutMaxShared);
     cudaFuncSetAttribute(hpvcd::k_residual<hpvcd::kIdctTensor>, cudaFuncAttributePreferredSharedMemoryCarveout,
                          (int)cudaSharedmemCarveoutMaxShared);
-    if (dev < 0) return recon_occupancy_of(cf, build);
+    if (dev < 0) return recon_occupancy_of(cf, cw);
     for (int f = 0; f < 3; ++f)
-        for (int b = 1; b <= 3; ++b) g_attr_occ[dev][f][b - 1] = recon_occupancy_of(f, b);
+        for (int b = 1; b <= 2; ++b) g_attr_occ[dev][f][b - 1] = recon_occupancy_of(f, b);
     g_attr_done[dev] = true;
-    return g_attr_occ[dev][cf][build - 1];
+    return g_attr_occ[dev][cf][cw - 1];
 }

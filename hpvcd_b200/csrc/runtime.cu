@@ -222,7 +222,7 @@ struct hpvcd_plan {
     // layout.  item_off / n_full: the wave's range of the CTU work list;
     // n_items: entries launched (one fewer while a test drops a CTU).
     // ready: CTUs of the wave that can be walked at once (per picture, the
-    // longest x + 2y diagonal of its CTB grid), which picks the build.
+    // longest x + 2y diagonal of its CTB grid), which sizes the grid.
     struct Wave {
         uint32_t seg;
         int cfmt;
@@ -232,12 +232,12 @@ struct hpvcd_plan {
     };
     std::vector<Wave> waves;
     // k_recon CTAs per SM by class and build (1 one walking warp for both
-    // chroma components, 2 and 3 one each; index build - 1)
-    int occ[3][3] = {{1, 1, 1}, {1, 1, 1}, {1, 1, 1}};
-    // Build of a wave's wavefront kernel (hpvcd_sched.chroma_warps; 0, the
-    // default, is one warp per chroma component: 24 mixed images 4305 us
-    // against 4597 with one warp for both, single pictures the same).
-    int build_of() const { return sched.chroma_warps >= 1 && sched.chroma_warps <= 3 ? (int)sched.chroma_warps : 2; }
+    // chroma components, 2 one each; index build - 1)
+    int occ[3][2] = {{1, 1}, {1, 1}, {1, 1}};
+    // Build of the wavefront kernel (hpvcd_sched.chroma_warps; 0, the default,
+    // and 3 are one warp per chroma component: 24 mixed images 4305 us against
+    // 4597 with one warp for both, single pictures the same).
+    int build_of() const { return sched.chroma_warps == 1 ? 1 : 2; }
     // CTAs of a wave's persistent grid, `slots` of them resident.  Intra
     // pictures walk at most `ready` CTUs at once; three CTAs for each keep the
     // set-up of the next ones off the chain, and CTAs beyond that (but one per
@@ -844,7 +844,7 @@ hpvcd_status plan_build(const hpvcd_picture* pics, uint32_t n, const hpvcd_outpu
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, P->device);
     P->sms = sms;
     for (int cls = 0; cls < 3; ++cls)
-        for (int cw = 1; cw <= 3; ++cw) P->occ[cls][cw - 1] = std::max(1, hpvcd_recon_occupancy(cls, cw));
+        for (int cw = 1; cw <= 2; ++cw) P->occ[cls][cw - 1] = std::max(1, hpvcd_recon_occupancy(cls, cw));
     {
         const cudaError_t fe = hpvcd_filter_tile_setup();
         if (fe != cudaSuccess) {

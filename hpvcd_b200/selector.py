@@ -3,10 +3,11 @@
 The schedule of a batch (include/hpvcd_gpu.h `hpvcd_sched`) picks kernel
 variants that never change pixels: the inverse transform of 16x16 / 32x32 TBs
 in k_residual (integer tensor-core products, or even-odd butterflies), the
-chroma warps of the wavefront kernel k_recon (one warp per chroma component
-in a CTA of three, or one warp walking Cb then Cr in a CTA of two) and the
-persistent k_recon CTAs per SM (occupancy maximum, or one).  Which is fastest depends on the batch: its TB-size mix,
-coefficient density, QP, intra share, size and picture count.
+chroma warps of the wavefront kernel k_recon (one warp per chroma component in
+a CTA of four, or one warp walking Cb then Cr in a CTA of three) and the
+persistent k_recon CTAs per SM (by the CTUs ready at once, or one).  Which is
+fastest depends on the batch: its TB-size mix, coefficient density, QP, intra
+share, size and picture count.
 
 * Exhaustive autotuning (`hpvcd_plan_autotune`) times every schedule on the
   batch itself: always right, but K decodes' worth of time.
